@@ -33,6 +33,8 @@ int32_t check_launch(const char* op);
 int32_t require_sm100(const char* op);
 // Number of SMs of the current device (cached).
 int sm_count();
+// Whether launches carry the programmatic-stream-serialization attribute (GEMB_TUNE_GEMV_PDL).
+bool pdl_enabled();
 // Tuning knobs owned by the GEMM translation unit (see gemb_set_tuning).
 int32_t gemm_set_tuning(int32_t knob, int32_t value);
 int32_t ep_set_tuning(int32_t knob, int32_t value);
@@ -71,12 +73,70 @@ inline bool positive_finite(float v) { return std::isfinite(v) && v > 0.0f; }
     if (gemb_rc_ != GEMB_OK) return gemb_rc_; \
   } while (0)
 
+// Programmatic dependent launch.  A kernel launched through launch_pdl may become resident while its
+// predecessor in the stream still runs, so it
+//   - lets its own successor do the same (pdl_trigger), first thing;
+//   - calls pdl_wait in every CTA before it reads or writes any global memory.  The only accesses
+//     allowed before are prefetches into L2, which is coherent: they cannot return stale bytes, whoever
+//     writes the line later.  Every kernel of the chain waits, so "my predecessor has completed" implies
+//     that everything before it has;
+//   - reads what an earlier kernel wrote with ld_dep, not __ldg: the read-only path promises that the data
+//     does not change while the kernel is resident, which starts before pdl_wait here.
+template <typename... P, typename... A>
+int32_t launch_pdl(const char* op, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(GEMB_INTERNAL, "%s: %s: %s", op, cudaGetErrorName(e), cudaGetErrorString(e));
+  }
+  return GEMB_OK;
+}
+
 // ---------------------------------------------------------------------------------------------
 // Device-side codecs.  E2M1/E4M3 conversions use the hardware cvt instructions, which round to
 // nearest with ties to the even code and saturate to the largest finite value: the same rule
 // as ChooseNearestE2M1 / ChooseNearestPositiveE4M3Fn in src/numeric/nvfp4.cpp:26-56.
 // ---------------------------------------------------------------------------------------------
 #ifdef __CUDACC__
+
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Loads of data an earlier kernel of the stream produced (volatile: they stay behind pdl_wait).
+__device__ __forceinline__ uint4 ld_dep(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float4 ld_dep(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float ld_dep(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint16_t ld_dep(const uint16_t* p) {
+  uint16_t v;
+  asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint8_t ld_dep(const uint8_t* p) {
+  uint16_t v;
+  asm volatile("ld.global.u8 %0, [%1];" : "=h"(v) : "l"(p));
+  return static_cast<uint8_t>(v);
+}
 
 __device__ __forceinline__ float bf16_bits_to_float(uint16_t bits) {
   return __uint_as_float(static_cast<uint32_t>(bits) << 16);
@@ -153,57 +213,104 @@ __device__ __forceinline__ float gelu_tanh_product(float g, float u) {
 
 constexpr float kInvSix = 1.0f / 6.0f;  // kE2M1MaxReciprocal, src/numeric/nvfp4.cpp:16
 
+// Scale byte of a 16-element block with the given amax, and the factors its elements are quantised with.
+// EXACT follows src/numeric/nvfp4.cpp:139-150, RCP_APPROX follows src/cuda/nvfp4/reference.cu:60-78.
+// Explicit _rn intrinsics keep the compiler from fusing the multiplies into fma, which would change the rounding.
+struct BlockScale {
+  uint8_t bits;
+  float ds;   // decoded scale byte
+  float r;    // EXACT: RN(1 / ds); RCP_APPROX: the multiplier of the elements; 0 for a zero scale
+};
+template <bool kRcp>
+__device__ __forceinline__ BlockScale block_scale(float amax, float g) {
+  BlockScale s;
+  if constexpr (kRcp) {
+    s.bits = e4m3_encode(__fmul_rn(__fmul_rn(amax, rcp_approx_ftz(6.0f)), g));
+    s.ds = e4m3_decode(s.bits);
+    s.r = s.ds == 0.0f ? 0.0f : rcp_approx_ftz(__fmul_rn(s.ds, rcp_approx_ftz(g)));
+  } else {
+    s.bits = e4m3_encode(__fmul_rn(__fmul_rn(amax, kInvSix), g));
+    s.ds = e4m3_decode(s.bits);
+    // RN(1 / ds) without the general division: ds is one of the 126 positive E4M3 values, i.e. one of
+    // eight mantissas times a power of two, and for those one Newton step from any start within six
+    // ulps gives the correctly rounded reciprocal (checked in tests/test_quant_gpu.py on every value).
+    const float y0 = rcp_approx_ftz(s.ds);
+    s.r = s.ds == 0.0f ? 0.0f : fmaf(fmaf(-s.ds, y0, 1.0f), y0, y0);
+  }
+  return s;
+}
+
+// E2M1 codes of two elements of a block.
+// EXACT: (x * g) / ds, correctly rounded, with one reciprocal per block: t = RN(x * g), q0 = RN(t * r),
+// e = t - ds * q0 (exact in one fma), q = RN(q0 + e * r).  With a correctly rounded reciprocal this
+// residual correction yields the correctly rounded quotient (Markstein); for the 126 values an E4M3
+// scale can take it is also checked exhaustively around every E2M1 rounding boundary in
+// tests/test_oracle.py.  Two elements per instruction (packed fp32 multiply and fma: one IEEE operation per
+// half, so the rounding of every step is that of the scalar form).  The signs are arranged (-t, -r, -e) so
+// that a zero keeps its sign through the correction: -0 is a code of its own in E2M1.
+template <bool kRcp>
+__device__ __forceinline__ uint32_t quantize_pair(float2 v, float g, const BlockScale& s) {
+  if constexpr (kRcp) {
+    const float2 n = __fmul2_rn(v, make_float2(s.r, s.r));
+    return e2m1x2_encode(n.x, n.y);
+  } else {
+    const float2 nr = make_float2(-s.r, -s.r);
+    const float2 nt = __fmul2_rn(v, make_float2(-g, -g));
+    const float2 q0 = __fmul2_rn(nt, nr);
+    const float2 ne = __ffma2_rn(make_float2(s.ds, s.ds), q0, nt);
+    const float2 q = __ffma2_rn(ne, nr, q0);
+    return e2m1x2_encode(q.x, q.y);
+  }
+}
+
 // Quantizes 16 values into 8 packed bytes (returned as two 32-bit words) and one scale byte.
-// EXACT follows src/numeric/nvfp4.cpp:139-150, RCP_APPROX follows
-// src/cuda/nvfp4/reference.cu:60-78.  Explicit _rn intrinsics keep the compiler from fusing
-// the multiplies into fma, which would change the rounding.
 template <bool kRcp>
 __device__ __forceinline__ void quantize_block16(const float (&v)[16], float g, uint32_t& lo,
                                                  uint32_t& hi, uint8_t& scale_bits) {
   float amax = 0.0f;
 #pragma unroll
   for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(v[i]));
-  float n[16];
-  bool zero_scale = false;
-  if constexpr (kRcp) {
-    scale_bits = e4m3_encode(__fmul_rn(__fmul_rn(amax, rcp_approx_ftz(6.0f)), g));
-    const float ds = e4m3_decode(scale_bits);
-    const float os = ds == 0.0f ? 0.0f : rcp_approx_ftz(__fmul_rn(ds, rcp_approx_ftz(g)));
-#pragma unroll
-    for (int i = 0; i < 16; ++i) n[i] = __fmul_rn(v[i], os);
-  } else {
-    scale_bits = e4m3_encode(__fmul_rn(__fmul_rn(amax, kInvSix), g));
-    const float ds = e4m3_decode(scale_bits);
-    // (x * g) / ds, correctly rounded, with ONE division per block: r = RN(1 / ds), then per element
-    // q0 = RN(t * r), e = t - ds * q0 (exact in one fma), q = RN(q0 + e * r).  With a correctly rounded
-    // reciprocal this residual correction yields the correctly rounded quotient (Markstein); for the
-    // 126 values an E4M3 scale can take it is also checked exhaustively around every E2M1 rounding
-    // boundary in tests/test_oracle.py.  Sixteen IEEE divisions per block kept the conversion pipe of
-    // the fused GEMM epilogue busier than the tensor pipe.
-    // Two elements per instruction (packed fp32 multiply and fma: one IEEE operation per half, so the
-    // rounding of every step is that of the scalar form).  A zero scale gives sixteen +0 codes, set after
-    // the packing below.
-    const float r = ds == 0.0f ? 0.0f : __fdiv_rn(1.0f, ds);
-    const float2 g2 = make_float2(g, g), r2 = make_float2(r, r), nds2 = make_float2(-ds, -ds);
-#pragma unroll
-    for (int i = 0; i < 16; i += 2) {
-      const float2 t = __fmul2_rn(make_float2(v[i], v[i + 1]), g2);
-      const float2 q0 = __fmul2_rn(t, r2);
-      const float2 q = __ffma2_rn(__ffma2_rn(nds2, q0, t), r2, q0);
-      // (the quotient has the sign of t, also when it is zero: -0 keeps its sign bit in E2M1, and the
-      // residual correction alone would turn -0 into +0)
-      n[i] = copysignf(q.x, t.x);
-      n[i + 1] = copysignf(q.y, t.y);
-    }
-    zero_scale = ds == 0.0f;
-  }
+  const BlockScale s = block_scale<kRcp>(amax, g);
+  scale_bits = s.bits;
   lo = hi = 0;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    lo |= static_cast<uint32_t>(e2m1x2_encode(n[2 * i], n[2 * i + 1])) << (8 * i);
-    hi |= static_cast<uint32_t>(e2m1x2_encode(n[8 + 2 * i], n[8 + 2 * i + 1])) << (8 * i);
+    lo |= quantize_pair<kRcp>(make_float2(v[2 * i], v[2 * i + 1]), g, s) << (8 * i);
+    hi |= quantize_pair<kRcp>(make_float2(v[8 + 2 * i], v[8 + 2 * i + 1]), g, s) << (8 * i);
   }
-  if (zero_scale) lo = hi = 0;
+  if (!kRcp && s.ds == 0.0f) lo = hi = 0;   // a zero scale gives sixteen +0 codes
+}
+
+// E4M3 codes of x / scale, the IEEE quotient rounded to nearest (src/numeric/fp8.cpp:41-58), without a division
+// per element: with inv = RN(1 / scale), q0 = RN(x * inv) is within two ulps of the quotient, one residual
+// correction q1 = RN(q0 + (x - scale * q0) * inv) makes it faithful and a second one correctly rounded
+// (Markstein).  The residuals are exact while x is above 2^-102; below, the quotient is under half the
+// smallest E4M3 value and its code is zero either way, as long as scale is at least 2^-90 -- callers send
+// smaller scales (q.tiny) to the division.  Everything is computed on -q (see quantize_pair: zeros keep their sign).
+// The conversion instruction is the scarce one (about ten results per clock and SM), hence one per pair.
+struct Quotient {
+  float scale, inv;
+  bool tiny;
+};
+__device__ __forceinline__ Quotient token_quotient(float amax) {
+  Quotient q;
+  q.scale = amax == 0.0f ? 1.0f : __fdiv_rn(amax, 448.0f);
+  q.inv = __fdiv_rn(1.0f, q.scale);
+  q.tiny = q.scale < 0x1p-90f;
+  return q;
+}
+__device__ __forceinline__ uint32_t e4m3x2(float2 v) {
+  return static_cast<uint16_t>(__nv_cvt_float2_to_fp8x2(v, __NV_SATFINITE, __NV_E4M3));
+}
+static __device__ __noinline__ uint32_t e4m3x2_divided(float x, float y, float scale) {
+  return e4m3x2(make_float2(__fdiv_rn(x, scale), __fdiv_rn(y, scale)));
+}
+__device__ __forceinline__ uint32_t e4m3_of_quotients(float2 x, const Quotient& q) {
+  const float2 ninv = make_float2(-q.inv, -q.inv), s2 = make_float2(q.scale, q.scale);
+  const float2 y0 = __fmul2_rn(x, ninv);
+  const float2 y1 = __ffma2_rn(__ffma2_rn(s2, y0, x), ninv, y0);
+  const float2 y2 = __ffma2_rn(__ffma2_rn(s2, y1, x), ninv, y1);
+  return e4m3x2(y2) ^ 0x8080u;
 }
 
 #endif  // __CUDACC__

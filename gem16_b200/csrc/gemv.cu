@@ -108,32 +108,14 @@ __device__ __forceinline__ void stage_fp8_activation(const uint8_t* act, uint64_
   zero_fp8_staging_tail<kW>(k, xs);
 }
 
-// A value y with E4M3(y) == E4M3(x / scale) for the IEEE quotient x / scale.  x * (1/scale) is
-// within two ulp of the quotient, so both round to the same E4M3 code unless y sits within a
-// few ulp of a rounding boundary of the 3-bit mantissa (fraction bits 0x80000) or in E4M3's
-// subnormal range (below 2^-6), where the true division is used.
-__device__ __forceinline__ float quotient_for_e4m3(float x, float scale, float inv_scale) {
-  const float y = __fmul_rn(x, inv_scale);
-  const uint32_t bits = __float_as_uint(y);
-  const uint32_t mag = bits & 0x7FFFFFFFu;
-  const bool near_boundary = ((bits & 0xFFFFFu) - 0x7FFFCu) <= 8u;
-  const bool tiny = mag < 0x3C800000u && mag != 0u;  // |y| < 2^-6 (and not an exact zero)
-  if (near_boundary || tiny) return __fdiv_rn(x, scale);
-  return y;
-}
-
 // Quantizes eight bf16 values (one 16-byte chunk) and stages them as fp16.
-__device__ __forceinline__ void stage_bf16_chunk(const uint4& v, uint64_t c, float scale,
-                                                 float inv_scale, __half* xs) {
+__device__ __forceinline__ void stage_bf16_chunk(const uint4& v, uint64_t c, const Quotient& q, __half* xs) {
   const uint32_t ww[4] = {v.x, v.y, v.z, v.w};
   uint32_t h[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const float lo = quotient_for_e4m3(__uint_as_float(ww[i] << 16), scale, inv_scale);
-    const float hi = quotient_for_e4m3(__uint_as_float(ww[i] & 0xFFFF0000u), scale, inv_scale);
-    const uint16_t q = static_cast<uint16_t>(
-        __nv_cvt_float2_to_fp8x2(make_float2(lo, hi), __NV_SATFINITE, __NV_E4M3));
-    h[i] = e4m3x2_to_half2(q);
+    const float2 x = make_float2(__uint_as_float(ww[i] << 16), __uint_as_float(ww[i] & 0xFFFF0000u));
+    h[i] = e4m3x2_to_half2(static_cast<uint16_t>(q.tiny ? e4m3x2_divided(x.x, x.y, q.scale) : e4m3_of_quotients(x, q)));
   }
   const uint64_t c16 = c / 2;
   *reinterpret_cast<uint4*>(xs + (c16 / 32) * 512 + (c % 2) * 256 + (c16 % 32) * 8) =
@@ -177,8 +159,7 @@ __device__ __forceinline__ float stage_bf16_activation(const uint16_t* x, uint64
   amax = red[0];
 #pragma unroll
   for (int i = 1; i < kW; ++i) amax = fmaxf(amax, red[i]);
-  const float scale = amax == 0.0f ? 1.0f : __fdiv_rn(amax, 448.0f);
-  const float inv_scale = __frcp_rn(scale);
+  const Quotient quot = token_quotient(amax);
   // Second pass: the token was just read by this CTA, so these loads hit L1.
   for (uint64_t base = threadIdx.x; base < chunks; base += 4ull * (kW * 32)) {
     uint4 v[4];
@@ -190,11 +171,11 @@ __device__ __forceinline__ float stage_bf16_activation(const uint16_t* x, uint64
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const uint64_t c = base + static_cast<uint64_t>(i) * (kW * 32);
-      if (c < chunks) stage_bf16_chunk(v[i], c, scale, inv_scale, xs);
+      if (c < chunks) stage_bf16_chunk(v[i], c, quot, xs);
     }
   }
   zero_fp8_staging_tail<kW>(k, xs);
-  return scale;
+  return quot.scale;
 }
 
 // Persistent FP8 GEMV.  The grid is one wave of CTAs (SM count x resident CTAs per SM); warp
@@ -758,9 +739,9 @@ fp8_gemv_ring_kernel(const void* __restrict__ act, const float* __restrict__ act
       amax = red[0];
 #pragma unroll
       for (int i = 1; i < kRingConsumers; ++i) amax = fmaxf(amax, red[i]);
-      a_scale = amax == 0.0f ? 1.0f : __fdiv_rn(amax, 448.0f);
-      const float inv_scale = __frcp_rn(a_scale);
-      for (uint32_t c = ctid; c < chunks8; c += cthreads) stage_bf16_chunk(__ldg(xp + c), c, a_scale, inv_scale, xs);
+      const Quotient quot = token_quotient(amax);
+      a_scale = quot.scale;
+      for (uint32_t c = ctid; c < chunks8; c += cthreads) stage_bf16_chunk(__ldg(xp + c), c, quot, xs);
     } else {
       const uint8_t* a8 = static_cast<const uint8_t*>(act);
       for (uint32_t c = ctid; c < k / 16; c += cthreads) {
@@ -1181,7 +1162,7 @@ int32_t validate_nvfp4_gemv(const char* op, uint64_t rows, uint64_t k, float ga,
 // ---------------------------------------------------------------------------------------------
 // Decode-time FP8 token quantizer: one 1024-thread CTA per token, the token held in registers
 // between the amax pass and the conversion (one global round trip), quotients through
-// quotient_for_e4m3 (bit-identical to the IEEE division of src/numeric/fp8.cpp:41-58).  It
+// e4m3_of_quotients (bit-identical to the IEEE division of src/numeric/fp8.cpp:41-58).  It
 // triggers its dependents at once and waits for its predecessor before touching the
 // activation, so under programmatic dependent launch the GEMV that follows can prefetch its
 // weights while this kernel runs.  bf16 input, K <= 16384, K % 8 == 0.
@@ -1209,9 +1190,8 @@ fp8_quantize_decode_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__
   amax = red[0];
 #pragma unroll
   for (int i = 1; i < 32; ++i) amax = fmaxf(amax, red[i]);
-  const float scale = amax == 0.0f ? 1.0f : __fdiv_rn(amax, 448.0f);
-  const float inv_scale = __frcp_rn(scale);
-  if (threadIdx.x == 0) scales[t] = scale;
+  const Quotient quot = token_quotient(amax);
+  if (threadIdx.x == 0) scales[t] = quot.scale;
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
     const uint32_t c = threadIdx.x + i * 1024;
@@ -1220,16 +1200,16 @@ fp8_quantize_decode_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__
     uint32_t q[2] = {0, 0};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const float lo = quotient_for_e4m3(__uint_as_float(ww[j] << 16), scale, inv_scale);
-      const float hi = quotient_for_e4m3(__uint_as_float(ww[j] & 0xFFFF0000u), scale, inv_scale);
-      const uint32_t pair = static_cast<uint16_t>(__nv_cvt_float2_to_fp8x2(make_float2(lo, hi), __NV_SATFINITE, __NV_E4M3));
-      q[j >> 1] |= pair << (16 * (j & 1));
+      const float2 pair = make_float2(__uint_as_float(ww[j] << 16), __uint_as_float(ww[j] & 0xFFFF0000u));
+      q[j >> 1] |= (quot.tiny ? e4m3x2_divided(pair.x, pair.y, quot.scale) : e4m3_of_quotients(pair, quot)) << (16 * (j & 1));
     }
     *reinterpret_cast<uint2*>(out + t * k + static_cast<uint64_t>(c) * 8) = make_uint2(q[0], q[1]);
   }
 }
 
 }  // namespace
+
+bool pdl_enabled() { return g_pdl != 0; }
 
 int32_t launch_fp8_quantize_decode(const char* op, const uint16_t* x, uint8_t* out, float* scales, uint64_t tokens,
                                    uint64_t k, cudaStream_t stream) {

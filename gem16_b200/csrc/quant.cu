@@ -3,32 +3,44 @@
 //
 // All of them are HBM-streaming kernels: every input element is read once with 128-bit loads,
 // every output byte written once.  Algorithmic bytes per element (bf16 input): NVFP4
-// 2 + 0.5 + 1/16 = 2.5625 B, FP8 2 + 2 (second pass hits L2 or L1) + 1 = 3 B (+4 B per token).
+// 2 + 0.5 + 1/16 = 2.5625 B, FP8 2 + 1 = 3 B (+4 B per token).
+#include <algorithm>
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace gemb {
 namespace {
 
-
+// Sixteen / eight consecutive elements of a dependent input (an earlier kernel may have written it).
+__device__ __forceinline__ void unpack8(const uint4& t, float (&v)[8]) {
+  const uint32_t w[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    v[2 * j] = __uint_as_float(w[j] << 16);
+    v[2 * j + 1] = __uint_as_float(w[j] & 0xFFFF0000u);
+  }
+}
 __device__ __forceinline__ void load16(const float* p, float (&v)[16]) {
   const float4* q = reinterpret_cast<const float4*>(p);
+  float4 t[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) t[i] = ld_dep(q + i);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    float4 t = __ldg(q + i);
-    v[4 * i] = t.x; v[4 * i + 1] = t.y; v[4 * i + 2] = t.z; v[4 * i + 3] = t.w;
+    v[4 * i] = t[i].x; v[4 * i + 1] = t[i].y; v[4 * i + 2] = t[i].z; v[4 * i + 3] = t[i].w;
   }
 }
 __device__ __forceinline__ void load16(const uint16_t* p, float (&v)[16]) {
   const uint4* q = reinterpret_cast<const uint4*>(p);
+  const uint4 t0 = ld_dep(q), t1 = ld_dep(q + 1);
+  float a[8], b[8];
+  unpack8(t0, a);
+  unpack8(t1, b);
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    uint4 t = __ldg(q + i);
-    const uint32_t w[4] = {t.x, t.y, t.z, t.w};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      v[8 * i + 2 * j] = __uint_as_float(w[j] << 16);
-      v[8 * i + 2 * j + 1] = __uint_as_float(w[j] & 0xFFFF0000u);
-    }
+  for (int i = 0; i < 8; ++i) {
+    v[i] = a[i];
+    v[8 + i] = b[i];
   }
 }
 
@@ -58,41 +70,53 @@ struct GatedGeluLoader {
   }
 };
 
-// One thread per group of four consecutive 16-blocks ("quad", 64 elements): it writes 32 packed
-// bytes and one 32-bit word of scales.  The thread grid covers rows_out x quads where, for the
-// interleaved layout, rows_out is `tokens` rounded up to 128 and padded cells get zero scales.
+// The four scale bytes of a quad (four consecutive 16-blocks, one per lane of an aligned group of four) in one
+// word, little end first; every lane of the group gets it.
+__device__ __forceinline__ uint32_t quad_scale_word(uint32_t byte) {
+  const int pos = threadIdx.x & 3;
+  uint32_t w = byte << (8 * pos);
+  w |= __shfl_xor_sync(0xFFFFFFFFu, w, 1);
+  w |= __shfl_xor_sync(0xFFFFFFFFu, w, 2);
+  return w;
+}
+
+// One thread per 16-element block: 32 (bf16) or 64 bytes in, 8 payload bytes out, so that a warp's loads
+// and stores cover whole lines; four lanes pool their scale bytes into one 32-bit store.  The thread grid
+// covers rows_out x blocks_pad where, for the interleaved layout, rows_out is `tokens` rounded up to 128 and
+// padded cells get zero scales.  Bound by HBM at prefill sizes (2.56 B per bf16 element); a thread per quad,
+// the former split, read 128 bytes per thread with 128-byte strides between lanes and left a one-token call
+// with a single CTA.
 template <class Loader, bool kRcp, bool kInterleaved>
 __global__ void __launch_bounds__(256)
 nvfp4_quantize_kernel(Loader loader, uint8_t* __restrict__ packed, uint8_t* __restrict__ scales,
-                      uint64_t tokens, uint64_t k, uint64_t rows_out, uint64_t quads, float g) {
+                      uint32_t tokens, uint64_t k, uint32_t blocks_pad, uint64_t cells, float g) {
+  pdl_trigger();
+  pdl_wait();
+  // blockDim and cells are multiples of 4: quads stay whole.  A 64-bit division costs as much as the
+  // quantisation of a block, so it is left to tensors that need it.
   const uint64_t idx = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (idx >= rows_out * quads) return;
-  const uint64_t r = idx / quads, q = idx % quads;
-  const uint64_t c_real = k / 16;
-  uint32_t scale_word = 0;
-  if (r < tokens) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const uint64_t c = q * 4 + j;
-      if (c < c_real) {
-        float v[16];
-        loader(r * k + c * 16, v);
-        uint32_t lo, hi;
-        uint8_t sb;
-        quantize_block16<kRcp>(v, g, lo, hi, sb);
-        *reinterpret_cast<uint2*>(packed + r * (k / 2) + c * 8) = make_uint2(lo, hi);
-        scale_word |= static_cast<uint32_t>(sb) << (8 * j);
-      }
-    }
+  const uint64_t r = (cells >> 32) == 0 ? static_cast<uint32_t>(idx) / blocks_pad : idx / blocks_pad;
+  const uint32_t c = static_cast<uint32_t>(idx - r * blocks_pad);
+  const uint32_t c_real = static_cast<uint32_t>(k / 16);
+  const bool live = idx < cells && r < tokens && c < c_real;
+  uint8_t sb = 0;
+  if (live) {
+    float v[16];
+    loader(r * k + static_cast<uint64_t>(c) * 16, v);
+    uint32_t lo, hi;
+    quantize_block16<kRcp>(v, g, lo, hi, sb);
+    *reinterpret_cast<uint2*>(packed + r * (k / 2) + static_cast<uint64_t>(c) * 8) = make_uint2(lo, hi);
   }
+  const uint32_t word = quad_scale_word(sb);
+  if (idx >= cells) return;
   if constexpr (kInterleaved) {
-    *reinterpret_cast<uint32_t*>(scales + interleaved_scale_offset(r, q * 4, quads * 4)) = scale_word;
+    if ((c & 3) == 0) *reinterpret_cast<uint32_t*>(scales + interleaved_scale_offset(r, c, blocks_pad)) = word;
   } else {
-    if (q * 4 + 4 <= c_real && c_real % 4 == 0) {
-      *reinterpret_cast<uint32_t*>(scales + r * c_real + q * 4) = scale_word;
-    } else {
-      for (int j = 0; j < 4 && q * 4 + j < c_real; ++j)
-        scales[r * c_real + q * 4 + j] = static_cast<uint8_t>(scale_word >> (8 * j));
+    uint8_t* row = scales + r * c_real;
+    if (c_real % 4 == 0) {
+      if ((c & 3) == 0) *reinterpret_cast<uint32_t*>(row + c) = word;
+    } else if (live) {
+      row[c] = sb;
     }
   }
 }
@@ -102,18 +126,15 @@ int32_t launch_nvfp4_quantize(const char* op, Loader loader, uint8_t* packed, ui
                               uint64_t tokens, uint64_t k, float g, int32_t layout, int32_t mode,
                               cudaStream_t stream) {
   const bool inter = layout == GEMB_SCALES_INTERLEAVED;
-  const uint64_t rows_out = inter ? (tokens + 127) / 128 * 128 : tokens;
-  const uint64_t quads = (k / 16 + 3) / 4;
-  const uint64_t threads = rows_out * quads;
-  const unsigned grid = static_cast<unsigned>((threads + 255) / 256);
+  const uint64_t blocks_pad = (k / 16 + 3) / 4 * 4;
   const bool rcp = mode == GEMB_QUANT_RCP_APPROX;
-  if (inter) {
-    if (rcp) nvfp4_quantize_kernel<Loader, true, true><<<grid, 256, 0, stream>>>(loader, packed, scales, tokens, k, rows_out, quads, g);
-    else nvfp4_quantize_kernel<Loader, false, true><<<grid, 256, 0, stream>>>(loader, packed, scales, tokens, k, rows_out, quads, g);
-  } else {
-    if (rcp) nvfp4_quantize_kernel<Loader, true, false><<<grid, 256, 0, stream>>>(loader, packed, scales, tokens, k, rows_out, quads, g);
-    else nvfp4_quantize_kernel<Loader, false, false><<<grid, 256, 0, stream>>>(loader, packed, scales, tokens, k, rows_out, quads, g);
-  }
+  auto kern = inter ? (rcp ? nvfp4_quantize_kernel<Loader, true, true> : nvfp4_quantize_kernel<Loader, false, true>)
+                    : (rcp ? nvfp4_quantize_kernel<Loader, true, false> : nvfp4_quantize_kernel<Loader, false, false>);
+  const uint64_t cells = (inter ? (tokens + 127) / 128 * 128 : tokens) * blocks_pad;
+  // Few cells (a decode token): small CTAs, so that they spread over the SMs and load side by side.
+  const unsigned threads = cells <= 16384 ? 64 : 256;
+  GEMB_TRY(launch_pdl(op, kern, dim3(static_cast<unsigned>((cells + threads - 1) / threads)), dim3(threads), 0, stream,
+                      loader, packed, scales, static_cast<uint32_t>(tokens), k, static_cast<uint32_t>(blocks_pad), cells, g));
   return check_launch(op);
 }
 
@@ -135,29 +156,281 @@ int32_t validate_nvfp4_quantize(const char* op, const void* in, const void* pack
 }
 
 // ---------------------------------------------------------------------------------------------
-// RMSNorm fused quantizers.  One CTA of 256 threads per token.  The sum of squares follows the
-// reference exactly: thread t fma-accumulates index t, t+256, ... and a power-of-two tree folds
-// the 256 partials (src/cuda/nvfp4/reference.cu:102-118), so the fp32 sum is bit-identical.
+// Row kernels: RMSNorm fused quantizers, RMSNorm + residual, the FP8 per-token quantizer.
+//
+// The sum of squares follows the reference exactly: residue t of the row (indices t, t + 256, ...) is one fma
+// chain, and a power-of-two tree folds the 256 partials (strides 128, 64, ..., 1;
+// src/cuda/nvfp4/reference.cu:102-118), so the fp32 sum is bit-identical.  Both forms below keep that order:
+//   warp form   one warp per row.  Lane l holds eight consecutive elements of every 256-element chunk, i.e. the
+//               residues 8l .. 8l+7: eight independent chains per lane, the chunks in order, then the tree as
+//               shuffles.  The row (bf16, at most 4,096 elements) stays in registers between the passes, so
+//               it is read once, with 16-byte loads that are all in flight together, and nothing
+//               waits at a CTA barrier.  For batches that give every SM several rows.
+//   CTA form    256 threads per row, thread t owns residue t.  For few rows (a decode token: eight warps
+//               share the arithmetic of one row), fp32 inputs and long rows.
 // ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ float load_scalar(const float* p, uint64_t i) { return __ldg(p + i); }
-__device__ __forceinline__ float load_scalar(const uint16_t* p, uint64_t i) {
-  return bf16_bits_to_float(__ldg(p + i));
+__device__ __forceinline__ float sqrt_inverse(float sum, uint64_t k, float eps) {
+  return rsqrtf(sum / static_cast<float>(k) + eps);
 }
+__device__ __forceinline__ float2 bf16x2_to_float2(uint32_t w) {
+  return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
+}
+__device__ __forceinline__ uint32_t float2_to_bf16x2(float2 v) {
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(v.y), "f"(v.x));
+  return r;
+}
+// acc += v * v for a bf16 v, one rounding (mixed-precision fma: no unpacking, and off the integer pipe).
+__device__ __forceinline__ void fma_bf16(float& acc, uint16_t v) {
+  asm("fma.rn.f32.bf16 %0, %1, %1, %0;" : "+f"(acc) : "h"(v));
+}
+// Larger magnitude per half of two bf16 pairs whose sign bits are already cleared.
+__device__ __forceinline__ uint32_t max_bf16x2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+__device__ __forceinline__ float max_of_halves(uint32_t w) {
+  return fmaxf(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
+}
+__device__ __forceinline__ uint32_t abs_max4(const uint32_t (&w)[4]) {
+  return max_bf16x2(max_bf16x2(w[0] & 0x7FFF7FFFu, w[1] & 0x7FFF7FFFu), max_bf16x2(w[2] & 0x7FFF7FFFu, w[3] & 0x7FFF7FFFu));
+}
+
+constexpr int kRowChunks = 16;       // 256-element chunks a warp keeps in registers
+constexpr int kRowWarps = 4;         // rows (warps) per CTA of the warp form
+enum { kRowFp8 = 0, kRowFp8Norm = 1, kRowNvfp4Compact = 2, kRowNvfp4Interleaved = 3, kRowResidual = 4 };
+
+struct RowArgs {
+  const void* x;
+  const uint16_t* w;         // RMSNorm weight, may be null
+  uint8_t* out8;             // E4M3 bytes or E2M1 payload
+  void* scales;              // fp32 per row (FP8) or E4M3 block scales
+  const void* residual;
+  float* normalized;
+  void* out;                 // RMSNorm + residual
+  const uint16_t* scalar;
+  uint64_t rows, k;
+  float eps, g;
+  uint32_t rows_out;         // interleaved scales: rows rounded up to 128 (the padding is written as zero)
+};
+
+// Eight normalised elements as bf16 pairs: bf16((x * inv) * w).
+__device__ __forceinline__ void normalise8(const uint4& raw, const uint4* w, bool has_w, float inv, uint32_t (&n)[4]) {
+  const uint32_t xw[4] = {raw.x, raw.y, raw.z, raw.w};
+  uint4 wv = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);   // ones
+  if (has_w) wv = __ldg(w);
+  const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w};
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    n[j] = float2_to_bf16x2(__fmul2_rn(__fmul2_rn(bf16x2_to_float2(xw[j]), make_float2(inv, inv)), bf16x2_to_float2(ww[j])));
+}
+
+// Warp form.  bf16 rows, k a multiple of 16 and at most 4,096, 16-byte aligned rows.
+// Measured on 16,384 x 3,840 (4,096 for the plain FP8 quantizer), before (one CTA per row: 2-byte loads for the sum,
+// eight barriers, every pass from memory again, a division per element) and now, against the bytes at the copy peak:
+//   RMSNorm + FP8     184 -> 58 us (29)       FP8            66 -> 36 us (31)
+//   RMSNorm + NVFP4   142 -> 66 us (25)       RMSNorm + residual   140 -> 65 us (59)
+// The FP8 and residual forms are bound by HBM; the normalising quantizers by the integer pipe (unpacking
+// bf16, amax, scale bytes: about nine instructions per element there).
+template <int kMode, bool kRcp>
+__global__ void __launch_bounds__(kRowWarps * 32, kMode == kRowResidual ? 4 : 5)
+row_warp_kernel(const __grid_constant__ RowArgs a) {
+  pdl_trigger();
+  pdl_wait();
+  constexpr bool kNorm = kMode != kRowFp8;
+  const int lane = threadIdx.x & 31;
+  const uint64_t r = static_cast<uint64_t>(blockIdx.x) * kRowWarps + (threadIdx.x >> 5);
+  const uint32_t k = static_cast<uint32_t>(a.k);
+  if constexpr (kMode == kRowNvfp4Interleaved) {
+    if (r >= a.rows) {   // padding row of the interleaved scale buffer
+      const uint32_t quads = (k / 16 + 3) / 4;
+      if (r < a.rows_out)
+        for (uint32_t q = lane; q < quads; q += 32)
+          *reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(a.scales) + interleaved_scale_offset(r, 4 * q, quads * 4)) = 0;
+      return;
+    }
+  } else {
+    if (r >= a.rows) return;
+  }
+  const uint16_t* row = static_cast<const uint16_t*>(a.x) + r * k;
+  uint4 raw[kRowChunks];
+#pragma unroll
+  for (int c = 0; c < kRowChunks; ++c) {
+    const uint32_t i = c * 256 + lane * 8;
+    raw[c] = make_uint4(0, 0, 0, 0);
+    if (i < k) raw[c] = ld_dep(reinterpret_cast<const uint4*>(row + i));
+  }
+  // The residual's first eight chunks are requested before the reduction, the others behind the first half of the output.
+  uint4 res[kMode == kRowResidual ? 8 : 1];
+  auto load_residual = [&](int c0) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const uint32_t i = (c0 + u) * 256 + lane * 8;
+      if (i < k) res[kMode == kRowResidual ? u : 0] = ld_dep(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(a.residual) + r * k + i));
+    }
+  };
+  if constexpr (kMode == kRowResidual) load_residual(0);
+  float inv = 1.0f;
+  if constexpr (kNorm) {
+    float ss[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) ss[j] = 0.0f;
+#pragma unroll
+    for (int c = 0; c < kRowChunks; ++c) {
+      if (c * 256 >= static_cast<int>(k)) break;   // elements past k are zero and add nothing
+      const uint32_t xw[4] = {raw[c].x, raw[c].y, raw[c].z, raw[c].w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        fma_bf16(ss[2 * j], static_cast<uint16_t>(xw[j]));
+        fma_bf16(ss[2 * j + 1], static_cast<uint16_t>(xw[j] >> 16));
+      }
+    }
+    // Tree over residues 8 * lane + j.  Strides 128, 64, 32 pair lanes 16, 8, 4 apart: each step keeps half of
+    // the lane's residues (the lane's bit picks which), so that the later steps carry one value instead of eight.
+    float h4[4], h2[2], s;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float mine = (lane & 16) ? ss[4 + j] : ss[j], theirs = (lane & 16) ? ss[j] : ss[4 + j];
+      h4[j] = mine + __shfl_xor_sync(0xFFFFFFFFu, theirs, 16);
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const float mine = (lane & 8) ? h4[2 + j] : h4[j], theirs = (lane & 8) ? h4[j] : h4[2 + j];
+      h2[j] = mine + __shfl_xor_sync(0xFFFFFFFFu, theirs, 8);
+    }
+    s = ((lane & 4) ? h2[1] : h2[0]) + __shfl_xor_sync(0xFFFFFFFFu, (lane & 4) ? h2[0] : h2[1], 4);
+    s += __shfl_xor_sync(0xFFFFFFFFu, s, 2);     // stride 16
+    s += __shfl_xor_sync(0xFFFFFFFFu, s, 1);     // stride 8
+    s += __shfl_xor_sync(0xFFFFFFFFu, s, 16);    // strides 4, 2, 1: the residue's low bits sit in lane bits 4, 3, 2
+    s += __shfl_xor_sync(0xFFFFFFFFu, s, 8);
+    s += __shfl_xor_sync(0xFFFFFFFFu, s, 4);
+    inv = sqrt_inverse(s, k, a.eps);
+  }
+  const bool has_w = a.w != nullptr;
+  const uint4* wp = reinterpret_cast<const uint4*>(a.w) + lane;
+
+  if constexpr (kMode == kRowFp8 || kMode == kRowFp8Norm) {
+    uint32_t amax2 = 0;
+#pragma unroll
+    for (int c = 0; c < kRowChunks; ++c) {
+      if (c * 256 >= static_cast<int>(k)) break;
+      if constexpr (kNorm) {
+        uint32_t n[4];
+        normalise8(raw[c], wp + c * 32, has_w && c * 256 + lane * 8 < static_cast<int>(k), inv, n);
+        raw[c] = make_uint4(n[0], n[1], n[2], n[3]);
+      }
+      const uint32_t n[4] = {raw[c].x, raw[c].y, raw[c].z, raw[c].w};
+      amax2 = max_bf16x2(amax2, abs_max4(n));
+    }
+    const Quotient q = token_quotient(warp_max(max_of_halves(amax2)));
+    if (lane == 0) static_cast<float*>(a.scales)[r] = q.scale;
+    uint8_t* out = a.out8 + r * k + lane * 8;
+    auto convert = [&](auto code) {
+#pragma unroll
+      for (int c = 0; c < kRowChunks; ++c) {
+        if (c * 256 + lane * 8 >= k) break;
+        const uint32_t n[4] = {raw[c].x, raw[c].y, raw[c].z, raw[c].w};
+        uint32_t p[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) p[j] = code(bf16x2_to_float2(n[j]));
+        *reinterpret_cast<uint2*>(out + c * 256) = make_uint2(__byte_perm(p[0], p[1], 0x5410), __byte_perm(p[2], p[3], 0x5410));
+      }
+    };
+    if (q.tiny) convert([&](float2 v) { return e4m3x2_divided(v.x, v.y, q.scale); });
+    else convert([&](float2 v) { return e4m3_of_quotients(v, q); });
+  } else if constexpr (kMode == kRowNvfp4Compact || kMode == kRowNvfp4Interleaved) {
+    const uint32_t c_real = k / 16, c_pad = (c_real + 3) / 4 * 4;
+    // Chunk c covers blocks 16c .. 16c + 15, one per lane pair; addresses advance by constants.
+    uint8_t* pay = a.out8 + r * (k / 2) + lane * 4;
+    uint8_t* sc = static_cast<uint8_t*>(a.scales);
+    if constexpr (kMode == kRowNvfp4Interleaved) sc += interleaved_scale_offset(r, (lane >> 3) * 4, c_pad);
+    else sc += r * c_real + (lane >> 1);
+#pragma unroll
+    for (int c = 0; c < kRowChunks; ++c) {
+      if (c * 256 >= static_cast<int>(k)) break;
+      const uint32_t i = c * 256 + lane * 8;   // lanes 2b and 2b + 1 share a 16-element block
+      uint32_t n[4];
+      normalise8(raw[c], wp + c * 32, has_w && i < k, inv, n);
+      uint32_t m = abs_max4(n);
+      m = max_bf16x2(m, __shfl_xor_sync(0xFFFFFFFFu, m, 1));
+      const BlockScale s = block_scale<kRcp>(max_of_halves(m), a.g);
+      uint32_t p[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) p[j] = quantize_pair<kRcp>(bf16x2_to_float2(n[j]), a.g, s);
+      uint32_t word = __byte_perm(__byte_perm(p[0], p[1], 0x0040), __byte_perm(p[2], p[3], 0x0040), 0x5410);
+      if (!kRcp && s.ds == 0.0f) word = 0;
+      if (i < k) *reinterpret_cast<uint32_t*>(pay + c * 128) = word;
+      if (kMode == kRowNvfp4Interleaved || c_real % 4 == 0) {
+        // four blocks = eight lanes: their scale bytes leave as one word
+        uint32_t sw = i < k ? static_cast<uint32_t>(s.bits) << (8 * ((lane >> 1) & 3)) : 0u;
+        sw |= __shfl_xor_sync(0xFFFFFFFFu, sw, 2);
+        sw |= __shfl_xor_sync(0xFFFFFFFFu, sw, 4);
+        if ((lane & 7) == 0 && i / 16 < c_pad)
+          *reinterpret_cast<uint32_t*>(sc + c * (kMode == kRowNvfp4Interleaved ? 2048 : 16)) = sw;
+      } else if ((lane & 1) == 0 && i < k) {
+        sc[c * 16] = s.bits;
+      }
+    }
+  } else {
+    const float layer_scale = a.scalar ? bf16_bits_to_float(__ldg(a.scalar)) : 1.0f;
+    uint16_t* out = static_cast<uint16_t*>(a.out) + r * k;
+#pragma unroll
+    for (int c0 = 0; c0 < kRowChunks; c0 += 8) {
+      if (c0 != 0) load_residual(c0);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int c = c0 + u;
+        const uint32_t i = c * 256 + lane * 8;
+        if (i >= k) break;
+        const uint32_t rw[4] = {res[u].x, res[u].y, res[u].z, res[u].w};
+        uint32_t n[4];
+        normalise8(raw[c], wp + c * 32, has_w, inv, n);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          n[j] = float2_to_bf16x2(__fadd2_rn(bf16x2_to_float2(n[j]), bf16x2_to_float2(rw[j])));
+          if (a.scalar) n[j] = float2_to_bf16x2(__fmul2_rn(bf16x2_to_float2(n[j]), make_float2(layer_scale, layer_scale)));
+        }
+        *reinterpret_cast<uint4*>(out + i) = make_uint4(n[0], n[1], n[2], n[3]);
+      }
+    }
+  }
+}
+
+// ---- CTA form ---------------------------------------------------------------------------------
+__device__ __forceinline__ float to_float(float v) { return v; }
+__device__ __forceinline__ float to_float(uint16_t v) { return bf16_bits_to_float(v); }
 
 template <typename In>
 __device__ __forceinline__ float rmsnorm_inverse(const In* row, uint64_t k, float eps, float* red) {
   float ss = 0.0f;
-  for (uint64_t i = threadIdx.x; i < k; i += 256) {
-    const float v = load_scalar(row, i);
-    ss = fmaf(v, v, ss);
+  // sixteen loads of the thread's chain in flight at a time; zeros past the end add nothing
+  for (uint64_t base = threadIdx.x; base < k; base += 256 * 16) {
+    In raw[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const uint64_t i = base + j * 256;
+      raw[j] = In(0);
+      if (i < k) raw[j] = ld_dep(row + i);
+    }
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const float v = to_float(raw[j]);
+      ss = fmaf(v, v, ss);
+    }
   }
   red[threadIdx.x] = ss;
   __syncthreads();
-  for (unsigned stride = 128; stride; stride >>= 1) {
-    if (threadIdx.x < stride) red[threadIdx.x] += red[threadIdx.x + stride];
-    __syncthreads();
-  }
-  return rsqrtf(red[0] / static_cast<float>(k) + eps);
+  // Every warp folds the 256 partials by itself, in the tree's order: strides 128, 64, 32 inside the lane, the
+  // rest as shuffles.  One barrier instead of eight.
+  const int lane = threadIdx.x & 31;
+  float p[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) p[j] = red[lane + 32 * j];
+  float s = ((p[0] + p[4]) + (p[2] + p[6])) + ((p[1] + p[5]) + (p[3] + p[7]));
+#pragma unroll
+  for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+  return sqrt_inverse(s, k, eps);
 }
 
 // RMSNorm + residual (+ layer scalar) with the bf16 boundaries of src/cuda/norm/reference.cu:66-160:
@@ -165,112 +438,162 @@ __device__ __forceinline__ float rmsnorm_inverse(const In* row, uint64_t k, floa
 __device__ __forceinline__ void store_scalar(float* p, uint64_t i, float v) { p[i] = v; }
 __device__ __forceinline__ void store_scalar(uint16_t* p, uint64_t i, float v) { p[i] = float_to_bf16_bits(v); }
 
+// Any width and alignment: the second pass takes one element per thread and step, eight steps in flight.
 template <typename In, typename Res, typename Out>
 __global__ void __launch_bounds__(256)
-rmsnorm_residual_kernel(const In* __restrict__ x, const uint16_t* __restrict__ w, const Res* __restrict__ residual,
-                        float* __restrict__ normalized, Out* __restrict__ out, uint64_t k, float eps,
-                        const uint16_t* __restrict__ scalar) {
+rmsnorm_residual_kernel(const In* x, const uint16_t* __restrict__ w, const Res* residual, float* normalized, Out* out,
+                        uint64_t k, float eps, const uint16_t* __restrict__ scalar) {
   __shared__ float red[256];
+  pdl_trigger();
+  pdl_wait();
   const uint64_t base = static_cast<uint64_t>(blockIdx.x) * k;
   const float inv = rmsnorm_inverse(x + base, k, eps, red);
   const float layer_scale = scalar ? bf16_bits_to_float(__ldg(scalar)) : 1.0f;
-  for (uint64_t i = threadIdx.x; i < k; i += 256) {
-    const float ws = w ? bf16_bits_to_float(__ldg(w + i)) : 1.0f;
-    const float n = bf16_round(__fmul_rn(__fmul_rn(load_scalar(x + base, i), inv), ws));
-    if (normalized) normalized[base + i] = n;
-    float v = bf16_round(__fadd_rn(n, load_scalar(residual + base, i)));
-    if (scalar) v = bf16_round(__fmul_rn(v, layer_scale));
-    store_scalar(out, base + i, v);
+  for (uint64_t i0 = threadIdx.x; i0 < k; i0 += 256 * 8) {
+    In xv[8];
+    Res rv[8];
+    uint16_t wv[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const uint64_t i = i0 + j * 256;
+      if (i >= k) continue;
+      xv[j] = ld_dep(x + base + i);
+      rv[j] = ld_dep(residual + base + i);
+      wv[j] = w ? __ldg(w + i) : uint16_t(0x3F80);
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const uint64_t i = i0 + j * 256;
+      if (i >= k) continue;
+      const float n = bf16_round(__fmul_rn(__fmul_rn(to_float(xv[j]), inv), bf16_bits_to_float(wv[j])));
+      if (normalized) normalized[base + i] = n;
+      float v = bf16_round(__fadd_rn(n, to_float(rv[j])));
+      if (scalar) v = bf16_round(__fmul_rn(v, layer_scale));
+      store_scalar(out, base + i, v);
+    }
   }
+}
+
+__device__ __forceinline__ float norm_weight(const uint16_t* w, uint64_t i) {
+  return w ? bf16_bits_to_float(__ldg(w + i)) : 1.0f;
 }
 
 template <typename In, bool kRcp, bool kInterleaved>
 __global__ void __launch_bounds__(256)
-rmsnorm_nvfp4_quantize_kernel(const In* __restrict__ x, const uint16_t* __restrict__ w,
-                              uint8_t* __restrict__ packed, uint8_t* __restrict__ scales,
-                              uint64_t k, float eps, float g, uint64_t c_pad) {
+rmsnorm_nvfp4_quantize_kernel(const In* x, const uint16_t* __restrict__ w, uint8_t* packed, uint8_t* scales,
+                              uint32_t rows, uint64_t k, float eps, float g, uint32_t c_pad) {
   __shared__ float red[256];
+  pdl_trigger();
+  pdl_wait();
   const uint64_t r = blockIdx.x;
+  const uint32_t c_real = static_cast<uint32_t>(k / 16);
+  const bool pad_row = r >= rows;   // interleaved layout only: rows up to a multiple of 128 get zero scales
   const In* row = x + r * k;
-  const float inv = rmsnorm_inverse(row, k, eps, red);
-  for (uint64_t c = threadIdx.x; c < k / 16; c += 256) {
-    float v[16];
-    load16(row + c * 16, v);
+  float inv = 0.0f;
+  if (!pad_row) inv = rmsnorm_inverse(row, k, eps, red);
+  for (uint32_t c0 = 0; c0 < c_pad; c0 += 256) {
+    const uint32_t c = c0 + threadIdx.x;
+    uint8_t sb = 0;
+    if (c < c_real && !pad_row) {
+      float v[16];
+      load16(row + static_cast<uint64_t>(c) * 16, v);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const float ws = w ? bf16_bits_to_float(__ldg(w + c * 16 + i)) : 1.0f;
-      v[i] = bf16_round(__fmul_rn(__fmul_rn(v[i], inv), ws));
+      for (int i = 0; i < 16; ++i) v[i] = bf16_round(__fmul_rn(__fmul_rn(v[i], inv), norm_weight(w, c * 16ull + i)));
+      uint32_t lo, hi;
+      quantize_block16<kRcp>(v, g, lo, hi, sb);
+      *reinterpret_cast<uint2*>(packed + r * (k / 2) + c * 8ull) = make_uint2(lo, hi);
     }
-    uint32_t lo, hi;
-    uint8_t sb;
-    quantize_block16<kRcp>(v, g, lo, hi, sb);
-    *reinterpret_cast<uint2*>(packed + r * (k / 2) + c * 8) = make_uint2(lo, hi);
-    if constexpr (kInterleaved) scales[interleaved_scale_offset(r, c, c_pad)] = sb;
-    else scales[r * (k / 16) + c] = sb;
+    const uint32_t word = quad_scale_word(sb);
+    if (c >= c_pad) continue;
+    if constexpr (kInterleaved) {
+      if ((c & 3) == 0) *reinterpret_cast<uint32_t*>(scales + interleaved_scale_offset(r, c, c_pad)) = word;
+    } else if (c_real % 4 == 0) {
+      if ((c & 3) == 0) *reinterpret_cast<uint32_t*>(scales + r * c_real + c) = word;
+    } else if (c < c_real) {
+      scales[r * c_real + c] = sb;
+    }
   }
 }
 
-// ---------------------------------------------------------------------------------------------
-// FP8 per-token quantizer.  One CTA per token; pass 1 finds amax (max is order independent),
-// pass 2 divides and converts.  src/numeric/fp8.cpp:41-58, src/cuda/fp8/reference.cu:39-69.
-// ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ float block_max_256(float v, float* red) {
-  v = warp_max(v);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  float m = red[0];
-#pragma unroll
-  for (int i = 1; i < 8; ++i) m = fmaxf(m, red[i]);
-  return m;
-}
-
+// FP8 per-token quantizer: pass 1 finds amax (max is order independent), pass 2 divides and converts.
+// src/numeric/fp8.cpp:41-58, src/cuda/fp8/reference.cu:39-69.  A thread keeps its first two 16-element
+// blocks (rows of up to 8,192 elements) between the passes; the rest of a longer row is read again from L2.
 template <typename In, bool kNorm>
 __global__ void __launch_bounds__(256)
-fp8_quantize_kernel(const In* __restrict__ x, const uint16_t* __restrict__ w,
-                    uint8_t* __restrict__ out, float* __restrict__ scales, uint64_t k, float eps) {
+fp8_quantize_kernel(const In* x, const uint16_t* __restrict__ w, uint8_t* out, float* scales, uint64_t k, float eps) {
   __shared__ float red[256];
   __shared__ float red2[8];
+  pdl_trigger();
+  pdl_wait();
   const uint64_t r = blockIdx.x;
   const In* row = x + r * k;
   float inv = 1.0f;
   if constexpr (kNorm) inv = rmsnorm_inverse(row, k, eps, red);
-  auto value = [&](uint64_t i, float raw) {
+  const uint32_t blocks = static_cast<uint32_t>(k / 16);
+  auto block_values = [&](uint32_t c, float (&v)[16]) {
+    load16(row + static_cast<uint64_t>(c) * 16, v);
     if constexpr (kNorm) {
-      const float ws = w ? bf16_bits_to_float(__ldg(w + i)) : 1.0f;
-      return bf16_round(__fmul_rn(__fmul_rn(raw, inv), ws));
-    } else {
-      return raw;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = bf16_round(__fmul_rn(__fmul_rn(v[i], inv), norm_weight(w, c * 16ull + i)));
     }
   };
+  float kept[2][16];
   float amax = 0.0f;
-  for (uint64_t c = threadIdx.x; c < k / 16; c += 256) {
-    float v[16];
-    load16(row + c * 16, v);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(value(c * 16 + i, v[i])));
+  for (int b = 0; b < 2; ++b) {
+    const uint32_t c = threadIdx.x + b * 256;
+    if (c >= blocks) continue;
+    block_values(c, kept[b]);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(kept[b][i]));
   }
-  for (uint64_t i = (k / 16) * 16 + threadIdx.x; i < k; i += 256)
-    amax = fmaxf(amax, fabsf(value(i, load_scalar(row, i))));
-  amax = block_max_256(amax, red2);
-  const float scale = amax == 0.0f ? 1.0f : __fdiv_rn(amax, 448.0f);
-  if (threadIdx.x == 0) scales[r] = scale;
-  uint8_t* orow = out + r * k;
-  for (uint64_t c = threadIdx.x; c < k / 16; c += 256) {
+  for (uint32_t c = threadIdx.x + 512; c < blocks; c += 256) {
     float v[16];
-    load16(row + c * 16, v);
+    block_values(c, v);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(v[i]));
+  }
+  amax = warp_max(amax);
+  if ((threadIdx.x & 31) == 0) red2[threadIdx.x >> 5] = amax;
+  __syncthreads();
+  amax = red2[0];
+#pragma unroll
+  for (int i = 1; i < 8; ++i) amax = fmaxf(amax, red2[i]);
+  const Quotient q = token_quotient(amax);
+  if (threadIdx.x == 0) scales[r] = q.scale;
+  uint8_t* orow = out + r * k;
+  auto code = [&](float x, float y) {
+    return q.tiny ? e4m3x2_divided(x, y, q.scale) : e4m3_of_quotients(make_float2(x, y), q);
+  };
+  auto emit = [&](uint32_t c, const float (&v)[16]) {
     uint32_t words[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      uint32_t word = 0;
+    for (int j = 0; j < 4; ++j)
+      words[j] = code(v[4 * j], v[4 * j + 1]) | (code(v[4 * j + 2], v[4 * j + 3]) << 16);
+    *reinterpret_cast<uint4*>(orow + static_cast<uint64_t>(c) * 16) = make_uint4(words[0], words[1], words[2], words[3]);
+  };
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        word |= static_cast<uint32_t>(e4m3_encode(__fdiv_rn(value(c * 16 + 4 * j + i, v[4 * j + i]), scale))) << (8 * i);
-      words[j] = word;
-    }
-    *reinterpret_cast<uint4*>(orow + c * 16) = make_uint4(words[0], words[1], words[2], words[3]);
+  for (int b = 0; b < 2; ++b)
+    if (threadIdx.x + b * 256 < blocks) emit(threadIdx.x + b * 256, kept[b]);
+  for (uint32_t c = threadIdx.x + 512; c < blocks; c += 256) {
+    float v[16];
+    block_values(c, v);
+    emit(c, v);
   }
-  for (uint64_t i = (k / 16) * 16 + threadIdx.x; i < k; i += 256)
-    orow[i] = e4m3_encode(__fdiv_rn(value(i, load_scalar(row, i)), scale));
+}
+
+// Which form a batch of bf16 rows takes: see the comment above the row kernels.
+// Two rows per SM is where a warp per row has as many rows in flight as CTAs per row would.
+bool warp_rows(const void* x, const void* w, uint64_t rows, uint64_t k) {
+  return rows >= static_cast<uint64_t>(sm_count()) * 2 && k % 16 == 0 && k <= 256 * kRowChunks && (reinterpret_cast<uintptr_t>(x) & 15) == 0 &&
+         (reinterpret_cast<uintptr_t>(w) & 15) == 0;
+}
+template <int kMode, bool kRcp>
+int32_t launch_row_warp(const char* op, const RowArgs& a, cudaStream_t stream) {
+  const uint64_t rows = kMode == kRowNvfp4Interleaved ? a.rows_out : a.rows;
+  GEMB_TRY(launch_pdl(op, row_warp_kernel<kMode, kRcp>, dim3(static_cast<unsigned>((rows + kRowWarps - 1) / kRowWarps)),
+                      dim3(kRowWarps * 32), 0, stream, a));
+  return check_launch(op);
 }
 
 __global__ void __launch_bounds__(256)
@@ -322,26 +645,32 @@ int32_t gemb_nvfp4_rmsnorm_quantize(const void* input, int32_t input_dtype, cons
   GEMB_TRY(validate_nvfp4_quantize(op, input, packed, scales, input_dtype, tokens, k, g, layout, mode));
   GEMB_REQUIRE(std::isfinite(eps) && eps >= 0.0f, "%s: epsilon must be finite and nonnegative", op);
   const bool inter = layout == GEMB_SCALES_INTERLEAVED;
-  const uint64_t c_pad = (k / 16 + 3) / 4 * 4;
-  if (inter) {
-    // Padded rows / columns of the interleaved buffer must read as zero.
-    cudaError_t e = cudaMemsetAsync(scales, 0, gemb_interleaved_scale_bytes(tokens, k), stream);
-    if (e != cudaSuccess) return fail(GEMB_INTERNAL, "%s: %s: %s", op, cudaGetErrorName(e), cudaGetErrorString(e));
-  }
-  const unsigned grid = static_cast<unsigned>(tokens);
   const bool rcp = mode == GEMB_QUANT_RCP_APPROX;
-#define GEMB_LAUNCH_RMS(T, RCP, INTER)                                                         \
-  rmsnorm_nvfp4_quantize_kernel<T, RCP, INTER><<<grid, 256, 0, stream>>>(                      \
-      static_cast<const T*>(input), weight, packed, scales, k, eps, g, c_pad)
-  if (input_dtype == GEMB_F32) {
-    if (inter) { if (rcp) GEMB_LAUNCH_RMS(float, true, true); else GEMB_LAUNCH_RMS(float, false, true); }
-    else { if (rcp) GEMB_LAUNCH_RMS(float, true, false); else GEMB_LAUNCH_RMS(float, false, false); }
-  } else {
-    if (inter) { if (rcp) GEMB_LAUNCH_RMS(uint16_t, true, true); else GEMB_LAUNCH_RMS(uint16_t, false, true); }
-    else { if (rcp) GEMB_LAUNCH_RMS(uint16_t, true, false); else GEMB_LAUNCH_RMS(uint16_t, false, false); }
+  const uint64_t c_real = k / 16, c_pad = inter ? (c_real + 3) / 4 * 4 : c_real;
+  const uint64_t rows_out = inter ? (tokens + 127) / 128 * 128 : tokens;
+  if (input_dtype == GEMB_BF16 && warp_rows(input, weight, tokens, k)) {
+    RowArgs a{};
+    a.x = input;
+    a.w = weight;
+    a.out8 = packed;
+    a.scales = scales;
+    a.rows = tokens;
+    a.k = k;
+    a.eps = eps;
+    a.g = g;
+    a.rows_out = static_cast<uint32_t>(rows_out);
+    if (inter) return rcp ? launch_row_warp<kRowNvfp4Interleaved, true>(op, a, stream) : launch_row_warp<kRowNvfp4Interleaved, false>(op, a, stream);
+    return rcp ? launch_row_warp<kRowNvfp4Compact, true>(op, a, stream) : launch_row_warp<kRowNvfp4Compact, false>(op, a, stream);
   }
-#undef GEMB_LAUNCH_RMS
-  return check_launch(op);
+  auto launch = [&](auto* x) -> int32_t {
+    using T = std::remove_const_t<std::remove_pointer_t<decltype(x)>>;
+    auto kern = inter ? (rcp ? rmsnorm_nvfp4_quantize_kernel<T, true, true> : rmsnorm_nvfp4_quantize_kernel<T, false, true>)
+                      : (rcp ? rmsnorm_nvfp4_quantize_kernel<T, true, false> : rmsnorm_nvfp4_quantize_kernel<T, false, false>);
+    GEMB_TRY(launch_pdl(op, kern, dim3(static_cast<unsigned>(rows_out)), dim3(256), 0, stream, x, weight, packed, scales,
+                        static_cast<uint32_t>(tokens), k, eps, g, static_cast<uint32_t>(c_pad)));
+    return check_launch(op);
+  };
+  return input_dtype == GEMB_F32 ? launch(static_cast<const float*>(input)) : launch(static_cast<const uint16_t*>(input));
 }
 
 int32_t gemb_nvfp4_interleave_scales(const uint8_t* compact, uint8_t* interleaved, uint64_t rows,
@@ -369,18 +698,41 @@ static int32_t validate_fp8_quantize(const char* op, const void* in, const void*
   return require_sm100(op);
 }
 
+}  // extern "C"
+namespace {
+template <bool kNorm>
+int32_t launch_fp8_rows(const char* op, const void* input, int32_t input_dtype, const uint16_t* weight, uint8_t* out,
+                        float* scales, uint64_t tokens, uint64_t k, float eps, cudaStream_t stream) {
+  if (input_dtype == GEMB_BF16 && warp_rows(input, weight, tokens, k)) {
+    RowArgs a{};
+    a.x = input;
+    a.w = weight;
+    a.out8 = out;
+    a.scales = scales;
+    a.rows = tokens;
+    a.k = k;
+    a.eps = eps;
+    return launch_row_warp<kNorm ? kRowFp8Norm : kRowFp8, false>(op, a, stream);
+  }
+  const dim3 grid(static_cast<unsigned>(tokens));
+  if (input_dtype == GEMB_F32)
+    GEMB_TRY(launch_pdl(op, fp8_quantize_kernel<float, kNorm>, grid, dim3(256), 0, stream, static_cast<const float*>(input), weight,
+                        out, scales, k, eps));
+  else
+    GEMB_TRY(launch_pdl(op, fp8_quantize_kernel<uint16_t, kNorm>, grid, dim3(256), 0, stream,
+                        static_cast<const uint16_t*>(input), weight, out, scales, k, eps));
+  return check_launch(op);
+}
+}  // namespace
+extern "C" {
+
 int32_t gemb_fp8_quantize(const void* input, int32_t input_dtype, uint8_t* out, float* scales,
                           uint64_t tokens, uint64_t k, gemb_stream_t stream) {
   const char* op = "gemb_fp8_quantize";
   GEMB_TRY(validate_fp8_quantize(op, input, out, scales, input_dtype, tokens, k));
-  const unsigned grid = static_cast<unsigned>(tokens);
   if (input_dtype == GEMB_BF16 && tokens <= 16 && k <= 16384)   // decode batches: latency-optimised kernel
     return launch_fp8_quantize_decode(op, static_cast<const uint16_t*>(input), out, scales, tokens, k, stream);
-  if (input_dtype == GEMB_F32)
-    fp8_quantize_kernel<float, false><<<grid, 256, 0, stream>>>(static_cast<const float*>(input), nullptr, out, scales, k, 0.0f);
-  else
-    fp8_quantize_kernel<uint16_t, false><<<grid, 256, 0, stream>>>(static_cast<const uint16_t*>(input), nullptr, out, scales, k, 0.0f);
-  return check_launch(op);
+  return launch_fp8_rows<false>(op, input, input_dtype, nullptr, out, scales, tokens, k, 0.0f, stream);
 }
 
 int32_t gemb_fp8_rmsnorm_quantize(const void* input, int32_t input_dtype, const uint16_t* weight,
@@ -389,12 +741,7 @@ int32_t gemb_fp8_rmsnorm_quantize(const void* input, int32_t input_dtype, const 
   const char* op = "gemb_fp8_rmsnorm_quantize";
   GEMB_TRY(validate_fp8_quantize(op, input, out, scales, input_dtype, tokens, k));
   GEMB_REQUIRE(std::isfinite(eps) && eps >= 0.0f, "%s: epsilon must be finite and nonnegative", op);
-  const unsigned grid = static_cast<unsigned>(tokens);
-  if (input_dtype == GEMB_F32)
-    fp8_quantize_kernel<float, true><<<grid, 256, 0, stream>>>(static_cast<const float*>(input), weight, out, scales, k, eps);
-  else
-    fp8_quantize_kernel<uint16_t, true><<<grid, 256, 0, stream>>>(static_cast<const uint16_t*>(input), weight, out, scales, k, eps);
-  return check_launch(op);
+  return launch_fp8_rows<true>(op, input, input_dtype, weight, out, scales, tokens, k, eps, stream);
 }
 
 int32_t gemb_rmsnorm_residual(const void* input, int32_t input_dtype, const uint16_t* weight_bf16, const void* residual,
@@ -409,19 +756,34 @@ int32_t gemb_rmsnorm_residual(const void* input, int32_t input_dtype, const uint
   GEMB_REQUIRE(residual_output_dtype == GEMB_F32 || (input_dtype == GEMB_BF16 && normalized_output == nullptr),
                "%s: bf16 residual and output go with a bf16 input and no separate normalised output", op);
   GEMB_ENTER(op);
-  const unsigned grid = static_cast<unsigned>(vectors);
-  if (residual_output_dtype == GEMB_BF16)
-    rmsnorm_residual_kernel<<<grid, 256, 0, stream>>>(static_cast<const uint16_t*>(input), weight_bf16,
-                                                      static_cast<const uint16_t*>(residual), normalized_output,
-                                                      static_cast<uint16_t*>(output), width, epsilon, scalar_bf16);
+  const bool bf16_out = residual_output_dtype == GEMB_BF16;
+  auto aligned16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  if (bf16_out && warp_rows(input, weight_bf16, vectors, width) && aligned16(residual) && aligned16(output)) {
+    RowArgs a{};
+    a.x = input;
+    a.w = weight_bf16;
+    a.residual = residual;
+    a.out = output;
+    a.scalar = scalar_bf16;
+    a.rows = vectors;
+    a.k = width;
+    a.eps = epsilon;
+    return launch_row_warp<kRowResidual, false>(op, a, stream);
+  }
+  const dim3 grid(static_cast<unsigned>(vectors));
+  const auto* xb = static_cast<const uint16_t*>(input);
+  if (bf16_out)
+    GEMB_TRY(launch_pdl(op, rmsnorm_residual_kernel<uint16_t, uint16_t, uint16_t>, grid, dim3(256), 0, stream, xb, weight_bf16,
+                        static_cast<const uint16_t*>(residual), normalized_output, static_cast<uint16_t*>(output), width,
+                        epsilon, scalar_bf16));
   else if (input_dtype == GEMB_BF16)
-    rmsnorm_residual_kernel<<<grid, 256, 0, stream>>>(static_cast<const uint16_t*>(input), weight_bf16,
-                                                      static_cast<const float*>(residual), normalized_output,
-                                                      static_cast<float*>(output), width, epsilon, scalar_bf16);
+    GEMB_TRY(launch_pdl(op, rmsnorm_residual_kernel<uint16_t, float, float>, grid, dim3(256), 0, stream, xb, weight_bf16,
+                        static_cast<const float*>(residual), normalized_output, static_cast<float*>(output), width, epsilon,
+                        scalar_bf16));
   else
-    rmsnorm_residual_kernel<<<grid, 256, 0, stream>>>(static_cast<const float*>(input), weight_bf16,
-                                                      static_cast<const float*>(residual), normalized_output,
-                                                      static_cast<float*>(output), width, epsilon, scalar_bf16);
+    GEMB_TRY(launch_pdl(op, rmsnorm_residual_kernel<float, float, float>, grid, dim3(256), 0, stream,
+                        static_cast<const float*>(input), weight_bf16, static_cast<const float*>(residual), normalized_output,
+                        static_cast<float*>(output), width, epsilon, scalar_bf16));
   return check_launch(op);
 }
 

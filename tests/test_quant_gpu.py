@@ -190,3 +190,76 @@ def test_quantizer_properties_at_full_size(lib, dev):
     assert int(s.max()) <= 0x7E
     # scale bytes are monotone in block amax: the block holding the global amax gets 448.
     assert int(s.max()) == 0x7E
+
+
+@pytest.mark.parametrize("rows,k", [(296, 16), (300, 272), (297, 3840), (513, 4096), (300, 4112)])
+def test_row_kernels_warp_form_equals_cta_form(lib, dev, orc, rows, k):
+    """Batches take one warp per row (up to 4,096 elements), single rows one CTA: same bytes, row by row, at the
+    edges of the 256-element chunks, with a partial last CTA and around the size where the forms change."""
+    rng = np.random.default_rng(rows + k)
+    x = bf16_round(rng.standard_normal((rows, k)).astype(np.float32) * 3)
+    x[3] = 0.0
+    w = to_dev(bf16_bits(1.0 + 0.1 * rng.standard_normal(k).astype(np.float32)), dev)
+    res = to_dev(bf16_bits(rng.standard_normal((rows, k)).astype(np.float32)), dev)
+    xd, g = to_dev(bf16_bits(x), dev), 400.0
+    u8 = dict(dtype=torch.uint8, device=dev)
+
+    def run(t, xin, rin):
+        nb = lib.cdll.gemb_interleaved_scale_bytes(t, k)
+        o = {"q": torch.full((t, k), 0xA5, **u8), "qs": torch.zeros((t,), device=dev), "n": torch.full((t, k), 0xA5, **u8),
+             "ns": torch.zeros((t,), device=dev), "p": torch.full((t, k // 2), 0xA5, **u8),
+             "s": torch.full((t, k // 16), 0xA5, **u8), "pi": torch.full((t, k // 2), 0xA5, **u8),
+             "r": torch.zeros((t, k), dtype=torch.int16, device=dev)}
+        si = torch.full((nb,), 0xA5, **u8)
+        lib.gemb_fp8_quantize(xin, BF16, o["q"], o["qs"], t, k, None)
+        lib.gemb_fp8_rmsnorm_quantize(xin, BF16, w, o["n"], o["ns"], t, k, 1e-6, None)
+        lib.gemb_nvfp4_rmsnorm_quantize(xin, BF16, w, o["p"], o["s"], t, k, 1e-6, g, COMPACT, EXACT, None)
+        lib.gemb_nvfp4_rmsnorm_quantize(xin, BF16, w, o["pi"], si, t, k, 1e-6, g, INTERLEAVED, EXACT, None)
+        lib.gemb_rmsnorm_residual(xin, BF16, w, rin, None, o["r"], BF16, t, k, 1e-6, None, None)
+        return o, si
+
+    batch, si = run(rows, xd, res)
+    for r in (0, 3, 128, rows - 1):
+        one, _ = run(1, xd[r:r + 1].contiguous(), res[r:r + 1].contiguous())
+        for name, v in one.items():
+            assert torch.equal(v[0], batch[name][r]), (name, r)
+    assert torch.equal(batch["p"], batch["pi"])
+    assert np.array_equal(to_np(si), orc.interleave_scales(to_np(batch["s"]), k))   # padding zero
+    qo, so = orc.fp8_quantize(x)
+    assert np.array_equal(to_np(batch["q"]), qo) and np.array_equal(to_np(batch["qs"]), so)
+
+
+def test_nvfp4_every_scale_byte_at_every_rounding_boundary(lib, dev, orc):
+    """All 126 nonzero scale bytes, each with values on and one ulp beside the E2M1 rounding boundaries, both signs
+    and signed zeros: the reciprocal and the residual correction give the oracle's bytes."""
+    b = np.array([0.25, 0.75, 1.25, 1.75, 2.5, 3.5, 5.0, 6.0], np.float32)
+    blocks = []
+    for code in range(1, 127):
+        ds = np.float32(orc.e4m3_decode(code))
+        for near in (np.float32(-np.inf), None, np.float32(np.inf)):
+            v = (b * ds).astype(np.float32)
+            v[:7] = v[:7] if near is None else np.nextafter(v[:7], near)
+            blocks.append(np.concatenate([v, -v[:7], np.array([-0.0], np.float32)]))
+    x = np.stack(blocks).astype(np.float32)
+    p, s = run_nvfp4(lib, dev, x, 1.0)
+    po, so = orc.nvfp4_quantize(x, 1.0)
+    assert len(np.unique(s)) == 126
+    assert np.array_equal(p, po) and np.array_equal(s.reshape(so.shape), so)
+
+
+@pytest.mark.parametrize("rows", [1, 300])
+@pytest.mark.parametrize("amax", [448.0, 3.3, 1e-20, 1e-30, 1e36])
+def test_fp8_quotients_at_rounding_boundaries(lib, dev, orc, rows, amax):
+    """Elements on and around the E4M3 rounding boundaries of their token's scale, from bf16 inputs; scales down to
+    where the quantiser falls back to the division."""
+    codes = np.array([orc.e4m3_decode(c) for c in range(0, 127)], np.float32)
+    mids = ((codes[1:] + codes[:-1]) / 2).astype(np.float32)
+    v = np.concatenate([codes, mids, -mids, [-0.0, 0.0]]).astype(np.float64) * (float(bf16_round(np.float32([amax]))[0]) / 448.0)
+    v = np.concatenate([v, np.zeros((-len(v)) % 16)]).astype(np.float32)
+    x = bf16_round(np.stack([v] * rows))
+    x[:, 0] = bf16_round(np.float32([amax]))[0]
+    q = torch.zeros(x.shape, dtype=torch.uint8, device=dev)
+    sc = torch.zeros((rows,), dtype=torch.float32, device=dev)
+    lib.gemb_fp8_quantize(to_dev(bf16_bits(x), dev), BF16, q, sc, rows, x.shape[1], None)
+    qo, so = orc.fp8_quantize(x)
+    assert np.array_equal(to_np(sc), so) and np.array_equal(to_np(q), qo)
