@@ -47,6 +47,7 @@ int32_t launch_fp8_quantize_decode(const char* op, const uint16_t* x, uint8_t* o
 int gemv_take_device_error();
 int ep_take_device_error();
 int moe_take_device_error();
+int router_input_take_device_error();
 
 inline bool positive_finite(float v) { return std::isfinite(v) && v > 0.0f; }
 

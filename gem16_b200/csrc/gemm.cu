@@ -1319,6 +1319,8 @@ int32_t gemb_check_device_status(void) {
     return fail(GEMB_INTERNAL, "%s: an expert-parallel flag barrier gave up waiting for a peer (check 5)", op);
   if (ep_code != 0)
     return fail(GEMB_INTERNAL, "%s: an expert-parallel kernel met positions outside its buffers and skipped or clamped them (check %d)", op, ep_code);
+  if (router_input_take_device_error() != 0)
+    return fail(GEMB_INTERNAL, "%s: the router's input transform gave up waiting for its rows", op);
   const int moe_code = moe_take_device_error();
   if (moe_code == 1)
     return fail(GEMB_DATA_LOSS, "%s: the router met a non-finite logit; the token got zero routing weights", op);

@@ -11,16 +11,129 @@
 
 #include "common.cuh"
 #include "moe_layer.h"
+#include "ptx.cuh"
 
 namespace gemb {
 
+__device__ int g_router_input_error = 0;   // 3 = the router's input transform gave up waiting for its rows
+
+int router_input_take_device_error() {
+  int code = 0;
+  if (cudaMemcpyFromSymbol(&code, g_router_input_error, sizeof code) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  if (code != 0) {
+    const int zero = 0;
+    cudaMemcpyToSymbol(g_router_input_error, &zero, sizeof zero);
+  }
+  return code;
+}
+
 namespace {
 
-// r = bf16(((x * inv) * scale) * root): one thread per token walks the row (the sum of squares is a
-// single fma chain in ascending k, which is the contract), then the CTA's threads rescale the
-// rows together.  A mode of the router, not a hot kernel.
+// r = bf16(((x * inv) * scale) * root), where the sum of squares behind inv is ONE fp32 fma chain in ascending k
+// (the contract).  The chain is the floor: hidden x 4 clocks, 6 us at 2,816, whatever the batch; everything
+// else has to hide behind it or be short.  A CTA takes eight tokens and keeps their rows in shared memory: one
+// thread requests them as 1,024-byte pieces with bulk copies, a warp whose lanes are the tokens follows the
+// pieces as they land, then all warps rescale the rows out of shared memory, so that x is read once.
+// Rows are padded by 16 bytes so that the eight lanes' 16-byte reads fall into different banks.
+// 45 KB per CTA at 2,816: five CTAs per SM, one's chain over another's loads and stores.  Measured on
+// 3,001 x 2,816: 15 us, against 821 us for a thread per token walking global memory.
+constexpr uint32_t kRiTokens = 8, kRiThreads = 256, kRiPiece = 1024;
+constexpr uint32_t kRiMaxHidden = 12288;   // eight rows have to fit the shared memory of a CTA
+__host__ __device__ constexpr uint32_t router_input_row_bytes(uint32_t hidden) { return hidden * 2 + 16; }
+__host__ __device__ constexpr uint32_t router_input_pieces(uint32_t hidden) { return (hidden * 2 + kRiPiece - 1) / kRiPiece; }
+constexpr uint32_t router_input_smem(uint32_t hidden) {
+  return kRiTokens * router_input_row_bytes(hidden) + router_input_pieces(hidden) * 8;
+}
+
+__device__ __forceinline__ void fma_square_bf16(float& acc, uint16_t v) {
+  asm("fma.rn.f32.bf16 %0, %1, %1, %0;" : "+f"(acc) : "h"(v));
+}
+
+__global__ void __launch_bounds__(kRiThreads)
+router_input_kernel(const uint16_t* x, const uint16_t* __restrict__ scale, uint16_t* out, uint32_t tokens,
+                    uint32_t hidden, float eps, float root, bool vector_access) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  __shared__ float inv_s[kRiTokens];
+  const uint32_t row_bytes = router_input_row_bytes(hidden), pieces = router_input_pieces(hidden);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kRiTokens * row_bytes);
+  const uint32_t t0 = blockIdx.x * kRiTokens, rows = min(kRiTokens, tokens - t0);
+  const int lane = threadIdx.x & 31;
+  pdl_trigger();
+  if (threadIdx.x < 32) {
+    if (lane == 0) {
+      for (uint32_t p = 0; p < pieces; ++p) ptx::mbar_init(&bars[p], 1);
+      ptx::fence_barrier_init();
+      pdl_wait();
+      for (uint32_t p = 0; p < pieces; ++p) {
+        const uint32_t bytes = min(kRiPiece, hidden * 2 - p * kRiPiece);
+        ptx::mbar_expect_tx(&bars[p], bytes * rows);
+        for (uint32_t r = 0; r < rows; ++r)
+          ptx::bulk_load_1d(smem + r * row_bytes + p * kRiPiece,
+                            reinterpret_cast<const uint8_t*>(x + static_cast<uint64_t>(t0 + r) * hidden) + p * kRiPiece, bytes, &bars[p]);
+      }
+    }
+    __syncwarp();
+    const uint8_t* row = smem + min(static_cast<uint32_t>(lane), rows - 1) * row_bytes;
+    float ss = 0.0f;
+    for (uint32_t p = 0; p < pieces; ++p) {
+      if (!ptx::mbar_wait(&bars[p], 0)) {
+        if (lane == 0) atomicCAS(&g_router_input_error, 0, 3);
+        for (int i = 0; i < 2000; ++i) __nanosleep(1000);   // copies in flight get time to land before the CTA ends
+        break;
+      }
+      const uint32_t n = min(kRiPiece, hidden * 2 - p * kRiPiece) / 16;
+      const uint4* src = reinterpret_cast<const uint4*>(row + p * kRiPiece);
+#pragma unroll 8
+      for (uint32_t i = 0; i < n; ++i) {
+        const uint4 v = src[i];
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          fma_square_bf16(ss, static_cast<uint16_t>(w[j]));
+          fma_square_bf16(ss, static_cast<uint16_t>(w[j] >> 16));
+        }
+      }
+    }
+    const float mean = __fadd_rn(__fdiv_rn(ss, static_cast<float>(hidden)), eps);
+    if (static_cast<uint32_t>(lane) < rows) inv_s[lane] = __fdiv_rn(1.0f, __fsqrt_rn(mean));
+  } else {
+    pdl_wait();
+  }
+  __syncthreads();   // the rows have landed (warp 0 waited for every piece), the factors are known
+  auto rescaled = [&](uint32_t bits, float inv, uint32_t s) {   // one element; arguments are bf16 bit patterns in the high half
+    return float_to_bf16_bits(__fmul_rn(__fmul_rn(__fmul_rn(__uint_as_float(bits), inv), __uint_as_float(s)), root));
+  };
+  if (vector_access) {
+    const uint32_t chunks = hidden / 8;
+    for (uint32_t c = threadIdx.x; c < chunks; c += kRiThreads) {   // a thread keeps its scales for all rows
+      const uint4 sv = __ldg(reinterpret_cast<const uint4*>(scale) + c);
+      const uint32_t sw[4] = {sv.x, sv.y, sv.z, sv.w};
+      for (uint32_t r = 0; r < rows; ++r) {
+        const uint4 v = *reinterpret_cast<const uint4*>(smem + r * row_bytes + c * 16);
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+        const float inv = inv_s[r];
+        uint32_t o[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          o[j] = rescaled(w[j] << 16, inv, sw[j] << 16) | (static_cast<uint32_t>(rescaled(w[j] & 0xFFFF0000u, inv, sw[j] & 0xFFFF0000u)) << 16);
+        reinterpret_cast<uint4*>(out + static_cast<uint64_t>(t0 + r) * hidden)[c] = make_uint4(o[0], o[1], o[2], o[3]);
+      }
+    }
+  } else {
+    for (uint32_t i = threadIdx.x; i < rows * hidden; i += kRiThreads) {
+      const uint32_t r = i / hidden, c = i % hidden;
+      const uint32_t v = *reinterpret_cast<const uint16_t*>(smem + r * row_bytes + c * 2);
+      out[static_cast<uint64_t>(t0 + r) * hidden + c] = rescaled(v << 16, inv_s[r], static_cast<uint32_t>(__ldg(scale + c)) << 16);
+    }
+  }
+}
+
+// Rows too long for shared memory: one thread per token walks its row, then the CTA rescales the rows together.
 __global__ void __launch_bounds__(128)
-router_input_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ scale, uint16_t* __restrict__ out,
+router_input_long_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ scale, uint16_t* __restrict__ out,
                     uint32_t tokens, uint32_t hidden, float eps, float root) {
   __shared__ float inv_s[128];
   const uint32_t t0 = blockIdx.x * 128;
@@ -267,8 +380,19 @@ int32_t gemb_moe_router_input(const uint16_t* x_bf16, const uint16_t* scale_bf16
   GEMB_REQUIRE(reinterpret_cast<uintptr_t>(x_bf16) % 16 == 0, "%s: input must be 16-byte aligned", op);
   GEMB_ENTER(op);
   const float root = 1.0f / std::sqrt(static_cast<float>(hidden));
-  router_input_kernel<<<static_cast<unsigned>((tokens + 127) / 128), 128, 0, stream>>>(
-      x_bf16, scale_bf16, out_bf16, static_cast<uint32_t>(tokens), static_cast<uint32_t>(hidden), epsilon, root);
+  const uint32_t h = static_cast<uint32_t>(hidden), t = static_cast<uint32_t>(tokens);
+  if (h > kRiMaxHidden) {
+    router_input_long_kernel<<<(t + 127) / 128, 128, 0, stream>>>(x_bf16, scale_bf16, out_bf16, t, h, epsilon, root);
+    return check_launch(op);
+  }
+  const uint32_t smem = router_input_smem(h);
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(router_input_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return fail(GEMB_INTERNAL, "%s: %s: %s", op, cudaGetErrorName(e), cudaGetErrorString(e));
+  }
+  const bool vec = reinterpret_cast<uintptr_t>(scale_bf16) % 16 == 0 && reinterpret_cast<uintptr_t>(out_bf16) % 16 == 0;
+  GEMB_TRY(launch_pdl(op, router_input_kernel, dim3((t + kRiTokens - 1) / kRiTokens), dim3(kRiThreads), smem, stream, x_bf16,
+                      scale_bf16, out_bf16, t, h, epsilon, root, vec));
   return check_launch(op);
 }
 

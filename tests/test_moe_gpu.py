@@ -394,3 +394,16 @@ def test_router_specification_mode(lib, dev, orc):
     assert np.array_equal(to_np(layer.logits).view(np.uint32), logits.view(np.uint32))
     assert np.array_equal(to_np(layer.ids), ids)
     assert np.array_equal(to_np(layer.weights).view(np.uint32), weights.view(np.uint32))
+
+
+@pytest.mark.parametrize("tokens,hidden,offset", [(1, 8, 0), (9, 520, 0), (13, 2816, 1), (3, 12288, 0), (2, 12296, 0)])
+def test_router_input_rows_in_shared_memory(lib, dev, orc, tokens, hidden, offset):
+    """Partial last CTA, rows that end inside a 1,024-byte piece, an output without 16-byte alignment, and the
+    row lengths on both sides of the shared-memory limit: the bits of the oracle's serial chain."""
+    rng = np.random.default_rng(tokens + hidden)
+    x = bf16_bits(rng.standard_normal((tokens, hidden)).astype(np.float32))
+    scale = bf16_bits(1.0 + 0.1 * rng.standard_normal(hidden).astype(np.float32))
+    got = torch.zeros((tokens * hidden + offset,), dtype=torch.int16, device=dev)
+    lib.gemb_moe_router_input(to_dev(x, dev), to_dev(scale, dev), got[offset:], tokens, hidden, 1e-6, None)
+    want = orc.moe_router_input(x, scale, 1e-6)
+    assert np.array_equal(to_np(got[offset:]).view(np.uint16).reshape(tokens, hidden), want)
