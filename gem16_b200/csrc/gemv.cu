@@ -1,13 +1,12 @@
-// Batch-1 decode projections: HBM-streaming, warp-reduced GEMV kernels for FP8 (W8A8) and NVFP4
-// (W4A4) weights in the checkpoint's row-major source layout.
+// Batch-1 decode projections: HBM-streaming, warp-reduced GEMV kernels for FP8 (W8A8) weights in the
+// checkpoint's row-major source layout (NVFP4 weights: nvfp4_gemv.cu).
 //
-// Shape of every kernel: a CTA of 8 warps stages the activation vector once in shared memory
-// (decoded to fp16, which holds every E4M3 and E2M1 value exactly), then each warp streams
-// kRows weight rows with coalesced 128-bit loads (lane l reads bytes [16 l, 16 l + 16) of each
-// 512-byte row segment, `no_allocate` so the stream does not evict the activation from L1),
-// accumulates in fp32 and folds the 32 lanes with an xor butterfly.  Weights are read exactly
-// once: algorithmic bytes per output row are K (FP8) or K/2 + K/16 (NVFP4) plus the scale and
-// the 4-byte result; the activation (K bytes or less) is re-read per CTA from L2.
+// A CTA of 8 warps stages the activation vector once in shared memory (decoded to fp16, which holds every
+// E4M3 value exactly), then each warp streams kRows weight rows with coalesced 128-bit loads (lane l reads
+// bytes [16 l, 16 l + 16) of each 512-byte row segment, `no_allocate` so the stream does not evict the
+// activation from L1), accumulates in fp32 and folds the 32 lanes with an xor butterfly.  Weights are read
+// exactly once: algorithmic bytes per output row are K plus the scale and the 4-byte result; the
+// activation (K bytes) is re-read per CTA from L2.
 #include <algorithm>
 #include <mutex>
 
@@ -906,260 +905,6 @@ int32_t validate_fp8_gemv(const char* op, const void* act, const void* w, const 
 }
 
 // ---------------------------------------------------------------------------------------------
-// NVFP4 GEMV.  Activation staged as fp16 values (decoded E2M1) plus fp32 decoded block scales.
-// A lane's 16-byte weight chunk is two 16-element blocks; within a block the sixteen E2M1
-// products are summed in fp16 (exact: each product is a multiple of 1/4 no larger than 36, a
-// half2 lane sums eight of them, at most 288), then the block sum is scaled by sa*sw in fp32.
-// ---------------------------------------------------------------------------------------------
-// All four bytes of a word -> four half2.
-__device__ __forceinline__ void e2m1x8_to_half2(uint32_t word, uint32_t (&h)[4]) {
-  asm("{ .reg .b8 t0, t1, t2, t3;\n"
-      "  mov.b32 {t0, t1, t2, t3}, %4;\n"
-      "  cvt.rn.f16x2.e2m1x2 %0, t0;\n"
-      "  cvt.rn.f16x2.e2m1x2 %1, t1;\n"
-      "  cvt.rn.f16x2.e2m1x2 %2, t2;\n"
-      "  cvt.rn.f16x2.e2m1x2 %3, t3; }"
-      : "=r"(h[0]), "=r"(h[1]), "=r"(h[2]), "=r"(h[3])
-      : "r"(word));
-}
-__device__ __forceinline__ uint32_t hfma2_bits(uint32_t a, uint32_t b, uint32_t c) {
-  uint32_t d;
-  asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-  return d;
-}
-__device__ __forceinline__ float half2_sum(uint32_t h) {
-  const __half2 v = *reinterpret_cast<const __half2*>(&h);
-  return __low2float(v) + __high2float(v);
-}
-// One 16-element block: w bytes (lo, hi words) against 16 staged fp16 activations.
-__device__ __forceinline__ float block_dot_fp4(uint32_t w_lo, uint32_t w_hi, const uint4& xa, const uint4& xb) {
-  uint32_t h[4];
-  uint32_t acc = 0;
-  e2m1x8_to_half2(w_lo, h);
-  acc = hfma2_bits(h[0], xa.x, acc);
-  acc = hfma2_bits(h[1], xa.y, acc);
-  acc = hfma2_bits(h[2], xa.z, acc);
-  acc = hfma2_bits(h[3], xa.w, acc);
-  e2m1x8_to_half2(w_hi, h);
-  acc = hfma2_bits(h[0], xb.x, acc);
-  acc = hfma2_bits(h[1], xb.y, acc);
-  acc = hfma2_bits(h[2], xb.z, acc);
-  acc = hfma2_bits(h[3], xb.w, acc);
-  return half2_sum(acc);
-}
-
-template <int kRows, bool kGateUp>
-__global__ void __launch_bounds__(kThreads)
-nvfp4_gemv_kernel(const uint8_t* __restrict__ act, const uint8_t* __restrict__ act_scales,
-                  const uint8_t* __restrict__ w0, const uint8_t* __restrict__ ws0,
-                  const uint8_t* __restrict__ w1, const uint8_t* __restrict__ ws1,
-                  float* __restrict__ out0, float* __restrict__ out1, float* __restrict__ product,
-                  uint64_t rows, uint64_t k, float div0, float div1) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  // Staged activation: per 1024-element segment (512 weight bytes), lane l's 32 values are
-  // stored as four 8-value parts at [p*256 + l*8, +8), p = 0..3 (conflict-free 128-bit loads).
-  const uint64_t k_pad = (k + 1023) / 1024 * 1024;
-  __half* xs = reinterpret_cast<__half*>(smem_raw);              // k_pad halves
-  float* sa = reinterpret_cast<float*>(smem_raw + k_pad * 2);    // k/16 decoded scales
-  for (uint64_t c = threadIdx.x; c < k / 32; c += kThreads) {
-    const uint4 v = __ldg(reinterpret_cast<const uint4*>(act) + c);  // 32 elements
-    const uint32_t ww[4] = {v.x, v.y, v.z, v.w};
-    uint32_t h[16];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      uint32_t t[4];
-      e2m1x8_to_half2(ww[i], t);
-      h[4 * i] = t[0]; h[4 * i + 1] = t[1]; h[4 * i + 2] = t[2]; h[4 * i + 3] = t[3];
-    }
-    __half* dst = xs + (c / 32) * 1024 + (c % 32) * 8;
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-      *reinterpret_cast<uint4*>(dst + i * 256) = make_uint4(h[4 * i], h[4 * i + 1], h[4 * i + 2], h[4 * i + 3]);
-  }
-  for (uint64_t c = threadIdx.x; c < k / 16; c += kThreads) sa[c] = e4m3_decode(__ldg(act_scales + c));
-  __syncthreads();
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint64_t row0 = (static_cast<uint64_t>(blockIdx.x) * kWarps + warp) * kRows;
-  if (row0 >= rows) return;
-  constexpr int kMats = kGateUp ? 2 : 1;
-  const uint64_t row_bytes = k / 2, srow_bytes = k / 16;
-  float acc[kMats][kRows];
-#pragma unroll
-  for (int m = 0; m < kMats; ++m)
-#pragma unroll
-    for (int r = 0; r < kRows; ++r) acc[m][r] = 0.0f;
-
-  // A lane owns 16 weight bytes = 32 elements = 2 blocks per 512-byte row segment.
-  for (uint64_t kb = lane * 16ull; kb < row_bytes; kb += 512) {
-    uint4 wv[kMats][kRows];
-    uint16_t sv[kMats][kRows];
-#pragma unroll
-    for (int m = 0; m < kMats; ++m)
-#pragma unroll
-      for (int r = 0; r < kRows; ++r) {
-        const uint64_t row = row0 + r < rows ? row0 + r : rows - 1;
-        const uint8_t* wp = (m == 0 ? w0 : w1) + row * row_bytes + kb;
-        const uint8_t* sp = (m == 0 ? ws0 : ws1) + row * srow_bytes + kb / 8;
-        wv[m][r] = ldg_stream(wp);
-        sv[m][r] = __ldg(reinterpret_cast<const uint16_t*>(sp));
-      }
-    const __half* xp = xs + (kb / 512) * 1024 + lane * 8;
-    const uint4 x0 = *reinterpret_cast<const uint4*>(xp), x1 = *reinterpret_cast<const uint4*>(xp + 256),
-                x2 = *reinterpret_cast<const uint4*>(xp + 512), x3 = *reinterpret_cast<const uint4*>(xp + 768);
-    const float sa0 = sa[kb / 8], sa1 = sa[kb / 8 + 1];
-#pragma unroll
-    for (int m = 0; m < kMats; ++m)
-#pragma unroll
-      for (int r = 0; r < kRows; ++r) {
-        const float d0 = block_dot_fp4(wv[m][r].x, wv[m][r].y, x0, x1);
-        const float d1 = block_dot_fp4(wv[m][r].z, wv[m][r].w, x2, x3);
-        const float sw0 = e4m3_decode(static_cast<uint8_t>(sv[m][r] & 0xFF));
-        const float sw1 = e4m3_decode(static_cast<uint8_t>(sv[m][r] >> 8));
-        acc[m][r] = fmaf(d0, sa0 * sw0, acc[m][r]);
-        acc[m][r] = fmaf(d1, sa1 * sw1, acc[m][r]);
-      }
-  }
-#pragma unroll
-  for (int m = 0; m < kMats; ++m)
-#pragma unroll
-    for (int r = 0; r < kRows; ++r) acc[m][r] = warp_sum(acc[m][r]);
-  if (lane == 0) {
-#pragma unroll
-    for (int r = 0; r < kRows; ++r) {
-      if (row0 + r >= rows) continue;
-      // Single final division by ga*gw: src/cuda/nvfp4/sm120.cu:243.
-      const float y0 = __fdiv_rn(acc[0][r], div0);
-      if constexpr (kGateUp) {
-        const float y1 = __fdiv_rn(acc[1][r], div1);
-        if (out0) out0[row0 + r] = y0;
-        if (out1) out1[row0 + r] = y1;
-        // bf16 boundaries and GELU-tanh product: src/cuda/nvfp4/sm120.cu:375-386.
-        const float g = bf16_round(y0), u = bf16_round(y1);
-        product[row0 + r] = gelu_tanh_product(g, u);
-      } else {
-        out0[row0 + r] = y0;
-      }
-    }
-  }
-}
-
-// Small-batch NVFP4 GEMV (2..8 tokens, the verifier's MLP projections): the weight chunk is
-// converted to fp16 once and meets kTok staged activations; per token the arithmetic and its
-// order are those of the single-token kernel, so each token's result is bit-identical to it.
-template <int kTok>
-__global__ void __launch_bounds__(kThreads)
-nvfp4_gemv_batch_kernel(const uint8_t* __restrict__ act, const uint8_t* __restrict__ act_scales,
-                        const uint8_t* __restrict__ w, const uint8_t* __restrict__ ws, float* __restrict__ out,
-                        uint64_t rows, uint64_t k, float div) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const uint64_t k_pad = (k + 1023) / 1024 * 1024;
-  const uint64_t tok_bytes = k_pad * 2 + (k / 16) * 4;   // staged fp16 values, then fp32 block scales
-  for (int t = 0; t < kTok; ++t) {
-    __half* xs = reinterpret_cast<__half*>(smem_raw + t * tok_bytes);
-    float* sa = reinterpret_cast<float*>(smem_raw + t * tok_bytes + k_pad * 2);
-    const uint8_t* a = act + static_cast<uint64_t>(t) * (k / 2);
-    for (uint64_t c = threadIdx.x; c < k / 32; c += kThreads) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4*>(a) + c);  // 32 elements
-      const uint32_t ww[4] = {v.x, v.y, v.z, v.w};
-      __half* dst = xs + (c / 32) * 1024 + (c % 32) * 8;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        uint32_t h[4];
-        e2m1x8_to_half2(ww[i], h);
-        *reinterpret_cast<uint4*>(dst + i * 256) = make_uint4(h[0], h[1], h[2], h[3]);
-      }
-    }
-    for (uint64_t c = threadIdx.x; c < k / 16; c += kThreads)
-      sa[c] = e4m3_decode(__ldg(act_scales + static_cast<uint64_t>(t) * (k / 16) + c));
-  }
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint64_t row = static_cast<uint64_t>(blockIdx.x) * kWarps + warp;
-  if (row >= rows) return;
-  const uint64_t row_bytes = k / 2, srow_bytes = k / 16;
-  float acc[kTok];
-#pragma unroll
-  for (int t = 0; t < kTok; ++t) acc[t] = 0.0f;
-  for (uint64_t kb = lane * 16ull; kb < row_bytes; kb += 512) {
-    const uint4 wv = ldg_stream(w + row * row_bytes + kb);
-    const uint16_t sv = __ldg(reinterpret_cast<const uint16_t*>(ws + row * srow_bytes + kb / 8));
-    const float sw0 = e4m3_decode(static_cast<uint8_t>(sv & 0xFF)), sw1 = e4m3_decode(static_cast<uint8_t>(sv >> 8));
-#pragma unroll
-    for (int t = 0; t < kTok; ++t) {
-      const __half* xp = reinterpret_cast<const __half*>(smem_raw + t * tok_bytes) + (kb / 512) * 1024 + lane * 8;
-      const float* sa = reinterpret_cast<const float*>(smem_raw + t * tok_bytes + k_pad * 2);
-      const uint4 x0 = *reinterpret_cast<const uint4*>(xp), x1 = *reinterpret_cast<const uint4*>(xp + 256),
-                  x2 = *reinterpret_cast<const uint4*>(xp + 512), x3 = *reinterpret_cast<const uint4*>(xp + 768);
-      const float d0 = block_dot_fp4(wv.x, wv.y, x0, x1);
-      const float d1 = block_dot_fp4(wv.z, wv.w, x2, x3);
-      acc[t] = fmaf(d0, sa[kb / 8] * sw0, acc[t]);
-      acc[t] = fmaf(d1, sa[kb / 8 + 1] * sw1, acc[t]);
-    }
-  }
-#pragma unroll
-  for (int t = 0; t < kTok; ++t) acc[t] = warp_sum(acc[t]);
-  if (lane == 0) {
-#pragma unroll
-    for (int t = 0; t < kTok; ++t) out[static_cast<uint64_t>(t) * rows + row] = __fdiv_rn(acc[t], div);
-  }
-}
-
-template <int kTok>
-int32_t launch_nvfp4_gemv_batch_variant(const char* op, const uint8_t* act, const uint8_t* act_scales, const uint8_t* w,
-                                        const uint8_t* ws, float* out, uint64_t rows, uint64_t k, float div,
-                                        cudaStream_t stream) {
-  auto kern = nvfp4_gemv_batch_kernel<kTok>;
-  const size_t smem = static_cast<size_t>(kTok) * ((k + 1023) / 1024 * 1024 * 2 + (k / 16) * 4);
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e != cudaSuccess) return fail(GEMB_INTERNAL, "%s: %s: %s", op, cudaGetErrorName(e), cudaGetErrorString(e));
-  }
-  const unsigned blocks = static_cast<unsigned>((rows + kWarps - 1) / kWarps);
-  kern<<<blocks, kThreads, smem, stream>>>(act, act_scales, w, ws, out, rows, k, div);
-  return check_launch(op);
-}
-
-template <bool kGateUp>
-int32_t launch_nvfp4_gemv(const char* op, const uint8_t* act, const uint8_t* act_scales,
-                          const uint8_t* w0, const uint8_t* ws0, const uint8_t* w1,
-                          const uint8_t* ws1, float* out0, float* out1, float* product,
-                          uint64_t rows, uint64_t k, float div0, float div1, cudaStream_t stream) {
-  const int rpw = kGateUp ? (rows / (kWarps * 2) >= 2ull * sm_count() ? 2 : 1)
-                          : (rows / (kWarps * 4) >= 2ull * sm_count() ? 4 : rows / (kWarps * 2) >= 2ull * sm_count() ? 2 : 1);
-  const unsigned blocks = static_cast<unsigned>((rows + kWarps * rpw - 1) / (kWarps * rpw));
-  const size_t smem = (k + 1023) / 1024 * 1024 * 2 + (k / 16) * 4;
-#define GEMB_LAUNCH_FP4_GEMV(R)                                                                   \
-  do {                                                                                            \
-    auto kern = nvfp4_gemv_kernel<R, kGateUp>;                                                    \
-    if (smem > 48 * 1024) {                                                                       \
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,     \
-                                           static_cast<int>(smem));                               \
-      if (e != cudaSuccess)                                                                       \
-        return fail(GEMB_INTERNAL, "%s: %s: %s", op, cudaGetErrorName(e), cudaGetErrorString(e)); \
-    }                                                                                             \
-    kern<<<blocks, kThreads, smem, stream>>>(act, act_scales, w0, ws0, w1, ws1, out0, out1,       \
-                                             product, rows, k, div0, div1);             \
-  } while (0)
-  if (rpw == 4) { if constexpr (!kGateUp) GEMB_LAUNCH_FP4_GEMV(4); }
-  else if (rpw == 2) GEMB_LAUNCH_FP4_GEMV(2);
-  else GEMB_LAUNCH_FP4_GEMV(1);
-#undef GEMB_LAUNCH_FP4_GEMV
-  return check_launch(op);
-}
-
-int32_t validate_nvfp4_gemv(const char* op, uint64_t rows, uint64_t k, float ga, float gw) {
-  GEMB_REQUIRE(rows > 0 && k > 0, "%s: geometry must be nonzero", op);
-  GEMB_REQUIRE(k % 64 == 0 && rows % 8 == 0,
-               "%s: requires K divisible by 64 and rows divisible by 8", op);
-  GEMB_REQUIRE(k <= 96 * 1024, "%s: contracting extent exceeds the shared-memory staging limit (98304)", op);
-  GEMB_REQUIRE(rows < (1ull << 31), "%s: too many rows", op);
-  GEMB_REQUIRE(positive_finite(ga) && positive_finite(gw), "%s: global divisors must be positive and finite", op);
-  GEMB_REQUIRE(std::isfinite(ga * gw), "%s: combined global divisor overflowed", op);
-  return GEMB_OK;
-}
-
-// ---------------------------------------------------------------------------------------------
 // Decode-time FP8 token quantizer: one 1024-thread CTA per token, the token held in registers
 // between the amax pass and the conversion (one global round trip), quotients through
 // e4m3_of_quotients (bit-identical to the IEEE division of src/numeric/fp8.cpp:41-58).  It
@@ -1355,83 +1100,6 @@ int32_t gemb_fp8_gemv_bf16in(const uint16_t* act_bf16, const uint8_t* w, const u
   grp.p[0] = {w, w_scales, out, rows};
   if (out_dtype == GEMB_BF16) return launch_fp8_gemv<true, true>(op, act_bf16, nullptr, grp, k, stream);
   return launch_fp8_gemv<true, false>(op, act_bf16, nullptr, grp, k, stream);
-}
-
-int32_t gemb_nvfp4_gemv(const uint8_t* act, const uint8_t* act_scales, const uint8_t* w,
-                        const uint8_t* w_scales, float* out, uint64_t rows, uint64_t k, float ga,
-                        float gw, gemb_stream_t stream) {
-  const char* op = "gemb_nvfp4_gemv";
-  GEMB_REQUIRE(act && act_scales && w && w_scales && out, "%s: pointers must be nonnull", op);
-  GEMB_TRY(validate_nvfp4_gemv(op, rows, k, ga, gw));
-  GEMB_REQUIRE(reinterpret_cast<uintptr_t>(act) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0 &&
-                   reinterpret_cast<uintptr_t>(w_scales) % 2 == 0,
-               "%s: activation and weight must be 16-byte aligned, weight scales 2-byte aligned", op);
-  GEMB_ENTER(op);
-  return launch_nvfp4_gemv<false>(op, act, act_scales, w, w_scales, nullptr, nullptr, out, nullptr,
-                                  nullptr, rows, k, ga * gw, 1.0f, stream);
-}
-
-int32_t gemb_nvfp4_gemv_batch(const uint8_t* act, const uint8_t* act_scales, const uint8_t* w, const uint8_t* w_scales,
-                              float* out, uint64_t tokens, uint64_t rows, uint64_t k, float ga, float gw,
-                              gemb_stream_t stream) {
-  const char* op = "gemb_nvfp4_gemv_batch";
-  GEMB_REQUIRE(act && act_scales && w && w_scales && out, "%s: pointers must be nonnull", op);
-  GEMB_TRY(validate_nvfp4_gemv(op, rows, k, ga, gw));
-  GEMB_REQUIRE(tokens >= 1 && tokens <= 8, "%s: between 1 and 8 tokens (larger batches go through gemb_nvfp4_gemm_bf16)", op);
-  GEMB_REQUIRE(tokens * ((k + 1023) / 1024 * 1024 * 2 + (k / 16) * 4) <= 200 * 1024,
-               "%s: tokens * K exceeds the shared-memory staging limit", op);
-  GEMB_REQUIRE(reinterpret_cast<uintptr_t>(act) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0 &&
-                   reinterpret_cast<uintptr_t>(w_scales) % 2 == 0,
-               "%s: activation and weight must be 16-byte aligned, weight scales 2-byte aligned", op);
-  GEMB_ENTER(op);
-  const float div = ga * gw;
-  switch (tokens) {
-    case 1: return launch_nvfp4_gemv<false>(op, act, act_scales, w, w_scales, nullptr, nullptr, out, nullptr, nullptr, rows,
-                                            k, div, 1.0f, stream);
-    case 2: return launch_nvfp4_gemv_batch_variant<2>(op, act, act_scales, w, w_scales, out, rows, k, div, stream);
-    case 3: return launch_nvfp4_gemv_batch_variant<3>(op, act, act_scales, w, w_scales, out, rows, k, div, stream);
-    case 4: return launch_nvfp4_gemv_batch_variant<4>(op, act, act_scales, w, w_scales, out, rows, k, div, stream);
-    case 5: return launch_nvfp4_gemv_batch_variant<5>(op, act, act_scales, w, w_scales, out, rows, k, div, stream);
-    case 6: return launch_nvfp4_gemv_batch_variant<6>(op, act, act_scales, w, w_scales, out, rows, k, div, stream);
-    case 7: return launch_nvfp4_gemv_batch_variant<7>(op, act, act_scales, w, w_scales, out, rows, k, div, stream);
-    default: return launch_nvfp4_gemv_batch_variant<8>(op, act, act_scales, w, w_scales, out, rows, k, div, stream);
-  }
-}
-
-int32_t gemb_nvfp4_gemv_gate_up(const uint8_t* act, const uint8_t* act_scales, const uint8_t* gate_w,
-                                const uint8_t* gate_s, const uint8_t* up_w, const uint8_t* up_s,
-                                float* gate_out, float* up_out, float* product, uint64_t rows,
-                                uint64_t k, float gate_ga, float gate_gw, float up_ga, float up_gw,
-                                gemb_stream_t stream) {
-  const char* op = "gemb_nvfp4_gemv_gate_up";
-  GEMB_REQUIRE(act && act_scales && gate_w && gate_s && up_w && up_s && product,
-               "%s: required pointers must be nonnull", op);
-  GEMB_REQUIRE((gate_out == nullptr) == (up_out == nullptr),
-               "%s: gate and up outputs must both be present or both null", op);
-  GEMB_TRY(validate_nvfp4_gemv(op, rows, k, gate_ga, gate_gw));
-  GEMB_TRY(validate_nvfp4_gemv(op, rows, k, up_ga, up_gw));
-  GEMB_REQUIRE(reinterpret_cast<uintptr_t>(act) % 16 == 0 && reinterpret_cast<uintptr_t>(gate_w) % 16 == 0 &&
-                   reinterpret_cast<uintptr_t>(up_w) % 16 == 0 && reinterpret_cast<uintptr_t>(gate_s) % 2 == 0 &&
-                   reinterpret_cast<uintptr_t>(up_s) % 2 == 0,
-               "%s: activation and weights must be 16-byte aligned, weight scales 2-byte aligned", op);
-  GEMB_ENTER(op);
-  return launch_nvfp4_gemv<true>(op, act, act_scales, gate_w, gate_s, up_w, up_s, gate_out, up_out,
-                                 product, rows, k, gate_ga * gate_gw, up_ga * up_gw, stream);
-}
-
-int32_t gemb_nvfp4_gemv_gate_up_batch(const uint8_t* act, const uint8_t* act_scales, const uint8_t* gate_w,
-                                      const uint8_t* gate_s, const uint8_t* up_w, const uint8_t* up_s, float* gate_out,
-                                      float* up_out, float* product, uint64_t tokens, uint64_t rows, uint64_t k,
-                                      float gate_ga, float gate_gw, float up_ga, float up_gw, gemb_stream_t stream) {
-  const char* op = "gemb_nvfp4_gemv_gate_up_batch";
-  GEMB_REQUIRE(tokens >= 1 && tokens <= 65535, "%s: between 1 and 65,535 tokens", op);
-  // One fused gate/up launch per token (the verifier's batches are a handful of tokens): every
-  // token's result is bit-identical to the single-token operator.
-  for (uint64_t t = 0; t < tokens; ++t)
-    GEMB_TRY(gemb_nvfp4_gemv_gate_up(act + t * (k / 2), act_scales + t * (k / 16), gate_w, gate_s, up_w, up_s,
-                                     gate_out ? gate_out + t * rows : nullptr, up_out ? up_out + t * rows : nullptr,
-                                     product + t * rows, rows, k, gate_ga, gate_gw, up_ga, up_gw, stream));
-  return GEMB_OK;
 }
 
 }  // extern "C"

@@ -1,0 +1,406 @@
+// Decode projections with NVFP4 weights (W4A4) for 1 .. 8 tokens: y = (sum_k qa sa qw sw) / (ga * gw), and the fused
+// gate / up form with the GELU-tanh product.  Weights in the checkpoint's row-major layout with COMPACT
+// block scales; every weight byte is read once whatever the token count.
+//
+// The dot products run on the warp-level tensor-core path (mma.sync m16n8k16, fp16 x fp16 -> fp32): the weights
+// are the M side as they lie in memory, the tokens its eight columns, so the arithmetic is the same for
+// one token and for eight.  E2M1 values times E4M3 scales have six significant bits and lie in
+// [2^-10, 2688]: they are exact in fp16, for weights and activations alike, and their products are exact in
+// fp32.  A chain of four MMAs (64 products) starts from zero and is added to the running sum with an IEEE
+// addition, so that the tensor core's own accumulation stays short.  A token's result depends on its own
+// column only: it is bit-identical for every batch size.  (E4M3 operands would spare the scaling of the weights,
+// but mma.sync with 8-bit floats measured twice as slow here.)
+//
+// A tile is 16 matrix rows -- sixteen weight rows, or eight gate rows over the same eight up rows -- cut into
+// 128-byte pieces along K.  The tiles are dealt out over the SMs and the pieces of an SM's tiles over its warps in
+// equal contiguous shares: the kernel is as much bound by the conversions as by the loads, so warps without
+// work cost as much as SMs without loads.  Measured, weights cold, in a chain of launches: gate / up 2 x 15,360 x 3,840 in
+// 18 us for one token and 20 us for five (23 us per token before, one launch each), down 3,840 x 15,360 in 12 and
+// 14 us (11 and 67 us before); without the loads the arithmetic takes 12 us, without the arithmetic
+// the loads 8.  Requesting all weights into L2 ahead of pdl_wait changed nothing: the kernels before
+// this one then wait for HBM instead.  Lane 4g + t loads 32 contiguous bytes of rows g and g + 8 per piece
+// (four scale blocks each) and the four scale bytes that go with them; MMA j takes bytes 2j, 2j + 1 of that run as
+// a0 / a2 (row g) and a1 / a3 (row g + 8).  That permutes k inside the piece, which is harmless because the
+// activations are staged in the same order: 16 bytes (eight fp16 values) per lane and MMA pair,
+// [piece][j / 2][token][t], conflict-free.
+#include <algorithm>
+
+#include "common.cuh"
+
+namespace gemb {
+namespace {
+
+constexpr uint32_t kFpWarps = 16, kFpThreads = kFpWarps * 32;
+constexpr uint32_t kPieceElems = 256;   // 128 bytes of a row
+
+__device__ __forceinline__ void e2m1x8_to_half2(uint32_t word, uint32_t (&h)[4]) {
+  asm("{ .reg .b8 t0, t1, t2, t3;\n"
+      "  mov.b32 {t0, t1, t2, t3}, %4;\n"
+      "  cvt.rn.f16x2.e2m1x2 %0, t0;\n"
+      "  cvt.rn.f16x2.e2m1x2 %1, t1;\n"
+      "  cvt.rn.f16x2.e2m1x2 %2, t2;\n"
+      "  cvt.rn.f16x2.e2m1x2 %3, t3; }"
+      : "=r"(h[0]), "=r"(h[1]), "=r"(h[2]), "=r"(h[3])
+      : "r"(word));
+}
+__device__ __forceinline__ uint32_t mul_half2(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
+// Two E4M3 scale bytes -> each as a pair of equal fp16 values.
+__device__ __forceinline__ void scale_pairs(uint32_t two_bytes, uint32_t& first, uint32_t& second) {
+  uint32_t h;
+  asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h) : "h"(static_cast<uint16_t>(two_bytes)));
+  first = __byte_perm(h, h, 0x1010);
+  second = __byte_perm(h, h, 0x3232);
+}
+// c = A B (first of a chain) and c += A B.
+__device__ __forceinline__ void mma_first(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.0f));
+}
+__device__ __forceinline__ void mma_next(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+struct Fp4Matrix {
+  const uint8_t* w;
+  const uint8_t* ws;
+  float* out;      // [tokens, rows], may be null in the gate / up form
+  float div;
+};
+struct Fp4GemvArgs {
+  const uint8_t* act;
+  const uint8_t* act_scales;
+  Fp4Matrix m[2];
+  float* product;  // gate / up form
+  uint32_t rows, k, tokens;
+  bool wide;       // weights 32-byte and scales 4-byte aligned
+};
+
+// One row's share of a piece: 32 weight bytes and four scale bytes.  Left as it is when `in` is false: the
+// activations past K are zero and pieces past the warp's share are not used.
+struct Run {
+  uint32_t w[8];
+  uint32_t s;
+};
+__device__ __forceinline__ void load_run(Run& r, const uint8_t* w, const uint8_t* s, bool in, bool wide) {
+  if (wide) {
+    asm volatile("{ .reg .pred p; setp.ne.b32 p, %11, 0;\n"
+                 "@p ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%9];\n"
+                 "@p ld.global.nc.b32 %8, [%10]; }"
+                 : "+r"(r.w[0]), "+r"(r.w[1]), "+r"(r.w[2]), "+r"(r.w[3]), "+r"(r.w[4]), "+r"(r.w[5]), "+r"(r.w[6]), "+r"(r.w[7]), "+r"(r.s)
+                 : "l"(w), "l"(s), "r"(static_cast<uint32_t>(in)));
+  } else if (in) {
+    asm volatile("ld.global.nc.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r.w[0]), "=r"(r.w[1]), "=r"(r.w[2]), "=r"(r.w[3]) : "l"(w));
+    asm volatile("ld.global.nc.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r.w[4]), "=r"(r.w[5]), "=r"(r.w[6]), "=r"(r.w[7]) : "l"(w + 16));
+    uint16_t lo, hi;
+    asm volatile("ld.global.nc.b16 %0, [%1];" : "=h"(lo) : "l"(s));
+    asm volatile("ld.global.nc.b16 %0, [%1];" : "=h"(hi) : "l"(s + 2));
+    r.s = lo | (static_cast<uint32_t>(hi) << 16);
+  }
+}
+
+// Stages the tokens' dequantised activations (fp16, exact) in MMA order; cells past K are zero.
+__device__ __forceinline__ void stage_fp4_activations(const Fp4GemvArgs& a, uint4* xs) {
+  const uint32_t halves = (a.k + kPieceElems - 1) / kPieceElems * 8;   // halves of the 64-element runs (piece, t) per token
+  for (uint32_t idx = threadIdx.x; idx < halves * a.tokens; idx += kFpThreads) {
+    const uint32_t token = idx / halves, half = idx - token * halves, piece = half / 8, t = (half / 2) & 3, q0 = (half & 1) * 4;
+    uint32_t h[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) h[i] = 0;
+    if (half * 32 < a.k) {
+      const uint4 v = ld_dep(reinterpret_cast<const uint4*>(a.act + static_cast<uint64_t>(token) * (a.k / 2)) + half);
+      const uint8_t* sp = a.act_scales + static_cast<uint64_t>(token) * (a.k / 16) + half * 2;
+      uint32_t s[2];
+      scale_pairs(ld_dep(sp) | (static_cast<uint32_t>(ld_dep(sp + 1)) << 8), s[0], s[1]);
+      const uint32_t words[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        uint32_t d[4];
+        e2m1x8_to_half2(words[i], d);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) h[4 * i + j] = mul_half2(d[j], s[i >> 1]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      xs[((piece * 8 + q0 + i) * a.tokens + token) * 4 + t] = make_uint4(h[4 * i], h[4 * i + 1], h[4 * i + 2], h[4 * i + 3]);
+  }
+}
+
+// acc += rows g and g + 8 of one piece against the staged tokens: `xp` advances by `step` bytes per MMA pair
+// (lanes of token columns past the batch stay on a zero cell).
+__device__ __forceinline__ void dot_piece(float (&acc)[4], const Run& ra, const Run& rb, const uint8_t* xp, uint32_t step) {
+#pragma unroll
+  for (int two = 0; two < 2; ++two) {
+    uint32_t sa[2], sb[2];
+    scale_pairs(ra.s >> (16 * two), sa[0], sa[1]);
+    scale_pairs(rb.s >> (16 * two), sb[0], sb[1]);
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      float c[4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int q = two * 4 + b * 2 + i;
+        const uint4 xv = *reinterpret_cast<const uint4*>(xp + q * step);
+        uint32_t ha[4], hb[4];
+        e2m1x8_to_half2(ra.w[q], ha);
+        e2m1x8_to_half2(rb.w[q], hb);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          ha[j] = mul_half2(ha[j], sa[b]);
+          hb[j] = mul_half2(hb[j], sb[b]);
+        }
+        if (i == 0) mma_first(c, ha[0], hb[0], ha[1], hb[1], xv.x, xv.y);
+        else mma_next(c, ha[0], hb[0], ha[1], hb[1], xv.x, xv.y);
+        mma_next(c, ha[2], hb[2], ha[3], hb[3], xv.z, xv.w);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[j] = __fadd_rn(acc[j], c[j]);
+    }
+  }
+}
+
+template <bool kGateUp>
+__global__ void __launch_bounds__(kFpThreads, 1)
+nvfp4_gemv_kernel(const __grid_constant__ Fp4GemvArgs a) {
+  constexpr int kAhead = 2;                          // pieces in flight per warp
+  constexpr uint32_t kTileRows = kGateUp ? 8 : 16;
+  extern __shared__ __align__(128) uint8_t smem[];
+  // zero cell (128 bytes), staged activations, partial sums [warp][continuation / start of a tile][lane]
+  uint4* xs = reinterpret_cast<uint4*>(smem + 128);
+  const uint32_t pieces = (a.k + kPieceElems - 1) / kPieceElems;
+  float4* partial = reinterpret_cast<float4*>(smem + 128 + static_cast<size_t>(pieces) * a.tokens * kPieceElems * 2);
+  const uint32_t warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const uint32_t tiles = (a.rows + kTileRows - 1) / kTileRows;
+  const uint32_t row_bytes = a.k / 2, srow_bytes = a.k / 16;
+  // The CTA owns the tiles blockIdx.x, + gridDim.x, ...; their pieces form one list, of which every warp takes
+  // an equal, contiguous share.
+  const uint64_t list = static_cast<uint64_t>((tiles - blockIdx.x + gridDim.x - 1) / gridDim.x) * pieces;
+  auto share = [&](uint32_t w) { return list * w / kFpWarps; };
+  const uint64_t lo = share(warp), hi = share(warp + 1);
+  pdl_trigger();
+  pdl_wait();
+  // Load cursor: piece `next` of the list = piece `np` of the tile whose rows the pointers stand on.
+  uint64_t next = lo;
+  uint32_t ntile = static_cast<uint32_t>(lo / pieces), np = static_cast<uint32_t>(lo % pieces);
+  const uint8_t* pw[2];
+  const uint8_t* ps[2];
+  auto aim = [&]() {
+    const uint32_t row0 = (blockIdx.x + gridDim.x * ntile) * kTileRows;
+    // rows are a multiple of 8: the second half of a 16-row tile may lie past the end; it then repeats the first
+    const uint64_t ra = min(row0 + g, a.rows - 1), rb = !kGateUp && row0 + 8 < a.rows ? ra + 8 : ra;
+    pw[0] = a.m[0].w + ra * row_bytes + t * 32;
+    pw[1] = a.m[kGateUp ? 1 : 0].w + rb * row_bytes + t * 32;
+    ps[0] = a.m[0].ws + ra * srow_bytes + t * 4;
+    ps[1] = a.m[kGateUp ? 1 : 0].ws + rb * srow_bytes + t * 4;
+  };
+  Run wa[kAhead], wb[kAhead];
+  auto load = [&](int u) {
+    const bool in = next < hi && np * 128 + t * 32 < row_bytes;
+    load_run(wa[u], pw[0] + np * 128, ps[0] + np * 16, in, a.wide);
+    load_run(wb[u], pw[1] + np * 128, ps[1] + np * 16, in, a.wide);
+    ++next;
+    if (++np == pieces) {
+      np = 0;
+      ++ntile;
+      aim();
+    }
+  };
+  aim();
+#pragma unroll
+  for (int u = 0; u < kAhead; ++u) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) wa[u].w[i] = wb[u].w[i] = 0;
+    wa[u].s = wb[u].s = 0;
+    load(u);
+  }
+  // under the first weight loads
+  if (threadIdx.x < 8) reinterpret_cast<uint4*>(smem)[threadIdx.x] = make_uint4(0, 0, 0, 0);
+  stage_fp4_activations(a, xs);
+  __syncthreads();
+
+  float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  // acc[0], acc[1]: row g, tokens 2t, 2t + 1; acc[2], acc[3]: row g + 8 (gate / up: the up projection of row g)
+  auto emit = [&](uint32_t local_tile) {
+    const uint32_t row = (blockIdx.x + gridDim.x * local_tile) * kTileRows + g;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const uint32_t token = 2 * t + j;
+      if (token >= a.tokens) continue;
+      const uint64_t o = static_cast<uint64_t>(token) * a.rows + row;
+      const float y0 = __fdiv_rn(acc[j], a.m[0].div);   // single final division by ga*gw: src/cuda/nvfp4/sm120.cu:243
+      const float y1 = __fdiv_rn(acc[2 + j], a.m[kGateUp ? 1 : 0].div);
+      if constexpr (kGateUp) {
+        if (a.m[0].out) a.m[0].out[o] = y0;
+        if (a.m[1].out) a.m[1].out[o] = y1;
+        // bf16 boundaries and GELU-tanh product: src/cuda/nvfp4/sm120.cu:375-386.
+        a.product[o] = gelu_tanh_product(bf16_round(y0), bf16_round(y1));
+      } else {
+        a.m[0].out[o] = y0;
+        if (row + 8 < a.rows) a.m[0].out[o + 8] = y1;
+      }
+    }
+  };
+  const bool token_live = static_cast<uint32_t>(g) < a.tokens;
+  const uint32_t step = token_live ? a.tokens * 64 : 0;
+  const uint8_t* const xl = token_live ? reinterpret_cast<const uint8_t*>(xs + g * 4 + t) : smem + (lane & 7) * 16;
+  uint32_t tile = static_cast<uint32_t>(lo / pieces), cp = static_cast<uint32_t>(lo % pieces);
+  const uint8_t* xp = xl + static_cast<size_t>(cp) * 8 * step;
+  bool from_start = cp == 0;
+  for (uint64_t c = lo; c < hi;) {
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      if (c >= hi) break;   // warp-uniform, as everything about the list
+      dot_piece(acc, wa[u], wb[u], xp, step);
+      load(u);
+      xp += 8 * step;
+      ++c;
+      if (++cp == pieces || c == hi) {
+        if (from_start && cp == pieces) emit(tile);
+        else partial[(warp * 2 + (from_start ? 1 : 0)) * 32 + lane] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        from_start = true;
+        cp = 0;
+        ++tile;
+        xp = xl;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[j] = 0.0f;
+      }
+    }
+  }
+  __syncthreads();
+  // A tile shared by several warps is finished by the one that holds its first piece, the others' sums added in
+  // warp order: the same bits on every launch.
+  const uint64_t last_start = hi > lo ? (hi - 1) / pieces * pieces : 0;
+  if (hi <= lo || last_start < lo || hi == last_start + pieces) return;
+  float4 v = partial[(warp * 2 + 1) * 32 + lane];
+  acc[0] = v.x, acc[1] = v.y, acc[2] = v.z, acc[3] = v.w;
+  for (uint32_t w = warp + 1; w < kFpWarps && share(w) < last_start + pieces; ++w) {
+    if (share(w + 1) == share(w)) continue;
+    v = partial[w * 2 * 32 + lane];
+    acc[0] = __fadd_rn(acc[0], v.x);
+    acc[1] = __fadd_rn(acc[1], v.y);
+    acc[2] = __fadd_rn(acc[2], v.z);
+    acc[3] = __fadd_rn(acc[3], v.w);
+  }
+  emit(static_cast<uint32_t>(last_start / pieces));
+}
+
+uint64_t fp4_stage_bytes(uint64_t tokens, uint64_t k) { return tokens * ((k + kPieceElems - 1) / kPieceElems * kPieceElems) * 2; }
+
+template <bool kGateUp>
+int32_t launch_nvfp4_gemv(const char* op, Fp4GemvArgs a, cudaStream_t stream) {
+  a.wide = true;
+  for (int m = 0; m < (kGateUp ? 2 : 1); ++m)
+    a.wide = a.wide && reinterpret_cast<uintptr_t>(a.m[m].w) % 32 == 0 && reinterpret_cast<uintptr_t>(a.m[m].ws) % 4 == 0;
+  const size_t smem = 128 + fp4_stage_bytes(a.tokens, a.k) + kFpWarps * 2 * 32 * sizeof(float4);
+  auto kern = nvfp4_gemv_kernel<kGateUp>;
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return fail(GEMB_INTERNAL, "%s: %s: %s", op, cudaGetErrorName(e), cudaGetErrorString(e));
+  }
+  // One CTA per SM (registers allow no second one), tiles dealt out round robin.
+  const uint32_t tile_rows = kGateUp ? 8 : 16, tiles = (a.rows + tile_rows - 1) / tile_rows;
+  GEMB_TRY(launch_pdl(op, kern, dim3(std::min(tiles, static_cast<uint32_t>(sm_count()))), dim3(kFpThreads), smem, stream, a));
+  return check_launch(op);
+}
+
+int32_t validate_nvfp4_gemv(const char* op, uint64_t rows, uint64_t k, float ga, float gw) {
+  GEMB_REQUIRE(rows > 0 && k > 0, "%s: geometry must be nonzero", op);
+  GEMB_REQUIRE(k % 64 == 0 && rows % 8 == 0,
+               "%s: requires K divisible by 64 and rows divisible by 8", op);
+  GEMB_REQUIRE(k <= 96 * 1024, "%s: contracting extent exceeds the shared-memory staging limit (98304)", op);
+  GEMB_REQUIRE(rows < (1ull << 31), "%s: too many rows", op);
+  GEMB_REQUIRE(positive_finite(ga) && positive_finite(gw), "%s: global divisors must be positive and finite", op);
+  GEMB_REQUIRE(std::isfinite(ga * gw), "%s: combined global divisor overflowed", op);
+  return GEMB_OK;
+}
+
+}  // namespace
+}  // namespace gemb
+
+using namespace gemb;
+
+extern "C" {
+
+int32_t gemb_nvfp4_gemv_batch(const uint8_t* act, const uint8_t* act_scales, const uint8_t* w, const uint8_t* w_scales,
+                              float* out, uint64_t tokens, uint64_t rows, uint64_t k, float ga, float gw,
+                              gemb_stream_t stream) {
+  const char* op = "gemb_nvfp4_gemv_batch";
+  GEMB_REQUIRE(act && act_scales && w && w_scales && out, "%s: pointers must be nonnull", op);
+  GEMB_TRY(validate_nvfp4_gemv(op, rows, k, ga, gw));
+  GEMB_REQUIRE(tokens >= 1 && tokens <= 8, "%s: between 1 and 8 tokens (larger batches go through gemb_nvfp4_gemm_bf16)", op);
+  GEMB_REQUIRE(tokens == 1 || tokens * ((k + 1023) / 1024 * 1024 * 2 + (k / 16) * 4) <= 200 * 1024,
+               "%s: tokens * K exceeds the shared-memory staging limit", op);
+  GEMB_REQUIRE(reinterpret_cast<uintptr_t>(act) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0 &&
+                   reinterpret_cast<uintptr_t>(w_scales) % 2 == 0,
+               "%s: activation and weight must be 16-byte aligned, weight scales 2-byte aligned", op);
+  GEMB_ENTER(op);
+  Fp4GemvArgs a{};
+  a.act = act;
+  a.act_scales = act_scales;
+  a.m[0] = {w, w_scales, out, ga * gw};
+  a.rows = static_cast<uint32_t>(rows);
+  a.k = static_cast<uint32_t>(k);
+  a.tokens = static_cast<uint32_t>(tokens);
+  return launch_nvfp4_gemv<false>(op, a, stream);
+}
+
+int32_t gemb_nvfp4_gemv(const uint8_t* act, const uint8_t* act_scales, const uint8_t* w,
+                        const uint8_t* w_scales, float* out, uint64_t rows, uint64_t k, float ga,
+                        float gw, gemb_stream_t stream) {
+  return gemb_nvfp4_gemv_batch(act, act_scales, w, w_scales, out, 1, rows, k, ga, gw, stream);
+}
+
+int32_t gemb_nvfp4_gemv_gate_up_batch(const uint8_t* act, const uint8_t* act_scales, const uint8_t* gate_w,
+                                      const uint8_t* gate_s, const uint8_t* up_w, const uint8_t* up_s, float* gate_out,
+                                      float* up_out, float* product, uint64_t tokens, uint64_t rows, uint64_t k,
+                                      float gate_ga, float gate_gw, float up_ga, float up_gw, gemb_stream_t stream) {
+  const char* op = "gemb_nvfp4_gemv_gate_up_batch";
+  GEMB_REQUIRE(tokens >= 1 && tokens <= 65535, "%s: between 1 and 65,535 tokens", op);
+  GEMB_REQUIRE(act && act_scales && gate_w && gate_s && up_w && up_s && product,
+               "%s: required pointers must be nonnull", op);
+  GEMB_REQUIRE((gate_out == nullptr) == (up_out == nullptr),
+               "%s: gate and up outputs must both be present or both null", op);
+  GEMB_TRY(validate_nvfp4_gemv(op, rows, k, gate_ga, gate_gw));
+  GEMB_TRY(validate_nvfp4_gemv(op, rows, k, up_ga, up_gw));
+  GEMB_REQUIRE(reinterpret_cast<uintptr_t>(act) % 16 == 0 && reinterpret_cast<uintptr_t>(gate_w) % 16 == 0 &&
+                   reinterpret_cast<uintptr_t>(up_w) % 16 == 0 && reinterpret_cast<uintptr_t>(gate_s) % 2 == 0 &&
+                   reinterpret_cast<uintptr_t>(up_s) % 2 == 0,
+               "%s: activation and weights must be 16-byte aligned, weight scales 2-byte aligned", op);
+  GEMB_ENTER(op);
+  // Up to eight tokens share a launch and with it one pass over the weights (the verifier's batches are a
+  // handful of tokens), fewer where their activations would not fit the shared memory of a CTA.
+  uint64_t group = std::min<uint64_t>(8, tokens);
+  while (group > 1 && fp4_stage_bytes(group, k) > 200 * 1024) --group;
+  for (uint64_t t0 = 0; t0 < tokens; t0 += group) {
+    Fp4GemvArgs a{};
+    a.act = act + t0 * (k / 2);
+    a.act_scales = act_scales + t0 * (k / 16);
+    a.m[0] = {gate_w, gate_s, gate_out ? gate_out + t0 * rows : nullptr, gate_ga * gate_gw};
+    a.m[1] = {up_w, up_s, up_out ? up_out + t0 * rows : nullptr, up_ga * up_gw};
+    a.product = product + t0 * rows;
+    a.rows = static_cast<uint32_t>(rows);
+    a.k = static_cast<uint32_t>(k);
+    a.tokens = static_cast<uint32_t>(std::min(group, tokens - t0));
+    GEMB_TRY(launch_nvfp4_gemv<true>(op, a, stream));
+  }
+  return GEMB_OK;
+}
+
+int32_t gemb_nvfp4_gemv_gate_up(const uint8_t* act, const uint8_t* act_scales, const uint8_t* gate_w,
+                                const uint8_t* gate_s, const uint8_t* up_w, const uint8_t* up_s,
+                                float* gate_out, float* up_out, float* product, uint64_t rows,
+                                uint64_t k, float gate_ga, float gate_gw, float up_ga, float up_gw,
+                                gemb_stream_t stream) {
+  return gemb_nvfp4_gemv_gate_up_batch(act, act_scales, gate_w, gate_s, up_w, up_s, gate_out, up_out, product, 1, rows, k, gate_ga,
+                                       gate_gw, up_ga, up_gw, stream);
+}
+
+}  // extern "C"

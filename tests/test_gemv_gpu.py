@@ -259,3 +259,34 @@ def test_nvfp4_gemv_small_batch(lib, dev, orc, tokens, rows, k):
     from gem16_b200.lib import GembError
     with pytest.raises(GembError):
         lib.gemb_nvfp4_gemv_batch(d[0], d[1], d[2], d[3], out, 9, rows, k, ga, gw, None)
+
+
+@pytest.mark.parametrize("rows,k,shift", [(8, 64, 0), (24, 192, 16), (16 * 149, 704, 0), (8 * 301, 3904, 16), (1192, 15360, 0)])
+def test_nvfp4_gemv_tiles_and_token_counts(lib, dev, orc, rows, k, shift):
+    """Half tiles, rows that end inside a 128-byte piece, fewer tiles than SMs and a few more, weights with 16-byte and
+    scales with 2-byte alignment only: against binary64, and bit-identical for every batch size."""
+    rng = np.random.default_rng(rows + k)
+    t_max = 8 if k < 8192 else 5
+    x = bf16_round(rng.standard_normal((t_max, k)).astype(np.float32))
+    xp, xs = orc.nvfp4_quantize(x, 400.0)
+    w = [orc.nvfp4_quantize((rng.standard_normal((rows, k)) * 0.03).astype(np.float32), 9000.0) for _ in range(2)]
+
+    def place(a, off):
+        buf = torch.zeros((a.size + 64,), dtype=torch.uint8, device=dev)
+        buf[off:off + a.size] = to_dev(np.ascontiguousarray(a).reshape(-1), dev)
+        return buf[off:off + a.size]
+
+    (gp, gs), (up, us) = [(place(p, shift), place(s, shift // 8)) for p, s in w]
+    dx, dxs = to_dev(xp, dev), to_dev(xs, dev)
+    want = orc.nvfp4_matmul(xp, xs, w[0][0], w[0][1], 400.0, 9000.0)
+    outs = {}
+    for t in (1, 2, 5, t_max):
+        y, p = torch.full((t, rows), 7.0, device=dev), torch.full((t, rows), 7.0, device=dev)
+        g, u = torch.zeros((t, rows), device=dev), torch.zeros((t, rows), device=dev)
+        lib.gemb_nvfp4_gemv_batch(dx, dxs, gp, gs, y, t, rows, k, 400.0, 9000.0, None)
+        lib.gemb_nvfp4_gemv_gate_up_batch(dx, dxs, gp, gs, up, us, g, u, p, t, rows, k, 400.0, 9000.0, 400.0, 9000.0, None)
+        outs[t] = (y, g, u, p)
+        assert np.linalg.norm(to_np(y) - want[:t]) <= 1e-6 * np.linalg.norm(want[:t])
+        assert np.linalg.norm(to_np(g) - want[:t]) <= 1e-6 * np.linalg.norm(want[:t])
+    for t, o in outs.items():
+        assert all(torch.equal(a, b[:t]) for a, b in zip(o, outs[t_max]))
