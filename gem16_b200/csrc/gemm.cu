@@ -150,22 +150,24 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   uint64_t* empty = full + kStages;
   uint64_t* acc_full = empty + kStages;
   uint64_t* acc_empty = acc_full + kAccStages;
-  uint64_t* sf_ready = acc_empty + kAccStages;   // per stage: its scales are in TMEM
-  uint64_t* peer_full = sf_ready + kStages;      // pairs, FP8: the odd CTA's operands have landed
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(peer_full + kStages);
+  uint64_t* sf_full = acc_empty + kAccStages;    // NVFP4, per stage: its scales have landed in shared memory,
+  uint64_t* sf_empty = sf_full + kStages;        // have been read from there by the movers,
+  uint64_t* sf_ready = sf_empty + kStages;       // are in TMEM
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(sf_ready + kStages);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // CTA pairs: the even CTA (rank 0) issues every MMA; the barriers that gate it (scales ready,
-  // accumulator drained, peer operands landed) live in its shared memory and collect arrivals
-  // from both CTAs.  The MMA's completion is committed to the same barrier in both CTAs.
+  // CTA pairs: the even CTA (rank 0) issues every MMA; the barriers that gate it (operands landed, scales
+  // ready, accumulator drained) live in its shared memory and collect arrivals from both CTAs, the
+  // odd CTA's TMA loads included.  The MMA's completion is committed to the same barrier in both CTAs.
   const uint32_t rank = kPair ? ptx::cluster_ctarank() : 0u;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       ptx::mbar_init(&full[s], 1);
       ptx::mbar_init(&empty[s], 1);
+      ptx::mbar_init(&sf_full[s], 1);
+      ptx::mbar_init(&sf_empty[s], 4);
       ptx::mbar_init(&sf_ready[s], kPair ? 8 : 4);
-      ptx::mbar_init(&peer_full[s], 1);
     }
     for (int s = 0; s < kAccStages; ++s) {
       ptx::mbar_init(&acc_full[s], 1);
@@ -238,6 +240,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   // Completion of the MMAs issued so far, signalled to the same barrier of both CTAs of a pair.
   const uint32_t bars_rank0 = kPair ? ptx::cluster_map(bars, 0) : 0u;
   const uint32_t bars_rank1 = kPair ? ptx::cluster_map(bars, 1) : 0u;
+  const uint32_t full_rank0 = bars_rank0;   // `full` comes first
   auto commit = [&](uint64_t* bar) {
     if constexpr (kPair) {
       const uint32_t off = static_cast<uint32_t>(reinterpret_cast<uint8_t*>(bar) - reinterpret_cast<uint8_t*>(bars));
@@ -262,15 +265,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     *abort_flag = 1;
   };
 
-  // NVFP4: 640 threads start with 96 registers each.  The control warpgroup (to 40) and the two
-  // mover warpgroups (to 72) hand back 128 * (56 + 2 * 24) = 13,312 registers; the two epilogue
-  // warpgroups (to 144) take 128 * 2 * 48 = 12,288 of them.  An inc can only be served from what
+  // NVFP4: 640 threads start with 96 registers each.  The control warpgroup (to 48) and the two
+  // mover warpgroups (to 72) hand back 128 * (48 + 2 * 24) = 12,288 registers; the two epilogue
+  // warpgroups (to 144) take 128 * 2 * 48 = 12,288.  An inc can only be served from what
   // the same CTA has released, so the decs must cover the incs (the inc waits for them).  Each
   // setmaxnreg is the first thing its whole warpgroup executes inside the branch it governs.
   const bool is_ctrl = kFp4 ? warp < 4 : warp < 2;
   const bool is_mover = kFp4 && ((warp >= 8 && warp < 12) || warp >= 16);
   if (is_ctrl) {
-  if constexpr (kFp4) ptx::reg_dec<40>();
+  if constexpr (kFp4) ptx::reg_dec<48>();
   if (warp == 0) {
     // ------------------------------- producer -------------------------------------------------
     if (ptx::elect_one()) {
@@ -281,49 +284,50 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         const uint32_t expert = tile_expert ? min(static_cast<uint32_t>(tile_expert_of(mt)), p.experts - 1) : 0u;
         for (uint32_t ks = 0; ks < k_stages; ++ks) {
           if (!ptx::mbar_wait(&empty[stage], phase ^ 1)) { fail_wait(1); break; }
-          const uint32_t k0 = ks * C::kKPerStage;
-          const uint32_t n_mma = min(4u, (p.k - k0) / C::kKPerMma);
-          uint32_t bytes = C::kABytes + C::kBBytes;
-          if constexpr (kFp4) {
-            const uint32_t groups_per_matrix = (p.n + 127) / 128;
-            const uint32_t g0 = expert * groups_per_matrix + (nt * BN) / 128;
-            const uint32_t total_groups = groups_per_matrix * (tile_expert ? p.experts : 1u);
-            const uint32_t n_groups = min(static_cast<uint32_t>(C::kSfbGroups), total_groups - g0);
-            bytes += n_mma * 512 * (1 + n_groups);
-            ptx::mbar_expect_tx(&full[stage], bytes);
-            // The odd CTA of a pair may sit past the last token tile: its rows are never stored,
-            // it just reads the last tile's scales again.
-            ptx::bulk_load_1d(stage_sfa + stage * C::kSfaBytes,
-                              p.sfa + (static_cast<uint64_t>(min(mt, (p.plan ? p.m / BM : m_tiles) - 1)) * k_groups_pad + ks * 4) * 512,
-                              n_mma * 512, &full[stage]);
-            for (uint32_t g = 0; g < n_groups; ++g)
-              ptx::bulk_load_1d(stage_sfb + stage * C::kSfbBytes + g * 2048,
-                                p.sfb + (static_cast<uint64_t>(g0 + g) * k_groups_pad + ks * 4) * 512,
-                                n_mma * 512, &full[stage]);
-          } else {
-            ptx::mbar_expect_tx(&full[stage], bytes);
-          }
-          ptx::tma_load_2d(stage_a + stage * C::kABytes, &map_a, &full[stage], static_cast<int32_t>(ks * 128),
-                           static_cast<int32_t>(mt * BM));
-          ptx::tma_load_2d(stage_b + stage * C::kBBytes, &map_b, &full[stage], static_cast<int32_t>(ks * 128),
-                           static_cast<int32_t>(expert * p.n + nt * BN + rank * C::kBRows));
+          // The even CTA announces the pair's bytes; both CTAs' loads complete on its barrier.
+          if (rank == 0) ptx::mbar_expect_tx(&full[stage], (kPair ? 2 : 1) * (C::kABytes + C::kBBytes));
+          const uint32_t bar = kPair ? full_rank0 + stage * 8 : ptx::smem_addr(&full[stage]);
+          ptx::tma_load_2d<kPair>(stage_a + stage * C::kABytes, &map_a, bar, static_cast<int32_t>(ks * 128),
+                                  static_cast<int32_t>(mt * BM));
+          ptx::tma_load_2d<kPair>(stage_b + stage * C::kBBytes, &map_b, bar, static_cast<int32_t>(ks * 128),
+                                  static_cast<int32_t>(expert * p.n + nt * BN + rank * C::kBRows));
+          if (++stage == kStages) { stage = 0; phase ^= 1; }
+        }
+      }
+    }
+  } else if (kFp4 && warp == 2) {
+    // ------------------------------- scale producer (NVFP4) -----------------------------------
+    // The block scales run through a ring of their own: a stage is free again as soon as the movers have read it,
+    // long before the MMAs that use the scales, so that the next scales are always waiting in shared memory
+    // and the operands' round trip (TMA, MMA, commit) does not pass through the movers.
+    if (ptx::elect_one()) {
+      uint32_t stage = 0, phase = 0;
+      for (uint32_t tile = first_tile; tile < num_tiles && !*abort_flag; tile += tile_stride) {
+        uint32_t mt, nt;
+        tile_coords(tile, mt, nt);
+        const uint32_t expert = tile_expert ? min(static_cast<uint32_t>(tile_expert_of(mt)), p.experts - 1) : 0u;
+        const uint32_t groups_per_matrix = (p.n + 127) / 128;
+        const uint32_t g0 = expert * groups_per_matrix + (nt * BN) / 128;
+        const uint32_t total_groups = groups_per_matrix * (tile_expert ? p.experts : 1u);
+        const uint32_t n_groups = min(static_cast<uint32_t>(C::kSfbGroups), total_groups - g0);
+        // The odd CTA of a pair may sit past the last token tile: its rows are never stored,
+        // it just reads the last tile's scales again.
+        const uint8_t* sfa = p.sfa + static_cast<uint64_t>(min(mt, (p.plan ? p.m / BM : m_tiles) - 1)) * k_groups_pad * 512;
+        const uint8_t* sfb = p.sfb + static_cast<uint64_t>(g0) * k_groups_pad * 512;
+        for (uint32_t ks = 0; ks < k_stages; ++ks) {
+          if (!ptx::mbar_wait(&sf_empty[stage], phase ^ 1)) { fail_wait(6); break; }
+          const uint32_t bytes = min(4u, (p.k - ks * C::kKPerStage) / C::kKPerMma) * 512;
+          ptx::mbar_expect_tx(&sf_full[stage], bytes * (1 + n_groups));
+          ptx::bulk_load_1d(stage_sfa + stage * C::kSfaBytes, sfa + static_cast<uint64_t>(ks) * 2048, bytes, &sf_full[stage]);
+          for (uint32_t g = 0; g < n_groups; ++g)
+            ptx::bulk_load_1d(stage_sfb + stage * C::kSfbBytes + g * 2048,
+                              sfb + (static_cast<uint64_t>(g) * k_groups_pad + ks * 4) * 512, bytes, &sf_full[stage]);
           if (++stage == kStages) { stage = 0; phase ^= 1; }
         }
       }
     }
   } else if (warp == 1 && rank != 0) {
-    // ------------------------------- odd CTA of a pair: relay (FP8) ---------------------------
-    // Tells the issuer in the even CTA that this CTA's operands have landed.  NVFP4 needs no
-    // relay: the scale movers, who wait for the operands, arrive on the issuer's barrier.
-    if (!kFp4 && ptx::elect_one()) {
-      const uint32_t total_steps = my_tiles * k_stages;
-      uint32_t stage = 0, phase = 0;
-      for (uint32_t step = 0; step < total_steps && !*abort_flag; ++step) {
-        if (!ptx::mbar_wait(&full[stage], phase)) { fail_wait(7); break; }
-        arrive_issuer(&peer_full[stage]);
-        if (++stage == kStages) { stage = 0; phase ^= 1; }
-      }
-    }
+    // the odd CTA of a pair issues no MMA
   } else if (warp == 1) {
     // ------------------------------- MMA issuer -----------------------------------------------
     // One thread issues everything.  Its instruction stream is on the critical path (an MMA
@@ -342,14 +346,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         uint32_t k_left = p.k;
         bool ok = true;
         for (uint32_t ks = 0; ks < k_stages; ++ks, k_left -= C::kKPerStage) {
-          // NVFP4 waits for the scale movers (who waited for the operands); FP8 for the operands.
-          if (!ready) {
-            if constexpr (kFp4) {
-              ok = wait_issuer(&sf_ready[stage], phase);
-            } else {
-              ok = ptx::mbar_wait(&full[stage], phase);
-              if constexpr (kPair) ok = ok && wait_issuer(&peer_full[stage], phase);
-            }
+          if (!ready) {   // the operands and, NVFP4, their scales
+            ok = wait_issuer(&full[stage], phase);
+            if constexpr (kFp4) ok = ok && wait_issuer(&sf_ready[stage], phase);
             if (!ok) { fail_wait(3); break; }
           }
           ptx::tc_fence_after();
@@ -358,10 +357,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
           const uint32_t n_mma = min(4u, k_left / C::kKPerMma);
           const uint64_t a_desc = ptx::smem_desc_k128_swizzled(ptx::smem_addr(stage_a + stage * C::kABytes));
           const uint64_t b_desc = ptx::smem_desc_k128_swizzled(ptx::smem_addr(stage_b + stage * C::kBBytes));
-          // What the next step will wait for: NVFP4 the scale movers (who waited for the operands),
-          // FP8 the operands of this CTA and, in a pair, of the odd CTA.
-          uint64_t* poll0 = kFp4 ? &sf_ready[next_stage] : &full[next_stage];
-          uint64_t* poll1 = (!kFp4 && kPair) ? &peer_full[next_stage] : poll0;
+          uint64_t* poll0 = &full[next_stage];   // what the next step will wait for
+          uint64_t* poll1 = kFp4 ? &sf_ready[next_stage] : poll0;
           if constexpr (kFp4) {
             const uint32_t tsfa = tmem_base + C::kAccCols + stage * C::kSfColsPerStage;
             const uint32_t tsfb = tsfa + C::kSfaCols;
@@ -425,14 +422,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
       const uint32_t total_steps = my_tiles * k_stages;
       static_assert(kStages % 2 == 1 && kStages >= 3, "the mover sets split an odd number of stages");
       const uint32_t mset = warp >= 16 ? 1u : 0u;
-      uint32_t stage = mset, phase = 0, step = mset, ks = mset % k_stages;
+      uint32_t stage = mset, phase = 0, step = mset;
       bool ready = false;
       while (step < total_steps && !*abort_flag) {
-        if (!ready && !ptx::mbar_wait(&full[stage], phase)) { fail_wait(5); break; }
-        // A full stage means its previous MMAs completed (the producer waited for that), so the
-        // stage's TMEM scale region is free as well.
-        ptx::tc_fence_after();
-        const uint32_t n_mma = min(4u, (p.k - ks * C::kKPerStage) / C::kKPerMma);
+        if (!ready && !ptx::mbar_wait(&sf_full[stage], phase)) { fail_wait(5); break; }
         const uint32_t tsfa = tmem_base + C::kAccCols + stage * C::kSfColsPerStage + lane_base;
         const uint32_t tsfb = tsfa + C::kSfaCols;
         const uint8_t* sfa_s = stage_sfa + stage * C::kSfaBytes + lane * 16;
@@ -445,29 +438,25 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
           next_phase ^= 1;
           delta = mset ? 3 : 1;
         }
-        if (n_mma == 4) {
-          uint4 a4[4], b4[4 * C::kSfbGroups];
+        // Four MMAs' worth always: behind the end of K a stage holds old bytes, which no MMA reads.
+        uint4 a4[4], b4[4 * C::kSfbGroups];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            a4[j] = *reinterpret_cast<const uint4*>(sfa_s + j * 512);
+        for (int j = 0; j < 4; ++j) {
+          a4[j] = *reinterpret_cast<const uint4*>(sfa_s + j * 512);
 #pragma unroll
-            for (int g = 0; g < C::kSfbGroups; ++g)
-              b4[j * C::kSfbGroups + g] = *reinterpret_cast<const uint4*>(sfb_s + g * 2048 + j * 512);
-          }
-          ready = ptx::mbar_test_wait(&full[next_stage], next_phase);
-          ptx::tc_st_32x32b_x16(tsfa, a4);
-          if constexpr (C::kSfbGroups == 2) ptx::tc_st_32x32b_x32(tsfb, b4);
-          else ptx::tc_st_32x32b_x16(tsfb, b4);
-        } else {
-          // Last stage of a K that is not a multiple of 256: fewer MMAs, fewer scale rows staged.
-          ready = false;
-          for (uint32_t j = 0; j < n_mma; ++j) {
-            ptx::tc_st_32x32b_x4(tsfa + j * 4, *reinterpret_cast<const uint4*>(sfa_s + j * 512));
-            for (int g = 0; g < C::kSfbGroups; ++g)
-              ptx::tc_st_32x32b_x4(tsfb + j * C::kSfbColsPerMma + g * 4,
-                                   *reinterpret_cast<const uint4*>(sfb_s + g * 2048 + j * 512));
-          }
+          for (int g = 0; g < C::kSfbGroups; ++g)
+            b4[j * C::kSfbGroups + g] = *reinterpret_cast<const uint4*>(sfb_s + g * 2048 + j * 512);
         }
+        // The scales are in registers: their shared-memory stage can be refilled.  The stage's TMEM region is free
+        // once the MMAs of its previous use have completed, which the commit of the operand stage says.
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(&sf_empty[stage]);
+        if (!ptx::mbar_wait(&empty[stage], phase ^ 1)) { fail_wait(7); break; }
+        ptx::tc_fence_after();
+        ready = ptx::mbar_test_wait(&sf_full[next_stage], next_phase);
+        ptx::tc_st_32x32b_x16(tsfa, a4);
+        if constexpr (C::kSfbGroups == 2) ptx::tc_st_32x32b_x32(tsfb, b4);
+        else ptx::tc_st_32x32b_x16(tsfb, b4);
         ptx::tc_wait_st();
         ptx::tc_fence_before();
         __syncwarp();
@@ -475,8 +464,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         stage = next_stage;
         phase = next_phase;
         step += delta;
-        ks += delta;
-        while (ks >= k_stages) ks -= k_stages;
       }
     }
   } else {

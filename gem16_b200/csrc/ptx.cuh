@@ -135,13 +135,20 @@ __device__ __forceinline__ void reg_inc() {
 __device__ __forceinline__ void prefetch_tensormap(const void* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
-// 2-D tiled load global -> shared of this CTA, completion on `bar` (transaction bytes).
-__device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* map, uint64_t* bar, int32_t x,
-                                            int32_t y) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(smem_addr(smem_dst)), "l"(map), "r"(smem_addr(bar)), "r"(x), "r"(y)
-      : "memory");
+// 2-D tiled load global -> shared of this CTA, completion (transaction bytes) on the barrier at shared address
+// `bar`: one of this CTA or, with kPair (cta_group::2), a cluster address of a barrier of either CTA of the pair.
+template <bool kPair>
+__device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* map, uint32_t bar, int32_t x, int32_t y) {
+  if constexpr (kPair)
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        ::"r"(smem_addr(smem_dst)), "l"(map), "r"(bar), "r"(x), "r"(y)
+        : "memory");
+  else
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        ::"r"(smem_addr(smem_dst)), "l"(map), "r"(bar), "r"(x), "r"(y)
+        : "memory");
 }
 // 1-D bulk copy global -> shared; both addresses 16-byte aligned, size a multiple of 16.
 __device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gmem_src, uint32_t bytes,
