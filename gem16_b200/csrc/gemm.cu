@@ -151,7 +151,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   uint64_t* acc_full = empty + kStages;
   uint64_t* acc_empty = acc_full + kAccStages;
   uint64_t* sf_full = acc_empty + kAccStages;    // NVFP4, per stage: its scales have landed in shared memory,
-  uint64_t* sf_empty = sf_full + kStages;        // have been read from there by the movers,
+  uint64_t* sf_empty = sf_full + kStages;        // have been copied from there by the movers,
   uint64_t* sf_ready = sf_empty + kStages;       // are in TMEM
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(sf_ready + kStages);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
@@ -297,8 +297,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     }
   } else if (kFp4 && warp == 2) {
     // ------------------------------- scale producer (NVFP4) -----------------------------------
-    // The block scales run through a ring of their own: a stage is free again as soon as the movers have read it,
-    // long before the MMAs that use the scales, so that the next scales are always waiting in shared memory
+    // The block scales run through a ring of their own: a stage is free again as soon as the movers have copied it
+    // to TMEM, before the MMAs that use the scales, so that the next scales are waiting in shared memory
     // and the operands' round trip (TMA, MMA, commit) does not pass through the movers.
     if (ptx::elect_one()) {
       uint32_t stage = 0, phase = 0;
@@ -447,10 +447,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
           for (int g = 0; g < C::kSfbGroups; ++g)
             b4[j * C::kSfbGroups + g] = *reinterpret_cast<const uint4*>(sfb_s + g * 2048 + j * 512);
         }
-        // The scales are in registers: their shared-memory stage can be refilled.  The stage's TMEM region is free
-        // once the MMAs of its previous use have completed, which the commit of the operand stage says.
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(&sf_empty[stage]);
+        // The stage's TMEM region is free once the MMAs of its previous use have completed, which the commit of
+        // the operand stage says.
         if (!ptx::mbar_wait(&empty[stage], phase ^ 1)) { fail_wait(7); break; }
         ptx::tc_fence_after();
         ready = ptx::mbar_test_wait(&sf_full[next_stage], next_phase);
@@ -460,7 +458,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         ptx::tc_wait_st();
         ptx::tc_fence_before();
         __syncwarp();
-        if (lane == 0) arrive_issuer(&sf_ready[stage]);
+        // Only here may the shared-memory stage be refilled: tcgen05.st has taken the registers, so the loads have
+        // returned.  Behind the loads alone the arrival can overtake them (they are still queued), and the
+        // refill then reaches a warp that wanted the old scales; waiting this long costs nothing measurable.
+        if (lane == 0) {
+          arrive_issuer(&sf_ready[stage]);
+          ptx::mbar_arrive(&sf_empty[stage]);
+        }
         stage = next_stage;
         phase = next_phase;
         step += delta;

@@ -407,3 +407,19 @@ def test_router_input_rows_in_shared_memory(lib, dev, orc, tokens, hidden, offse
     lib.gemb_moe_router_input(to_dev(x, dev), to_dev(scale, dev), got[offset:], tokens, hidden, 1e-6, None)
     want = orc.moe_router_input(x, scale, 1e-6)
     assert np.array_equal(to_np(got[offset:]).view(np.uint16).reshape(tokens, hidden), want)
+
+
+@pytest.mark.parametrize("tokens", [192, 3001])
+def test_layer_bytes_do_not_change_between_calls(lib, dev, tokens):
+    """The GEMM's operand and scale rings under two streams and changing inputs: same input, same bytes, every call."""
+    from gem16_b200.moe import synthetic_weights
+    layer = MoeLayer(synthetic_weights(dev, 7), tokens, 8, 600.0, 336.0, 336.0, stages=False)
+    layer.fused = True
+    g = torch.Generator(device=dev).manual_seed(tokens)
+    x, other = (torch.randn((tokens, 2816), device=dev, generator=g).bfloat16().view(torch.int16) for _ in range(2))
+    want = layer.forward(x).clone()
+    outs = []
+    for _ in range(100 if tokens < 1000 else 20):
+        layer.forward(other)
+        outs.append(layer.forward(x).clone())
+    assert all(torch.equal(o, want) for o in outs)
