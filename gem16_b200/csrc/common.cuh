@@ -111,6 +111,12 @@ int32_t launch_pdl(const char* op, void (*kern)(P...), dim3 grid, dim3 block, si
 #ifdef __CUDACC__
 
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
+// The decode GEMVs read their weights ahead of pdl_wait.  A quantiser, whose output may be a weight matrix, therefore lets
+// its dependents start early only for a decode batch's few rows; otherwise they start when
+// its CTAs have ended.
+__device__ __forceinline__ void pdl_trigger_few_rows(uint32_t rows) {
+  if (rows <= 16) pdl_trigger();
+}
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Loads of data an earlier kernel of the stream produced (volatile: they stay behind pdl_wait).
 __device__ __forceinline__ uint4 ld_dep(const uint4* p) {
@@ -131,6 +137,16 @@ __device__ __forceinline__ float ld_dep(const float* p) {
 __device__ __forceinline__ uint16_t ld_dep(const uint16_t* p) {
   uint16_t v;
   asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ int32_t ld_dep(const int32_t* p) {
+  int32_t v;
+  asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ int2 ld_dep(const int2* p) {
+  int2 v;
+  asm volatile("ld.global.v2.s32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
   return v;
 }
 __device__ __forceinline__ uint8_t ld_dep(const uint8_t* p) {

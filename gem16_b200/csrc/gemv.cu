@@ -92,7 +92,7 @@ __device__ __forceinline__ void zero_fp8_staging_tail(uint64_t k, __half* xs) {
 template <int kW>
 __device__ __forceinline__ void stage_fp8_activation(const uint8_t* act, uint64_t k, __half* xs) {
   for (uint64_t c = threadIdx.x; c < k / 16; c += kW * 32) {
-    const uint4 v = __ldg(reinterpret_cast<const uint4*>(act) + c);
+    const uint4 v = ld_dep(reinterpret_cast<const uint4*>(act) + c);
     const uint32_t ww[4] = {v.x, v.y, v.z, v.w};
     uint32_t h[8];
 #pragma unroll
@@ -147,7 +147,7 @@ __device__ __forceinline__ float stage_bf16_activation(const uint16_t* x, uint64
 #pragma unroll
     for (int i = 0; i < kBatch; ++i) {
       const uint64_t c = base + static_cast<uint64_t>(i) * (kW * 32);
-      v[i] = c < chunks ? __ldg(xp + c) : make_uint4(0, 0, 0, 0);
+      v[i] = c < chunks ? ld_dep(xp + c) : make_uint4(0, 0, 0, 0);
     }
 #pragma unroll
     for (int i = 0; i < kBatch; ++i) amax = fmaxf(amax, chunk_amax(v[i]));
@@ -165,7 +165,7 @@ __device__ __forceinline__ float stage_bf16_activation(const uint16_t* x, uint64
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const uint64_t c = base + static_cast<uint64_t>(i) * (kW * 32);
-      v[i] = c < chunks ? __ldg(xp + c) : make_uint4(0, 0, 0, 0);
+      v[i] = c < chunks ? ld_dep(xp + c) : make_uint4(0, 0, 0, 0);
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -224,22 +224,24 @@ fp8_gemv_kernel(const void* __restrict__ act, const float* __restrict__ act_scal
 
   // Programmatic dependent launch: let the next kernel in the stream start its own weight
   // prefetch as soon as SM slots free up; weights are immutable so they may be read before the
-  // previous kernel has finished, everything else waits for it.
-  asm volatile("griddepcontrol.launch_dependents;");
+  // previous kernel has finished, everything else waits for it.  (Loading them behind the wait, with an L2
+  // prefetch in front of it, cost a four-layer FP8 decode pass 21 of 209 us.)  No kernel that could be writing
+  // weights triggers its dependents early: the quantisers do so for a decode batch only.
+  pdl_trigger();
   uint64_t task = static_cast<uint64_t>(blockIdx.x) * kW + warp;
   bool prefetched = false;
   if (task < num_tasks) {
     load_step(task, 0);
     prefetched = true;
   }
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_wait();
 
   float a_scale;
   if constexpr (kFusedQuant) {
     a_scale = stage_bf16_activation<kW>(static_cast<const uint16_t*>(act), k, xs, red);
   } else {
     stage_fp8_activation<kW>(static_cast<const uint8_t*>(act), k, xs);
-    a_scale = __ldg(act_scale);
+    a_scale = ld_dep(act_scale);
   }
   __syncthreads();
 
@@ -369,19 +371,19 @@ fp8_gemv_batch_kernel(const uint8_t* __restrict__ act, const float* __restrict__
     for (int u = 0; u < kUnroll; ++u)
       wv[u] = kb + u * 512 + lane * 16 < k ? ldg_stream(wp + u * 512) : make_uint4(0, 0, 0, 0);
   };
-  asm volatile("griddepcontrol.launch_dependents;");
+  pdl_trigger();
   uint64_t task = static_cast<uint64_t>(blockIdx.x) * kWarps + warp;
   bool prefetched = false;
   if (task < total_rows) {
     load_step(task, 0);
     prefetched = true;
   }
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_wait();
 #pragma unroll 1
   for (int t = 0; t < kTok; ++t) stage_fp8_activation<kWarps>(act + static_cast<uint64_t>(t) * k, k, xs + t * k_pad);
   float a_scale[kTok];
 #pragma unroll
-  for (int t = 0; t < kTok; ++t) a_scale[t] = __ldg(act_scales + t);
+  for (int t = 0; t < kTok; ++t) a_scale[t] = ld_dep(act_scales + t);
   __syncthreads();
   for (; task < total_rows; task += task_stride) {
     float acc[kTok];
@@ -515,7 +517,7 @@ fp8_gemv_mma_kernel(const uint8_t* __restrict__ act, const float* __restrict__ a
       wb[u] = in ? ldg_stream(rb + off) : make_uint4(0, 0, 0, 0);
     }
   };
-  asm volatile("griddepcontrol.launch_dependents;");
+  pdl_trigger();
   uint64_t task = blockIdx.x;
   const uint64_t first_kb = static_cast<uint64_t>(warp) * kMmaSpan;
   const uint8_t* ra = nullptr;
@@ -527,11 +529,11 @@ fp8_gemv_mma_kernel(const uint8_t* __restrict__ act, const float* __restrict__ a
     load_span(ra, rb, first_kb);
     prefetched = true;
   }
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_wait();
   const bool token_live = static_cast<uint32_t>(g) < tokens;   // B column g = token g; columns past the batch are zero
   const uint8_t* xrow = act + static_cast<uint64_t>(token_live ? g : 0) * k + t4 * 16;
-  const float s0 = 2 * t4 < static_cast<int>(tokens) ? __ldg(act_scales + 2 * t4) : 0.0f;
-  const float s1 = 2 * t4 + 1 < static_cast<int>(tokens) ? __ldg(act_scales + 2 * t4 + 1) : 0.0f;
+  const float s0 = 2 * t4 < static_cast<int>(tokens) ? ld_dep(act_scales + 2 * t4) : 0.0f;
+  const float s1 = 2 * t4 + 1 < static_cast<int>(tokens) ? ld_dep(act_scales + 2 * t4 + 1) : 0.0f;
   for (; task < num_tasks; task += gridDim.x) {
     if (!prefetched) {
       ra = row_pointer(task * 16 + g);
@@ -545,7 +547,7 @@ fp8_gemv_mma_kernel(const uint8_t* __restrict__ act, const float* __restrict__ a
       for (int u = 0; u < kMmaPieces; ++u) {
         if (kb + u * 64 < k) {   // warp-uniform; K is a multiple of 16, lanes past it hold zero weights
           uint4 xv = make_uint4(0, 0, 0, 0);
-          if (token_live && kb + u * 64 + t4 * 16 < k) xv = __ldg(reinterpret_cast<const uint4*>(xrow + kb + u * 64));
+          if (token_live && kb + u * 64 + t4 * 16 < k) xv = ld_dep(reinterpret_cast<const uint4*>(xrow + kb + u * 64));
           mma_e4m3_m16n8k32(acc, wa[u].x, wb[u].x, wa[u].y, wb[u].y, xv.x, xv.y);
           mma_e4m3_m16n8k32(acc, wa[u].z, wb[u].z, wa[u].w, wb[u].w, xv.z, xv.w);
         }
@@ -916,8 +918,8 @@ __global__ void __launch_bounds__(1024)
 fp8_quantize_decode_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ out,
                            float* __restrict__ scales, uint32_t k) {
   __shared__ float red[32];
-  asm volatile("griddepcontrol.launch_dependents;");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_trigger();
+  pdl_wait();
   const uint64_t t = blockIdx.x;
   const uint4* xp = reinterpret_cast<const uint4*>(x + t * k);
   const uint32_t chunks = k / 8;
@@ -926,7 +928,7 @@ fp8_quantize_decode_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
     const uint32_t c = threadIdx.x + i * 1024;
-    v[i] = c < chunks ? __ldg(xp + c) : make_uint4(0, 0, 0, 0);
+    v[i] = c < chunks ? ld_dep(xp + c) : make_uint4(0, 0, 0, 0);
     amax = fmaxf(amax, chunk_amax(v[i]));
   }
   amax = warp_max(amax);

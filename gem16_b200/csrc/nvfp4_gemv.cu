@@ -17,7 +17,8 @@
 // work cost as much as SMs without loads.  Measured, weights cold, in a chain of launches: gate / up 2 x 15,360 x 3,840 in
 // 18 us for one token and 20 us for five (23 us per token before, one launch each), down 3,840 x 15,360 in 12 and
 // 14 us (11 and 67 us before); without the loads the arithmetic takes 12 us, without the arithmetic
-// the loads 8.  Requesting all weights into L2 ahead of pdl_wait changed nothing: the kernels before
+// the loads 8.  A warp's first pieces are loaded ahead of pdl_wait (weights are immutable): 7 % of a decode pass.
+// Requesting all weights into L2 ahead of it changed nothing: the kernels before
 // this one then wait for HBM instead.  Lane 4g + t loads 32 contiguous bytes of rows g and g + 8 per piece
 // (four scale blocks each) and the four scale bytes that go with them; MMA j takes bytes 2j, 2j + 1 of that run as
 // a0 / a2 (row g) and a1 / a3 (row g + 8).  That permutes k inside the piece, which is harmless because the
@@ -82,8 +83,7 @@ struct Fp4GemvArgs {
   bool wide;       // weights 32-byte and scales 4-byte aligned
 };
 
-// One row's share of a piece: 32 weight bytes and four scale bytes.  Left as it is when `in` is false: the
-// activations past K are zero and pieces past the warp's share are not used.
+// One row's share of a piece: 32 weight bytes and four scale bytes.  Left as it is when `in` is false.
 struct Run {
   uint32_t w[8];
   uint32_t s;
@@ -186,7 +186,6 @@ nvfp4_gemv_kernel(const __grid_constant__ Fp4GemvArgs a) {
   auto share = [&](uint32_t w) { return list * w / kFpWarps; };
   const uint64_t lo = share(warp), hi = share(warp + 1);
   pdl_trigger();
-  pdl_wait();
   // Load cursor: piece `next` of the list = piece `np` of the tile whose rows the pointers stand on.
   uint64_t next = lo;
   uint32_t ntile = static_cast<uint32_t>(lo / pieces), np = static_cast<uint32_t>(lo % pieces);
@@ -204,6 +203,7 @@ nvfp4_gemv_kernel(const __grid_constant__ Fp4GemvArgs a) {
   Run wa[kAhead], wb[kAhead];
   auto load = [&](int u) {
     const bool in = next < hi && np * 128 + t * 32 < row_bytes;
+    wa[u].s = wb[u].s = 0;   // past K: old codes with zero scales against zero activations
     load_run(wa[u], pw[0] + np * 128, ps[0] + np * 16, in, a.wide);
     load_run(wb[u], pw[1] + np * 128, ps[1] + np * 16, in, a.wide);
     ++next;
@@ -221,6 +221,7 @@ nvfp4_gemv_kernel(const __grid_constant__ Fp4GemvArgs a) {
     wa[u].s = wb[u].s = 0;
     load(u);
   }
+  pdl_wait();   // the weights do not depend on the kernels before this one
   // under the first weight loads
   if (threadIdx.x < 8) reinterpret_cast<uint4*>(smem)[threadIdx.x] = make_uint4(0, 0, 0, 0);
   stage_fp4_activations(a, xs);

@@ -90,7 +90,7 @@ template <class Loader, bool kRcp, bool kInterleaved>
 __global__ void __launch_bounds__(256)
 nvfp4_quantize_kernel(Loader loader, uint8_t* __restrict__ packed, uint8_t* __restrict__ scales,
                       uint32_t tokens, uint64_t k, uint32_t blocks_pad, uint64_t cells, float g) {
-  pdl_trigger();
+  pdl_trigger_few_rows(tokens);
   pdl_wait();
   // blockDim and cells are multiples of 4: quads stay whole.  A 64-bit division costs as much as the
   // quantisation of a block, so it is left to tensors that need it.
@@ -236,9 +236,9 @@ __device__ __forceinline__ void normalise8(const uint4& raw, const uint4* w, boo
 template <int kMode, bool kRcp>
 __global__ void __launch_bounds__(kRowWarps * 32, kMode == kRowResidual ? 4 : 5)
 row_warp_kernel(const __grid_constant__ RowArgs a) {
-  pdl_trigger();
-  pdl_wait();
   constexpr bool kNorm = kMode != kRowFp8;
+  if constexpr (kNorm) pdl_trigger();   // a normalised tensor is no weight
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const uint64_t r = static_cast<uint64_t>(blockIdx.x) * kRowWarps + (threadIdx.x >> 5);
   const uint32_t k = static_cast<uint32_t>(a.k);
@@ -523,7 +523,8 @@ __global__ void __launch_bounds__(256)
 fp8_quantize_kernel(const In* x, const uint16_t* __restrict__ w, uint8_t* out, float* scales, uint64_t k, float eps) {
   __shared__ float red[256];
   __shared__ float red2[8];
-  pdl_trigger();
+  if constexpr (kNorm) pdl_trigger();
+  else pdl_trigger_few_rows(gridDim.x);
   pdl_wait();
   const uint64_t r = blockIdx.x;
   const In* row = x + r * k;
