@@ -95,11 +95,15 @@ def _ctype(t: str):
     return _SCALARS[t.replace("const ", "")]
 
 
+_PLAIN = frozenset((int, float, type(None)))
+
+
 def _as_arg(v):
     if v is None:
         return None
-    if hasattr(v, "data_ptr"):
-        return v.data_ptr()
+    data_ptr = getattr(v, "data_ptr", None)
+    if data_ptr is not None:
+        return data_ptr()
     if hasattr(v, "cuda_stream"):
         return v.cuda_stream
     if isinstance(v, C.Structure):
@@ -131,17 +135,23 @@ class Lib:
         return getattr(self.cdll, name)(*[_as_arg(a) for a in args])
 
     def __getattr__(self, name: str):
+        """The checked call of an entry point, built once and kept on the instance: a decode call is a few
+        microseconds on the GPU, so the host path must not cost more.  Plain numbers, None and
+        tensors (by far the most arguments) are converted without going through _as_arg."""
         if not name.startswith("gemb_"):
             raise AttributeError(name)
-        ret = self.protos[name][0]
         fn = getattr(self.cdll, name)
-
-        def call(*args):
-            rc = fn(*[_as_arg(a) for a in args])
-            if ret == "int32_t" and rc != 0:
-                raise GembError(rc, self.last_error())
-            return rc
-
+        plain, convert = _PLAIN, _as_arg
+        if self.protos[name][0] == "int32_t":
+            def call(*args):
+                rc = fn(*[a if type(a) in plain else convert(a) for a in args])
+                if rc:
+                    raise GembError(rc, self.last_error())
+                return rc
+        else:
+            def call(*args):
+                return fn(*[a if type(a) in plain else convert(a) for a in args])
+        setattr(self, name, call)
         return call
 
 
