@@ -161,6 +161,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   // ready, accumulator drained) live in its shared memory and collect arrivals from both CTAs, the
   // odd CTA's TMA loads included.  The MMA's completion is committed to the same barrier in both CTAs.
   const uint32_t rank = kPair ? ptx::cluster_ctarank() : 0u;
+  pdl_trigger();
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       ptx::mbar_init(&full[s], 1);
@@ -188,6 +189,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   else __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
+  pdl_wait();   // barriers, tensor memory and descriptors are set up while the kernel before this one finishes
 
   // A device-side plan is clamped to the buffers' capacity (p.m rows): whatever it holds, no tile
   // beyond the activation, scale and output buffers is touched.
@@ -197,8 +199,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   // plan entries behind the expert offsets: {expert of tile i (-1: padding only), i-th tile that holds real rows},
   // then, behind the last tile's pair, the number of tiles that hold real rows.
   const int32_t* tile_info = p.plan ? p.plan + 3 + p.experts : nullptr;
-  const uint32_t plan_tiles = p.plan ? min(static_cast<uint32_t>(__ldg(p.plan)), p.m / BM) : 0u;
-  const uint32_t m_tiles = p.plan ? (kPair ? plan_tiles : min(static_cast<uint32_t>(__ldg(tile_info + 2 * plan_tiles)), plan_tiles))
+  const uint32_t plan_tiles = p.plan ? min(static_cast<uint32_t>(ld_dep(p.plan)), p.m / BM) : 0u;
+  const uint32_t m_tiles = p.plan ? (kPair ? plan_tiles : min(static_cast<uint32_t>(ld_dep(tile_info + 2 * plan_tiles)), plan_tiles))
                                   : (p.m + BM - 1) / BM;
   const uint32_t n_tiles = (p.n + BN - 1) / BN;
   const int32_t* tile_expert = tile_info;   // stride 2
@@ -207,8 +209,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   uint32_t unit0 = 0;   // first 256-row unit of the call's expert range
   if constexpr (kPair) {
     if (p.plan != nullptr && p.expert_hi != 0) {   // padded offsets are multiples of 256 rows: whole units
-      const uint32_t lo_t = min(static_cast<uint32_t>(__ldg(p.plan + 2 + min(p.expert_lo, p.experts))) / BM, plan_tiles);
-      const uint32_t hi_t = min(static_cast<uint32_t>(__ldg(p.plan + 2 + min(p.expert_hi, p.experts))) / BM, plan_tiles);
+      const uint32_t lo_t = min(static_cast<uint32_t>(ld_dep(p.plan + 2 + min(p.expert_lo, p.experts))) / BM, plan_tiles);
+      const uint32_t hi_t = min(static_cast<uint32_t>(ld_dep(p.plan + 2 + min(p.expert_hi, p.experts))) / BM, plan_tiles);
       unit0 = lo_t / 2;
       m_units = hi_t > lo_t ? (hi_t - lo_t + 1) / 2 : 0u;
     }
@@ -220,7 +222,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   const uint32_t k_stages = (p.k + C::kKPerStage - 1) / C::kKPerStage;
   const uint32_t k_groups_pad = (p.k / 16 + 3) / 4;  // 512-byte scale chunks per 128-row group
   auto tile_expert_of = [&](uint32_t mt) -> int32_t {
-    return __ldg(tile_expert + 2 * (kPair ? (mt & ~1u) : mt));
+    return ld_dep(tile_expert + 2 * (kPair ? (mt & ~1u) : mt));
   };
 
   // Tile order: groups of 16 token tiles; inside a group the token tile runs fastest, so the
@@ -234,7 +236,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     const uint32_t within = tile % per_group;
     mt = first_m + within % gm;
     if constexpr (kPair) mt = (mt + unit0) * 2 + rank;
-    else if (tile_info != nullptr) mt = min(static_cast<uint32_t>(__ldg(tile_info + 2 * mt + 1)), p.m / BM - 1);
+    else if (tile_info != nullptr) mt = min(static_cast<uint32_t>(ld_dep(tile_info + 2 * mt + 1)), p.m / BM - 1);
     nt = within / gm;
   };
   // Completion of the MMAs issued so far, signalled to the same barrier of both CTAs of a pair.
@@ -482,18 +484,18 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
       uint32_t mt, nt;
       tile_coords(tile, mt, nt);
       // In a pair the odd CTA may own a padding-only tile: it takes part in the barriers, nothing else.
-      const bool dead = kPair && tile_expert != nullptr && (mt >= p.m / BM || __ldg(tile_expert + 2 * mt) < 0);
-      // The staging buffer must be free again (the previous tile's last store has read it); checked
-      // here, while the tile is still being computed, rather than after the accumulator is full.
+      const bool dead = kPair && tile_expert != nullptr && (mt >= p.m / BM || ld_dep(tile_expert + 2 * mt) < 0);
+      // The scales are fetched, and the staging buffer checked to be free again (the previous tile's last store has
+      // read it), here, while the tile is still being computed, rather than after the accumulator is full.
+      const uint32_t row0 = mt * BM + quarter * 32;
+      float row_scale = p.alpha;
+      if constexpr (!kFp4) row_scale = row0 + lane < p.m ? ld_dep(p.a_scales + row0 + lane) : 0.0f;
+      if (kFp4 && p.w_divisors != nullptr)
+        row_scale = __fdiv_rn(1.0f, __fmul_rn(p.ga, __ldg(p.w_divisors + (tile_expert ? min(static_cast<uint32_t>(tile_expert_of(mt)), p.experts - 1) : 0u))));
       if (lane == 0) ptx::bulk_wait_group_read<0>();
       __syncwarp();
       if (!ptx::mbar_wait(&acc_full[as], aphase)) { fail_wait(4); break; }
       ptx::tc_fence_after();
-      const uint32_t row0 = mt * BM + quarter * 32;
-      float row_scale = p.alpha;
-      if constexpr (!kFp4) row_scale = row0 + lane < p.m ? __ldg(p.a_scales + row0 + lane) : 0.0f;
-      if (kFp4 && p.w_divisors != nullptr)
-        row_scale = __fdiv_rn(1.0f, __fmul_rn(p.ga, __ldg(p.w_divisors + (tile_expert ? min(static_cast<uint32_t>(tile_expert_of(mt)), p.experts - 1) : 0u))));
       const uint32_t tmem_acc = tmem_base + as * BN + ((quarter * 32) << 16);
       bool released = false, pending = false;
       uint32_t pending_col = 0;
@@ -503,10 +505,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
       int2 push_to = make_int2(-1, 0);
       uint32_t push_valid = 0;
       if (kFp4 && p.push_meta != nullptr && !dead) {
-        const uint32_t tile_rows = min(static_cast<uint32_t>(__ldg(p.push_tile_rows + mt)), static_cast<uint32_t>(BM));
+        const uint32_t tile_rows = min(static_cast<uint32_t>(ld_dep(p.push_tile_rows + mt)), static_cast<uint32_t>(BM));
         push_valid = tile_rows > quarter * 32 ? min(32u, tile_rows - quarter * 32) : 0u;
         if (static_cast<uint32_t>(lane) < push_valid) {
-          push_to = __ldg(p.push_meta + row0 + lane);
+          push_to = ld_dep(p.push_meta + row0 + lane);
           if (static_cast<uint32_t>(push_to.x) >= p.push_ranks || static_cast<uint32_t>(push_to.y) >= p.push_rows) {
             atomicCAS(&g_gemm_error, 0, 8);   // a destination outside the buffers: recorded, the row is dropped
             push_to.x = -1;
@@ -627,7 +629,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
 #pragma unroll
             for (int b = 0; b < 4; ++b) {
               if (col0 + b * 16 >= p.n) break;
-              const uint4 ga4 = __ldg(gp + 2 * b), gb4 = __ldg(gp + 2 * b + 1);
+              const uint4 ga4 = ld_dep(gp + 2 * b), gb4 = ld_dep(gp + 2 * b + 1);
               const uint32_t gw[8] = {ga4.x, ga4.y, ga4.z, ga4.w, gb4.x, gb4.y, gb4.z, gb4.w};
               float prod[16];
 #pragma unroll
@@ -847,17 +849,19 @@ int32_t launch_gemm(const char* op, const void* a, const void* b, const GemmPara
   cudaGetDevice(&dev);
   dev &= 63;
   std::lock_guard<std::mutex> configure_lock(configure_mutex);
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = 2;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg{};
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = C::kSmemBytes;
   cfg.stream = stream;
   cfg.attrs = attr;
-  cfg.numAttrs = kPair ? 1 : 0;
+  cfg.numAttrs = kPair ? 2 : 1;
   if (!configured[dev]) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
     if (e != cudaSuccess) return fail(GEMB_INTERNAL, "%s: %s: %s", op, cudaGetErrorName(e), cudaGetErrorString(e));

@@ -1,4 +1,4 @@
-// Mixture-of-experts routing path: router logits, softmax / top-k / renormalise, histogram +
+// Mixture-of-experts routing path behind the router logits (moe_router.cu): softmax / top-k / renormalise, histogram +
 // exclusive prefix + stable permutation of the (token, slot) assignments, quantise-and-dispatch
 // of expert inputs into the padded per-expert row layout the grouped GEMM consumes, and the
 // deterministic weighted combine.
@@ -20,10 +20,6 @@ namespace gemb {
 // in-range value, never dereferenced; gemb_check_device_status() reports and clears the word.
 __device__ int g_moe_error = 0;
 
-// Benchmark hook (GEMB_TUNE_ROUTER_TILE): 0 = automatic, 1 = expert-per-thread kernels wherever they
-// apply, 8 / 16 / 32 = the tiled kernel with that many tokens per CTA.  All give the same bits.
-int g_router_tile = 0;
-
 int moe_take_device_error() {
   int code = 0;
   if (cudaMemcpyFromSymbol(&code, g_moe_error, sizeof code) != cudaSuccess) {
@@ -38,282 +34,6 @@ int moe_take_device_error() {
 }
 
 namespace {
-
-// ---------------------------------------------------------------------------------------------
-// Router logits: logits[t][e] = fma(x[t][H-1], w[e][H-1], ... fma(x[t][0], w[e][0], bias[e])),
-// one fp32 fma per k in ascending k (the order is the contract; it rules out tensor cores and
-// K-splitting).  CTA = 32 tokens x 128 experts, 128 threads, thread = 8 tokens x 4 experts
-// (32 independent fma chains).  K is walked in shared-memory tiles of 32; the next tile's global
-// loads are issued into registers before the current tile is consumed.
-// ---------------------------------------------------------------------------------------------
-constexpr int kRtExp = 128, kRtK = 32, kRtThreads = 128;
-
-// kTok = tokens per CTA (64, 56 or 32 for prefill batches -- 64 halves the weight reads from shared memory per
-// fma, at 64 accumulators per thread; 56 is the same with 14 tokens per thread, for batches that 64-token
-// CTAs would spread unevenly over the SMs -- 8 for decode batches so that a few dozen tokens
-// still spread over many SMs).  Shared tiles are stored k-major with an xor swizzle of the column
-// (multiples of 4 / 8 keep each thread's float4 groups intact) so that both the transposing
-// stores and the float4 loads are bank-conflict free.
-template <int kTok>
-__global__ void __launch_bounds__(kRtThreads, kTok >= 56 ? 3 : 4)
-router_logits_kernel(const uint16_t* __restrict__ x, const float* __restrict__ w,
-                     const float* __restrict__ bias, float* __restrict__ logits, uint32_t tokens,
-                     uint32_t hidden, uint32_t experts) {
-  constexpr int kPerThread = kTok / 4;  // tokens per thread: 16, 14, 8, 4 or 2
-  // A warp's tokens occupy a slot of kSlot columns of the shared tile (kSlot = kPerThread rounded up to a
-  // multiple of four, so that the float4 reads stay aligned: 16 columns for the 14 tokens of the 56-token tile).
-  constexpr int kSlot = kPerThread >= 4 ? (kPerThread + 3) / 4 * 4 : kPerThread;
-  constexpr int kXCols = 4 * kSlot > 32 ? 4 * kSlot : 32;
-  constexpr int kXLoads = kTok > 32 ? (kTok + 31) / 32 : 1;   // staged 16-byte pieces of the token tile per thread
-  __shared__ __align__(16) float xs[kRtK][kXCols];
-  __shared__ __align__(16) float ws[kRtK][kRtExp];
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // experts tx*4.., tokens ty*kPerThread..
-  const uint32_t tok0 = blockIdx.x * kTok, exp0 = blockIdx.y * kRtExp;
-  float acc[kPerThread][4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const uint32_t e = exp0 + tx * 4 + j;
-    const float b = (bias != nullptr && e < experts) ? __ldg(bias + e) : 0.0f;
-#pragma unroll
-    for (int i = 0; i < kPerThread; ++i) acc[i][j] = b;
-  }
-  // Global -> register staging: X tile kTok tokens x 32 k bf16 = one uint4 per thread (token
-  // tid/4, k chunk (tid%4)*8); W tile 128 experts x 32 k fp32 = eight float4 per thread
-  // (expert tid/8 + 16 i, k chunk (tid%8)*4).
-  const int xt = threadIdx.x >> 2, xq = threadIdx.x & 3, xk = xq * 8;
-  const int we = threadIdx.x >> 3, wm = threadIdx.x & 7, wk = wm * 4;
-  uint4 xr[kXLoads];
-  float4 wr[8];
-  auto load_tile = [&](uint32_t k0) {
-#pragma unroll
-    for (int l = 0; l < kXLoads; ++l) {
-      xr[l] = make_uint4(0, 0, 0, 0);
-      const int tk = xt + 32 * l;   // token of the tile
-      if (tk < kTok && tok0 + tk < tokens) {
-        const uint16_t* src = x + static_cast<uint64_t>(tok0 + tk) * hidden + k0 + xk;
-        if (k0 + xk + 8 <= hidden) {
-          if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
-            xr[l] = __ldg(reinterpret_cast<const uint4*>(src));
-          } else {
-            const uint2 a = __ldg(reinterpret_cast<const uint2*>(src)), b2 = __ldg(reinterpret_cast<const uint2*>(src) + 1);
-            xr[l] = make_uint4(a.x, a.y, b2.x, b2.y);
-          }
-        } else if (k0 + xk + 4 <= hidden) {
-          const uint2 a = __ldg(reinterpret_cast<const uint2*>(src));
-          xr[l] = make_uint4(a.x, a.y, 0, 0);
-        }
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      wr[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-      const uint32_t e = exp0 + we + 16 * i;
-      if (e < experts && k0 + wk < hidden)
-        wr[i] = __ldg(reinterpret_cast<const float4*>(w + static_cast<uint64_t>(e) * hidden + k0 + wk));
-    }
-  };
-  auto store_tile = [&]() {
-#pragma unroll
-    for (int l = 0; l < kXLoads; ++l) {
-      const uint32_t xw[4] = {xr[l].x, xr[l].y, xr[l].z, xr[l].w};
-      const int tk = xt + 32 * l;
-      if (tk >= kTok) continue;
-      const int xcol = ((tk / kPerThread) * kSlot + tk % kPerThread) ^ (8 * xq);  // rows xk..xk+7 all have (k / 8) & 3 == xq
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        xs[xk + 2 * i][xcol] = __uint_as_float(xw[i] << 16);
-        xs[xk + 2 * i + 1][xcol] = __uint_as_float(xw[i] & 0xFFFF0000u);
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int col = (we + 16 * i) ^ (4 * wm);  // rows wk..wk+3 all have k / 4 == wm
-      ws[wk + 0][col] = wr[i].x;
-      ws[wk + 1][col] = wr[i].y;
-      ws[wk + 2][col] = wr[i].z;
-      ws[wk + 3][col] = wr[i].w;
-    }
-  };
-  load_tile(0);
-  for (uint32_t k0 = 0; k0 < hidden; k0 += kRtK) {
-    store_tile();
-    __syncthreads();
-    if (k0 + kRtK < hidden) load_tile(k0 + kRtK);
-    const uint32_t kmax = min(static_cast<uint32_t>(kRtK), hidden - k0);
-    // One k: four weights, kPerThread activations, kPerThread x 4 fma.  With four or eight tokens per
-    // thread two tokens share an instruction: the packed fp32 fma is one IEEE fma per half, so every
-    // chain keeps its order and rounding while the issue slots carry half the instructions.
-    auto step = [&](uint32_t k) {
-      const float4 wv4 = *reinterpret_cast<const float4*>(&ws[k][(tx * 4) ^ (4 * (k >> 2))]);
-      const float wv[4] = {wv4.x, wv4.y, wv4.z, wv4.w};
-      const int col = (ty * kPerThread) ^ (8 * ((k >> 3) & 3));
-      if constexpr (kPerThread >= 4) {
-        float2 xp[kPerThread / 2];
-#pragma unroll
-        for (int q = 0; q < kSlot / 4; ++q) {   // the swizzle moves groups of eight columns: a group of four stays whole
-          const float4 xa = *reinterpret_cast<const float4*>(&xs[k][(ty * kSlot + 4 * q) ^ (8 * ((k >> 3) & 3))]);
-          xp[2 * q] = make_float2(xa.x, xa.y);
-          if (2 * q + 1 < kPerThread / 2) xp[2 * q + 1] = make_float2(xa.z, xa.w);
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 wp = make_float2(wv[j], wv[j]);
-#pragma unroll
-          for (int i = 0; i < kPerThread / 2; ++i) {
-            const float2 r = __ffma2_rn(xp[i], wp, make_float2(acc[2 * i][j], acc[2 * i + 1][j]));
-            acc[2 * i][j] = r.x;
-            acc[2 * i + 1][j] = r.y;
-          }
-        }
-      } else {
-        const float2 xa = *reinterpret_cast<const float2*>(&xs[k][col]);
-        const float xv[2] = {xa.x, xa.y};
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(xv[i], wv[j], acc[i][j]);
-      }
-    };
-    if (kmax == kRtK) {
-#pragma unroll
-      for (uint32_t k = 0; k < kRtK; ++k) step(k);
-    } else {
-#pragma unroll 4
-      for (uint32_t k = 0; k < kmax; ++k) step(k);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < kPerThread; ++i) {
-    const uint32_t t = tok0 + ty * kPerThread + i;
-    if (t >= tokens) continue;
-    float* dst = logits + static_cast<uint64_t>(t) * experts + exp0 + tx * 4;
-    if (exp0 + tx * 4 + 4 <= experts && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-      *reinterpret_cast<float4*>(dst) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (exp0 + tx * 4 + j < experts) dst[j] = acc[i][j];
-    }
-  }
-}
-
-// Decode-size and small-batch form of the same contract.  With few tokens the tile above leaves
-// most SMs idle (one CTA per 8 or 32 tokens, each walking all of K).  Here a thread owns ONE
-// expert and kTpt tokens (kTpt independent fma chains), a warp 32 experts, a CTA of two warps
-// 2 * kTpt tokens of the same 32 experts.  K is walked in tiles of 128.  The chain over k is
-// serial, so a tile's arithmetic (about 600 clocks) is all there is to hide a load behind, and
-// an L2 round trip takes longer than that: the CTA's weight tiles (32 experts x 128 k, fetched
-// as coalesced 16-byte cp.async pieces) and the tokens' raw bf16 activations therefore run
-// through a ring of kRsDepth shared-memory buffers, three tiles ahead of the arithmetic.  Same
-// chain, same order: bias, then one fma per k ascending.
-constexpr int kRsK = 128, kRsThreads = 64, kRsPad = 4, kRsDepth = 4;
-
-__device__ __forceinline__ void cp_async_16(void* smem_dst, const void* src, bool valid) {
-  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst));
-  const uint32_t n = valid ? 16u : 0u;   // 0 source bytes: the destination is zero filled
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
-}
-__device__ __forceinline__ void cp_async_8(void* smem_dst, const void* src, bool valid) {
-  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst));
-  const uint32_t n = valid ? 8u : 0u;
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int kPending>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory"); }
-
-template <int kTpt>
-struct RouterSmallSmem {
-  static constexpr int kTokCta = 2 * kTpt;
-  float ws[kRsDepth][32][kRsK + kRsPad];     // row stride 132 words: float4 reads of one k by 32 rows are conflict free
-  uint16_t xraw[kRsDepth][kTokCta][kRsK];    // bf16 as loaded
-  float xs[kTokCta][kRsK];                   // the current tile's activations as fp32
-};
-
-template <int kTpt>
-__global__ void __launch_bounds__(kRsThreads)
-router_logits_small_kernel(const uint16_t* __restrict__ x, const float* __restrict__ w,
-                           const float* __restrict__ bias, float* __restrict__ logits, uint32_t tokens,
-                           uint32_t hidden, uint32_t experts) {
-  constexpr int kTokCta = 2 * kTpt;
-  extern __shared__ __align__(16) uint8_t router_small_smem[];
-  auto& sm = *reinterpret_cast<RouterSmallSmem<kTpt>*>(router_small_smem);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t tok0 = blockIdx.x * kTokCta, exp0 = blockIdx.y * 32;
-  const uint32_t e = exp0 + lane;
-  const bool live = e < experts;
-  float acc[kTpt];
-  const float b = (bias != nullptr && live) ? __ldg(bias + e) : 0.0f;
-#pragma unroll
-  for (int i = 0; i < kTpt; ++i) acc[i] = b;
-  const uint32_t tiles = (hidden + kRsK - 1) / kRsK;
-  // Warp `warp` fetches rows warp*16 .. warp*16+15 of the weight tile (lane = 16-byte piece of the
-  // row); the activation tile is kTokCta rows of 32 eight-byte pieces shared out over the CTA.
-  auto issue_tile = [&](uint32_t t) {
-    if (t < tiles) {
-      const uint32_t k0 = t * kRsK, buf = t % kRsDepth;
-      const uint32_t kmax = min(static_cast<uint32_t>(kRsK), hidden - k0);   // a multiple of 4
-#pragma unroll
-      for (int r = 0; r < 16; ++r) {
-        const uint32_t row = exp0 + warp * 16 + r;
-        const bool ok = row < experts && static_cast<uint32_t>(lane) * 4 < kmax;
-        const float* src = w + static_cast<uint64_t>(ok ? row : 0) * hidden + (ok ? k0 + lane * 4 : 0);
-        cp_async_16(&sm.ws[buf][warp * 16 + r][lane * 4], src, ok);
-      }
-#pragma unroll
-      for (int q = 0; q < kTokCta * 32 / kRsThreads; ++q) {
-        const uint32_t idx = threadIdx.x + q * kRsThreads;
-        const uint32_t tk = idx / 32, c = (idx % 32) * 4;
-        const bool ok = tok0 + tk < tokens && c < kmax;
-        const uint16_t* src = x + static_cast<uint64_t>(ok ? tok0 + tk : 0) * hidden + (ok ? k0 + c : 0);
-        cp_async_8(&sm.xraw[buf][tk][c], src, ok);
-      }
-    }
-    cp_async_commit();   // one group per call, empty past the last tile, so the counting stays uniform
-  };
-#pragma unroll
-  for (int t = 0; t < kRsDepth - 1; ++t) issue_tile(t);
-  for (uint32_t t = 0; t < tiles; ++t) {
-    const uint32_t buf = t % kRsDepth;
-    const uint32_t groups = min(static_cast<uint32_t>(kRsK), hidden - t * kRsK) / 4;
-    cp_async_wait<kRsDepth - 2>();   // this thread's pieces of tile t have landed
-    __syncthreads();                 // everyone's have; and tile t-1 has been consumed
-    issue_tile(t + kRsDepth - 1);    // refills the buffer tile t-1 used
-    for (uint32_t idx = threadIdx.x; idx < kTokCta * (kRsK / 4); idx += kRsThreads) {
-      const uint32_t tk = idx / (kRsK / 4), c = (idx % (kRsK / 4)) * 4;
-      const uint2 raw = *reinterpret_cast<const uint2*>(&sm.xraw[buf][tk][c]);
-      *reinterpret_cast<float4*>(&sm.xs[tk][c]) =
-          make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xFFFF0000u),
-                      __uint_as_float(raw.y << 16), __uint_as_float(raw.y & 0xFFFF0000u));
-    }
-    __syncthreads();
-#pragma unroll 8
-    for (uint32_t g = 0; g < groups; ++g) {
-      const float4 wv = *reinterpret_cast<const float4*>(&sm.ws[buf][lane][g * 4]);
-      float4 xv[kTpt];
-#pragma unroll
-      for (int i = 0; i < kTpt; ++i) xv[i] = *reinterpret_cast<const float4*>(&sm.xs[warp * kTpt + i][g * 4]);
-      // k-major: the kTpt chains advance together, so consecutive instructions are independent
-      // (a chain's own steps are four clocks apart at best).
-#pragma unroll
-      for (int i = 0; i < kTpt; ++i) acc[i] = fmaf(xv[i].x, wv.x, acc[i]);
-#pragma unroll
-      for (int i = 0; i < kTpt; ++i) acc[i] = fmaf(xv[i].y, wv.y, acc[i]);
-#pragma unroll
-      for (int i = 0; i < kTpt; ++i) acc[i] = fmaf(xv[i].z, wv.z, acc[i]);
-#pragma unroll
-      for (int i = 0; i < kTpt; ++i) acc[i] = fmaf(xv[i].w, wv.w, acc[i]);
-    }
-  }
-  cp_async_wait<0>();
-  if (!live) return;
-#pragma unroll
-  for (int i = 0; i < kTpt; ++i) {
-    const uint32_t t = tok0 + warp * kTpt + i;
-    if (t < tokens) logits[static_cast<uint64_t>(t) * experts + e] = acc[i];
-  }
-}
 
 // ---------------------------------------------------------------------------------------------
 // Softmax over all experts, top-k with the lower id winning ties, renormalise, optional
@@ -343,22 +63,24 @@ __device__ __forceinline__ float det_exp(float x) {
 constexpr int kMaxPerLane = 8;  // up to 256 experts
 
 __global__ void __launch_bounds__(128)
-route_kernel(const float* __restrict__ logits, const float* __restrict__ per_expert_scale,
+route_kernel(const float* logits, const float* __restrict__ per_expert_scale,
              int32_t* __restrict__ ids, float* __restrict__ weights, float* __restrict__ probs,
              uint32_t tokens, uint32_t experts, uint32_t topk) {
+  pdl_trigger();
+  pdl_wait();
   const uint32_t t = blockIdx.x * 4 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (t >= tokens) return;
   const int per_lane = static_cast<int>(experts / 32);
   const float* lg = logits + static_cast<uint64_t>(t) * experts;
   float p[kMaxPerLane];
-  float m = __ldg(lg + lane);
+  float m = ld_dep(lg + lane);
   p[0] = m;
   bool finite = isfinite(m);
 #pragma unroll
   for (int j = 1; j < kMaxPerLane; ++j) {
     if (j < per_lane) {
-      p[j] = __ldg(lg + lane + 32 * j);
+      p[j] = ld_dep(lg + lane + 32 * j);
       finite = finite && isfinite(p[j]);
       m = fmaxf(m, p[j]);
     }
@@ -408,15 +130,11 @@ route_kernel(const float* __restrict__ logits, const float* __restrict__ per_exp
         best_id = lane + 32 * j;
       }
     }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-      const float ob = __shfl_xor_sync(0xFFFFFFFFu, best, o);
-      const int oi = __shfl_xor_sync(0xFFFFFFFFu, best_id, o);
-      if (ob > best || (ob == best && oi < best_id)) {
-        best = ob;
-        best_id = oi;
-      }
-    }
+    // Probabilities are >= 0 and taken entries -1: their bit patterns order as signed integers.  The largest one over the
+    // warp, then the lowest id that has it: two warp reductions instead of ten shuffles and as many selects.
+    const int top = __reduce_max_sync(0xFFFFFFFFu, __float_as_int(best));
+    best_id = __reduce_min_sync(0xFFFFFFFFu, __float_as_int(best) == top ? best_id : 0x7FFFFFFF);
+    best = __int_as_float(top);
     if ((best_id & 31) == lane) {
 #pragma unroll
       for (int j = 0; j < kMaxPerLane; ++j)
@@ -451,15 +169,23 @@ constexpr int kSegment = 1024;  // assignments per CTA: 4 warps x 8 chunks x 32
 constexpr int kRowAlign = 256;  // every expert's padded rows start on a multiple of this
 
 __global__ void __launch_bounds__(128)
-permute_count_kernel(const int32_t* __restrict__ ids, int32_t* __restrict__ block_counts,
-                     uint32_t total, uint32_t experts) {
+permute_count_kernel(const int32_t* ids, int32_t* __restrict__ block_counts, uint32_t total, uint32_t experts) {
   extern __shared__ int smem_counts[];
+  pdl_trigger();
   for (uint32_t e = threadIdx.x; e < experts; e += 128) smem_counts[e] = 0;
+  pdl_wait();
   __syncthreads();
   const uint32_t base = blockIdx.x * kSegment;
-  for (uint32_t i = threadIdx.x; i < kSegment; i += 128) {
-    if (base + i >= total) continue;
-    uint32_t e = static_cast<uint32_t>(__ldg(ids + base + i));
+  uint32_t mine[kSegment / 128];
+#pragma unroll
+  for (int c = 0; c < kSegment / 128; ++c) {
+    const uint32_t i = base + threadIdx.x + c * 128;
+    if (i < total) mine[c] = static_cast<uint32_t>(ld_dep(ids + i));
+  }
+#pragma unroll
+  for (int c = 0; c < kSegment / 128; ++c) {
+    if (base + threadIdx.x + c * 128 >= total) continue;
+    uint32_t e = mine[c];
     if (e >= experts) {   // recorded, and counted under the last expert so that every position stays in range
       atomicCAS(&g_moe_error, 0, 2);
       e = experts - 1;
@@ -471,59 +197,57 @@ permute_count_kernel(const int32_t* __restrict__ ids, int32_t* __restrict__ bloc
     block_counts[static_cast<uint64_t>(blockIdx.x) * experts + e] = smem_counts[e];
 }
 
+// From the experts' counts (shared memory, cnt[experts]) to their offsets, padded offsets and first entries in the list
+// of real tiles (off / poff / loff, [experts + 1] each), and the plan.  All threads of the CTA together: a scan over
+// the experts by warp shuffles, then one thread per tile.  `totals` holds 3 x 33 ints.
 // plan layout (int32): [0] number T of 128-row tiles, [1] padded rows in total, [2 .. 2+E] padded
 // offset of every expert (+ the end), then T pairs {expert of tile i (-1: padding only), i-th tile
 // that holds real rows (what a single-CTA grouped GEMM walks)}, then the number of such tiles.
-__global__ void __launch_bounds__(256)
-permute_scan_kernel(int32_t* __restrict__ block_counts, int32_t* __restrict__ counts,
-                    int32_t* __restrict__ offsets, int32_t* __restrict__ plan, uint32_t segments,
-                    uint32_t experts, uint32_t max_tiles) {
-  extern __shared__ int sm[];
-  int* cnt = sm;                 // [experts]
-  int* off = sm + experts;       // [experts + 1]
-  int* poff = off + experts + 1; // [experts + 1]
-  int* loff = poff + experts + 1; // [experts + 1] first entry of the expert in the list of real tiles
-  for (uint32_t e = threadIdx.x; e < experts; e += blockDim.x) {
-    int run = 0;
-    // sixteen loads in flight at a time: a thread that consumes each count before it asks for the
-    // next one waits a full memory round trip per segment
-    for (uint32_t b0 = 0; b0 < segments; b0 += 16) {
-      int c[16];
+__device__ __forceinline__ void plan_from_counts(const int* cnt, int* off, int* poff, int* loff, int* totals, uint32_t experts,
+                                                 int32_t* __restrict__ counts, int32_t* __restrict__ offsets, int32_t* __restrict__ plan) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  int carry[3] = {0, 0, 0};
+  for (uint32_t e0 = 0; e0 < experts; e0 += blockDim.x) {
+    const uint32_t e = e0 + threadIdx.x;
+    const int c = e < experts ? cnt[e] : 0;
+    const int v[3] = {c, (c + kRowAlign - 1) / kRowAlign * kRowAlign, (c + 127) / 128};
+    int incl[3];
 #pragma unroll
-      for (int j = 0; j < 16; ++j)
-        c[j] = b0 + j < segments ? block_counts[static_cast<uint64_t>(b0 + j) * experts + e] : 0;
+    for (int q = 0; q < 3; ++q) {
+      int x = v[q];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        if (b0 + j < segments) block_counts[static_cast<uint64_t>(b0 + j) * experts + e] = run;  // exclusive prefix over segments
-        run += c[j];
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+        if (lane >= o) x += y;
+      }
+      incl[q] = x;
+      if (lane == 31) totals[q * 33 + warp] = x;
+    }
+    __syncthreads();
+    int before[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      before[q] = carry[q];
+      for (int w = 0; w < warps; ++w) {
+        const int t = totals[q * 33 + w];
+        if (w < warp) before[q] += t;
+        carry[q] += t;
       }
     }
-    cnt[e] = run;
-    counts[e] = run;
+    if (e < experts) {
+      off[e] = before[0] + incl[0] - v[0];
+      poff[e] = before[1] + incl[1] - v[1];
+      loff[e] = before[2] + incl[2] - v[2];
+      counts[e] = c;
+    }
+    __syncthreads();
   }
-  __syncthreads();
   if (threadIdx.x == 0) {
-    int o = 0, po = 0, lo = 0;
-    for (uint32_t e0 = 0; e0 < experts; e0 += 8) {   // eight counts at a time: one add per expert instead of one shared-memory round trip
-      int c[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) c[j] = e0 + j < experts ? cnt[e0 + j] : 0;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        if (e0 + j >= experts) break;
-        off[e0 + j] = o;
-        poff[e0 + j] = po;
-        loff[e0 + j] = lo;
-        o += c[j];
-        po += (c[j] + kRowAlign - 1) / kRowAlign * kRowAlign;
-        lo += (c[j] + 127) / 128;
-      }
-    }
-    off[experts] = o;
-    poff[experts] = po;
-    plan[0] = po / 128;
-    plan[1] = po;
-    plan[3 + experts + 2 * (po / 128)] = lo;
+    off[experts] = carry[0];
+    poff[experts] = carry[1];
+    plan[0] = carry[1] / 128;
+    plan[1] = carry[1];
+    plan[3 + experts + 2 * (carry[1] / 128)] = carry[2];
   }
   __syncthreads();
   for (uint32_t e = threadIdx.x; e <= experts; e += blockDim.x) {
@@ -531,30 +255,88 @@ permute_scan_kernel(int32_t* __restrict__ block_counts, int32_t* __restrict__ co
     plan[2 + e] = poff[e];
   }
   int32_t* info = plan + 3 + experts;
-  for (uint32_t e = threadIdx.x; e < experts; e += blockDim.x)
-    for (int tile = poff[e] / 128, j = 0; tile < poff[e + 1] / 128; ++tile, ++j) {
-      const bool real = tile * 128 - poff[e] < cnt[e];
-      info[2 * tile] = real ? static_cast<int32_t>(e) : -1;
-      if (real) info[2 * (loff[e] + j) + 1] = tile;
+  for (int tile = threadIdx.x; tile < carry[1] / 128; tile += blockDim.x) {
+    uint32_t lo = 0, hi = experts;   // the last expert whose padded rows start at or before the tile owns it
+    while (hi - lo > 1) {
+      const uint32_t mid = (lo + hi) / 2;
+      if (poff[mid] <= tile * 128) lo = mid;
+      else hi = mid;
     }
+    const int j = tile - poff[lo] / 128;
+    const bool real = j * 128 < cnt[lo];
+    info[2 * tile] = real ? static_cast<int32_t>(lo) : -1;
+    if (real) info[2 * (loff[lo] + j) + 1] = tile;
+  }
+}
+
+constexpr int kScanThreads = 1024;
+uint32_t permute_scan_smem(uint32_t experts) { return (4 * experts + 3 + 3 * 33 + kScanThreads) * sizeof(int); }
+__global__ void __launch_bounds__(kScanThreads)
+permute_scan_kernel(int32_t* block_counts, int32_t* __restrict__ counts, int32_t* __restrict__ offsets, int32_t* __restrict__ plan,
+                    uint32_t segments, uint32_t experts) {
+  extern __shared__ int sm[];
+  int* cnt = sm;                  // [experts]
+  int* off = sm + experts;        // [experts + 1]
+  int* poff = off + experts + 1;
+  int* loff = poff + experts + 1;
+  int* totals = loff + experts + 1;
+  int* group_sum = totals + 3 * 33;   // [groups][experts]
+  pdl_trigger();
+  pdl_wait();
+  // Exclusive prefix over the segments, per expert: `groups` threads per expert take contiguous shares of the
+  // segments, sixteen loads in flight each.
+  const uint32_t groups = kScanThreads / experts, share = (segments + groups - 1) / groups;
+  const uint32_t e = threadIdx.x % experts, grp = threadIdx.x / experts;
+  const uint32_t b_lo = min(segments, grp * share), b_hi = grp < groups ? min(segments, b_lo + share) : b_lo;
+  int sum = 0;
+  for (uint32_t b0 = b_lo; b0 < b_hi; b0 += 16) {
+    int c[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) c[j] = b0 + j < b_hi ? ld_dep(block_counts + static_cast<uint64_t>(b0 + j) * experts + e) : 0;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) sum += c[j];
+  }
+  if (grp < groups) group_sum[grp * experts + e] = sum;
+  __syncthreads();
+  int run = 0;
+  if (grp < groups)
+    for (uint32_t q = 0; q < grp; ++q) run += group_sum[q * experts + e];
+  if (grp + 1 == groups) cnt[e] = run + sum;
+  for (uint32_t b0 = b_lo; b0 < b_hi; b0 += 16) {
+    int c[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) c[j] = b0 + j < b_hi ? ld_dep(block_counts + static_cast<uint64_t>(b0 + j) * experts + e) : 0;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      if (b0 + j < b_hi) block_counts[static_cast<uint64_t>(b0 + j) * experts + e] = run;
+      run += c[j];
+    }
+  }
+  __syncthreads();
+  plan_from_counts(cnt, off, poff, loff, totals, experts, counts, offsets, plan);
 }
 
 __global__ void __launch_bounds__(128)
-permute_scatter_kernel(const int32_t* __restrict__ ids, const int32_t* __restrict__ block_prefix,
-                       const int32_t* __restrict__ offsets, const int32_t* __restrict__ plan,
+permute_scatter_kernel(const int32_t* ids, const int32_t* block_prefix, const int32_t* offsets, const int32_t* plan,
                        int32_t* __restrict__ perm, int32_t* __restrict__ slot_rows, uint32_t total,
                        uint32_t experts) {
   extern __shared__ int sm[];
   int* warp_counts = sm;  // [4][experts], becomes each warp's running base
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  pdl_trigger();
   for (uint32_t i = threadIdx.x; i < 4 * experts; i += 128) warp_counts[i] = 0;
+  pdl_wait();
   __syncthreads();
   const uint32_t base = blockIdx.x * kSegment + warp * 256;
   int my_ids[8];
 #pragma unroll
   for (int c = 0; c < 8; ++c) {
     const uint32_t i = base + c * 32 + lane;
-    my_ids[c] = i < total ? __ldg(ids + i) : -1;
+    my_ids[c] = i < total ? ld_dep(ids + i) : -1;
+  }
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    const uint32_t i = base + c * 32 + lane;
     if (i < total && static_cast<uint32_t>(my_ids[c]) >= experts)
       my_ids[c] = static_cast<int>(experts) - 1;   // same clamp as the count kernel, which recorded it
     if (my_ids[c] >= 0) atomicAdd(&warp_counts[warp * experts + my_ids[c]], 1);
@@ -562,7 +344,7 @@ permute_scatter_kernel(const int32_t* __restrict__ ids, const int32_t* __restric
   __syncthreads();
   // exclusive prefix over the four warps, plus the segment's own prefix
   for (uint32_t e = threadIdx.x; e < experts; e += 128) {
-    int run = block_prefix[static_cast<uint64_t>(blockIdx.x) * experts + e];
+    int run = ld_dep(block_prefix + static_cast<uint64_t>(blockIdx.x) * experts + e);
     for (int wq = 0; wq < 4; ++wq) {
       const int c = warp_counts[wq * experts + e];
       warp_counts[wq * experts + e] = run;
@@ -580,8 +362,8 @@ permute_scatter_kernel(const int32_t* __restrict__ ids, const int32_t* __restric
       const int rank = __popc(peers & ((1u << lane) - 1));
       const int within = running[e] + rank;  // position inside the expert
       const uint32_t i = base + c * 32 + lane;
-      perm[__ldg(offsets + e) + within] = static_cast<int32_t>(i);
-      slot_rows[i] = __ldg(plan + 2 + e) + within;
+      perm[ld_dep(offsets + e) + within] = static_cast<int32_t>(i);
+      slot_rows[i] = ld_dep(plan + 2 + e) + within;
       __syncwarp(active);
       if (rank == 0) running[e] += __popc(peers);
     }
@@ -592,23 +374,30 @@ permute_scatter_kernel(const int32_t* __restrict__ ids, const int32_t* __restric
 // The three steps above in ONE launch of one CTA, for batches of at most kSegment assignments (the
 // decode-size layer, where three launches cost more than the work): same records, same order.
 __global__ void __launch_bounds__(128)
-permute_small_kernel(const int32_t* __restrict__ ids, int32_t* __restrict__ counts, int32_t* __restrict__ offsets,
+permute_small_kernel(const int32_t* ids, int32_t* __restrict__ counts, int32_t* __restrict__ offsets,
                      int32_t* __restrict__ plan, int32_t* __restrict__ perm, int32_t* __restrict__ slot_rows,
-                     uint32_t total, uint32_t experts, uint32_t max_tiles) {
+                     uint32_t total, uint32_t experts) {
   extern __shared__ int sm[];
   int* cnt = sm;                        // [experts]
   int* off = cnt + experts;             // [experts + 1]
   int* poff = off + experts + 1;        // [experts + 1]
   int* loff = poff + experts + 1;       // [experts + 1]
-  int* warp_counts = loff + experts + 1;  // [4][experts]
+  int* totals = loff + experts + 1;     // [3 * 33]
+  int* warp_counts = totals + 3 * 33;   // [4][experts]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  pdl_trigger();
   for (uint32_t i = threadIdx.x; i < 5 * experts; i += 128) (i < experts ? cnt[i] : warp_counts[i - experts]) = 0;
+  pdl_wait();
   __syncthreads();
   int my_ids[8];
 #pragma unroll
   for (int c = 0; c < 8; ++c) {
     const uint32_t i = warp * 256 + c * 32 + lane;
-    my_ids[c] = i < total ? __ldg(ids + i) : -1;
+    my_ids[c] = i < total ? ld_dep(ids + i) : -1;
+  }
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    const uint32_t i = warp * 256 + c * 32 + lane;
     if (i < total && static_cast<uint32_t>(my_ids[c]) >= experts) {
       atomicCAS(&g_moe_error, 0, 2);
       my_ids[c] = static_cast<int>(experts) - 1;
@@ -619,41 +408,8 @@ permute_small_kernel(const int32_t* __restrict__ ids, int32_t* __restrict__ coun
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int o = 0, po = 0, lo = 0;
-    for (uint32_t e0 = 0; e0 < experts; e0 += 8) {   // eight counts at a time, as in permute_scan_kernel
-      int c[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) c[j] = e0 + j < experts ? cnt[e0 + j] : 0;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        if (e0 + j >= experts) break;
-        off[e0 + j] = o;
-        poff[e0 + j] = po;
-        loff[e0 + j] = lo;
-        o += c[j];
-        po += (c[j] + kRowAlign - 1) / kRowAlign * kRowAlign;
-        lo += (c[j] + 127) / 128;
-      }
-    }
-    off[experts] = o;
-    poff[experts] = po;
-    plan[0] = po / 128;
-    plan[1] = po;
-    plan[3 + experts + 2 * (po / 128)] = lo;
-  }
-  __syncthreads();
-  int32_t* info = plan + 3 + experts;
-  for (uint32_t e = threadIdx.x; e <= experts; e += 128) {
-    offsets[e] = off[e];
-    plan[2 + e] = poff[e];
-    if (e == experts) break;
-    counts[e] = cnt[e];
-    for (int tile = poff[e] / 128, j = 0; tile < poff[e + 1] / 128; ++tile, ++j) {
-      const bool real = tile * 128 - poff[e] < cnt[e];
-      info[2 * tile] = real ? static_cast<int32_t>(e) : -1;
-      if (real) info[2 * (loff[e] + j) + 1] = tile;
-    }
+  plan_from_counts(cnt, off, poff, loff, totals, experts, counts, offsets, plan);
+  for (uint32_t e = threadIdx.x; e < experts; e += 128) {
     int run = 0;   // exclusive prefix of the expert over the four warps
     for (int wq = 0; wq < 4; ++wq) {
       const int c = warp_counts[wq * experts + e];
@@ -688,20 +444,22 @@ permute_small_kernel(const int32_t* __restrict__ ids, int32_t* __restrict__ coun
 // ---------------------------------------------------------------------------------------------
 constexpr uint32_t kDispatchMaxBlocks = 1024;   // 16-element blocks of a token whose scales are staged in shared memory
 __global__ void __launch_bounds__(256)
-dispatch_quantize_kernel(const uint16_t* __restrict__ x, const int32_t* __restrict__ slot_rows,
+dispatch_quantize_kernel(const uint16_t* x, const int32_t* slot_rows,
                          uint8_t* __restrict__ packed, uint8_t* __restrict__ scales, uint32_t hidden,
                          uint32_t topk, float g, uint32_t c_pad) {
+  pdl_trigger();
+  pdl_wait();
   const uint32_t t = blockIdx.x;
   __shared__ int rows[32];
   // The token's scale bytes meet here, so that they leave as 4-byte words (four consecutive K blocks are
   // contiguous in the interleaved layout) instead of one byte store per block and assignment.
   __shared__ __align__(4) uint8_t token_scales[kDispatchMaxBlocks];
   const bool words = hidden / 16 <= kDispatchMaxBlocks && (hidden / 16) % 4 == 0;
-  if (threadIdx.x < topk) rows[threadIdx.x] = __ldg(slot_rows + static_cast<uint64_t>(t) * topk + threadIdx.x);
+  if (threadIdx.x < topk) rows[threadIdx.x] = ld_dep(slot_rows + static_cast<uint64_t>(t) * topk + threadIdx.x);
   __syncthreads();
   for (uint32_t c = threadIdx.x; c < hidden / 16; c += blockDim.x) {
     const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<uint64_t>(t) * hidden + c * 16);
-    const uint4 a = __ldg(src), b = __ldg(src + 1);
+    const uint4 a = ld_dep(src), b = ld_dep(src + 1);
     const uint32_t ww[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
     float v[16];
 #pragma unroll
@@ -806,9 +564,10 @@ scatter_quantized_kernel(const uint8_t* __restrict__ payload, const uint8_t* __r
 // One thread per 8 output columns.
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-combine_kernel(const uint16_t* __restrict__ y, const int32_t* __restrict__ slot_rows,
-               const float* __restrict__ weights, const uint16_t* __restrict__ shared_out,
+combine_kernel(const uint16_t* y, const int32_t* slot_rows, const float* weights, const uint16_t* shared_out,
                uint16_t* __restrict__ out, uint32_t tokens, uint32_t hidden, uint32_t topk) {
+  pdl_trigger();
+  pdl_wait();
   const uint32_t chunks = hidden / 8;
   const uint64_t idx = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= static_cast<uint64_t>(tokens) * chunks) return;
@@ -816,20 +575,31 @@ combine_kernel(const uint16_t* __restrict__ y, const int32_t* __restrict__ slot_
   float acc[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) acc[i] = 0.0f;
-  for (uint32_t s = 0; s < topk; ++s) {
-    const float wv = __ldg(weights + static_cast<uint64_t>(t) * topk + s);
-    const int64_t r = slot_rows ? static_cast<int64_t>(__ldg(slot_rows + static_cast<uint64_t>(t) * topk + s))
-                                : static_cast<int64_t>(t) * topk + s;
-    const uint4 v = __ldg(reinterpret_cast<const uint4*>(y + r * hidden) + c);
-    const uint32_t ww[4] = {v.x, v.y, v.z, v.w};
+  // eight slots' rows in flight at a time, added in slot order
+  for (uint32_t s0 = 0; s0 < topk; s0 += 8) {
+    float wv[8];
+    uint4 v[8];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      acc[2 * i] = fmaf(wv, __uint_as_float(ww[i] << 16), acc[2 * i]);
-      acc[2 * i + 1] = fmaf(wv, __uint_as_float(ww[i] & 0xFFFF0000u), acc[2 * i + 1]);
+    for (int s = 0; s < 8; ++s) {
+      if (s0 + s >= topk) break;
+      const uint64_t slot = static_cast<uint64_t>(t) * topk + s0 + s;
+      wv[s] = ld_dep(weights + slot);
+      const int64_t r = slot_rows ? static_cast<int64_t>(ld_dep(slot_rows + slot)) : static_cast<int64_t>(slot);
+      v[s] = ld_dep(reinterpret_cast<const uint4*>(y + r * hidden) + c);
+    }
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+      if (s0 + s >= topk) break;
+      const uint32_t ww[4] = {v[s].x, v[s].y, v[s].z, v[s].w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        acc[2 * i] = fmaf(wv[s], __uint_as_float(ww[i] << 16), acc[2 * i]);
+        acc[2 * i + 1] = fmaf(wv[s], __uint_as_float(ww[i] & 0xFFFF0000u), acc[2 * i + 1]);
+      }
     }
   }
   if (shared_out) {
-    const uint4 v = __ldg(reinterpret_cast<const uint4*>(shared_out + static_cast<uint64_t>(t) * hidden) + c);
+    const uint4 v = ld_dep(reinterpret_cast<const uint4*>(shared_out + static_cast<uint64_t>(t) * hidden) + c);
     const uint32_t ww[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -864,22 +634,6 @@ int32_t validate_permute_geometry(const char* op, uint64_t tokens, uint64_t expe
   return GEMB_OK;
 }
 
-// The small-batch router kernel's ring needs more than the 48 KB a kernel gets without opting in.
-template <int kTpt>
-int32_t router_small_configure(const char* op) {
-  static std::atomic<bool> configured[64];   // racing first calls both set the (idempotent) attribute
-  int dev = 0;
-  cudaGetDevice(&dev);
-  dev &= 63;
-  if (!configured[dev].load(std::memory_order_acquire)) {
-    cudaError_t e = cudaFuncSetAttribute(router_logits_small_kernel<kTpt>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(sizeof(RouterSmallSmem<kTpt>)));
-    if (e != cudaSuccess) return fail(GEMB_INTERNAL, "%s: %s: %s", op, cudaGetErrorName(e), cudaGetErrorString(e));
-    configured[dev].store(true, std::memory_order_release);
-  }
-  return GEMB_OK;
-}
-
 int32_t validate_moe_geometry(const char* op, uint64_t tokens, uint64_t experts, uint64_t topk) {
   GEMB_REQUIRE(tokens > 0 && tokens * topk < (1ull << 31), "%s: token count must be nonzero and fit 31 bits", op);
   GEMB_REQUIRE(experts >= 32 && experts % 32 == 0 && experts <= 256, "%s: experts must be a multiple of 32 in [32, 256]", op);
@@ -888,86 +642,19 @@ int32_t validate_moe_geometry(const char* op, uint64_t tokens, uint64_t experts,
 }
 }  // namespace
 
-extern "C" {
-
-int32_t gemb_moe_router_logits(const uint16_t* x_bf16, const float* router_weight, const float* bias,
-                               float* logits, uint64_t tokens, uint64_t hidden, uint64_t experts,
-                               gemb_stream_t stream) {
-  const char* op = "gemb_moe_router_logits";
-  GEMB_REQUIRE(x_bf16 && router_weight && logits, "%s: pointers must be nonnull", op);
-  GEMB_REQUIRE(tokens > 0 && tokens < (1ull << 31) && experts > 0 && experts < (1ull << 20), "%s: bad geometry", op);
-  GEMB_REQUIRE(hidden > 0 && hidden % 4 == 0 && hidden < (1ull << 31), "%s: hidden must be a nonzero multiple of 4", op);
-  GEMB_REQUIRE(reinterpret_cast<uintptr_t>(x_bf16) % 8 == 0 && reinterpret_cast<uintptr_t>(router_weight) % 16 == 0,
-               "%s: activations must be 8-byte and router weights 16-byte aligned", op);
-  GEMB_ENTER(op);
-  // Up to a thousand tokens: one expert per thread, weight rows streamed from L2 (the tiled kernel
-  // would occupy a fraction of the SMs).  Its L2 traffic grows with the token count (one pass over
-  // the router weight per 2 * kTpt tokens), so larger batches use the tiled kernel.  Measured on
-  // 2,816 x 128: 25 / 31 / 43 / 56 us at 64 / 256 / 512 / 1,024 tokens here, against 64 us for the
-  // tiled kernel; at 2,048 tokens 105 us against 72 us for the 16-token tile.
-  if ((tokens <= 1024 && g_router_tile == 0) || (tokens <= 2048 && g_router_tile == 1)) {
-    if (tokens <= 256) {
-      dim3 g(static_cast<unsigned>((tokens + 3) / 4), static_cast<unsigned>((experts + 31) / 32));
-      GEMB_TRY(router_small_configure<2>(op));
-      router_logits_small_kernel<2><<<g, kRsThreads, sizeof(RouterSmallSmem<2>), stream>>>(x_bf16, router_weight, bias, logits,
-                                                                   static_cast<uint32_t>(tokens), static_cast<uint32_t>(hidden),
-                                                                   static_cast<uint32_t>(experts));
-    } else if (tokens <= 512) {
-      dim3 g(static_cast<unsigned>((tokens + 7) / 8), static_cast<unsigned>((experts + 31) / 32));
-      GEMB_TRY(router_small_configure<4>(op));
-      router_logits_small_kernel<4><<<g, kRsThreads, sizeof(RouterSmallSmem<4>), stream>>>(x_bf16, router_weight, bias, logits,
-                                                                   static_cast<uint32_t>(tokens), static_cast<uint32_t>(hidden),
-                                                                   static_cast<uint32_t>(experts));
-    } else {
-      dim3 g(static_cast<unsigned>((tokens + 15) / 16), static_cast<unsigned>((experts + 31) / 32));
-      GEMB_TRY(router_small_configure<8>(op));
-      router_logits_small_kernel<8><<<g, kRsThreads, sizeof(RouterSmallSmem<8>), stream>>>(x_bf16, router_weight, bias, logits,
-                                                                   static_cast<uint32_t>(tokens), static_cast<uint32_t>(hidden),
-                                                                   static_cast<uint32_t>(experts));
-    }
-    return check_launch(op);
-  }
-  // 8- and 16-token CTAs only while they do not outnumber the SMs; beyond that the larger tiles do more
-  // arithmetic per shared-memory load: 32 tokens, and 64 once there is a 64-token CTA for most SMs
-  // (measured on 2,816 x 128: 303 / 268 us at 16,384 tokens, 166 / 158 us at 8,192, 114 / 158 us at 4,096).
-  const uint64_t expert_tiles = (experts + kRtExp - 1) / kRtExp;
-  unsigned tile = 32;
-  if ((tokens + 7) / 8 * expert_tiles <= static_cast<uint64_t>(sm_count())) tile = 8;
-  else if ((tokens + 15) / 16 * expert_tiles <= static_cast<uint64_t>(sm_count())) tile = 16;
-  else if ((tokens + 63) / 64 * expert_tiles * 8 >= static_cast<uint64_t>(sm_count()) * 6) tile = 64;
-  // 56-token CTAs where they even out the load: with up to two of the large CTAs per SM, an SM's time goes with
-  // the tokens it holds (16,384 tokens: 256 CTAs of 64 leave 40 SMs with one CTA and 108 with two, 293 CTAs
-  // of 56 give every SM two).
-  if (tile == 64) {
-    const uint64_t sms = static_cast<uint64_t>(sm_count());
-    const uint64_t c64 = (tokens + 63) / 64 * expert_tiles, c56 = (tokens + 55) / 56 * expert_tiles;
-    if ((c56 + sms - 1) / sms * 56 < (c64 + sms - 1) / sms * 64) tile = 56;
-  }
-  if (g_router_tile == 8 || g_router_tile == 16 || g_router_tile == 32 || g_router_tile == 56 || g_router_tile == 64)
-    tile = static_cast<unsigned>(g_router_tile);
-  dim3 grid(static_cast<unsigned>((tokens + tile - 1) / tile), static_cast<unsigned>((experts + kRtExp - 1) / kRtExp));
-  if (tile == 8)
-    router_logits_kernel<8><<<grid, kRtThreads, 0, stream>>>(x_bf16, router_weight, bias, logits,
-                                                            static_cast<uint32_t>(tokens), static_cast<uint32_t>(hidden),
-                                                            static_cast<uint32_t>(experts));
-  else if (tile == 16)
-    router_logits_kernel<16><<<grid, kRtThreads, 0, stream>>>(x_bf16, router_weight, bias, logits,
-                                                             static_cast<uint32_t>(tokens), static_cast<uint32_t>(hidden),
-                                                             static_cast<uint32_t>(experts));
-  else if (tile == 56)
-    router_logits_kernel<56><<<grid, kRtThreads, 0, stream>>>(x_bf16, router_weight, bias, logits,
-                                                             static_cast<uint32_t>(tokens), static_cast<uint32_t>(hidden),
-                                                             static_cast<uint32_t>(experts));
-  else if (tile == 64)
-    router_logits_kernel<64><<<grid, kRtThreads, 0, stream>>>(x_bf16, router_weight, bias, logits,
-                                                             static_cast<uint32_t>(tokens), static_cast<uint32_t>(hidden),
-                                                             static_cast<uint32_t>(experts));
-  else
-    router_logits_kernel<32><<<grid, kRtThreads, 0, stream>>>(x_bf16, router_weight, bias, logits,
-                                                             static_cast<uint32_t>(tokens), static_cast<uint32_t>(hidden),
-                                                             static_cast<uint32_t>(experts));
+namespace {
+int32_t launch_permute(const char* op, const int32_t* ids, int32_t* block_counts, int32_t* counts, int32_t* offsets, int32_t* plan,
+                       int32_t* perm, int32_t* slot_rows, uint32_t segments, uint32_t total, uint32_t e, cudaStream_t stream) {
+  GEMB_TRY(launch_pdl(op, permute_count_kernel, dim3(segments), dim3(128), e * sizeof(int), stream, ids, block_counts, total, e));
+  GEMB_TRY(launch_pdl(op, permute_scan_kernel, dim3(1), dim3(kScanThreads), permute_scan_smem(e), stream, block_counts, counts, offsets,
+                      plan, segments, e));
+  GEMB_TRY(launch_pdl(op, permute_scatter_kernel, dim3(segments), dim3(128), 4 * e * sizeof(int), stream, ids, block_counts, offsets, plan,
+                      perm, slot_rows, total, e));
   return check_launch(op);
 }
+}  // namespace
+
+extern "C" {
 
 int32_t gemb_moe_route(const float* logits, const float* per_expert_scale, int32_t* top_ids, float* top_weights,
                        float* probabilities, uint64_t tokens, uint64_t experts, uint64_t topk,
@@ -976,9 +663,9 @@ int32_t gemb_moe_route(const float* logits, const float* per_expert_scale, int32
   GEMB_REQUIRE(logits && top_ids && top_weights, "%s: pointers must be nonnull", op);
   GEMB_TRY(validate_moe_geometry(op, tokens, experts, topk));
   GEMB_ENTER(op);
-  route_kernel<<<static_cast<unsigned>((tokens + 3) / 4), 128, 0, stream>>>(
-      logits, per_expert_scale, top_ids, top_weights, probabilities, static_cast<uint32_t>(tokens),
-      static_cast<uint32_t>(experts), static_cast<uint32_t>(topk));
+  GEMB_TRY(launch_pdl(op, route_kernel, dim3(static_cast<unsigned>((tokens + 3) / 4)), dim3(128), 0, stream, logits, per_expert_scale,
+                      top_ids, top_weights, probabilities, static_cast<uint32_t>(tokens), static_cast<uint32_t>(experts),
+                      static_cast<uint32_t>(topk)));
   return check_launch(op);
 }
 
@@ -1005,19 +692,12 @@ int32_t gemb_moe_permute(const int32_t* top_ids, int32_t* counts, int32_t* offse
   const uint32_t total = static_cast<uint32_t>(tokens * topk), e = static_cast<uint32_t>(experts);
   const uint32_t segments = static_cast<uint32_t>(moe_segments(tokens, topk));
   if (segments == 1) {   // decode-size batch: count, scan and scatter in one launch
-    permute_small_kernel<<<1, 128, (8 * e + 3) * sizeof(int), stream>>>(
-        top_ids, counts, offsets, plan, perm, slot_rows, total, e, static_cast<uint32_t>(moe_max_tiles(tokens, experts, topk)));
+    GEMB_TRY(launch_pdl(op, permute_small_kernel, dim3(1), dim3(128), (8 * e + 3 + 3 * 33) * sizeof(int), stream, top_ids, counts, offsets,
+                        plan, perm, slot_rows, total, e));
     return check_launch(op);
   }
   int32_t* block_counts = static_cast<int32_t*>(workspace);
-  permute_count_kernel<<<segments, 128, e * sizeof(int), stream>>>(top_ids, block_counts, total, e);
-  GEMB_TRY(check_launch(op));
-  permute_scan_kernel<<<1, 256, (4 * e + 3) * sizeof(int), stream>>>(block_counts, counts, offsets, plan, segments, e,
-                                                                     static_cast<uint32_t>(moe_max_tiles(tokens, experts, topk)));
-  GEMB_TRY(check_launch(op));
-  permute_scatter_kernel<<<segments, 128, 4 * e * sizeof(int), stream>>>(top_ids, block_counts, offsets, plan, perm,
-                                                                        slot_rows, total, e);
-  return check_launch(op);
+  return launch_permute(op, top_ids, block_counts, counts, offsets, plan, perm, slot_rows, segments, total, e, stream);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1080,14 +760,7 @@ int32_t gemb_moe_permute_static(const int32_t* top_ids, int32_t* counts, int32_t
   const uint32_t segments = static_cast<uint32_t>(segments64);
   // The count kernel overwrites every (segment, expert) cell this call reads, so nothing has to
   // be cleared even though the array still holds the previous call's values.
-  permute_count_kernel<<<segments, 128, e * sizeof(int), stream>>>(top_ids, block_counts, total, e);
-  GEMB_TRY(check_launch(op));
-  permute_scan_kernel<<<1, 256, (4 * e + 3) * sizeof(int), stream>>>(block_counts, counts, offsets, plan, segments, e,
-                                                                     static_cast<uint32_t>(moe_max_tiles(tokens, experts, topk)));
-  GEMB_TRY(check_launch(op));
-  permute_scatter_kernel<<<segments, 128, 4 * e * sizeof(int), stream>>>(top_ids, block_counts, offsets, plan, perm,
-                                                                        slot_rows, total, e);
-  return check_launch(op);
+  return launch_permute(op, top_ids, block_counts, counts, offsets, plan, perm, slot_rows, segments, total, e, stream);
 }
 
 int32_t gemb_moe_dispatch_quantize(const uint16_t* x_bf16, const int32_t* slot_rows, uint8_t* packed_e2m1,
@@ -1103,9 +776,8 @@ int32_t gemb_moe_dispatch_quantize(const uint16_t* x_bf16, const int32_t* slot_r
   GEMB_ENTER(op);
   const uint32_t c_pad = static_cast<uint32_t>((hidden / 16 + 3) / 4 * 4);
   const unsigned threads = static_cast<unsigned>(std::min<uint64_t>(256, (hidden / 16 + 31) / 32 * 32));
-  dispatch_quantize_kernel<<<static_cast<unsigned>(tokens), threads, 0, stream>>>(
-      x_bf16, slot_rows, packed_e2m1, interleaved_scales, static_cast<uint32_t>(hidden), static_cast<uint32_t>(topk),
-      global_divisor, c_pad);
+  GEMB_TRY(launch_pdl(op, dispatch_quantize_kernel, dim3(static_cast<unsigned>(tokens)), dim3(threads), 0, stream, x_bf16, slot_rows,
+                      packed_e2m1, interleaved_scales, static_cast<uint32_t>(hidden), static_cast<uint32_t>(topk), global_divisor, c_pad));
   return check_launch(op);
 }
 
@@ -1182,9 +854,9 @@ int32_t gemb_moe_combine(const uint16_t* y_bf16, const int32_t* slot_rows, const
                "%s: buffers must be 16-byte aligned", op);
   GEMB_ENTER(op);
   const uint64_t work = tokens * (hidden / 8);
-  combine_kernel<<<static_cast<unsigned>((work + 255) / 256), 256, 0, stream>>>(
-      y_bf16, slot_rows, top_weights, shared_bf16, out_bf16, static_cast<uint32_t>(tokens),
-      static_cast<uint32_t>(hidden), static_cast<uint32_t>(topk));
+  GEMB_TRY(launch_pdl(op, combine_kernel, dim3(static_cast<unsigned>((work + 255) / 256)), dim3(256), 0, stream, y_bf16, slot_rows,
+                      top_weights, shared_bf16, out_bf16, static_cast<uint32_t>(tokens), static_cast<uint32_t>(hidden),
+                      static_cast<uint32_t>(topk)));
   return check_launch(op);
 }
 
