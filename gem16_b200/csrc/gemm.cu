@@ -161,7 +161,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   // ready, accumulator drained) live in its shared memory and collect arrivals from both CTAs, the
   // odd CTA's TMA loads included.  The MMA's completion is committed to the same barrier in both CTAs.
   const uint32_t rank = kPair ? ptx::cluster_ctarank() : 0u;
-  pdl_trigger();
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       ptx::mbar_init(&full[s], 1);
@@ -189,7 +188,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   else __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
-  pdl_wait();   // barriers, tensor memory and descriptors are set up while the kernel before this one finishes
+  // Barriers, tensor memory and descriptors are set up while the kernel before this one finishes.  The kernel itself does
+  // not let its dependents start early: their CTAs would sit beside its own for its whole run (a 16,384-token
+  // dense layer 2,122 -> 2,195 us, 77 tokens 93 -> 101 us with a trigger here).
+  pdl_wait();
 
   // A device-side plan is clamped to the buffers' capacity (p.m rows): whatever it holds, no tile
   // beyond the activation, scale and output buffers is touched.
