@@ -97,8 +97,8 @@ int32_t gemb_device_check(void);
  * GEMM of the first half on C SMs beside the gate/up GEMM of the second half, the second half's pushing down GEMM
  * beside the shared branch (0, the default: one pass over all local experts; at two GPUs the two-half schedule
  * measured 1.23-1.35 ms per layer against 1.00 ms, because neither push is light enough on the SMs);
- * GEMB_TUNE_ROUTER_TILE = which router-logits kernel runs: 0 automatic, 1 the expert-per-thread kernels
- * wherever they apply, 8 / 16 / 32 / 56 / 64 the tiled kernel with that many tokens per CTA (same bits from all). */
+ * GEMB_TUNE_ROUTER_TILE = which router-logits tile runs: 0 automatic, 1 .. 4 the small-batch shapes in ascending
+ * order, 8 / 16 / 24 / 32 / 40 / 48 / 56 / 64 a shape with that many tokens per CTA (same bits from all). */
 enum {
   GEMB_TUNE_GEMV_ROWS = 1,
   GEMB_TUNE_GEMV_PDL = 2,

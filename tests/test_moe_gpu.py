@@ -423,3 +423,22 @@ def test_layer_bytes_do_not_change_between_calls(lib, dev, tokens):
         layer.forward(other)
         outs.append(layer.forward(x).clone())
     assert all(torch.equal(o, want) for o in outs)
+
+
+@pytest.mark.parametrize("tile", [1, 2, 3, 4, 24, 40, 48])
+@pytest.mark.parametrize("tokens,hidden,experts,offset", [(131, 132, 160, 0), (97, 260, 32, 1), (9, 2816, 128, 0), (1, 4, 32, 0)])
+def test_router_shapes_at_their_edges(lib, dev, orc, tile, tokens, hidden, experts, offset):
+    """Token, expert and K remainders of the shapes the sweep above does not force; rows only 8-byte aligned."""
+    rng = np.random.default_rng(tokens + tile)
+    x = bf16_bits(rng.standard_normal((tokens, hidden)).astype(np.float32))
+    w = (rng.standard_normal((experts, hidden)) * 0.02).astype(np.float32)
+    b = rng.standard_normal(experts).astype(np.float32)
+    xd = torch.zeros(tokens * hidden + 4, dtype=torch.int16, device=dev)[4 * offset:][:tokens * hidden].view(tokens, hidden)
+    xd.copy_(to_dev(x, dev).view(torch.int16))
+    out = torch.full((tokens, experts), float("nan"), device=dev)
+    try:
+        lib.gemb_set_tuning(8, tile)
+        lib.gemb_moe_router_logits(xd, to_dev(w, dev), to_dev(b, dev), out, tokens, hidden, experts, None)
+    finally:
+        lib.gemb_set_tuning(8, 0)
+    assert np.array_equal(to_np(out).view(np.uint32), orc.moe_router_logits(x, w, b).view(np.uint32))
