@@ -447,7 +447,8 @@ __global__ void __launch_bounds__(256)
 dispatch_quantize_kernel(const uint16_t* x, const int32_t* slot_rows,
                          uint8_t* __restrict__ packed, uint8_t* __restrict__ scales, uint32_t hidden,
                          uint32_t topk, float g, uint32_t c_pad) {
-  pdl_trigger();
+  // No early start of the dependents: the GEMM's CTAs would take the SMs that the shared branch on the other stream
+  // needs meanwhile, and wait there (64-token layer 102 us against 97).
   pdl_wait();
   const uint32_t t = blockIdx.x;
   __shared__ int rows[32];
@@ -577,19 +578,22 @@ combine_kernel(const uint16_t* y, const int32_t* slot_rows, const float* weights
   for (int i = 0; i < 8; ++i) acc[i] = 0.0f;
   // eight slots' rows in flight at a time, added in slot order
   for (uint32_t s0 = 0; s0 < topk; s0 += 8) {
+    const uint64_t slot = static_cast<uint64_t>(t) * topk + s0;
+    const int n = static_cast<int>(min(8u, topk - s0));
     float wv[8];
+    int32_t r[8];
     uint4 v[8];
 #pragma unroll
-    for (int s = 0; s < 8; ++s) {
-      if (s0 + s >= topk) break;
-      const uint64_t slot = static_cast<uint64_t>(t) * topk + s0 + s;
-      wv[s] = ld_dep(weights + slot);
-      const int64_t r = slot_rows ? static_cast<int64_t>(ld_dep(slot_rows + slot)) : static_cast<int64_t>(slot);
-      v[s] = ld_dep(reinterpret_cast<const uint4*>(y + r * hidden) + c);
+    for (int s = 0; s < 8; ++s) {   // all eight before the first row is asked for: these loads keep their order
+      wv[s] = s < n ? ld_dep(weights + slot + s) : 0.0f;
+      r[s] = s < n && slot_rows ? ld_dep(slot_rows + slot + s) : static_cast<int32_t>(slot) + s;
     }
 #pragma unroll
+    for (int s = 0; s < 8; ++s)
+      if (s < n) v[s] = ld_dep(reinterpret_cast<const uint4*>(y + static_cast<int64_t>(r[s]) * hidden) + c);
+#pragma unroll
     for (int s = 0; s < 8; ++s) {
-      if (s0 + s >= topk) break;
+      if (s >= n) break;
       const uint32_t ww[4] = {v[s].x, v[s].y, v[s].z, v[s].w};
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
