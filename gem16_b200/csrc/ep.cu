@@ -205,7 +205,9 @@ ep_plan_body(const int32_t* counts_all_global, uint32_t ranks, uint32_t experts,
   __syncthreads();
   for (uint32_t e = threadIdx.x; e < experts; e += blockDim.x)
     out_base[e] = pad[e] + before_me[e] - my_pad[e];
-  int32_t* info = plan + 3 + el;   // pairs {expert of tile i, i-th tile with real rows}, then the number of those
+  int32_t* info = plan + 3 + el;   // pairs {expert of tile i, i-th tile with real rows}, the number of those, rows of every tile
+  const uint32_t last = me * el + el - 1;
+  int32_t* rows_of_tile = info + 2 * ((pad[last] + (tot[last] + 255) / 256 * 256) / 128) + 1;
   for (uint32_t e = threadIdx.x; e < el; e += blockDim.x) {
     const uint32_t ge = me * el + e;
     plan[2 + e] = pad[ge];
@@ -214,6 +216,7 @@ ep_plan_body(const int32_t* counts_all_global, uint32_t ranks, uint32_t experts,
       const int real = max(0, min(128, tot[ge] - (tile * 128 - pad[ge])));
       info[2 * tile] = real > 0 ? static_cast<int32_t>(e) : -1;   // -1: padding only
       if (real > 0) info[2 * (live_off[e] + j) + 1] = tile;
+      rows_of_tile[tile] = real;
       if (tile_rows != nullptr) tile_rows[tile] = real;
     }
   }
@@ -598,7 +601,8 @@ uint64_t gemb_moe_ep_plan_ints(uint64_t capacity_rows, uint64_t local_experts) {
   // tiles, padded rows, local_experts + 1 padded offsets, one expert id per possible tile (every
   // expert's rows are padded to a multiple of 256: at most capacity / 128 + 2 per expert tiles)
   // the same again for the list of tiles that hold real rows, plus its length
-  return 3 + local_experts + 2 * ((capacity_rows + 127) / 128 + 2 * local_experts) + 1;
+  // and the real rows of every tile
+  return 3 + local_experts + 3 * ((capacity_rows + 127) / 128 + 2 * local_experts) + 1;
 }
 
 int32_t gemb_moe_ep_plan(const int32_t* counts_all, uint64_t ranks, uint64_t experts, uint64_t rank,

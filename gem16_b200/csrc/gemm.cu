@@ -136,7 +136,7 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 template <bool kFp4, int BN, int kStages, int kAccStages, bool kPair>
 __global__ void __launch_bounds__(kFp4 ? kGemmThreadsFp4 : kGemmThreadsFp8, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-            const __grid_constant__ CUtensorMap map_out, const GemmParams p) {
+            const __grid_constant__ CUtensorMap map_part, const __grid_constant__ CUtensorMap map_out, const GemmParams p) {
   using C = Cfg<kFp4, BN, kStages, kAccStages, kPair>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -177,6 +177,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     ptx::fence_barrier_init();
     ptx::prefetch_tensormap(&map_a);
     ptx::prefetch_tensormap(&map_b);
+    if (p.plan != nullptr) ptx::prefetch_tensormap(&map_part);
     ptx::prefetch_tensormap(&map_out);
   }
   if (warp == 1) {
@@ -225,6 +226,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   const uint32_t k_groups_pad = (p.k / 16 + 3) / 4;  // 512-byte scale chunks per 128-row group
   auto tile_expert_of = [&](uint32_t mt) -> int32_t {
     return ld_dep(tile_expert + 2 * (kPair ? (mt & ~1u) : mt));
+  };
+
+  // Rows of a grouped tile that hold assignments, in steps of 32 (the plan lists them behind the number of real tiles).
+  // With a few tokens per expert most of a tile is padding: only the 32-row blocks that hold something are
+  // fetched -- the others' accumulators are computed from whatever the stage held and never leave TMEM -- and written
+  // (64 tokens, 128 experts top-8: gate/up 38 -> 33 us, down 25 -> 21 us).
+  auto tile_blocks_of = [&](uint32_t mt) -> uint32_t {
+    const int32_t rows = ld_dep(tile_info + 2 * plan_tiles + 1 + mt);
+    return rows <= 32 ? 1u : min((static_cast<uint32_t>(rows) + 31) / 32, 4u);
   };
 
   // Tile order: groups of 16 token tiles; inside a group the token tile runs fastest, so the
@@ -286,13 +296,20 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         uint32_t mt, nt;
         tile_coords(tile, mt, nt);
         const uint32_t expert = tile_expert ? min(static_cast<uint32_t>(tile_expert_of(mt)), p.experts - 1) : 0u;
+        const uint32_t blocks = !kPair && tile_info != nullptr ? tile_blocks_of(mt) : 4u;
         for (uint32_t ks = 0; ks < k_stages; ++ks) {
           if (!ptx::mbar_wait(&empty[stage], phase ^ 1)) { fail_wait(1); break; }
           // The even CTA announces the pair's bytes; both CTAs' loads complete on its barrier.
-          if (rank == 0) ptx::mbar_expect_tx(&full[stage], (kPair ? 2 : 1) * (C::kABytes + C::kBBytes));
+          if (rank == 0) ptx::mbar_expect_tx(&full[stage], (kPair ? 2 : 1) * (C::kABytes / 4 * blocks + C::kBBytes));
           const uint32_t bar = kPair ? full_rank0 + stage * 8 : ptx::smem_addr(&full[stage]);
-          ptx::tma_load_2d<kPair>(stage_a + stage * C::kABytes, &map_a, bar, static_cast<int32_t>(ks * 128),
-                                  static_cast<int32_t>(mt * BM));
+          if (blocks == 4) {
+            ptx::tma_load_2d<kPair>(stage_a + stage * C::kABytes, &map_a, bar, static_cast<int32_t>(ks * 128),
+                                    static_cast<int32_t>(mt * BM));
+          } else {
+            for (uint32_t b = 0; b < blocks; ++b)
+              ptx::tma_load_2d<kPair>(stage_a + stage * C::kABytes + b * (C::kABytes / 4), &map_part, bar,
+                                      static_cast<int32_t>(ks * 128), static_cast<int32_t>(mt * BM + b * 32));
+          }
           ptx::tma_load_2d<kPair>(stage_b + stage * C::kBBytes, &map_b, bar, static_cast<int32_t>(ks * 128),
                                   static_cast<int32_t>(expert * p.n + nt * BN + rank * C::kBRows));
           if (++stage == kStages) { stage = 0; phase ^= 1; }
@@ -486,7 +503,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
       uint32_t mt, nt;
       tile_coords(tile, mt, nt);
       // In a pair the odd CTA may own a padding-only tile: it takes part in the barriers, nothing else.
-      const bool dead = kPair && tile_expert != nullptr && (mt >= p.m / BM || ld_dep(tile_expert + 2 * mt) < 0);
+      // So does, single CTAs, a warp whose 32 rows are all padding (pairs run where experts hold many full tiles:
+      // looking the rows up costs them more than the padding, 2 % at 16,384 tokens).
+      const bool dead = tile_info != nullptr && (kPair ? mt >= p.m / BM || ld_dep(tile_expert + 2 * mt) < 0 : quarter >= tile_blocks_of(mt));
       // The scales are fetched, and the staging buffer checked to be free again (the previous tile's last store has
       // read it), here, while the tile is still being computed, rather than after the accumulator is full.
       const uint32_t row0 = mt * BM + quarter * 32;
@@ -881,8 +900,10 @@ int32_t launch_gemm(const char* op, const void* a, const void* b, const GemmPara
     configured[dev] = true;
   }
   const uint64_t row_bytes = kFp4 ? p.k / 2 : p.k;
-  CUtensorMap map_a, map_b, map_out;
+  CUtensorMap map_a, map_b, map_part, map_out;
   GEMB_TRY(make_byte_map(op, &map_a, a, p.m, row_bytes, BM));
+  if (p.plan != nullptr && !kPair) GEMB_TRY(make_byte_map(op, &map_part, a, p.m, row_bytes, BM / 4));
+  else map_part = map_a;
   GEMB_TRY(make_byte_map(op, &map_b, b, static_cast<uint64_t>(p.n) * (p.plan ? p.experts : 1u), row_bytes, C::kBRows));
   if (p.out_f32)
     GEMB_TRY(make_out_map_f32(op, &map_out, p.out, p.m, p.n));
@@ -903,7 +924,7 @@ int32_t launch_gemm(const char* op, const void* a, const void* b, const GemmPara
     if (g_gemm_cta_cap != 0) ctas_max = std::max(1u, std::min(ctas_max, g_gemm_cta_cap));
     cfg.gridDim = dim3(std::min<uint32_t>(m_tiles * n_tiles, ctas_max));
   }
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, map_a, map_b, map_out, p);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, map_a, map_b, map_part, map_out, p);
   if (e != cudaSuccess) return fail(GEMB_INTERNAL, "%s: %s: %s", op, cudaGetErrorName(e), cudaGetErrorString(e));
   return check_launch(op);
 }
@@ -914,9 +935,9 @@ int32_t launch_gemm(const char* op, const void* a, const void* b, const GemmPara
 //
 // Automatic choice: 256 wide, except where that leaves SMs without a tile or the tiles are too coarse to
 // balance -- a dense call with fewer 256-wide tiles than SMs (decode-size batches of the shared branch: 23 us
-// instead of 29), and the grouped gate/up GEMM with the GELU epilogue up to 128 announced assignments per
-// expert (its 1,408 interleaved columns are 5.5 tiles of 256 but 11 of 128; on 128 experts 37 us instead
-// of 41 at 64 tokens, 89 instead of 92 at 2,048; from 4,096 tokens, 256 rows per expert, the wide tile wins).
+// instead of 29), and the grouped gate/up GEMM with the GELU epilogue up to 320 announced assignments per
+// expert (its 1,408 interleaved columns are 5.5 tiles of 256 but 11 of 128; whole layer, 128 experts top-8: 370 us
+// instead of 379 at 3,001 tokens; about even at 6,000).
 int32_t launch_fp4(const char* op, const void* act, const void* w, const GemmParams& params, bool pairs, cudaStream_t stream) {
   GemmParams p = params;
   if (p.plan != nullptr) {
@@ -927,7 +948,7 @@ int32_t launch_fp4(const char* op, const void* act, const void* w, const GemmPar
   if (bn == 0) {
     bool narrow;
     if (p.plan != nullptr)
-      narrow = p.gated && g_grouped_rows_hint != 0 && g_grouped_rows_hint <= 128ull * p.experts;
+      narrow = p.gated && g_grouped_rows_hint != 0 && g_grouped_rows_hint <= 320ull * p.experts;
     else
       narrow = static_cast<uint64_t>((p.m + BM - 1) / BM) * ((p.n + 255) / 256) < static_cast<uint64_t>(sm_count());
     bn = narrow ? 128 : 256;

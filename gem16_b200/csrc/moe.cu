@@ -202,7 +202,8 @@ permute_count_kernel(const int32_t* ids, int32_t* __restrict__ block_counts, uin
 // the experts by warp shuffles, then one thread per tile.  `totals` holds 3 x 33 ints.
 // plan layout (int32): [0] number T of 128-row tiles, [1] padded rows in total, [2 .. 2+E] padded
 // offset of every expert (+ the end), then T pairs {expert of tile i (-1: padding only), i-th tile
-// that holds real rows (what a single-CTA grouped GEMM walks)}, then the number of such tiles.
+// that holds real rows (what a single-CTA grouped GEMM walks)}, then the number of such tiles, then
+// the number of real rows of every tile.
 __device__ __forceinline__ void plan_from_counts(const int* cnt, int* off, int* poff, int* loff, int* totals, uint32_t experts,
                                                  int32_t* __restrict__ counts, int32_t* __restrict__ offsets, int32_t* __restrict__ plan) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
@@ -266,6 +267,7 @@ __device__ __forceinline__ void plan_from_counts(const int* cnt, int* off, int* 
     const bool real = j * 128 < cnt[lo];
     info[2 * tile] = real ? static_cast<int32_t>(lo) : -1;
     if (real) info[2 * (loff[lo] + j) + 1] = tile;
+    info[2 * (carry[1] / 128) + 1 + tile] = max(0, min(128, cnt[lo] - j * 128));
   }
 }
 
@@ -677,7 +679,7 @@ uint64_t gemb_moe_permute_workspace_bytes(uint64_t tokens, uint64_t experts, uin
   return moe_segments(tokens, topk) * experts * sizeof(int32_t);
 }
 uint64_t gemb_moe_plan_ints(uint64_t tokens, uint64_t experts, uint64_t topk) {
-  return 2 + experts + 1 + 2 * moe_max_tiles(tokens, experts, topk) + 1;
+  return 2 + experts + 1 + 3 * moe_max_tiles(tokens, experts, topk) + 1;
 }
 uint64_t gemb_moe_padded_rows_max(uint64_t tokens, uint64_t experts, uint64_t topk) {
   return moe_max_tiles(tokens, experts, topk) * 128;

@@ -410,7 +410,8 @@ uint64_t gemb_moe_padded_rows_max(uint64_t tokens, uint64_t experts, uint64_t to
  *   counts[experts], offsets[experts + 1], perm[tokens * topk] (perm[pos] = i)   -- the spec's
  *   records;  slot_rows[i] = row of assignment i in the padded per-expert row space;
  *   plan = {tiles, padded rows, padded_offsets[experts + 1], tiles x {expert of the tile or -1 for a
- *   tile of padding only, i-th tile that holds real rows}, number of tiles that hold real rows},
+ *   tile of padding only, i-th tile that holds real rows}, number of tiles that hold real rows, tiles x
+ *   rows of the tile that hold assignments},
  *   consumed on the device by the grouped GEMM (no host readback).  Every expert's rows start on a
  *   multiple of 256, so a 128-row tile and the 256-row tile of a CTA pair never mix experts.
  *   1 <= experts <= 1024, topk <= 32.
@@ -463,7 +464,8 @@ int32_t gemb_moe_scatter_quantized(const uint8_t* packed_rows, const uint8_t* co
                                    uint64_t src_row_stride, gemb_stream_t stream);
 
 /* Grouped expert projection over the padded row space: for every 128-row tile t of the plan,
- * out[rows of t] = bf16( A[rows of t] . W[tile_expert[t]]^T / (ga * w_divisors[expert]) ).
+ * out[rows of t] = bf16( A[rows of t] . W[tile_expert[t]]^T / (ga * w_divisors[expert]) ).  Rows behind an
+ * expert's last assignment hold nothing that is read again: they may be left unwritten.
  * A: NVFP4 payload [padded_rows_max, K/2] + INTERLEAVED scales; W: [experts, rows_per_expert, K/2]
  * with each expert's scales INTERLEAVED back to back; w_divisors: fp32 [experts] on the device.
  * Experts with no assignment own no tile and cost nothing; nothing is read back to the host.

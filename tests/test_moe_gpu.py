@@ -442,3 +442,18 @@ def test_router_shapes_at_their_edges(lib, dev, orc, tile, tokens, hidden, exper
     finally:
         lib.gemb_set_tuning(8, 0)
     assert np.array_equal(to_np(out).view(np.uint32), orc.moe_router_logits(x, w, b).view(np.uint32))
+
+
+def test_plan_lists_the_rows_of_every_tile(lib, dev):
+    """Behind the number of real tiles: rows of each 128-row tile that hold assignments (0, partial, full)."""
+    experts, t, k = 32, 300, 2
+    ids = torch.zeros((t, k), dtype=torch.int32, device=dev)      # expert 0: 300 rows, expert 5: 33, the rest on 31
+    ids[:33, 1], ids[33:, 1] = 5, 31
+    c = lib.cdll
+    plan = torch.full((c.gemb_moe_plan_ints(t, experts, k),), -1, dtype=torch.int32, device=dev)
+    counts, offsets = torch.zeros(experts, dtype=torch.int32, device=dev), torch.zeros(experts + 1, dtype=torch.int32, device=dev)
+    perm, rows = (torch.zeros(t * k, dtype=torch.int32, device=dev) for _ in range(2))
+    ws = torch.empty((c.gemb_moe_permute_workspace_bytes(t, experts, k),), dtype=torch.uint8, device=dev)
+    lib.gemb_moe_permute(ids, counts, offsets, perm, rows, plan, ws, ws.numel(), t, experts, k, None)
+    p = to_np(plan)
+    assert p[3 + experts + 2 * p[0] + 1:][:p[0]].tolist() == [128, 128, 44, 0, 33, 0, 128, 128, 11, 0]
