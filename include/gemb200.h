@@ -273,7 +273,7 @@ int32_t gemb_nvfp4_gemv_gate_up(const uint8_t* packed_activation_e2m1,
 
 /* The same for 1..65,535 tokens (the verifier's batches are a handful): activation [tokens, K/2]
  * with COMPACT scales [tokens, K/16], outputs [tokens, rows]; per token bit-identical to
- * gemb_nvfp4_gemv_gate_up, which it launches once per token.
+ * gemb_nvfp4_gemv_gate_up; up to eight tokens share one pass over the weights.
  * Replaces LaunchNvfp4Sm120FusedGateUpBatch, src/cuda/nvfp4/sm120.h:75-92. */
 int32_t gemb_nvfp4_gemv_gate_up_batch(const uint8_t* packed_activation_e2m1, const uint8_t* activation_scales,
                                       const uint8_t* packed_gate_weight, const uint8_t* gate_weight_scales,
