@@ -133,7 +133,9 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   return r;
 }
 
-template <bool kFp4, int BN, int kStages, int kAccStages, bool kPair>
+// kSplit > 1: a cluster of that many CTAs shares one tile of a dense call, each a contiguous part of K; the fp32 partial
+// accumulators meet in shared memory (see the epilogue).
+template <bool kFp4, int BN, int kStages, int kAccStages, bool kPair, int kSplit = 1>
 __global__ void __launch_bounds__(kFp4 ? kGemmThreadsFp4 : kGemmThreadsFp8, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
             const __grid_constant__ CUtensorMap map_part, const __grid_constant__ CUtensorMap map_out, const GemmParams p) {
@@ -219,10 +221,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     }
   }
   const uint32_t num_tiles = m_units * n_tiles;
-  const uint32_t first_tile = kPair ? blockIdx.x >> 1 : blockIdx.x;
-  const uint32_t tile_stride = kPair ? gridDim.x >> 1 : gridDim.x;
+  static_assert(kSplit == 1 || !kPair, "a tile is shared along K or along its rows");
+  const uint32_t first_tile = kPair ? blockIdx.x >> 1 : blockIdx.x / kSplit;
+  const uint32_t tile_stride = kPair ? gridDim.x >> 1 : gridDim.x / kSplit;
   const uint32_t my_tiles = first_tile < num_tiles ? (num_tiles - first_tile + tile_stride - 1) / tile_stride : 0;
-  const uint32_t k_stages = (p.k + C::kKPerStage - 1) / C::kKPerStage;
+  const uint32_t k_stages_all = (p.k + C::kKPerStage - 1) / C::kKPerStage;
+  const uint32_t split = kSplit > 1 ? ptx::cluster_ctarank() : 0u;
+  const uint32_t ks0 = kSplit > 1 ? split * k_stages_all / kSplit : 0u;   // this CTA's part of K
+  const uint32_t k_stages = kSplit > 1 ? (split + 1) * k_stages_all / kSplit - ks0 : k_stages_all;
   const uint32_t k_groups_pad = (p.k / 16 + 3) / 4;  // 512-byte scale chunks per 128-row group
   auto tile_expert_of = [&](uint32_t mt) -> int32_t {
     return ld_dep(tile_expert + 2 * (kPair ? (mt & ~1u) : mt));
@@ -303,14 +309,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
           if (rank == 0) ptx::mbar_expect_tx(&full[stage], (kPair ? 2 : 1) * (C::kABytes / 4 * blocks + C::kBBytes));
           const uint32_t bar = kPair ? full_rank0 + stage * 8 : ptx::smem_addr(&full[stage]);
           if (blocks == 4) {
-            ptx::tma_load_2d<kPair>(stage_a + stage * C::kABytes, &map_a, bar, static_cast<int32_t>(ks * 128),
+            ptx::tma_load_2d<kPair>(stage_a + stage * C::kABytes, &map_a, bar, static_cast<int32_t>((ks0 + ks) * 128),
                                     static_cast<int32_t>(mt * BM));
           } else {
             for (uint32_t b = 0; b < blocks; ++b)
               ptx::tma_load_2d<kPair>(stage_a + stage * C::kABytes + b * (C::kABytes / 4), &map_part, bar,
                                       static_cast<int32_t>(ks * 128), static_cast<int32_t>(mt * BM + b * 32));
           }
-          ptx::tma_load_2d<kPair>(stage_b + stage * C::kBBytes, &map_b, bar, static_cast<int32_t>(ks * 128),
+          ptx::tma_load_2d<kPair>(stage_b + stage * C::kBBytes, &map_b, bar, static_cast<int32_t>((ks0 + ks) * 128),
                                   static_cast<int32_t>(expert * p.n + nt * BN + rank * C::kBRows));
           if (++stage == kStages) { stage = 0; phase ^= 1; }
         }
@@ -337,12 +343,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         const uint8_t* sfb = p.sfb + static_cast<uint64_t>(g0) * k_groups_pad * 512;
         for (uint32_t ks = 0; ks < k_stages; ++ks) {
           if (!ptx::mbar_wait(&sf_empty[stage], phase ^ 1)) { fail_wait(6); break; }
-          const uint32_t bytes = min(4u, (p.k - ks * C::kKPerStage) / C::kKPerMma) * 512;
+          const uint32_t bytes = min(4u, (p.k - (ks0 + ks) * C::kKPerStage) / C::kKPerMma) * 512;
           ptx::mbar_expect_tx(&sf_full[stage], bytes * (1 + n_groups));
-          ptx::bulk_load_1d(stage_sfa + stage * C::kSfaBytes, sfa + static_cast<uint64_t>(ks) * 2048, bytes, &sf_full[stage]);
+          ptx::bulk_load_1d(stage_sfa + stage * C::kSfaBytes, sfa + static_cast<uint64_t>(ks0 + ks) * 2048, bytes, &sf_full[stage]);
           for (uint32_t g = 0; g < n_groups; ++g)
             ptx::bulk_load_1d(stage_sfb + stage * C::kSfbBytes + g * 2048,
-                              sfb + (static_cast<uint64_t>(g) * k_groups_pad + ks * 4) * 512, bytes, &sf_full[stage]);
+                              sfb + (static_cast<uint64_t>(g) * k_groups_pad + (ks0 + ks) * 4) * 512, bytes, &sf_full[stage]);
           if (++stage == kStages) { stage = 0; phase ^= 1; }
         }
       }
@@ -364,7 +370,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
       for (uint32_t t = 0; t < my_tiles && !*abort_flag; ++t) {
         if (!wait_issuer(&acc_empty[as], aphase ^ 1)) { fail_wait(2); break; }
         const uint32_t tmem_acc = tmem_base + as * BN;
-        uint32_t k_left = p.k;
+        uint32_t k_left = p.k - ks0 * C::kKPerStage;
         bool ok = true;
         for (uint32_t ks = 0; ks < k_stages; ++ks, k_left -= C::kKPerStage) {
           if (!ready) {   // the operands and, NVFP4, their scales
@@ -499,6 +505,68 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     const uint32_t set = warp >= (kFp4 ? 12 : 6) ? 1u : 0u;
     uint8_t* my_stage = epi_stage + (set * 4 + quarter) * 4096;
     uint32_t as = 0, aphase = 0;
+    if constexpr (kSplit > 1) {
+      // Every CTA leaves its partial accumulator in shared memory (the operand stages are free: its last MMA has
+      // completed; rows of 132 words are conflict-free for a lane per row), then takes BN / kSplit columns and adds the
+      // parts of all CTAs in K order, read through the cluster's shared window.  Plain bf16 output only.
+      uint32_t mt, nt;
+      tile_coords(first_tile, mt, nt);
+      constexpr int kStride = BN + 4;
+      static_assert(128 * kStride * 4 <= kStages * (C::kABytes + C::kBBytes), "the partial sums replace the operand stages");
+      float* part = reinterpret_cast<float*>(smem) + (quarter * 32 + lane) * kStride;
+      if (!ptx::mbar_wait(&acc_full[0], 0)) fail_wait(4);
+      ptx::tc_fence_after();
+#pragma unroll 1
+      for (uint32_t c = set; c < BN / 64; c += 2) {
+        if (mt * BM + quarter * 32 >= p.m) break;   // warp-uniform
+        uint32_t v0[32], v1[32];
+        ptx::tc_ld_32x32b_x32(tmem_base + ((quarter * 32) << 16) + c * 64, v0);
+        ptx::tc_ld_32x32b_x32(tmem_base + ((quarter * 32) << 16) + c * 64 + 32, v1);
+        ptx::tc_wait_ld();
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          *reinterpret_cast<uint4*>(part + c * 64 + 4 * q) = make_uint4(v0[4 * q], v0[4 * q + 1], v0[4 * q + 2], v0[4 * q + 3]);
+          *reinterpret_cast<uint4*>(part + c * 64 + 32 + 4 * q) = make_uint4(v1[4 * q], v1[4 * q + 1], v1[4 * q + 2], v1[4 * q + 3]);
+        }
+      }
+      ptx::tc_fence_before();
+      __syncwarp();
+      ptx::cluster_sync();
+      // Eight or sixteen lanes per row: whole 128-byte lines through the shared window, whole sectors out.
+      constexpr uint32_t kLanes = BN / kSplit / 4, kRows = 32 / kLanes;
+      const uint32_t col = split * (BN / kSplit) + lane % kLanes * 4, gcol = nt * BN + col;
+      uint2 ws = make_uint2(0, 0);
+      if constexpr (!kFp4) {
+        if (gcol < p.n) ws = make_uint2(__ldg(reinterpret_cast<const uint32_t*>(p.w_scales + gcol)), __ldg(reinterpret_cast<const uint32_t*>(p.w_scales + gcol) + 1));
+      }
+      const uint32_t rows = min(static_cast<uint32_t>(BM), p.m - mt * BM);
+#pragma unroll 2
+      for (uint32_t r0 = (set * 4 + quarter) * kRows; r0 < rows; r0 += 8 * kRows) {   // rows past `rows` of a trip: old bytes, not stored
+        const uint32_t r = r0 + lane / kLanes, row = mt * BM + r;
+        float4 v[kSplit];
+#pragma unroll
+        for (int c = 0; c < kSplit; ++c) v[c] = ptx::ld_cluster_f4(ptx::cluster_map(reinterpret_cast<float*>(smem) + r * kStride + col, c));
+        if (r >= rows || gcol >= p.n) continue;   // n is a multiple of 8
+        float row_scale = p.alpha;
+        if constexpr (!kFp4) row_scale = ld_dep(p.a_scales + row);
+#pragma unroll
+        for (int c = 1; c < kSplit; ++c) {
+          v[0].x = __fadd_rn(v[0].x, v[c].x);
+          v[0].y = __fadd_rn(v[0].y, v[c].y);
+          v[0].z = __fadd_rn(v[0].z, v[c].z);
+          v[0].w = __fadd_rn(v[0].w, v[c].w);
+        }
+        float o[4] = {__fmul_rn(v[0].x, row_scale), __fmul_rn(v[0].y, row_scale), __fmul_rn(v[0].z, row_scale), __fmul_rn(v[0].w, row_scale)};
+        if constexpr (!kFp4) {
+          o[0] = __fmul_rn(o[0], __uint_as_float(ws.x << 16));
+          o[1] = __fmul_rn(o[1], __uint_as_float(ws.x & 0xFFFF0000u));
+          o[2] = __fmul_rn(o[2], __uint_as_float(ws.y << 16));
+          o[3] = __fmul_rn(o[3], __uint_as_float(ws.y & 0xFFFF0000u));
+        }
+        *reinterpret_cast<uint2*>(static_cast<uint16_t*>(p.out) + static_cast<uint64_t>(row) * p.n + gcol) =
+            make_uint2(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]));
+      }
+    } else
     for (uint32_t tile = first_tile; tile < num_tiles && !*abort_flag; tile += tile_stride) {
       uint32_t mt, nt;
       tile_coords(tile, mt, nt);
@@ -746,6 +814,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     if (lane == 0) ptx::bulk_wait_group_all();
   }
 
+  if constexpr (kSplit > 1) {
+    if (is_ctrl || is_mover) {   // the epilogue warps' barrier between writing and reading the partial sums
+      __syncwarp();
+      ptx::cluster_sync();
+    }
+  }
+
   // ------------------------------- teardown ---------------------------------------------------
   ptx::tc_fence_before();
   __syncthreads();
@@ -754,8 +829,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     for (int i = 0; i < 2000; ++i) __nanosleep(1000);
     __syncthreads();
   }
-  // Neither CTA of a pair may leave while the other can still reach its shared memory or barriers.
-  if constexpr (kPair) ptx::cluster_sync();
+  // No CTA of a cluster may leave while another can still reach its shared memory or barriers.
+  if constexpr (kPair || kSplit > 1) ptx::cluster_sync();
   if (warp == 1) {
     ptx::tc_fence_after();
     if constexpr (kPair) ptx::tmem_dealloc_pair(tmem_base, 512);
@@ -856,10 +931,10 @@ bool grouped_pairs(uint64_t padded_rows_max, uint64_t experts) {
   return g_gemm_pair == 2 || rows >= 768 * experts;
 }
 
-template <bool kFp4, int BN, int kStages, int kAccStages, bool kPair = false>
+template <bool kFp4, int BN, int kStages, int kAccStages, bool kPair = false, int kSplit = 1>
 int32_t launch_gemm(const char* op, const void* a, const void* b, const GemmParams& p, cudaStream_t stream) {
   using C = Cfg<kFp4, BN, kStages, kAccStages, kPair>;
-  auto kern = gemm_kernel<kFp4, BN, kStages, kAccStages, kPair>;
+  auto kern = gemm_kernel<kFp4, BN, kStages, kAccStages, kPair, kSplit>;
   constexpr unsigned kThreads = kFp4 ? kGemmThreadsFp4 : kGemmThreadsFp8;
   // First call per device and kernel variant: shared-memory opt-in and the pair occupancy,
   // serialised so that two host threads cannot race on it.
@@ -874,7 +949,7 @@ int32_t launch_gemm(const char* op, const void* a, const void* b, const GemmPara
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
   attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = 2;
+  attr[1].val.clusterDim.x = kPair ? 2 : kSplit;
   attr[1].val.clusterDim.y = 1;
   attr[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg{};
@@ -882,7 +957,7 @@ int32_t launch_gemm(const char* op, const void* a, const void* b, const GemmPara
   cfg.dynamicSmemBytes = C::kSmemBytes;
   cfg.stream = stream;
   cfg.attrs = attr;
-  cfg.numAttrs = kPair ? 2 : 1;
+  cfg.numAttrs = kPair || kSplit > 1 ? 2 : 1;
   if (!configured[dev]) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
     if (e != cudaSuccess) return fail(GEMB_INTERNAL, "%s: %s: %s", op, cudaGetErrorName(e), cudaGetErrorString(e));
@@ -919,6 +994,8 @@ int32_t launch_gemm(const char* op, const void* a, const void* b, const GemmPara
     uint32_t pairs_max = static_cast<uint32_t>(max_pairs[dev]);
     if (g_gemm_cta_cap != 0) pairs_max = std::max(1u, std::min(pairs_max, g_gemm_cta_cap / 2));
     cfg.gridDim = dim3(2 * std::min<uint32_t>(units, pairs_max));
+  } else if constexpr (kSplit > 1) {
+    cfg.gridDim = dim3(m_tiles * n_tiles * kSplit);   // one tile per cluster
   } else {
     uint32_t ctas_max = static_cast<uint32_t>(sm_count());
     if (g_gemm_cta_cap != 0) ctas_max = std::max(1u, std::min(ctas_max, g_gemm_cta_cap));
@@ -933,6 +1010,19 @@ int32_t launch_gemm(const char* op, const void* a, const void* b, const GemmPara
 // fill the 512); 256 x 128 pair tiles hold two, so a tile's epilogue runs under the next tile's MMAs, at
 // the operand traffic per flop of the single-CTA 128 x 256 tile.
 //
+// How many CTAs share a tile of a dense call along K.  A token tile of 128 rows and a few thousand columns are a few dozen
+// tiles: without the split most SMs idle while a few CTAs stream the weights.  Four or two parts where all of
+// them are resident at once (a few SMs are left: clusters cannot use every one) and each keeps at least eight K steps to cover
+// the ring's fill.  77 tokens, weights cold: FP8 8,192 x 3,840 15.4 -> 10.8 us (two parts), 3,840 x 4,096 15.2 -> 7.8 and NVFP4
+// 3,840 x 15,360 20.8 -> 12.4 (four).  (A lane per row instead of eight or sixteen in the reduction: 5-6 us more.)
+int dense_split(const GemmParams& p, uint32_t k_per_stage) {
+  if (p.plan != nullptr || p.gated || p.gate_in != nullptr || p.out_f32 || g_gemm_bn != 0 || g_gemm_pair != 0 || g_gemm_cta_cap != 0) return 1;
+  const uint64_t tiles = static_cast<uint64_t>((p.m + BM - 1) / BM) * ((p.n + 127) / 128), steps = (p.k + k_per_stage - 1) / k_per_stage;
+  for (int parts = 4; parts >= 2; parts /= 2)
+    if (tiles * parts + 8 <= static_cast<uint64_t>(sm_count()) && steps >= 8ull * parts) return parts;
+  return 1;
+}
+
 // Automatic choice: 256 wide, except where that leaves SMs without a tile or the tiles are too coarse to
 // balance -- a dense call with fewer 256-wide tiles than SMs (decode-size batches of the shared branch: 23 us
 // instead of 29), and the grouped gate/up GEMM with the GELU epilogue up to 320 announced assignments per
@@ -943,6 +1033,11 @@ int32_t launch_fp4(const char* op, const void* act, const void* w, const GemmPar
   if (p.plan != nullptr) {
     p.expert_lo = g_expert_lo;
     p.expert_hi = g_expert_hi;
+  }
+  switch (dense_split(p, 256)) {
+    case 4: return launch_gemm<true, 128, 5, 2, false, 4>(op, act, w, p, stream);
+    case 2: return launch_gemm<true, 128, 5, 2, false, 2>(op, act, w, p, stream);
+    default: break;
   }
   int bn = g_gemm_bn;
   if (bn == 0) {
@@ -1313,6 +1408,11 @@ int32_t gemb_fp8_gemm_bf16(const uint8_t* act, const float* act_scales, const ui
   p.alpha = 1.0f;
   const int bn = g_gemm_bn == 128 ? 128 : 256;
   if (bn == 128) return launch_gemm<false, 128, 6, 2>(op, act, w, p, stream);
+  switch (dense_split(p, 128)) {
+    case 4: return launch_gemm<false, 128, 6, 2, false, 4>(op, act, w, p, stream);
+    case 2: return launch_gemm<false, 128, 6, 2, false, 2>(op, act, w, p, stream);
+    default: break;
+  }
   if (use_pairs()) return launch_gemm<false, 256, 6, 2, true>(op, act, w, p, stream);
   return launch_gemm<false, 256, 4, 2>(op, act, w, p, stream);
 }

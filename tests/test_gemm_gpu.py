@@ -192,3 +192,32 @@ def test_cta_pair_and_single_cta_tiles_agree_bit_for_bit(lib, dev, tokens, rows,
         assert torch.equal(x, y), name
         assert torch.equal(x, z), name + " (256 x 128 pair tiles)"
         assert not torch.isnan(y.float() if y.dtype == torch.float32 else y.view(torch.bfloat16).float()).any(), name
+
+
+# Dense calls of a few tiles, shared along K by clusters of four (the first three) and two CTAs: token, column and K
+# remainders, two token tiles, the largest grids of each; a second call must give the same bytes.
+@pytest.mark.parametrize("fmt", ["nvfp4", "fp8"])
+@pytest.mark.parametrize("tokens,rows,steps,rest", [(1, 8, 32, 0), (77, 264, 33, 1), (130, 2176, 35, 2), (9, 4480, 32, 1),
+                                                    (200, 4480, 17, 3), (77, 8192, 16, 0)])
+def test_tiles_shared_along_k(lib, dev, orc, fmt, tokens, rows, steps, rest):
+    k = steps * (256 if fmt == "nvfp4" else 128) + rest * (64 if fmt == "nvfp4" else 32)
+    outs = [torch.full((tokens, rows), 0x7FC0, dtype=torch.int16, device=dev) for _ in range(2)]
+    if fmt == "nvfp4":
+        a, w = nvfp4_operand(lib, dev, tokens, k, 1.0, 3), nvfp4_operand(lib, dev, rows, k, 0.02, 4)
+        for out in outs:
+            lib.gemb_nvfp4_gemm_bf16(a["packed"], a["inter"], w["packed"], w["inter"], out, tokens, rows, k, a["div"], w["div"], None)
+    else:
+        a, w = fp8_operand(lib, dev, tokens, k, 1.0, 3), fp8_operand(lib, dev, rows, k, 0.02, 4)
+        for out in outs:
+            lib.gemb_fp8_gemm_bf16(a["q"], a["scales"], w["q"], w["scales_bf16"], out, tokens, rows, k, None)
+    lib.gemb_check_device_status()
+    assert torch.equal(outs[0], outs[1])
+    idx = sample_tokens(tokens, 6)
+    if fmt == "nvfp4":
+        want = orc.nvfp4_matmul(to_np(a["packed"])[idx], to_np(a["compact"])[idx], to_np(w["packed"]), to_np(w["compact"]), a["div"], w["div"])
+    else:
+        want = orc.fp8_matmul(to_np(a["q"])[idx], to_np(a["scales"])[idx], to_np(w["q"]), to_np(w["scales_bf16"], np.uint16))
+    got = bf16_tensor_to_f32(outs[0])
+    assert np.isfinite(got).all()
+    st = error_stats(got[idx], want)
+    assert st["rel_fro"] <= REL_FRO and st["cos"] > 0.9999, st
