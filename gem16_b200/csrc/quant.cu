@@ -401,6 +401,81 @@ row_warp_kernel(const __grid_constant__ RowArgs a) {
 __device__ __forceinline__ float to_float(float v) { return v; }
 __device__ __forceinline__ float to_float(uint16_t v) { return bf16_bits_to_float(v); }
 
+// Few rows of up to kShortRow elements are read once: thread t holds elements t, t + 256, ... (the sum's order) in registers
+// and, where the second half of the kernel wants sixteen neighbours, hands them over through shared memory.  A decode
+// step's row kernels are a chain of memory round trips: norm weights come before the wait for the previous kernel and
+// the second read of the row is gone (3,840 elements: RMSNorm + residual 4.0 -> 3.1 us behind its predecessor,
+// + FP8 3.3 -> 3.0; a decode pass 231 -> 218 us).
+constexpr uint32_t kShortRow = 256 * 16;
+// For the few rows of a decode step only: behind a GEMM, which starts nothing early, there is no wait to load weights under, and
+// the wider second read is the faster one (77-token layer 72.8 us against 74.3).
+bool short_rows(uint64_t rows, uint64_t k) { return k <= kShortRow && rows <= 16; }
+
+// Every warp folds the 256 partials by itself, in the tree's order: strides 128, 64, 32 inside the lane, the
+// rest as shuffles.  One barrier instead of eight.
+__device__ __forceinline__ float rmsnorm_fold(float ss, uint64_t k, float eps, float* red) {
+  red[threadIdx.x] = ss;
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  float p[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) p[j] = red[lane + 32 * j];
+  float s = ((p[0] + p[4]) + (p[2] + p[6])) + ((p[1] + p[5]) + (p[3] + p[7]));
+#pragma unroll
+  for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+  return sqrt_inverse(s, k, eps);
+}
+
+// A short row into registers, its sum of squares in the same order as below.
+template <typename In>
+__device__ __forceinline__ float load_short_row(const In* row, uint32_t k, float (&v)[16]) {
+  In raw[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    const uint32_t i = threadIdx.x + j * 256;
+    raw[j] = In(0);
+    if (i < k) raw[j] = ld_dep(row + i);
+  }
+  float ss = 0.0f;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    v[j] = to_float(raw[j]);
+    ss = fmaf(v[j], v[j], ss);
+  }
+  return ss;
+}
+// The norm weights of elements 16 c .. 16 c + 15, before the wait for the previous kernel (weights are immutable).
+__device__ __forceinline__ void load_norm_weights(const uint16_t* w, uint32_t c, uint32_t k, uint16_t (&wv)[16]) {
+  if (w && c * 16 < k && (reinterpret_cast<uintptr_t>(w) & 15) == 0) {   // k is a multiple of 16
+    const uint4 a = __ldg(reinterpret_cast<const uint4*>(w) + 2 * c), b = __ldg(reinterpret_cast<const uint4*>(w) + 2 * c + 1);
+    const uint32_t words[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int i = 0; i < 16; ++i) wv[i] = static_cast<uint16_t>(words[i / 2] >> (16 * (i & 1)));
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < 16; ++i) wv[i] = w && c * 16 + i < k ? __ldg(w + c * 16 + i) : uint16_t(0x3F80);
+}
+// 1 / rms of a short row whose elements it leaves in xs.
+template <typename In>
+__device__ __forceinline__ float stage_short_row(const In* row, uint32_t k, float eps, float* xs, float* red) {
+  float v[16];
+  const float ss = load_short_row(row, k, v);
+#pragma unroll
+  for (int j = 0; j < 16; ++j)
+    if (threadIdx.x + j * 256 < k) xs[threadIdx.x + j * 256] = v[j];
+  return rmsnorm_fold(ss, k, eps, red);   // its barrier covers xs
+}
+__device__ __forceinline__ void normalise_staged(const float* xs, uint32_t c, const uint16_t (&wv)[16], float inv, float (&v)[16]) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float4 x = *reinterpret_cast<const float4*>(xs + c * 16 + 4 * q);
+    v[4 * q] = x.x, v[4 * q + 1] = x.y, v[4 * q + 2] = x.z, v[4 * q + 3] = x.w;
+  }
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v[i] = bf16_round(__fmul_rn(__fmul_rn(v[i], inv), bf16_bits_to_float(wv[i])));
+}
+
 template <typename In>
 __device__ __forceinline__ float rmsnorm_inverse(const In* row, uint64_t k, float eps, float* red) {
   float ss = 0.0f;
@@ -419,18 +494,7 @@ __device__ __forceinline__ float rmsnorm_inverse(const In* row, uint64_t k, floa
       ss = fmaf(v, v, ss);
     }
   }
-  red[threadIdx.x] = ss;
-  __syncthreads();
-  // Every warp folds the 256 partials by itself, in the tree's order: strides 128, 64, 32 inside the lane, the
-  // rest as shuffles.  One barrier instead of eight.
-  const int lane = threadIdx.x & 31;
-  float p[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) p[j] = red[lane + 32 * j];
-  float s = ((p[0] + p[4]) + (p[2] + p[6])) + ((p[1] + p[5]) + (p[3] + p[7]));
-#pragma unroll
-  for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
-  return sqrt_inverse(s, k, eps);
+  return rmsnorm_fold(ss, k, eps, red);
 }
 
 // RMSNorm + residual (+ layer scalar) with the bf16 boundaries of src/cuda/norm/reference.cu:66-160:
@@ -439,14 +503,41 @@ __device__ __forceinline__ void store_scalar(float* p, uint64_t i, float v) { p[
 __device__ __forceinline__ void store_scalar(uint16_t* p, uint64_t i, float v) { p[i] = float_to_bf16_bits(v); }
 
 // Any width and alignment: the second pass takes one element per thread and step, eight steps in flight.
-template <typename In, typename Res, typename Out>
+template <typename In, typename Res, typename Out, bool kShort>
 __global__ void __launch_bounds__(256)
 rmsnorm_residual_kernel(const In* x, const uint16_t* __restrict__ w, const Res* residual, float* normalized, Out* out,
                         uint64_t k, float eps, const uint16_t* __restrict__ scalar) {
   __shared__ float red[256];
   pdl_trigger();
-  pdl_wait();
   const uint64_t base = static_cast<uint64_t>(blockIdx.x) * k;
+  if constexpr (kShort) {
+    uint16_t wv[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) wv[j] = w && threadIdx.x + j * 256 < k ? __ldg(w + threadIdx.x + j * 256) : uint16_t(0x3F80);
+    const float layer_scale = scalar ? bf16_bits_to_float(__ldg(scalar)) : 1.0f;
+    pdl_wait();
+    Res rv[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      rv[j] = Res(0);
+      if (threadIdx.x + j * 256 < k) rv[j] = ld_dep(residual + base + threadIdx.x + j * 256);
+    }
+    float xv[16];
+    const float ss = load_short_row(x + base, static_cast<uint32_t>(k), xv);
+    const float inv = rmsnorm_fold(ss, k, eps, red);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const uint64_t i = threadIdx.x + j * 256;
+      if (i >= k) continue;
+      const float n = bf16_round(__fmul_rn(__fmul_rn(xv[j], inv), bf16_bits_to_float(wv[j])));
+      if (normalized) normalized[base + i] = n;
+      float v = bf16_round(__fadd_rn(n, to_float(rv[j])));
+      if (scalar) v = bf16_round(__fmul_rn(v, layer_scale));
+      store_scalar(out, base + i, v);
+    }
+    return;
+  }
+  pdl_wait();
   const float inv = rmsnorm_inverse(x + base, k, eps, red);
   const float layer_scale = scalar ? bf16_bits_to_float(__ldg(scalar)) : 1.0f;
   for (uint64_t i0 = threadIdx.x; i0 < k; i0 += 256 * 8) {
@@ -478,27 +569,35 @@ __device__ __forceinline__ float norm_weight(const uint16_t* w, uint64_t i) {
   return w ? bf16_bits_to_float(__ldg(w + i)) : 1.0f;
 }
 
-template <typename In, bool kRcp, bool kInterleaved>
+template <typename In, bool kRcp, bool kInterleaved, bool kShort>
 __global__ void __launch_bounds__(256)
 rmsnorm_nvfp4_quantize_kernel(const In* x, const uint16_t* __restrict__ w, uint8_t* packed, uint8_t* scales,
                               uint32_t rows, uint64_t k, float eps, float g, uint32_t c_pad) {
   __shared__ float red[256];
+  __shared__ __align__(16) float xs[kShort ? kShortRow : 4];
   pdl_trigger();
-  pdl_wait();
   const uint64_t r = blockIdx.x;
   const uint32_t c_real = static_cast<uint32_t>(k / 16);
   const bool pad_row = r >= rows;   // interleaved layout only: rows up to a multiple of 128 get zero scales
+  constexpr bool short_row = kShort;
   const In* row = x + r * k;
   float inv = 0.0f;
-  if (!pad_row) inv = rmsnorm_inverse(row, k, eps, red);
+  uint16_t wv[16];
+  if (short_row && !pad_row) load_norm_weights(w, threadIdx.x, static_cast<uint32_t>(k), wv);
+  pdl_wait();
+  if (!pad_row) inv = short_row ? stage_short_row(row, static_cast<uint32_t>(k), eps, xs, red) : rmsnorm_inverse(row, k, eps, red);
   for (uint32_t c0 = 0; c0 < c_pad; c0 += 256) {
     const uint32_t c = c0 + threadIdx.x;
     uint8_t sb = 0;
     if (c < c_real && !pad_row) {
       float v[16];
-      load16(row + static_cast<uint64_t>(c) * 16, v);
+      if (short_row) {   // one trip: c = threadIdx.x
+        normalise_staged(xs, c, wv, inv, v);
+      } else {
+        load16(row + static_cast<uint64_t>(c) * 16, v);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) v[i] = bf16_round(__fmul_rn(__fmul_rn(v[i], inv), norm_weight(w, c * 16ull + i)));
+        for (int i = 0; i < 16; ++i) v[i] = bf16_round(__fmul_rn(__fmul_rn(v[i], inv), norm_weight(w, c * 16ull + i)));
+      }
       uint32_t lo, hi;
       quantize_block16<kRcp>(v, g, lo, hi, sb);
       *reinterpret_cast<uint2*>(packed + r * (k / 2) + c * 8ull) = make_uint2(lo, hi);
@@ -518,20 +617,28 @@ rmsnorm_nvfp4_quantize_kernel(const In* x, const uint16_t* __restrict__ w, uint8
 // FP8 per-token quantizer: pass 1 finds amax (max is order independent), pass 2 divides and converts.
 // src/numeric/fp8.cpp:41-58, src/cuda/fp8/reference.cu:39-69.  A thread keeps its first two 16-element
 // blocks (rows of up to 8,192 elements) between the passes; the rest of a longer row is read again from L2.
-template <typename In, bool kNorm>
+template <typename In, bool kNorm, bool kShort>
 __global__ void __launch_bounds__(256)
 fp8_quantize_kernel(const In* x, const uint16_t* __restrict__ w, uint8_t* out, float* scales, uint64_t k, float eps) {
   __shared__ float red[256];
   __shared__ float red2[8];
+  __shared__ __align__(16) float xs[kNorm && kShort ? kShortRow : 4];
   if constexpr (kNorm) pdl_trigger();
   else pdl_trigger_few_rows(gridDim.x);
-  pdl_wait();
   const uint64_t r = blockIdx.x;
   const In* row = x + r * k;
+  constexpr bool short_row = kNorm && kShort;
   float inv = 1.0f;
-  if constexpr (kNorm) inv = rmsnorm_inverse(row, k, eps, red);
+  uint16_t wv[16];
+  if (short_row) load_norm_weights(w, threadIdx.x, static_cast<uint32_t>(k), wv);
+  pdl_wait();
+  if constexpr (kNorm) inv = short_row ? stage_short_row(row, static_cast<uint32_t>(k), eps, xs, red) : rmsnorm_inverse(row, k, eps, red);
   const uint32_t blocks = static_cast<uint32_t>(k / 16);
   auto block_values = [&](uint32_t c, float (&v)[16]) {
+    if (short_row) {   // c = threadIdx.x: a short row has at most 256 blocks
+      normalise_staged(xs, c, wv, inv, v);
+      return;
+    }
     load16(row + static_cast<uint64_t>(c) * 16, v);
     if constexpr (kNorm) {
 #pragma unroll
@@ -665,8 +772,10 @@ int32_t gemb_nvfp4_rmsnorm_quantize(const void* input, int32_t input_dtype, cons
   }
   auto launch = [&](auto* x) -> int32_t {
     using T = std::remove_const_t<std::remove_pointer_t<decltype(x)>>;
-    auto kern = inter ? (rcp ? rmsnorm_nvfp4_quantize_kernel<T, true, true> : rmsnorm_nvfp4_quantize_kernel<T, false, true>)
-                      : (rcp ? rmsnorm_nvfp4_quantize_kernel<T, true, false> : rmsnorm_nvfp4_quantize_kernel<T, false, false>);
+    auto kern = inter ? (rcp ? rmsnorm_nvfp4_quantize_kernel<T, true, true, false> : rmsnorm_nvfp4_quantize_kernel<T, false, true, false>)
+                      : (rcp ? rmsnorm_nvfp4_quantize_kernel<T, true, false, false> : rmsnorm_nvfp4_quantize_kernel<T, false, false, false>);
+    if (short_rows(rows_out, k))   // the interleaved layout pads to 128 rows: never
+      kern = rcp ? rmsnorm_nvfp4_quantize_kernel<T, true, false, true> : rmsnorm_nvfp4_quantize_kernel<T, false, false, true>;
     GEMB_TRY(launch_pdl(op, kern, dim3(static_cast<unsigned>(rows_out)), dim3(256), 0, stream, x, weight, packed, scales,
                         static_cast<uint32_t>(tokens), k, eps, g, static_cast<uint32_t>(c_pad)));
     return check_launch(op);
@@ -716,12 +825,12 @@ int32_t launch_fp8_rows(const char* op, const void* input, int32_t input_dtype, 
     return launch_row_warp<kNorm ? kRowFp8Norm : kRowFp8, false>(op, a, stream);
   }
   const dim3 grid(static_cast<unsigned>(tokens));
-  if (input_dtype == GEMB_F32)
-    GEMB_TRY(launch_pdl(op, fp8_quantize_kernel<float, kNorm>, grid, dim3(256), 0, stream, static_cast<const float*>(input), weight,
-                        out, scales, k, eps));
-  else
-    GEMB_TRY(launch_pdl(op, fp8_quantize_kernel<uint16_t, kNorm>, grid, dim3(256), 0, stream,
-                        static_cast<const uint16_t*>(input), weight, out, scales, k, eps));
+  auto launch = [&](auto* x) -> int32_t {
+    using T = std::remove_const_t<std::remove_pointer_t<decltype(x)>>;
+    auto kern = kNorm && short_rows(tokens, k) ? fp8_quantize_kernel<T, kNorm, kNorm> : fp8_quantize_kernel<T, kNorm, false>;
+    return launch_pdl(op, kern, grid, dim3(256), 0, stream, x, weight, out, scales, k, eps);
+  };
+  GEMB_TRY(input_dtype == GEMB_F32 ? launch(static_cast<const float*>(input)) : launch(static_cast<const uint16_t*>(input)));
   return check_launch(op);
 }
 }  // namespace
@@ -772,19 +881,20 @@ int32_t gemb_rmsnorm_residual(const void* input, int32_t input_dtype, const uint
     return launch_row_warp<kRowResidual, false>(op, a, stream);
   }
   const dim3 grid(static_cast<unsigned>(vectors));
+  auto launch = [&](auto* x, auto* res, auto* o) -> int32_t {
+    using In = std::remove_const_t<std::remove_pointer_t<decltype(x)>>;
+    using Res = std::remove_const_t<std::remove_pointer_t<decltype(res)>>;
+    using Out = std::remove_pointer_t<decltype(o)>;
+    auto kern = short_rows(vectors, width) ? rmsnorm_residual_kernel<In, Res, Out, true> : rmsnorm_residual_kernel<In, Res, Out, false>;
+    return launch_pdl(op, kern, grid, dim3(256), 0, stream, x, weight_bf16, res, normalized_output, o, width, epsilon, scalar_bf16);
+  };
   const auto* xb = static_cast<const uint16_t*>(input);
   if (bf16_out)
-    GEMB_TRY(launch_pdl(op, rmsnorm_residual_kernel<uint16_t, uint16_t, uint16_t>, grid, dim3(256), 0, stream, xb, weight_bf16,
-                        static_cast<const uint16_t*>(residual), normalized_output, static_cast<uint16_t*>(output), width,
-                        epsilon, scalar_bf16));
+    GEMB_TRY(launch(xb, static_cast<const uint16_t*>(residual), static_cast<uint16_t*>(output)));
   else if (input_dtype == GEMB_BF16)
-    GEMB_TRY(launch_pdl(op, rmsnorm_residual_kernel<uint16_t, float, float>, grid, dim3(256), 0, stream, xb, weight_bf16,
-                        static_cast<const float*>(residual), normalized_output, static_cast<float*>(output), width, epsilon,
-                        scalar_bf16));
+    GEMB_TRY(launch(xb, static_cast<const float*>(residual), static_cast<float*>(output)));
   else
-    GEMB_TRY(launch_pdl(op, rmsnorm_residual_kernel<float, float, float>, grid, dim3(256), 0, stream,
-                        static_cast<const float*>(input), weight_bf16, static_cast<const float*>(residual), normalized_output,
-                        static_cast<float*>(output), width, epsilon, scalar_bf16));
+    GEMB_TRY(launch(static_cast<const float*>(input), static_cast<const float*>(residual), static_cast<float*>(output)));
   return check_launch(op);
 }
 
