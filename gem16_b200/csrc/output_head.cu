@@ -157,6 +157,175 @@ output_head_kernel(const uint16_t* __restrict__ weights, const float* __restrict
   }
 }
 
+// ---------------------------------------------------------------------------------------------
+// Three to eight hidden rows on the warp-level tensor-core path (mma.sync m16n8k16, bf16 x bf16 -> fp32): the weights are the M
+// side as they lie in memory, the hidden rows its eight columns.  An fp32 hidden value is the exact sum of three bf16 values
+// (its mantissa cut into eight bits each), so three MMAs per 16 k give the fp32 products; two chains of two (32 products each)
+// start from zero and join the running fp32 sum with IEEE additions.  The fma form above spends an fma and its share of
+// the unpacking per hidden row and weight: 262,144 x 3,840 with 3 / 5 / 8 rows 437 / 507 / 1,045 us there, 322 here (2.01 GB: 312 at the
+// copy rate).
+//
+// One CTA of sixteen warps per SM, the split hidden rows in shared memory in MMA order.  A task is sixteen vocabulary rows = the
+// eight tokens that two neighbouring candidate blocks take in one of their steps; a CTA owns whole pairs of blocks and
+// deals their tasks to its warps, so that a block's candidate is found inside the CTA.  Lane 4g + t loads 32 bytes of rows g
+// and g + 8 per 64 k, three such pieces ahead.
+// ---------------------------------------------------------------------------------------------
+constexpr int kHmWarps = 16, kHmThreads = kHmWarps * 32, kHmAhead = 3;
+constexpr uint32_t kHmMinRows = 3;   // two rows: 311 us in the fma form, 320 here
+constexpr uint32_t kHmPairs = kOhBlocks / 2;               // pairs of candidate blocks
+constexpr uint32_t kHmStepTokens = kOhBlocks * kOhWarps;   // tokens all blocks take in one step
+
+__device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void load_32_bytes(uint32_t (&r)[8], const uint16_t* w, bool in) {
+  asm volatile("{ .reg .pred p; setp.ne.b32 p, %9, 0;\n"
+               "@p ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8]; }"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
+               : "l"(w), "r"(static_cast<uint32_t>(in)));
+}
+__host__ __device__ inline uint32_t head_mma_tasks(uint32_t ctas, uint32_t vocab) {   // of the CTA that has the most
+  return (kHmPairs + ctas - 1) / ctas * ((vocab + kHmStepTokens - 1) / kHmStepTokens);
+}
+
+__global__ void __launch_bounds__(kHmThreads, 1)
+output_head_mma_kernel(const uint16_t* __restrict__ weights, const float* __restrict__ hidden_rows, uint32_t rows,
+                       const uint32_t* __restrict__ suppressed, uint32_t suppressed_count,
+                       const uint32_t* __restrict__ dynamic_suppressed_count, Candidate* __restrict__ candidates,
+                       float* __restrict__ logits_out, uint32_t vocab, uint32_t hidden) {
+  extern __shared__ __align__(16) uint4 hm_smem[];
+  const uint32_t chunks = (hidden + 63) / 64, steps = (vocab + kHmStepTokens - 1) / kHmStepTokens;
+  uint4* bs = hm_smem;   // [chunk][split][half of the chunk's MMAs][lane]
+  Candidate* best = reinterpret_cast<Candidate*>(bs + static_cast<size_t>(chunks) * 3 * 2 * 32);   // [task][block of the pair][8]
+  const uint32_t warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const uint32_t pairs = (kHmPairs - blockIdx.x + gridDim.x - 1) / gridDim.x, tasks = pairs * steps;
+  // Load cursor: piece `lc` of task `lt`.
+  uint32_t lt = warp, lc = 0;
+  const uint16_t* pw[2] = {weights, weights};
+  auto first_token = [&](uint32_t task) { return task % steps * kHmStepTokens + (blockIdx.x + gridDim.x * (task / steps)) * 16; };
+  auto aim = [&]() {
+    if (lt >= tasks) return;
+    const uint32_t tok0 = first_token(lt);
+    pw[0] = weights + static_cast<uint64_t>(min(tok0 + g, vocab - 1)) * hidden + t * 16;
+    pw[1] = weights + static_cast<uint64_t>(min(tok0 + 8 + g, vocab - 1)) * hidden + t * 16;
+  };
+  uint32_t wa[kHmAhead][8], wb[kHmAhead][8];
+  auto load = [&](int u) {
+    const bool in = lt < tasks && lc * 64 + t * 16 < hidden;
+    if (lc * 64 + 64 > hidden) {   // past K zero weights meet zero activations
+#pragma unroll
+      for (int i = 0; i < 8; ++i) wa[u][i] = wb[u][i] = 0;
+    }
+    load_32_bytes(wa[u], pw[0] + lc * 64, in);
+    load_32_bytes(wb[u], pw[1] + lc * 64, in);
+    if (++lc == chunks) {
+      lc = 0;
+      lt += kHmWarps;
+      aim();
+    }
+  };
+  aim();
+#pragma unroll
+  for (int u = 0; u < kHmAhead; ++u) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) wa[u][i] = wb[u][i] = 0;
+    load(u);
+  }
+  // under the first loads
+  for (uint32_t idx = threadIdx.x; idx < chunks * 64; idx += kHmThreads) {
+    const uint32_t chunk = idx / 64, half = idx / 32 & 1, cg = (idx & 31) >> 2, ct = idx & 3, k = chunk * 64 + ct * 16 + half * 8;
+    uint32_t out[3][4] = {};
+    if (cg < rows && k < hidden) {
+      const float4 a = __ldg(reinterpret_cast<const float4*>(hidden_rows + static_cast<uint64_t>(cg) * hidden + k));
+      const float4 b = __ldg(reinterpret_cast<const float4*>(hidden_rows + static_cast<uint64_t>(cg) * hidden + k) + 1);
+      const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        float rest = v[i];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          const uint32_t top = __float_as_uint(rest) & 0xFFFF0000u;
+          out[q][i / 2] |= (i & 1) ? top : top >> 16;
+          rest = isfinite(v[i]) ? __fsub_rn(rest, __uint_as_float(top)) : 0.0f;
+        }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q) bs[((chunk * 3 + q) * 2 + half) * 32 + (idx & 31)] = make_uint4(out[q][0], out[q][1], out[q][2], out[q][3]);
+  }
+  __syncthreads();
+  const uint32_t n_sup = dynamic_suppressed_count != nullptr ? __ldg(dynamic_suppressed_count) : suppressed_count;
+
+  float acc[3][4] = {};
+  // acc[.][0], acc[.][1]: token g, hidden rows 2t, 2t + 1; acc[.][2], acc[.][3]: token g + 8
+  auto emit = [&](uint32_t task) {
+    const uint32_t tok0 = first_token(task);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t token = tok0 + g + 8 * h;
+      const bool live = token < vocab, allowed = live && !is_suppressed(token, suppressed, n_sup);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const uint32_t r = 2 * t + j;
+        const int i = 2 * h + j;
+        const float capped = tanhf(__fadd_rn(acc[0][i], __fadd_rn(acc[1][i], acc[2][i])) / 30.0f) * 30.0f;   // src/cuda/output_head.cu:53,88
+        if (logits_out != nullptr && live && r < rows) logits_out[static_cast<uint64_t>(r) * vocab + token] = capped;
+        Candidate c{-FLT_MAX, 0u};
+        if (allowed && better(capped, token, c)) c = {capped, token};
+#pragma unroll
+        for (int off = 4; off <= 16; off <<= 1) {   // the eight tokens of the block
+          const float ov = __shfl_xor_sync(0xFFFFFFFFu, c.value, off);
+          const uint32_t ot = __shfl_xor_sync(0xFFFFFFFFu, c.token, off);
+          if (better(ov, ot, c)) c = {ov, ot};
+        }
+        if (g == 0) best[(task * 2 + h) * 8 + r] = c;
+      }
+    }
+  };
+  uint32_t task = warp, cc = 0;
+  while (task < tasks) {
+#pragma unroll
+    for (int u = 0; u < kHmAhead; ++u) {
+      if (task >= tasks) break;   // warp-uniform
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        const uint4 b0 = bs[((cc * 3 + q) * 2) * 32 + lane], b1 = bs[((cc * 3 + q) * 2 + 1) * 32 + lane];
+        float c[4] = {0.0f, 0.0f, 0.0f, 0.0f}, d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        mma_bf16(c, wa[u][0], wb[u][0], wa[u][1], wb[u][1], b0.x, b0.y);
+        mma_bf16(d, wa[u][4], wb[u][4], wa[u][5], wb[u][5], b1.x, b1.y);
+        mma_bf16(c, wa[u][2], wb[u][2], wa[u][3], wb[u][3], b0.z, b0.w);
+        mma_bf16(d, wa[u][6], wb[u][6], wa[u][7], wb[u][7], b1.z, b1.w);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[q][i] = __fadd_rn(acc[q][i], __fadd_rn(c[i], d[i]));
+      }
+      load(u);
+      if (++cc == chunks) {
+        emit(task);
+        cc = 0;
+        task += kHmWarps;
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) acc[q][i] = 0.0f;
+      }
+    }
+  }
+  __syncthreads();
+  if (candidates == nullptr) return;
+  for (uint32_t idx = threadIdx.x; idx < pairs * 2 * rows; idx += kHmThreads) {
+    const uint32_t r = idx % rows, h = idx / rows & 1, pair = idx / rows / 2;
+    Candidate c{-FLT_MAX, 0u};
+    for (uint32_t step = 0; step < steps; ++step) {
+      const Candidate o = best[((pair * steps + step) * 2 + h) * 8 + r];
+      if (better(o.value, o.token, c)) c = o;
+    }
+    candidates[static_cast<uint64_t>(r) * kOhBlocks + (blockIdx.x + gridDim.x * pair) * 2 + h] = c;
+  }
+}
+
 // One CTA per hidden row: best of its 4,096 candidates.
 __global__ void __launch_bounds__(kOhThreads)
 output_head_argmax_kernel(const Candidate* __restrict__ candidates, uint32_t* __restrict__ selected) {
@@ -207,6 +376,14 @@ int32_t launch_output_head(const char* op, const uint16_t* weights, const float*
   return check_launch(op);
 }
 
+// false: the shapes the tensor-core form does not take (rows that are not whole 32-byte pieces, hidden rows or candidates that do
+// not fit the shared memory of one CTA).
+bool head_mma_fits(const uint16_t* weights, uint32_t rows, uint32_t vocab, uint32_t hidden, size_t* smem) {
+  *smem = static_cast<size_t>((hidden + 63) / 64) * 3 * 2 * 32 * sizeof(uint4) +
+          static_cast<size_t>(head_mma_tasks(static_cast<uint32_t>(sm_count()), vocab)) * 2 * 8 * sizeof(Candidate);
+  return rows >= kHmMinRows && hidden % 16 == 0 && reinterpret_cast<uintptr_t>(weights) % 32 == 0 && *smem <= 227 * 1024;
+}
+
 }  // namespace
 }  // namespace gemb
 
@@ -237,6 +414,14 @@ int32_t gemb_output_head_candidates(const uint16_t* weights_bf16, const float* h
   Candidate* c = static_cast<Candidate*>(candidates);
   const uint32_t sc = static_cast<uint32_t>(suppressed_count), v = static_cast<uint32_t>(vocabulary),
                  h = static_cast<uint32_t>(hidden);
+  size_t smem = 0;
+  if (head_mma_fits(weights_bf16, static_cast<uint32_t>(rows), v, h, &smem)) {
+    const cudaError_t e = cudaFuncSetAttribute(output_head_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return fail(GEMB_INTERNAL, "%s: %s: %s", op, cudaGetErrorName(e), cudaGetErrorString(e));
+    output_head_mma_kernel<<<sm_count(), kHmThreads, smem, stream>>>(weights_bf16, hidden_rows, static_cast<uint32_t>(rows), suppressed, sc,
+                                                                     dynamic_suppressed_count, c, diagnostic_logits, v, h);
+    return check_launch(op);
+  }
   switch (rows) {
     case 1: return launch_output_head<1>(op, weights_bf16, hidden_rows, suppressed, sc, dynamic_suppressed_count, c, diagnostic_logits, v, h, stream);
     case 2: return launch_output_head<2>(op, weights_bf16, hidden_rows, suppressed, sc, dynamic_suppressed_count, c, diagnostic_logits, v, h, stream);

@@ -105,3 +105,26 @@ def test_output_head_ties_and_validation(lib, dev, orc):
         lib.gemb_output_head_candidates(wd, hd, 1, None, 0, None, cand, None, 2048, 100, None)     # hidden % 8
     with pytest.raises(GembError):
         lib.gemb_output_head_argmax(None, 1, sel, None)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,vocab,hidden", [(3, 17, 16), (4, 32769, 80), (8, 65536 + 9, 144), (7, 5, 3840), (3, 300, 24)])
+def test_output_head_rows_sharing_a_pass_at_the_edges(lib, dev, orc, rows, vocab, hidden):
+    """Token, step and K remainders of the tensor-core form, one shape it does not take; every candidate is written."""
+    w, h = make_case(orc, rows, vocab, hidden, rows + hidden)
+    want, _ = orc.output_head(w, h)
+    cand = torch.full((rows, 4096, 2), -1, dtype=torch.int32, device=dev)
+    logits = torch.full((rows, vocab), float("nan"), device=dev)
+    selected = torch.full((rows,), -1, dtype=torch.int32, device=dev)
+    lib.gemb_output_head_candidates(torch.from_numpy(w.view(np.int16)).to(dev), torch.from_numpy(h).to(dev), rows, None, 0, None, cand,
+                                    logits, vocab, hidden, None)
+    lib.gemb_output_head_argmax(cand, rows, selected, None)
+    got = logits.cpu().numpy()
+    assert np.abs(got - want).max() <= 2e-5 * max(1.0, np.abs(want).max())
+    assert np.array_equal(selected.cpu().numpy().astype(np.uint32), select(got, []))
+    block = (np.arange(vocab) % 32768) // 8
+    values = cand[:, :, 0].contiguous().view(torch.float32).cpu().numpy()
+    for r in range(rows):
+        best = np.full(4096, -np.finfo(np.float32).max, np.float32)
+        np.maximum.at(best, block, got[r])
+        assert np.array_equal(values[r], best)
