@@ -74,15 +74,18 @@ inline bool positive_finite(float v) { return std::isfinite(v) && v > 0.0f; }
     if (gemb_rc_ != GEMB_OK) return gemb_rc_; \
   } while (0)
 
-// Programmatic dependent launch.  A kernel launched through launch_pdl may become resident while its
-// predecessor in the stream still runs, so it
-//   - lets its own successor do the same (pdl_trigger), first thing;
-//   - calls pdl_wait in every CTA before it reads or writes any global memory.  The only accesses
-//     allowed before are prefetches into L2, which is coherent: they cannot return stale bytes, whoever
-//     writes the line later.  Every kernel of the chain waits, so "my predecessor has completed" implies
-//     that everything before it has;
-//   - reads what an earlier kernel wrote with ld_dep, not __ldg: the read-only path promises that the data
-//     does not change while the kernel is resident, which starts before pdl_wait here.
+// Programmatic dependent launch.  A kernel launched through launch_pdl may become resident while its predecessor in the
+// stream still runs.
+//   - pdl_trigger lets the successor do the same.  Row kernels, GEMVs and the routing kernels call it first thing, the plain
+//     quantisers for few rows only (pdl_trigger_few_rows); the GEMM and the expert dispatch never do (see there), nor do kernels
+//     launched with <<<>>>: their successors start when they have ended.
+//   - pdl_wait comes in every CTA before anything is written and before anything is read that another kernel of a running
+//     stream may still be writing.  Every kernel of the chain waits, so "my predecessor has completed" implies that
+//     everything before it has.
+//   - What may be read before pdl_wait is what no early-triggering kernel writes: weight matrices with their scales (the GEMVs'
+//     first pieces) and norm weights, straight into registers.  A kernel that writes such data must not trigger.
+//   - What an earlier kernel wrote is read with ld_dep, not __ldg: the read-only path promises that the data does not change
+//     while the kernel is resident, which starts before pdl_wait here.
 template <typename... P, typename... A>
 int32_t launch_pdl(const char* op, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
   cudaLaunchConfig_t cfg{};
@@ -112,10 +115,12 @@ int32_t launch_pdl(const char* op, void (*kern)(P...), dim3 grid, dim3 block, si
 
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
 // The decode GEMVs read their weights ahead of pdl_wait.  A quantiser, whose output may be a weight matrix, therefore lets
-// its dependents start early only for a decode batch's few rows; otherwise they start when
-// its CTAs have ended.
+// its dependents start early only for fewer rows than an NVFP4 weight matrix can have (its rows are a multiple of 8; an FP8
+// matrix gets its bf16 scales from a kernel outside this library, which lets nothing start early); otherwise they start
+// when its CTAs have ended.  Kernels whose output is no weight (norms, GEMVs, the expert path) trigger always.
+constexpr uint32_t kFewRows = 7;
 __device__ __forceinline__ void pdl_trigger_few_rows(uint32_t rows) {
-  if (rows <= 16) pdl_trigger();
+  if (rows <= kFewRows) pdl_trigger();
 }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Loads of data an earlier kernel of the stream produced (volatile: they stay behind pdl_wait).

@@ -226,7 +226,7 @@ fp8_gemv_kernel(const void* __restrict__ act, const float* __restrict__ act_scal
   // prefetch as soon as SM slots free up; weights are immutable so they may be read before the
   // previous kernel has finished, everything else waits for it.  (Loading them behind the wait, with an L2
   // prefetch in front of it, cost a four-layer FP8 decode pass 21 of 209 us.)  No kernel that could be writing
-  // weights triggers its dependents early: the quantisers do so for a decode batch only.
+  // weights triggers its dependents early: see pdl_trigger_few_rows.
   pdl_trigger();
   uint64_t task = static_cast<uint64_t>(blockIdx.x) * kW + warp;
   bool prefetched = false;
@@ -909,16 +909,16 @@ int32_t validate_fp8_gemv(const char* op, const void* act, const void* w, const 
 // ---------------------------------------------------------------------------------------------
 // Decode-time FP8 token quantizer: one 1024-thread CTA per token, the token held in registers
 // between the amax pass and the conversion (one global round trip), quotients through
-// e4m3_of_quotients (bit-identical to the IEEE division of src/numeric/fp8.cpp:41-58).  It
-// triggers its dependents at once and waits for its predecessor before touching the
-// activation, so under programmatic dependent launch the GEMV that follows can prefetch its
+// e4m3_of_quotients (bit-identical to the IEEE division of src/numeric/fp8.cpp:41-58).  For a
+// decode step's few rows it triggers its dependents at once and waits for its predecessor before
+// touching the activation, so under programmatic dependent launch the GEMV that follows can prefetch its
 // weights while this kernel runs.  bf16 input, K <= 16384, K % 8 == 0.
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(1024)
 fp8_quantize_decode_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ out,
                            float* __restrict__ scales, uint32_t k) {
   __shared__ float red[32];
-  pdl_trigger();
+  pdl_trigger_few_rows(gridDim.x);
   pdl_wait();
   const uint64_t t = blockIdx.x;
   const uint4* xp = reinterpret_cast<const uint4*>(x + t * k);

@@ -189,6 +189,14 @@ int32_t gemb_add_residual_f32(const float* values, const float* residual, float*
 /* ------------------------------------------------------------------------------------------
  * Batch-1 decode projections (HBM-streaming GEMV).  Weights are row-major [rows, K] in the
  * checkpoint's source layout; NVFP4 block scales are COMPACT [rows, K/16].
+ *
+ * Weights are taken to be at rest: these calls request their first weight bytes (gemb_rmsnorm_residual and the
+ * RMSNorm quantizers their norm weights) while the kernels in front of them in the stream still run.  What a copy, a memset,
+ * a kernel from elsewhere or a call of this library that writes a whole weight matrix has written by then is
+ * always seen (gemb_nvfp4_quantize and gemb_fp8_quantize of eight rows or more, gemb_nvfp4_interleave_scales,
+ * gemb_nvfp4_pack_gate_up).  Only a matrix that is being quantised in pieces of fewer than eight rows -- the size of a
+ * decode step's activations, whose quantizers overlap the projection behind them -- must be separated from
+ * the first call that uses it as a weight by a synchronisation or a copy, or be used with GEMB_TUNE_GEMV_PDL 0.
  * ---------------------------------------------------------------------------------------- */
 
 /* y[row] = (sum_k qa qw) * a_scale * bf16(w_scale[row]), fp32 out.  K % 16 == 0.

@@ -290,3 +290,55 @@ def test_nvfp4_gemv_tiles_and_token_counts(lib, dev, orc, rows, k, shift):
         assert np.linalg.norm(to_np(g) - want[:t]) <= 1e-6 * np.linalg.norm(want[:t])
     for t, o in outs.items():
         assert all(torch.equal(a, b[:t]) for a, b in zip(o, outs[t_max]))
+
+
+@pytest.mark.parametrize("rows,k", [(8, 64), (8, 15360), (16, 3840), (24, 8192)])
+@pytest.mark.parametrize("act_first", [False, True])
+def test_weight_quantised_on_the_device_is_seen_at_once(lib, dev, rows, k, act_first):
+    """A whole weight matrix, however small, may be quantised right in front of the GEMV that uses it, although the GEMV
+    requests weights while the kernels before it still run: the same buffers take two matrices in turn, and every
+    product equals the one computed with the device idle in between."""
+    gen = torch.Generator(device=dev).manual_seed(rows + k)
+    w = [(torch.randn((rows, k), device=dev, generator=gen) * 0.02).to(torch.bfloat16).view(torch.int16) for _ in range(2)]
+    x = torch.randn((1, k), device=dev, generator=gen).to(torch.bfloat16).view(torch.int16)
+    ga, gw, reps = 500.0, 20000.0, 24
+    u8, f32 = torch.uint8, torch.float32
+    xp, xs = torch.zeros((1, k // 2), dtype=u8, device=dev), torch.zeros((1, k // 16), dtype=u8, device=dev)
+    wp, ws = torch.zeros((rows, k // 2), dtype=u8, device=dev), torch.zeros((rows, k // 16), dtype=u8, device=dev)
+    xq, xsc = torch.zeros((1, k), dtype=u8, device=dev), torch.zeros((1,), dtype=f32, device=dev)
+    wq, wsc = torch.zeros((rows, k), dtype=u8, device=dev), torch.zeros((rows,), dtype=f32, device=dev)
+    ones = torch.full((rows,), 0x3F80, dtype=torch.int16, device=dev)   # bf16 row scales known beforehand
+    y4, y8 = torch.zeros((reps, rows), device=dev), torch.zeros((reps, rows), device=dev)
+
+    def sync(on):
+        if on:
+            torch.cuda.synchronize()
+
+    def nvfp4(i, y, idle):
+        steps = [lambda: lib.gemb_nvfp4_quantize(w[i % 2], 1, wp, ws, rows, k, gw, 0, 0, None),
+                 lambda: lib.gemb_nvfp4_quantize(x, 1, xp, xs, 1, k, ga, 0, 0, None)]
+        for step in (steps[::-1] if act_first else steps):
+            step()
+        sync(idle)
+        lib.gemb_nvfp4_gemv(xp, xs, wp, ws, y, rows, k, ga, gw, None)
+        sync(idle)
+
+    def fp8(i, y, idle):
+        steps = [lambda: lib.gemb_fp8_quantize(w[i % 2], 1, wq, wsc, rows, k, None),
+                 lambda: lib.gemb_fp8_quantize(x, 1, xq, xsc, 1, k, None)]
+        for step in (steps[::-1] if act_first else steps):
+            step()
+        sync(idle)
+        lib.gemb_fp8_gemv(xq, xsc, wq, ones, y, rows, k, None)
+        sync(idle)
+
+    for run, y in ((nvfp4, y4), (fp8, y8)):
+        want = torch.zeros((2, rows), device=dev)
+        for i in range(2):
+            run(i, want[i], True)
+        assert not torch.equal(want[0], want[1])
+        for i in range(reps):
+            run(i, y[i], False)
+        torch.cuda.synchronize()
+        for i in range(reps):
+            assert torch.equal(y[i], want[i % 2]), i
