@@ -7,6 +7,7 @@
 #include <cuda_fp8.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cmath>
 #include <cstdint>
 
@@ -73,6 +74,29 @@ inline bool positive_finite(float v) { return std::isfinite(v) && v > 0.0f; }
     int32_t gemb_rc_ = (expr);           \
     if (gemb_rc_ != GEMB_OK) return gemb_rc_; \
   } while (0)
+
+// Lets kKernel use all the dynamic shared memory that a CTA of the current device can have, once per device.  Never the size
+// of the call at hand: the limit belongs to the kernel, and a second host thread with a smaller size would lower it between
+// the first one's set and its launch.
+template <auto kKernel>
+int32_t allow_full_smem(const char* op) {
+  static std::atomic<uint64_t> done{0};
+  int dev = 0, optin = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  const uint64_t bit = 1ull << (dev & 63);
+  if (e == cudaSuccess && (done.load(std::memory_order_relaxed) & bit) != 0) return GEMB_OK;
+  cudaFuncAttributes attr{};
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, kKernel);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - static_cast<int>(attr.sharedSizeBytes));
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(GEMB_INTERNAL, "%s: %s: %s", op, cudaGetErrorName(e), cudaGetErrorString(e));
+  }
+  done.fetch_or(bit, std::memory_order_relaxed);
+  return GEMB_OK;
+}
 
 // Programmatic dependent launch.  A kernel launched through launch_pdl may become resident while its predecessor in the
 // stream still runs.

@@ -293,33 +293,38 @@ int pick_rows_per_warp(uint64_t total_rows, uint64_t k) {
   return 1;
 }
 
+// CTAs of `threads` threads and `smem` bytes that an SM holds; the last answer is kept per device, size and count in one word so
+// that threads with different sizes cannot mix them up.
+template <auto kKernel>
+int32_t resident_ctas(const char* op, int threads, size_t smem, int* ctas) {
+  static std::atomic<uint64_t> last[64];
+  GEMB_TRY(allow_full_smem<kKernel>(op));
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const uint64_t seen = last[dev & 63].load(std::memory_order_relaxed);
+  if ((seen & 0xFFFF) != 0 && seen >> 16 == smem) {
+    *ctas = static_cast<int>(seen & 0xFFFF);
+    return GEMB_OK;
+  }
+  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas, kKernel, threads, smem);
+  if (e != cudaSuccess || *ctas < 1) {
+    cudaGetLastError();
+    return fail(GEMB_INTERNAL, "%s: occupancy query failed: %s", op, cudaGetErrorName(e));
+  }
+  last[dev & 63].store(static_cast<uint64_t>(smem) << 16 | static_cast<uint64_t>(*ctas), std::memory_order_relaxed);
+  return GEMB_OK;
+}
+
 template <int kRows, int kUnroll, bool kFusedQuant, bool kBf16Out>
 int32_t launch_fp8_gemv_variant(const char* op, const void* act, const float* act_scale,
                                 const Fp8Group& grp, uint64_t k, cudaStream_t stream) {
   constexpr int kW = fp8_gemv_warps<kFusedQuant>();
   auto kern = fp8_gemv_kernel<kRows, kUnroll, kFusedQuant, kBf16Out>;
   const size_t smem = (k + 511) / 512 * 512 * sizeof(__half);
-  static int resident[64] = {0};      // CTAs per SM, per device, for the smem size last seen
-  static size_t resident_smem[64] = {0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  dev &= 63;
-  if (resident[dev] == 0 || smem != resident_smem[dev]) {
-    if (smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           static_cast<int>(smem));
-      if (e != cudaSuccess)
-        return fail(GEMB_INTERNAL, "%s: %s: %s", op, cudaGetErrorName(e), cudaGetErrorString(e));
-    }
-    int occ = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kW * 32, smem);
-    if (e != cudaSuccess || occ < 1)
-      return fail(GEMB_INTERNAL, "%s: occupancy query failed: %s", op, cudaGetErrorName(e));
-    resident[dev] = occ;
-    resident_smem[dev] = smem;
-  }
+  int resident = 0;
+  GEMB_TRY((resident_ctas<fp8_gemv_kernel<kRows, kUnroll, kFusedQuant, kBf16Out>>(op, kW * 32, smem, &resident)));
   const uint64_t tasks = (grp.row_start[grp.n] + kRows - 1) / kRows;
-  const uint64_t wave = static_cast<uint64_t>(sm_count()) * resident[dev];
+  const uint64_t wave = static_cast<uint64_t>(sm_count()) * resident;
   const unsigned blocks = static_cast<unsigned>(std::min<uint64_t>((tasks + kW - 1) / kW, wave));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(blocks);
@@ -424,24 +429,10 @@ int32_t launch_fp8_gemv_batch_variant(const char* op, const uint8_t* act, const 
                                       uint64_t k, cudaStream_t stream) {
   auto kern = fp8_gemv_batch_kernel<kTok>;
   const size_t smem = static_cast<size_t>(kTok) * ((k + 511) / 512 * 512) * sizeof(__half);
-  static int resident[64] = {0};
-  static size_t resident_smem[64] = {0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  dev &= 63;
-  if (resident[dev] == 0 || smem != resident_smem[dev]) {
-    if (smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-      if (e != cudaSuccess) return fail(GEMB_INTERNAL, "%s: %s: %s", op, cudaGetErrorName(e), cudaGetErrorString(e));
-    }
-    int occ = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kWarps * 32, smem);
-    if (e != cudaSuccess || occ < 1) return fail(GEMB_INTERNAL, "%s: occupancy query failed: %s", op, cudaGetErrorName(e));
-    resident[dev] = occ;
-    resident_smem[dev] = smem;
-  }
+  int resident = 0;
+  GEMB_TRY((resident_ctas<fp8_gemv_batch_kernel<kTok>>(op, kWarps * 32, smem, &resident)));
   const uint64_t tasks = grp.row_start[grp.n];
-  const uint64_t wave = static_cast<uint64_t>(sm_count()) * resident[dev];
+  const uint64_t wave = static_cast<uint64_t>(sm_count()) * resident;
   const unsigned blocks = static_cast<unsigned>(std::min<uint64_t>((tasks + kWarps - 1) / kWarps, wave));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(blocks);
@@ -846,15 +837,7 @@ int32_t launch_fp8_gemv_ring(const char* op, const void* act, const float* act_s
   const uint32_t stages = kRingConsumers;
   const size_t smem = x_bytes + static_cast<size_t>(stages) * kRingStageBytes + 2 * stages * 8 + kRingConsumers * 4 + 64;
   auto kern = fp8_gemv_ring_kernel<kFusedQuant, kBf16Out>;
-  static bool configured[64] = {false};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  dev &= 63;
-  if (!configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    if (e != cudaSuccess) return fail(GEMB_INTERNAL, "%s: %s: %s", op, cudaGetErrorName(e), cudaGetErrorString(e));
-    configured[dev] = true;
-  }
+  GEMB_TRY((allow_full_smem<fp8_gemv_ring_kernel<kFusedQuant, kBf16Out>>(op)));
   uint64_t chunks = 0;
   for (int i = 0; i < grp.n; ++i) chunks += (grp.p[i].rows + rows_per_chunk - 1) / rows_per_chunk;
   cudaLaunchConfig_t cfg{};

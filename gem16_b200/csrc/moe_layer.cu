@@ -386,10 +386,7 @@ int32_t gemb_moe_router_input(const uint16_t* x_bf16, const uint16_t* scale_bf16
     return check_launch(op);
   }
   const uint32_t smem = router_input_smem(h);
-  if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(router_input_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e != cudaSuccess) return fail(GEMB_INTERNAL, "%s: %s: %s", op, cudaGetErrorName(e), cudaGetErrorString(e));
-  }
+  GEMB_TRY(allow_full_smem<router_input_kernel>(op));
   const bool vec = reinterpret_cast<uintptr_t>(scale_bf16) % 16 == 0 && reinterpret_cast<uintptr_t>(out_bf16) % 16 == 0;
   GEMB_TRY(launch_pdl(op, router_input_kernel, dim3((t + kRiTokens - 1) / kRiTokens), dim3(kRiThreads), smem, stream, x_bf16,
                       scale_bf16, out_bf16, t, h, epsilon, root, vec));

@@ -356,8 +356,7 @@ template <int kTok, int kExp>
 int32_t launch_router(const char* op, const RouterArgs& a, cudaStream_t stream) {
   using S = RouterShape<kTok, kExp>;
   auto kern = router_logits_kernel<kTok, kExp>;
-  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(typename S::Smem)));
-  if (e != cudaSuccess) return fail(GEMB_INTERNAL, "%s: %s: %s", op, cudaGetErrorName(e), cudaGetErrorString(e));
+  GEMB_TRY((allow_full_smem<router_logits_kernel<kTok, kExp>>(op)));
   const bool x_wide = a.hidden % 8 == 0 && reinterpret_cast<uintptr_t>(a.x) % 16 == 0;
   // Not a dependent launch: CTAs placed while the kernel before this one still fills SMs end up two on one SM and none on
   // another (2,048 tokens: 57 us this way, 81 us behind a kernel that triggers early).

@@ -302,10 +302,7 @@ int32_t launch_nvfp4_gemv(const char* op, Fp4GemvArgs a, cudaStream_t stream) {
     a.wide = a.wide && reinterpret_cast<uintptr_t>(a.m[m].w) % 32 == 0 && reinterpret_cast<uintptr_t>(a.m[m].ws) % 4 == 0;
   const size_t smem = 128 + fp4_stage_bytes(a.tokens, a.k) + kFpWarps * 2 * 32 * sizeof(float4);
   auto kern = nvfp4_gemv_kernel<kGateUp>;
-  if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e != cudaSuccess) return fail(GEMB_INTERNAL, "%s: %s: %s", op, cudaGetErrorName(e), cudaGetErrorString(e));
-  }
+  GEMB_TRY(allow_full_smem<nvfp4_gemv_kernel<kGateUp>>(op));
   // One CTA per SM (registers allow no second one), tiles dealt out round robin.
   const uint32_t tile_rows = kGateUp ? 8 : 16, tiles = (a.rows + tile_rows - 1) / tile_rows;
   GEMB_TRY(launch_pdl(op, kern, dim3(std::min(tiles, static_cast<uint32_t>(sm_count()))), dim3(kFpThreads), smem, stream, a));

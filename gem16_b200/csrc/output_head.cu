@@ -362,15 +362,7 @@ int32_t launch_output_head(const char* op, const uint16_t* weights, const float*
                            uint32_t suppressed_count, const uint32_t* dynamic_count, Candidate* candidates,
                            float* logits, uint32_t vocab, uint32_t hidden, cudaStream_t stream) {
   const size_t smem = static_cast<size_t>(kRows) * hidden * sizeof(float);
-  static bool configured[64] = {false};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  dev &= 63;
-  if (!configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(output_head_kernel<kRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (e != cudaSuccess) return fail(GEMB_INTERNAL, "%s: %s: %s", op, cudaGetErrorName(e), cudaGetErrorString(e));
-    configured[dev] = true;
-  }
+  GEMB_TRY(allow_full_smem<output_head_kernel<kRows>>(op));
   output_head_kernel<kRows><<<kOhBlocks, kOhThreads, smem, stream>>>(weights, hidden_rows, suppressed, suppressed_count,
                                                                     dynamic_count, candidates, logits, vocab, hidden);
   return check_launch(op);
@@ -416,8 +408,7 @@ int32_t gemb_output_head_candidates(const uint16_t* weights_bf16, const float* h
                  h = static_cast<uint32_t>(hidden);
   size_t smem = 0;
   if (head_mma_fits(weights_bf16, static_cast<uint32_t>(rows), v, h, &smem)) {
-    const cudaError_t e = cudaFuncSetAttribute(output_head_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e != cudaSuccess) return fail(GEMB_INTERNAL, "%s: %s: %s", op, cudaGetErrorName(e), cudaGetErrorString(e));
+    GEMB_TRY(allow_full_smem<output_head_mma_kernel>(op));
     output_head_mma_kernel<<<sm_count(), kHmThreads, smem, stream>>>(weights_bf16, hidden_rows, static_cast<uint32_t>(rows), suppressed, sc,
                                                                      dynamic_suppressed_count, c, diagnostic_logits, v, h);
     return check_launch(op);
