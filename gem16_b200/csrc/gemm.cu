@@ -508,7 +508,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     if constexpr (kSplit > 1) {
       // Every CTA leaves its partial accumulator in shared memory (the operand stages are free: its last MMA has
       // completed; rows of 132 words are conflict-free for a lane per row), then takes BN / kSplit columns and adds the
-      // parts of all CTAs in K order, read through the cluster's shared window.  Plain bf16 output only.
+      // parts of all CTAs in K order, read through the cluster's shared window.  The forms that quantise the GELU product need whole
+      // blocks of columns: there a CTA takes every kSplit-th row.
       uint32_t mt, nt;
       tile_coords(first_tile, mt, nt);
       constexpr int kStride = BN + 4;
@@ -532,23 +533,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
       ptx::tc_fence_before();
       __syncwarp();
       ptx::cluster_sync();
-      // Eight or sixteen lanes per row: whole 128-byte lines through the shared window, whole sectors out.
-      constexpr uint32_t kLanes = BN / kSplit / 4, kRows = 32 / kLanes;
-      const uint32_t col = split * (BN / kSplit) + lane % kLanes * 4, gcol = nt * BN + col;
-      uint2 ws = make_uint2(0, 0);
-      if constexpr (!kFp4) {
-        if (gcol < p.n) ws = make_uint2(__ldg(reinterpret_cast<const uint32_t*>(p.w_scales + gcol)), __ldg(reinterpret_cast<const uint32_t*>(p.w_scales + gcol) + 1));
-      }
       const uint32_t rows = min(static_cast<uint32_t>(BM), p.m - mt * BM);
-#pragma unroll 2
-      for (uint32_t r0 = (set * 4 + quarter) * kRows; r0 < rows; r0 += 8 * kRows) {   // rows past `rows` of a trip: old bytes, not stored
-        const uint32_t r = r0 + lane / kLanes, row = mt * BM + r;
+      auto row_sum = [&](uint32_t r, uint32_t col) {   // four columns of a row, the parts added in K order
         float4 v[kSplit];
 #pragma unroll
         for (int c = 0; c < kSplit; ++c) v[c] = ptx::ld_cluster_f4(ptx::cluster_map(reinterpret_cast<float*>(smem) + r * kStride + col, c));
-        if (r >= rows || gcol >= p.n) continue;   // n is a multiple of 8
-        float row_scale = p.alpha;
-        if constexpr (!kFp4) row_scale = ld_dep(p.a_scales + row);
 #pragma unroll
         for (int c = 1; c < kSplit; ++c) {
           v[0].x = __fadd_rn(v[0].x, v[c].x);
@@ -556,15 +545,70 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
           v[0].z = __fadd_rn(v[0].z, v[c].z);
           v[0].w = __fadd_rn(v[0].w, v[c].w);
         }
-        float o[4] = {__fmul_rn(v[0].x, row_scale), __fmul_rn(v[0].y, row_scale), __fmul_rn(v[0].z, row_scale), __fmul_rn(v[0].w, row_scale)};
-        if constexpr (!kFp4) {
-          o[0] = __fmul_rn(o[0], __uint_as_float(ws.x << 16));
-          o[1] = __fmul_rn(o[1], __uint_as_float(ws.x & 0xFFFF0000u));
-          o[2] = __fmul_rn(o[2], __uint_as_float(ws.y << 16));
-          o[3] = __fmul_rn(o[3], __uint_as_float(ws.y & 0xFFFF0000u));
+        return v[0];
+      };
+      if (kFp4 && (p.gated || p.gate_in != nullptr)) {
+        // A warp per row, four columns per lane; a block of 16 product features is four neighbouring lanes.  Gated: of the
+        // sixteen lanes of a 64-column group the upper eight hold the up values of the lower eight's gate features.
+        // The arithmetic is that of the epilogues below, value for value.
+        const uint32_t col = lane * 4, feats = p.gated ? p.n / 2 : p.n, c_pad = (feats / 16 + 3) / 4 * 4;
+        const uint32_t f = p.gated ? nt * (BN / 2) + lane / 16 * 32 + lane % 8 * 4 : nt * BN + col;
+        const bool holds_up = p.gated && (lane & 8) != 0, live = f < feats && !holds_up;
+        const float alpha = holds_up ? p.alpha_up : p.alpha;
+        for (uint32_t r = split + kSplit * (set * 4 + quarter); r < rows; r += kSplit * 8) {   // warp-uniform
+          const uint64_t row = mt * BM + r;
+          uint2 gate = make_uint2(0, 0);
+          if (!p.gated && live) {
+            const uint16_t* gp = p.gate_in + row * p.n + f;
+            gate = make_uint2(ld_dep(reinterpret_cast<const int32_t*>(gp)), ld_dep(reinterpret_cast<const int32_t*>(gp) + 1));
+          }
+          const float4 sum = row_sum(r, col);
+          const float v[4] = {bf16_round(__fmul_rn(sum.x, alpha)), bf16_round(__fmul_rn(sum.y, alpha)), bf16_round(__fmul_rn(sum.z, alpha)),
+                              bf16_round(__fmul_rn(sum.w, alpha))};
+          const float given[4] = {__uint_as_float(gate.x << 16), __uint_as_float(gate.x & 0xFFFF0000u), __uint_as_float(gate.y << 16),
+                                  __uint_as_float(gate.y & 0xFFFF0000u)};
+          float prod[4], amax = 0.0f;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float up = __shfl_down_sync(0xFFFFFFFFu, v[i], 8);
+            prod[i] = p.gated ? gelu_tanh_product(v[i], up) : gelu_tanh_product(given[i], v[i]);
+            amax = fmaxf(amax, fabsf(prod[i]));
+          }
+          amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
+          amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 2));
+          const BlockScale s = block_scale<false>(amax, p.g_product);
+          uint32_t codes = quantize_pair<false>(make_float2(prod[0], prod[1]), p.g_product, s) |
+                           quantize_pair<false>(make_float2(prod[2], prod[3]), p.g_product, s) << 8;
+          if (s.ds == 0.0f) codes = 0;
+          if (!live) continue;
+          *reinterpret_cast<uint16_t*>(p.out_packed + row * (feats / 2) + f / 2) = static_cast<uint16_t>(codes);
+          if ((lane & 3) == 0) p.out_scales[interleaved_scale_offset(row, f / 16, c_pad)] = s.bits;
         }
-        *reinterpret_cast<uint2*>(static_cast<uint16_t*>(p.out) + static_cast<uint64_t>(row) * p.n + gcol) =
-            make_uint2(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]));
+      } else {
+        // Eight or sixteen lanes per row: whole 128-byte lines through the shared window, whole sectors out.
+        constexpr uint32_t kLanes = BN / kSplit / 4, kRows = 32 / kLanes;
+        const uint32_t col = split * (BN / kSplit) + lane % kLanes * 4, gcol = nt * BN + col;
+        uint2 ws = make_uint2(0, 0);
+        if constexpr (!kFp4) {
+          if (gcol < p.n) ws = make_uint2(__ldg(reinterpret_cast<const uint32_t*>(p.w_scales + gcol)), __ldg(reinterpret_cast<const uint32_t*>(p.w_scales + gcol) + 1));
+        }
+#pragma unroll 2
+        for (uint32_t r0 = (set * 4 + quarter) * kRows; r0 < rows; r0 += 8 * kRows) {   // rows past `rows` of a trip: old bytes, not stored
+          const uint32_t r = r0 + lane / kLanes, row = mt * BM + r;
+          float row_scale = p.alpha;
+          if constexpr (!kFp4) row_scale = r < rows ? ld_dep(p.a_scales + row) : 0.0f;   // in flight beside the parts
+          const float4 v = row_sum(r, col);
+          if (r >= rows || gcol >= p.n) continue;   // n is a multiple of 8
+          float o[4] = {__fmul_rn(v.x, row_scale), __fmul_rn(v.y, row_scale), __fmul_rn(v.z, row_scale), __fmul_rn(v.w, row_scale)};
+          if constexpr (!kFp4) {
+            o[0] = __fmul_rn(o[0], __uint_as_float(ws.x << 16));
+            o[1] = __fmul_rn(o[1], __uint_as_float(ws.x & 0xFFFF0000u));
+            o[2] = __fmul_rn(o[2], __uint_as_float(ws.y << 16));
+            o[3] = __fmul_rn(o[3], __uint_as_float(ws.y & 0xFFFF0000u));
+          }
+          *reinterpret_cast<uint2*>(static_cast<uint16_t*>(p.out) + static_cast<uint64_t>(row) * p.n + gcol) =
+              make_uint2(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]));
+        }
       }
     } else
     for (uint32_t tile = first_tile; tile < num_tiles && !*abort_flag; tile += tile_stride) {
@@ -922,6 +966,8 @@ thread_local uint64_t g_grouped_rows_hint = 0;
 // Upper bound on the persistent grid of the GEMMs this thread launches (0 = none): lets a caller run two
 // GEMMs side by side on disjoint sets of SMs instead of having their CTAs take turns.
 thread_local uint32_t g_gemm_cta_cap = 0;
+// Whether the dense GEMMs this thread launches keep a tile's K in one CTA (see dense_split).
+thread_local bool g_whole_k = false;
 // Expert range of the grouped GEMMs this thread launches next on CTA pairs ({0, 0}: all experts).
 thread_local uint32_t g_expert_lo = 0, g_expert_hi = 0;
 bool grouped_pairs(uint64_t padded_rows_max, uint64_t experts) {
@@ -1015,9 +1061,14 @@ int32_t launch_gemm(const char* op, const void* a, const void* b, const GemmPara
 // them are resident at once (a few SMs are left: clusters cannot use every one) and each keeps at least eight K steps to cover
 // the ring's fill.  77 tokens, weights cold: FP8 8,192 x 3,840 15.4 -> 10.8 us (two parts), 3,840 x 4,096 15.2 -> 7.8 and NVFP4
 // 3,840 x 15,360 20.8 -> 12.4 (four).  (A lane per row instead of eight or sixteen in the reduction: 5-6 us more.)
+// The parts of a row's sum are part of the result: a call that fuses the GELU product shares its tiles exactly where the separate
+// gate and up projections (half the columns each) would, whatever that does to its own number of tiles, so that both forms
+// give the same bytes.  The shared branch of a mixture-of-experts layer never shares (g_whole_k): its bits must depend neither on how
+// the layer's tokens are spread over ranks nor on the form its weights are stored in.
 int dense_split(const GemmParams& p, uint32_t k_per_stage) {
-  if (p.plan != nullptr || p.gated || p.gate_in != nullptr || p.out_f32 || g_gemm_bn != 0 || g_gemm_pair != 0 || g_gemm_cta_cap != 0) return 1;
-  const uint64_t tiles = static_cast<uint64_t>((p.m + BM - 1) / BM) * ((p.n + 127) / 128), steps = (p.k + k_per_stage - 1) / k_per_stage;
+  if (p.plan != nullptr || p.out_f32 || g_whole_k || g_gemm_bn != 0 || g_gemm_pair != 0) return 1;
+  const uint32_t columns = p.gated ? p.n / 2 : p.n;
+  const uint64_t tiles = static_cast<uint64_t>((p.m + BM - 1) / BM) * ((columns + 127) / 128), steps = (p.k + k_per_stage - 1) / k_per_stage;
   for (int parts = 4; parts >= 2; parts /= 2)
     if (tiles * parts + 8 <= static_cast<uint64_t>(sm_count()) && steps >= 8ull * parts) return parts;
   return 1;
@@ -1070,6 +1121,7 @@ int32_t validate_gemm(const char* op, uint64_t tokens, uint64_t rows, uint64_t k
 
 void set_grouped_rows_hint(uint64_t rows) { g_grouped_rows_hint = rows; }
 void set_gemm_cta_cap(uint32_t ctas) { g_gemm_cta_cap = ctas; }
+void set_gemm_whole_k(bool whole) { g_whole_k = whole; }
 void set_grouped_expert_range(uint32_t lo, uint32_t hi) {
   g_expert_lo = lo;
   g_expert_hi = hi;

@@ -286,6 +286,11 @@ int32_t moe_shared_stage(const gemb_moe_layer_weights* w, const uint16_t* x, uin
   const gemb_nvfp4_binding& sg = w->shared_gate_up;
   const gemb_nvfp4_binding& sd = w->shared_down;
   const uint64_t h = w->hidden, si = w->shared_intermediate;
+  // The same bits for every token count (an expert-parallel rank has a part of the tokens) and for both weight forms.
+  struct WholeK {
+    WholeK() { set_gemm_whole_k(true); }
+    ~WholeK() { set_gemm_whole_k(false); }
+  } whole_k;
   GEMB_TRY(gemb_nvfp4_quantize(x, GEMB_BF16, b.s_packed, b.s_scales, tokens, h, sg.input_divisor, GEMB_SCALES_INTERLEAVED,
                                GEMB_QUANT_EXACT, stream));
   if (w->shared_gate_up_fused != nullptr) {

@@ -51,6 +51,9 @@ void set_grouped_rows_hint(uint64_t rows);
 // Upper bound on the persistent grid of the GEMMs the calling thread launches next (0: none), so that two
 // GEMMs on two streams can each keep a set of SMs to themselves.
 void set_gemm_cta_cap(uint32_t ctas);
+// Whether the calling thread's next dense GEMMs keep each output tile's K in one CTA, so that a token's bits do not depend on how many
+// tokens the call has.
+void set_gemm_whole_k(bool whole);
 // Restricts the calling thread's next grouped GEMMs to the experts [lo, hi) ({0, 0}: all).  Takes effect on
 // CTA pairs only, which grouped_uses_pairs predicts for the rows announced with set_grouped_rows_hint.
 void set_grouped_expert_range(uint32_t lo, uint32_t hi);

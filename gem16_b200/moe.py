@@ -4,7 +4,8 @@
 and the fork / join of the shared branch live in the library (csrc/moe_layer.cu).  The stage
 methods (`route`, `experts`, `shared_branch`, `combine`, `forward_stages`) issue the same
 operator launches one by one from here, for stage timing and for tests that look at the
-intermediate buffers; both ways give identical bytes.  Stage order:
+intermediate buffers; both ways give identical bytes (shared branch: up to a hidden and intermediate size
+of 3,840, beyond which a dense GEMM call of few tokens adds a sum in parts and the layer call does not).  Stage order:
 docs/plans/gemma4-26b/specs/MOE_PREFILL_KERNEL_SPEC.md:34-47.
 """
 from __future__ import annotations

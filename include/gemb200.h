@@ -82,6 +82,7 @@ int32_t gemb_device_check(void);
  * results are bit-identical to gemb_fp8_gemv) or 2 (bulk-copy ring through shared memory wherever it fits);
  * GEMB_TUNE_GEMM_PAIR = dense prefill GEMMs on CTA pairs (two SMs share one 256 x 256 tile and
  * each stages half of the weight tile), 0 (automatic), 1 (never) or 2 (always, when the tile is 256 wide);
+ * with either of these two set no tile is shared along K;
  * GEMB_TUNE_EP_BARRIER_SPINS = how many times gemb_moe_ep_barrier polls its flags before it gives
  * up and records the fact (about 500 ns per poll; 0 = the default of 2^22, about three seconds) --
  * a deployment's failure-detection latency, and what lets a test see the give-up path quickly;
@@ -308,7 +309,10 @@ int32_t gemb_bf16_gemv(const float* input, const uint16_t* weight_bf16, float* o
  * Replaces LaunchNvfp4CutlassProjectionBf16Batch, src/cuda/nvfp4/cutlass_sm120.h:24-39.  The
  * reference re-tiles its Row8/K64 weights into scratch on every call (PrepareWeightKernel,
  * src/cuda/nvfp4/cutlass_sm120.cu:196-252); here weights are stored once, row-major with
- * interleaved scales, so the scratch and workspace arguments disappear. */
+ * interleaved scales, so the scratch and workspace arguments disappear.
+ * A call of few tokens and few rows with a long K adds a row's sum in two or four parts (so do gemb_fp8_gemm_bf16 and,
+ * where the separate projections would, the two fused forms below): how many follows from tokens, rows and K alone, never
+ * from what else runs.  A token's value may therefore differ in its last bit between batch sizes. */
 int32_t gemb_nvfp4_gemm_bf16(const uint8_t* packed_activation_e2m1,
                              const uint8_t* interleaved_activation_scales,
                              const uint8_t* packed_weight_e2m1,
@@ -681,6 +685,7 @@ int32_t gemb_checkpoint_bind_fp8(const gemb_checkpoint* checkpoint, const char* 
  * *_fused pointers are set (weights re-ordered once by gemb_nvfp4_pack_gate_up) the gate/up GEMM,
  * the GELU and the requantisation run as ONE kernel and gate_up.packed_weight / scales_interleaved
  * may be null; otherwise they run as GEMM + gemb_moe_expert_gelu_quantize (byte-identical results).
+ * A token's output depends on that token alone, not on how many others the call has.
  * Under expert parallelism the stacks hold this rank's experts only (gate_up.experts = experts / ranks).
  * Router: logits = x . router_weight^T + router_bias, or, when router_input_scale is set, the
  * specification's form  r = bf16(rmsnorm_noweight(x) * router_input_scale * hidden^-1/2),

@@ -221,3 +221,38 @@ def test_tiles_shared_along_k(lib, dev, orc, fmt, tokens, rows, steps, rest):
     assert np.isfinite(got).all()
     st = error_stats(got[idx], want)
     assert st["rel_fro"] <= REL_FRO and st["cos"] > 0.9999, st
+
+
+# Around the rule that shares tiles along K: clusters of four and two CTAs, token, column and K remainders, the largest grid of the
+# separate projections (140 tiles of the fused one: several clusters per SM), and just past it (not shared).
+@pytest.mark.parametrize("tokens,inter,k", [(1, 64, 8192), (77, 192, 8192 + 192), (130, 1088, 8192), (77, 3840, 8192), (77, 3840, 4096),
+                                            (128, 4480, 4096 + 64), (200, 2240, 4096), (77, 8960, 4096), (129, 9024, 4096)])
+def test_fused_gelu_forms_share_tiles_like_the_plain_gemm(lib, dev, tokens, inter, k):
+    """gemb_nvfp4_gemm_gated_quant and gemb_nvfp4_gemm_up_gated_quant give the bytes of the plain projections + the GELU
+    quantiser where K is long and tiles are few."""
+    a = nvfp4_operand(lib, dev, tokens, k, 1.0, 3)
+    gate, up = nvfp4_operand(lib, dev, inter, k, 0.02, 4), nvfp4_operand(lib, dev, inter, k, 0.03, 5)
+    fused = torch.zeros((2 * inter, k // 2), dtype=torch.uint8, device=dev)
+    fused_s = torch.zeros((lib.cdll.gemb_interleaved_scale_bytes(2 * inter, k),), dtype=torch.uint8, device=dev)
+    lib.gemb_nvfp4_pack_gate_up(gate["packed"], gate["compact"], up["packed"], up["compact"], fused, fused_s, inter, k, None)
+    ys = []
+    for w in (gate, up):
+        y = torch.full((tokens, inter), 0x7FC0, dtype=torch.int16, device=dev)
+        lib.gemb_nvfp4_gemm_bf16(a["packed"], a["inter"], w["packed"], w["inter"], y, tokens, inter, k, a["div"], w["div"], None)
+        ys.append(y)
+    prod = ys[1].view(torch.bfloat16).float().abs().max().item() * 2
+    g = 2688.0 / prod
+    n_scales = lib.cdll.gemb_interleaved_scale_bytes(tokens, inter)
+
+    def outputs():
+        return torch.full((tokens, inter // 2), 0xA5, dtype=torch.uint8, device=dev), torch.zeros((n_scales,), dtype=torch.uint8, device=dev)
+
+    want, got, got_up = outputs(), outputs(), outputs()
+    lib.gemb_nvfp4_gated_gelu_quantize(ys[0], ys[1], 1, want[0], want[1], tokens, inter, g, 1, 0, None)
+    lib.gemb_nvfp4_gemm_gated_quant(a["packed"], a["inter"], fused, fused_s, got[0], got[1], tokens, inter, k, a["div"], gate["div"],
+                                    up["div"], g, None)
+    lib.gemb_nvfp4_gemm_up_gated_quant(a["packed"], a["inter"], up["packed"], up["inter"], ys[0], got_up[0], got_up[1], tokens, inter, k,
+                                       a["div"], up["div"], g, None)
+    lib.gemb_check_device_status()
+    for name, out in (("gated", got), ("up gated", got_up)):
+        assert torch.equal(out[0], want[0]) and torch.equal(out[1], want[1]), name

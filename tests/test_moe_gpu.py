@@ -368,6 +368,26 @@ def test_library_layer_call_equals_the_stage_launches(lib, dev, fused):
         lib.gemb_moe_layer_forward(desc, x, out, tokens, b.c_base, b.c_workspace.numel() - 256, None, None, None, None)
 
 
+def test_shared_branch_bits_depend_on_the_token_alone(lib, dev):
+    """A layer whose shared branch has a long K and few tiles: the first 77 of 300 tokens by themselves (an expert-parallel
+    rank holds a part of the tokens) and with the others, through the fused epilogue and without it, give the same bytes."""
+    from gem16_b200.moe import synthetic_weights
+    w = synthetic_weights(dev, 3, hidden=4096, experts=32, inter=64, shared_inter=4096)
+    g = torch.Generator(device=dev)
+    g.manual_seed(4)
+    x = torch.randn((300, 4096), device=dev, generator=g).to(torch.bfloat16).view(torch.int16)
+    outs = []
+    for tokens in (300, 77):
+        for fused in (True, False):
+            layer = MoeLayer(w, tokens, 4, 650.0, 336.0, 336.0)
+            layer.fused = fused
+            outs.append(layer.forward(x[:tokens].contiguous())[:77].clone())
+    torch.cuda.synchronize()
+    lib.gemb_check_device_status()
+    for o in outs[1:]:
+        assert torch.equal(o, outs[0])
+
+
 def test_router_specification_mode(lib, dev, orc):
     """The router as docs/plans/gemma4-26b/specs/MOE_ROUTER_SPEC.md:3-13,41-63 writes it: r =
     rmsnorm_noweight(x) * scale * hidden^-1/2, logits = W r (no bias), softmax, top-8, renormalise,
