@@ -332,17 +332,19 @@ __device__ __forceinline__ void quantize_block16(const float (&v)[16], float g, 
 // correction q1 = RN(q0 + (x - scale * q0) * inv) makes it faithful and a second one correctly rounded
 // (Markstein).  The residuals are exact while x is above 2^-102; below, the quotient is under half the
 // smallest E4M3 value and its code is zero either way, as long as scale is at least 2^-90 -- callers send
-// smaller scales (q.tiny) to the division.  Everything is computed on -q (see quantize_pair: zeros keep their sign).
+// smaller scales, and the infinite one of a row with an infinity (the residual would turn its finite elements into NaN), to
+// the division (q.divide).  The signs are arranged (-x, -inv, -residual) so that zeros keep their sign, as in quantize_pair, but
+// the quotient comes out with its own: the NaN code is the conversion's.
 // The conversion instruction is the scarce one (about ten results per clock and SM), hence one per pair.
 struct Quotient {
   float scale, inv;
-  bool tiny;
+  bool divide;
 };
 __device__ __forceinline__ Quotient token_quotient(float amax) {
   Quotient q;
   q.scale = amax == 0.0f ? 1.0f : __fdiv_rn(amax, 448.0f);
   q.inv = __fdiv_rn(1.0f, q.scale);
-  q.tiny = q.scale < 0x1p-90f;
+  q.divide = !(q.scale >= 0x1p-90f && q.scale <= 3.402823466e+38f);
   return q;
 }
 __device__ __forceinline__ uint32_t e4m3x2(float2 v) {
@@ -352,11 +354,11 @@ static __device__ __noinline__ uint32_t e4m3x2_divided(float x, float y, float s
   return e4m3x2(make_float2(__fdiv_rn(x, scale), __fdiv_rn(y, scale)));
 }
 __device__ __forceinline__ uint32_t e4m3_of_quotients(float2 x, const Quotient& q) {
-  const float2 ninv = make_float2(-q.inv, -q.inv), s2 = make_float2(q.scale, q.scale);
-  const float2 y0 = __fmul2_rn(x, ninv);
-  const float2 y1 = __ffma2_rn(__ffma2_rn(s2, y0, x), ninv, y0);
-  const float2 y2 = __ffma2_rn(__ffma2_rn(s2, y1, x), ninv, y1);
-  return e4m3x2(y2) ^ 0x8080u;
+  const float2 ninv = make_float2(-q.inv, -q.inv), s2 = make_float2(q.scale, q.scale), nx = make_float2(-x.x, -x.y);
+  const float2 y0 = __fmul2_rn(nx, ninv);
+  const float2 y1 = __ffma2_rn(__ffma2_rn(s2, y0, nx), ninv, y0);
+  const float2 y2 = __ffma2_rn(__ffma2_rn(s2, y1, nx), ninv, y1);
+  return e4m3x2(y2);
 }
 
 #endif  // __CUDACC__

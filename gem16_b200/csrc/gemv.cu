@@ -114,7 +114,7 @@ __device__ __forceinline__ void stage_bf16_chunk(const uint4& v, uint64_t c, con
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const float2 x = make_float2(__uint_as_float(ww[i] << 16), __uint_as_float(ww[i] & 0xFFFF0000u));
-    h[i] = e4m3x2_to_half2(static_cast<uint16_t>(q.tiny ? e4m3x2_divided(x.x, x.y, q.scale) : e4m3_of_quotients(x, q)));
+    h[i] = e4m3x2_to_half2(static_cast<uint16_t>(q.divide ? e4m3x2_divided(x.x, x.y, q.scale) : e4m3_of_quotients(x, q)));
   }
   const uint64_t c16 = c / 2;
   *reinterpret_cast<uint4*>(xs + (c16 / 32) * 512 + (c % 2) * 256 + (c16 % 32) * 8) =
@@ -922,19 +922,21 @@ fp8_quantize_decode_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__
   for (int i = 1; i < 32; ++i) amax = fmaxf(amax, red[i]);
   const Quotient quot = token_quotient(amax);
   if (threadIdx.x == 0) scales[t] = quot.scale;
+  auto convert = [&](auto code) {
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const uint32_t c = threadIdx.x + i * 1024;
-    if (c >= chunks) continue;
-    const uint32_t ww[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
-    uint32_t q[2] = {0, 0};
+    for (int i = 0; i < 2; ++i) {
+      const uint32_t c = threadIdx.x + i * 1024;
+      if (c >= chunks) continue;
+      const uint32_t ww[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+      uint32_t q[2] = {0, 0};
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float2 pair = make_float2(__uint_as_float(ww[j] << 16), __uint_as_float(ww[j] & 0xFFFF0000u));
-      q[j >> 1] |= (quot.tiny ? e4m3x2_divided(pair.x, pair.y, quot.scale) : e4m3_of_quotients(pair, quot)) << (16 * (j & 1));
+      for (int j = 0; j < 4; ++j)
+        q[j >> 1] |= code(make_float2(__uint_as_float(ww[j] << 16), __uint_as_float(ww[j] & 0xFFFF0000u))) << (16 * (j & 1));
+      *reinterpret_cast<uint2*>(out + t * k + static_cast<uint64_t>(c) * 8) = make_uint2(q[0], q[1]);
     }
-    *reinterpret_cast<uint2*>(out + t * k + static_cast<uint64_t>(c) * 8) = make_uint2(q[0], q[1]);
-  }
+  };
+  if (quot.divide) convert([&](float2 x) { return e4m3x2_divided(x.x, x.y, quot.scale); });
+  else convert([&](float2 x) { return e4m3_of_quotients(x, quot); });
 }
 
 }  // namespace

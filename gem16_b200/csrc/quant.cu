@@ -337,7 +337,7 @@ row_warp_kernel(const __grid_constant__ RowArgs a) {
         *reinterpret_cast<uint2*>(out + c * 256) = make_uint2(__byte_perm(p[0], p[1], 0x5410), __byte_perm(p[2], p[3], 0x5410));
       }
     };
-    if (q.tiny) convert([&](float2 v) { return e4m3x2_divided(v.x, v.y, q.scale); });
+    if (q.divide) convert([&](float2 v) { return e4m3x2_divided(v.x, v.y, q.scale); });
     else convert([&](float2 v) { return e4m3_of_quotients(v, q); });
   } else if constexpr (kMode == kRowNvfp4Compact || kMode == kRowNvfp4Interleaved) {
     const uint32_t c_real = k / 16, c_pad = (c_real + 3) / 4 * 4;
@@ -671,7 +671,7 @@ fp8_quantize_kernel(const In* x, const uint16_t* __restrict__ w, uint8_t* out, f
   if (threadIdx.x == 0) scales[r] = q.scale;
   uint8_t* orow = out + r * k;
   auto code = [&](float x, float y) {
-    return q.tiny ? e4m3x2_divided(x, y, q.scale) : e4m3_of_quotients(make_float2(x, y), q);
+    return q.divide ? e4m3x2_divided(x, y, q.scale) : e4m3_of_quotients(make_float2(x, y), q);
   };
   auto emit = [&](uint32_t c, const float (&v)[16]) {
     uint32_t words[4];

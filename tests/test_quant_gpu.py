@@ -263,3 +263,30 @@ def test_fp8_quotients_at_rounding_boundaries(lib, dev, orc, rows, amax):
     lib.gemb_fp8_quantize(to_dev(bf16_bits(x), dev), BF16, q, sc, rows, x.shape[1], None)
     qo, so = orc.fp8_quantize(x)
     assert np.array_equal(to_np(sc), so) and np.array_equal(to_np(q), qo)
+
+
+# The forms of the FP8 quantiser: decode (bf16, few rows), a CTA per row (fp32; bf16 rows between), a warp per row (from two rows per SM on).
+@pytest.mark.parametrize("tokens,k,dtype", [(1, 3840, BF16), (3, 16400, BF16), (2, 48, F32), (40, 3840, BF16), (400, 3840, BF16), (400, 272, BF16)])
+def test_fp8_rows_with_infinities_and_nans(lib, dev, tokens, k, dtype):
+    """Outside the reference's contract (it refuses them), but defined: the quotient of the IEEE division.  In a row with an infinity
+    (scale infinite) finite elements are zeros of their sign and infinities NaN; a NaN is NaN (0x7F) and does not touch the scale."""
+    rng = np.random.default_rng(tokens + k)
+    x = bf16_round(rng.standard_normal((tokens, k)).astype(np.float32))
+    x[0, 3], x[0, 17], x[0, 5], x[0, 6] = np.inf, -np.inf, 0.0, -0.0
+    x[-1, 2] = np.nan
+    d = to_dev(bf16_bits(x) if dtype == BF16 else x, dev)
+    if dtype == BF16:
+        d[-1, 2] = 0x7FC0
+    q, s = torch.zeros((tokens, k), dtype=torch.uint8, device=dev), torch.zeros((tokens,), device=dev)
+    lib.gemb_fp8_quantize(d, dtype, q, s, tokens, k, None)
+    q, s = to_np(q), to_np(s)
+    assert np.isinf(s[0]) and (tokens == 1 or np.isfinite(s[1:]).all())
+    finite = np.isfinite(x[0])
+    assert np.array_equal(q[0][finite], np.where(np.signbit(x[0][finite]), 0x80, 0))
+    assert (q[0][~finite] == 0x7F).all()
+    assert q[-1, 2] == 0x7F
+    if tokens > 1:
+        others = x[1:].copy()
+        others[-1, 2] = 0
+        assert np.array_equal(s[1:], np.abs(others).max(axis=1) / np.float32(448.0))
+        assert ((q[1:] & 0x7F) == 0x7F).sum() == 1
