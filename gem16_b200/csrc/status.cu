@@ -93,7 +93,7 @@ const char* gemb_status_name(int32_t status) {
   }
 }
 
-int32_t gemb_abi_version(void) { return 1; }
+int32_t gemb_abi_version(void) { return GEMB_ABI_VERSION; }
 
 int32_t gemb_device_check(void) { return gemb::require_sm100("gemb_device_check"); }
 

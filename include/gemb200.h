@@ -66,7 +66,11 @@ enum { GEMB_QUANT_EXACT = 0, GEMB_QUANT_RCP_APPROX = 1 };
 
 const char* gemb_last_error(void);
 const char* gemb_status_name(int32_t status);
-/* ABI version of this header; bumped on any signature change. */
+/* ABI version of this header and of the library; bumped on any change of a signature or of a record that calls hand to one
+ * another.  2: the plan of gemb_moe_permute (and of gemb_moe_ep_plan) ends with one count per tile, which the grouped GEMMs read, and
+ * gemb_moe_plan_ints grew by as much; a plan of version 1 is too short for them.  A host that keeps plans in buffers of its own
+ * sizes them with gemb_moe_plan_ints and compares the two numbers once. */
+#define GEMB_ABI_VERSION 2
 int32_t gemb_abi_version(void);
 /* GEMB_OK when the current CUDA device is compute capability 10.x, else GEMB_UNSUPPORTED.
  * Counterpart of the device gate at src/cuda/engine/inference_engine_initialize.cuh:14-19. */

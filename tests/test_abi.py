@@ -102,3 +102,16 @@ def test_shim_defines_every_launcher_of_the_operator_headers():
         declared |= set(re.findall(r"Status (Launch\w+)\(", open(os.path.join(ref, "src", "cuda", h + ".h")).read()))
     assert declared and not (declared - defined), sorted(declared - defined)
     assert {"LaunchRmsNormResidualBf16", "LaunchRmsNormResidualBf16Input", "LaunchRmsNormResidualPhysicalBf16"} <= defined
+
+
+def test_plan_record_and_abi_version(lib):
+    """The plan as the header describes it (per tile: expert, list of real tiles, count) came with version 2, and the
+    integers the library asks for hold it: a host that sized plans for version 1 learns of the change."""
+    import re
+
+    from gem16_b200.lib import HEADER
+    assert lib.cdll.gemb_abi_version() == int(re.search(r"#define GEMB_ABI_VERSION (\d+)", open(HEADER).read()).group(1)) >= 2
+    for tokens, experts, topk in ((1, 32, 1), (64, 128, 8), (3001, 128, 8), (16384, 256, 32)):
+        tiles = lib.cdll.gemb_moe_padded_rows_max(tokens, experts, topk) // 128
+        assert lib.cdll.gemb_moe_plan_ints(tokens, experts, topk) == 2 + experts + 1 + 2 * tiles + 1 + tiles
+        assert lib.cdll.gemb_moe_ep_plan_ints(tokens * topk, experts) >= 2 + experts + 1 + 2 * (tokens * topk // 128) + 1 + tokens * topk // 128
