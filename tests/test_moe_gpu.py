@@ -368,6 +368,33 @@ def test_library_layer_call_equals_the_stage_launches(lib, dev, fused):
         lib.gemb_moe_layer_forward(desc, x, out, tokens, b.c_base, b.c_workspace.numel() - 256, None, None, None, None)
 
 
+@pytest.mark.parametrize("tokens,hidden,topk,offset", [(1, 8, 1, 0), (37, 2816, 8, 0), (37, 2816, 8, 1), (300, 136, 5, 0), (65, 264, 32, 0),
+                                                       (9, 1032, 6, 0), (130, 72, 4, 3)])
+@pytest.mark.parametrize("by_row", [True, False])
+def test_combine_forms(lib, dev, orc, tokens, hidden, topk, offset, by_row):
+    """Four slots to a load and one by one (top-k no multiple of four, records off a 16-byte boundary, rows in assignment order),
+    with and without the shared branch: the oracle's fma chain, bit for bit."""
+    rng = np.random.default_rng(tokens * 100 + topk)
+    n = tokens * topk
+    rows = n + 77 if by_row else n
+    y = bf16_bits(rng.standard_normal((rows, hidden)).astype(np.float32))
+    slots = rng.permutation(rows)[:n].astype(np.int32) if by_row else np.arange(n, dtype=np.int32)
+    weights = rng.random((tokens, topk)).astype(np.float32)
+    shared = bf16_bits(rng.standard_normal((tokens, hidden)).astype(np.float32))
+
+    def shifted(a):
+        buf = torch.zeros((n + 4,), dtype=torch.float32 if a.dtype == np.float32 else torch.int32, device=dev)
+        buf[offset:offset + n] = to_dev(a.reshape(-1), dev)
+        return buf[offset:offset + n]
+
+    d_slots, d_weights = (shifted(slots) if by_row else None), shifted(weights)
+    for sh in (shared, None):
+        out = torch.full((tokens, hidden), 0x7FC0, dtype=torch.int16, device=dev)
+        lib.gemb_moe_combine(to_dev(y, dev), d_slots, d_weights, None if sh is None else to_dev(sh, dev), out, tokens, hidden, topk, None)
+        want = orc.moe_combine(y[slots].reshape(tokens, topk, hidden), weights, sh)
+        assert np.array_equal(to_np(out, np.uint16), np.asarray(want).view(np.uint16).reshape(tokens, hidden))
+
+
 def test_shared_branch_bits_depend_on_the_token_alone(lib, dev):
     """A layer whose shared branch has a long K and few tiles: the first 77 of 300 tokens by themselves (an expert-parallel
     rank holds a part of the tokens) and with the others, through the fused epilogue and without it, give the same bytes."""
