@@ -670,24 +670,25 @@ fp8_quantize_kernel(const In* x, const uint16_t* __restrict__ w, uint8_t* out, f
   const Quotient q = token_quotient(amax);
   if (threadIdx.x == 0) scales[r] = q.scale;
   uint8_t* orow = out + r * k;
-  auto code = [&](float x, float y) {
-    return q.divide ? e4m3x2_divided(x, y, q.scale) : e4m3_of_quotients(make_float2(x, y), q);
-  };
-  auto emit = [&](uint32_t c, const float (&v)[16]) {
-    uint32_t words[4];
+  auto convert = [&](auto code) {
+    auto emit = [&](uint32_t c, const float (&v)[16]) {
+      uint32_t words[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      words[j] = code(v[4 * j], v[4 * j + 1]) | (code(v[4 * j + 2], v[4 * j + 3]) << 16);
-    *reinterpret_cast<uint4*>(orow + static_cast<uint64_t>(c) * 16) = make_uint4(words[0], words[1], words[2], words[3]);
-  };
+      for (int j = 0; j < 4; ++j)
+        words[j] = code(make_float2(v[4 * j], v[4 * j + 1])) | (code(make_float2(v[4 * j + 2], v[4 * j + 3])) << 16);
+      *reinterpret_cast<uint4*>(orow + static_cast<uint64_t>(c) * 16) = make_uint4(words[0], words[1], words[2], words[3]);
+    };
 #pragma unroll
-  for (int b = 0; b < 2; ++b)
-    if (threadIdx.x + b * 256 < blocks) emit(threadIdx.x + b * 256, kept[b]);
-  for (uint32_t c = threadIdx.x + 512; c < blocks; c += 256) {
-    float v[16];
-    block_values(c, v);
-    emit(c, v);
-  }
+    for (int b = 0; b < 2; ++b)
+      if (threadIdx.x + b * 256 < blocks) emit(threadIdx.x + b * 256, kept[b]);
+    for (uint32_t c = threadIdx.x + 512; c < blocks; c += 256) {
+      float v[16];
+      block_values(c, v);
+      emit(c, v);
+    }
+  };
+  if (q.divide) convert([&](float2 v) { return e4m3x2_divided(v.x, v.y, q.scale); });
+  else convert([&](float2 v) { return e4m3_of_quotients(v, q); });
 }
 
 // Which form a batch of bf16 rows takes: see the comment above the row kernels.
