@@ -171,7 +171,10 @@ output_head_kernel(const uint16_t* __restrict__ weights, const float* __restrict
 // and g + 8 per 64 k, three such pieces ahead.
 // ---------------------------------------------------------------------------------------------
 constexpr int kHmWarps = 16, kHmThreads = kHmWarps * 32, kHmAhead = 3;
-constexpr uint32_t kHmMinRows = 3;   // two rows: 311 us in the fma form, 320 here
+// Two rows take the fma form: 262,144 / 131,072 / 100,000 / 50,000 x 3,840 take 326 / 178 / 154 / 96 us there and 342 / 197 / 156 / 102
+// here (2,048 wide: 178 / 100 / 92 / 59 and 199 / 119 / 94 / 61); only where all blocks have one step (32,000 tokens) is it 80
+// there and 66 here.  Three rows are faster here at every size (8,000 x 2,048: 51 and 25; 262,144 x 3,840: 424 and 342; all cold).
+constexpr uint32_t kHmMinRows = 3;
 constexpr uint32_t kHmPairs = kOhBlocks / 2;               // pairs of candidate blocks
 constexpr uint32_t kHmStepTokens = kOhBlocks * kOhWarps;   // tokens all blocks take in one step
 
@@ -201,11 +204,15 @@ output_head_mma_kernel(const uint16_t* __restrict__ weights, const float* __rest
   Candidate* best = reinterpret_cast<Candidate*>(bs + static_cast<size_t>(chunks) * 3 * 2 * 32);   // [task][block of the pair][8]
   const uint32_t warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const uint32_t pairs = (kHmPairs - blockIdx.x + gridDim.x - 1) / gridDim.x, tasks = pairs * steps;
+  // Tasks in the order of their steps: every step but the last is whole, and of the last one the pairs that still hold tokens come
+  // first, so that no task lies past the vocabulary (50,000 x 2,048 would spend a quarter of its tasks there).
+  const uint32_t pairs = (kHmPairs - blockIdx.x + gridDim.x - 1) / gridDim.x;
+  const uint32_t last_live = (vocab - (steps - 1) * kHmStepTokens + 15) / 16;   // pairs of the whole grid that the last step reaches
+  const uint32_t tasks = pairs * (steps - 1) + (last_live > blockIdx.x ? (last_live - blockIdx.x + gridDim.x - 1) / gridDim.x : 0);
   // Load cursor: piece `lc` of task `lt`.
   uint32_t lt = warp, lc = 0;
   const uint16_t* pw[2] = {weights, weights};
-  auto first_token = [&](uint32_t task) { return task % steps * kHmStepTokens + (blockIdx.x + gridDim.x * (task / steps)) * 16; };
+  auto first_token = [&](uint32_t task) { return task / pairs * kHmStepTokens + (blockIdx.x + gridDim.x * (task % pairs)) * 16; };
   auto aim = [&]() {
     if (lt >= tasks) return;
     const uint32_t tok0 = first_token(lt);
@@ -318,8 +325,8 @@ output_head_mma_kernel(const uint16_t* __restrict__ weights, const float* __rest
   for (uint32_t idx = threadIdx.x; idx < pairs * 2 * rows; idx += kHmThreads) {
     const uint32_t r = idx % rows, h = idx / rows & 1, pair = idx / rows / 2;
     Candidate c{-FLT_MAX, 0u};
-    for (uint32_t step = 0; step < steps; ++step) {
-      const Candidate o = best[((pair * steps + step) * 2 + h) * 8 + r];
+    for (uint32_t task = pair; task < tasks; task += pairs) {
+      const Candidate o = best[(task * 2 + h) * 8 + r];
       if (better(o.value, o.token, c)) c = o;
     }
     candidates[static_cast<uint64_t>(r) * kOhBlocks + (blockIdx.x + gridDim.x * pair) * 2 + h] = c;
@@ -369,7 +376,8 @@ int32_t launch_output_head(const char* op, const uint16_t* weights, const float*
 }
 
 // false: the shapes the tensor-core form does not take (rows that are not whole 32-byte pieces, hidden rows or candidates that do
-// not fit the shared memory of one CTA).
+// not fit the shared memory of one CTA: 48 bytes per hidden element whatever the number of rows, so hidden up to 4,544 at
+// 262,144 tokens and 4,736 at 65,536).  They run in the fma form, which takes 1.2 (three rows) to 3 times (eight) as long.
 bool head_mma_fits(const uint16_t* weights, uint32_t rows, uint32_t vocab, uint32_t hidden, size_t* smem) {
   *smem = static_cast<size_t>((hidden + 63) / 64) * 3 * 2 * 32 * sizeof(uint4) +
           static_cast<size_t>(head_mma_tasks(static_cast<uint32_t>(sm_count()), vocab)) * 2 * 8 * sizeof(Candidate);

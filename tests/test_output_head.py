@@ -108,7 +108,8 @@ def test_output_head_ties_and_validation(lib, dev, orc):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("rows,vocab,hidden", [(3, 17, 16), (4, 32769, 80), (8, 65536 + 9, 144), (7, 5, 3840), (3, 300, 24)])
+@pytest.mark.parametrize("rows,vocab,hidden", [(3, 17, 16), (4, 32769, 80), (8, 65536 + 9, 144), (7, 5, 3840), (3, 300, 24),
+                                               (8, 32768 + 16 * 300 + 5, 64), (5, 50000, 32), (3, 2 * 32768, 16), (6, 100000, 48)])
 def test_output_head_rows_sharing_a_pass_at_the_edges(lib, dev, orc, rows, vocab, hidden):
     """Token, step and K remainders of the tensor-core form, one shape it does not take; every candidate is written."""
     w, h = make_case(orc, rows, vocab, hidden, rows + hidden)
