@@ -293,6 +293,9 @@ nvfp4_gemv_kernel(const __grid_constant__ Fp4GemvArgs a) {
   emit(static_cast<uint32_t>(last_start / pieces));
 }
 
+// The tokens that share a launch: their staged fp16 activations, beside which the partial sums have to fit.
+constexpr uint64_t kFpMaxStageBytes = 200 * 1024;
+static_assert(kFpMaxStageBytes + 128 + kFpWarps * 2 * 32 * sizeof(float4) <= 227 * 1024);
 uint64_t fp4_stage_bytes(uint64_t tokens, uint64_t k) { return tokens * ((k + kPieceElems - 1) / kPieceElems * kPieceElems) * 2; }
 
 template <bool kGateUp>
@@ -334,8 +337,8 @@ int32_t gemb_nvfp4_gemv_batch(const uint8_t* act, const uint8_t* act_scales, con
   GEMB_REQUIRE(act && act_scales && w && w_scales && out, "%s: pointers must be nonnull", op);
   GEMB_TRY(validate_nvfp4_gemv(op, rows, k, ga, gw));
   GEMB_REQUIRE(tokens >= 1 && tokens <= 8, "%s: between 1 and 8 tokens (larger batches go through gemb_nvfp4_gemm_bf16)", op);
-  GEMB_REQUIRE(tokens == 1 || tokens * ((k + 1023) / 1024 * 1024 * 2 + (k / 16) * 4) <= 200 * 1024,
-               "%s: tokens * K exceeds the shared-memory staging limit", op);
+  GEMB_REQUIRE(tokens == 1 || fp4_stage_bytes(tokens, k) <= kFpMaxStageBytes,
+               "%s: tokens * K (K padded to 256) exceeds the shared-memory staging limit (102400)", op);
   GEMB_REQUIRE(reinterpret_cast<uintptr_t>(act) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0 &&
                    reinterpret_cast<uintptr_t>(w_scales) % 2 == 0,
                "%s: activation and weight must be 16-byte aligned, weight scales 2-byte aligned", op);
@@ -376,7 +379,7 @@ int32_t gemb_nvfp4_gemv_gate_up_batch(const uint8_t* act, const uint8_t* act_sca
   // Up to eight tokens share a launch and with it one pass over the weights (the verifier's batches are a
   // handful of tokens), fewer where their activations would not fit the shared memory of a CTA.
   uint64_t group = std::min<uint64_t>(8, tokens);
-  while (group > 1 && fp4_stage_bytes(group, k) > 200 * 1024) --group;
+  while (group > 1 && fp4_stage_bytes(group, k) > kFpMaxStageBytes) --group;
   for (uint64_t t0 = 0; t0 < tokens; t0 += group) {
     Fp4GemvArgs a{};
     a.act = act + t0 * (k / 2);

@@ -262,7 +262,8 @@ int32_t gemb_nvfp4_gemv(const uint8_t* packed_activation_e2m1, const uint8_t* ac
 
 /* Small-batch form (1..8 tokens, the verifier's MLP projections): activation [tokens, K/2] with
  * COMPACT scales [tokens, K/16], output fp32 [tokens, rows]; per token bit-identical to
- * gemb_nvfp4_gemv.  Replaces LaunchNvfp4Sm120DirectProjectionBatch (src/cuda/nvfp4/sm120.h:26-37)
+ * gemb_nvfp4_gemv.  With two or more tokens, tokens * K (K padded to 256) <= 102,400.
+ * Replaces LaunchNvfp4Sm120DirectProjectionBatch (src/cuda/nvfp4/sm120.h:26-37)
  * for tokens <= 8; larger batches are prefill and belong to gemb_nvfp4_gemm_bf16. */
 int32_t gemb_nvfp4_gemv_batch(const uint8_t* packed_activation_e2m1, const uint8_t* activation_scales,
                               const uint8_t* packed_weight_e2m1, const uint8_t* weight_scales,

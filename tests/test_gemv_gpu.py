@@ -342,3 +342,19 @@ def test_weight_quantised_on_the_device_is_seen_at_once(lib, dev, rows, k, act_f
         torch.cuda.synchronize()
         for i in range(reps):
             assert torch.equal(y[i], want[i % 2]), i
+
+
+def test_nvfp4_gemv_batch_takes_what_fits_the_staging(lib, dev):
+    """The largest batch of a long K, and one token more."""
+    from gem16_b200.lib import GembError
+    rows, k = 24, 15360
+    gen = torch.Generator(device=dev).manual_seed(1)
+    act, w = (torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device=dev, generator=gen) for n in (8, rows))
+    acts, ws = (torch.randint(0x30, 0x40, (n, k // 16), dtype=torch.uint8, device=dev, generator=gen) for n in (8, rows))
+    y, one = torch.zeros((6, rows), device=dev), torch.zeros((rows,), device=dev)
+    lib.gemb_nvfp4_gemv_batch(act, acts, w, ws, y, 6, rows, k, 100.0, 100.0, None)
+    for t in range(6):
+        lib.gemb_nvfp4_gemv(act[t], acts[t], w, ws, one, rows, k, 100.0, 100.0, None)
+        assert torch.equal(one, y[t]), t
+    with pytest.raises(GembError):
+        lib.gemb_nvfp4_gemv_batch(act, acts, w, ws, torch.zeros((7, rows), device=dev), 7, rows, k, 100.0, 100.0, None)
