@@ -9,27 +9,30 @@
 // One persistent CTA per SM.  Dense calls pair the CTAs (clusters of two, tcgen05 cta_group::2):
 // the pair owns a 256 x 256 tile, each CTA stages its own 128 activation rows and 128 of the 256
 // weight rows, the even CTA issues every MMA, each CTA accumulates and stores its own 128 rows.
-// Grouped (mixture-of-experts) calls keep one CTA per 128 x 256 tile.  Warp roles:
-//   producer (warp 0): one elected lane issues TMA tile loads (128-byte swizzle, no multicast)
-//            for A and B and 1-D bulk copies for the interleaved block scales into a ring of
-//            kStages shared-memory stages, each guarded by a full/empty mbarrier pair;
+// Grouped (mixture-of-experts) calls keep one CTA per 128 x 256 tile unless the experts hold many rows; dense calls of few tiles
+// share each 128 x 128 tile along K in clusters of two or four (dense_split).  Warp roles:
+//   producer (warp 0): one elected lane issues TMA tile loads (128-byte swizzle, no multicast) for A and
+//            B into a ring of kStages shared-memory stages, each guarded by a full/empty mbarrier pair.  The loads of both
+//            CTAs of a pair complete on the even CTA's barrier;
 //   MMA issuer (warp 1): per stage one tcgen05.mma per 32 bytes of K, then a commit of the stage's
 //            empty barrier; after the last K step a commit of the accumulator barrier.  In the odd
-//            CTA of a pair this warp only relays "operands landed" to the issuer (FP8);
+//            CTA of a pair this warp does nothing;
+//   scale producer (NVFP4, warp 2): one elected lane issues the 1-D bulk copies of the interleaved block
+//            scales into a ring of their own (sf_full / sf_empty);
 //   epilogue, two sets of four warps: each warp drains its 32 TMEM lanes 64 columns at a time,
 //            the sets taking alternate 64-column sub-tiles; scales, rounds to bf16, stages a
 //            32 x 128-byte block in its own swizzled buffer and issues a TMA store (which also
-//            clips the token / row tails).  FP8 double-buffers the accumulator; NVFP4 has room
-//            for one (256 columns + the scale regions), so its epilogue releases the accumulator
+//            clips the token / row tails).  FP8 double-buffers the accumulator; 256-wide NVFP4 tiles have room
+//            for one (256 columns + the scale regions), so the epilogue releases the accumulator
 //            as early as it can: first sub-tile converted in registers, second loaded, release,
 //            and only then the staging and the stores;
 //   scale movers (NVFP4), two sets of four warps: copy a stage's block scales from shared memory
 //            into the stage's TMEM region with tcgen05.st and arrive on its scales-ready barrier.
 //            Doing this with tcgen05.cp from the MMA thread costs a third of the tensor-pipe
 //            time, because those copies queue in front of the MMAs.
-// NVFP4 lays the roles out on warpgroup boundaries (warps 0-3 producer / issuer / two idle, 4-7
+// NVFP4 lays the roles out on warpgroup boundaries (warps 0-3 producer / issuer / scale producer / idle, 4-7
 // and 12-15 epilogue, 8-11 and 16-19 movers) so that setmaxnreg can move registers from the
-// producer, issuer and movers to the epilogue, which holds 96 accumulator values per thread
+// control warps and movers to the epilogue, which holds 96 accumulator values per thread
 // between the accumulator becoming full and its release.
 // Tiles are walked with the token-tile index fastest so CTAs running at the same time share the
 // same weight tile through L2.
@@ -55,7 +58,7 @@ __device__ int g_gemm_error = 0;
 namespace {
 
 constexpr int kGemmThreadsFp8 = 320;   // producer, MMA, 2 x 4 epilogue warps
-constexpr int kGemmThreadsFp4 = 640;   // warpgroups: control (producer, MMA, 2 idle), epilogue, movers, epilogue, movers
+constexpr int kGemmThreadsFp4 = 640;   // warpgroups: control (producer, MMA, scale producer, idle), epilogue, movers, epilogue, movers
 constexpr int BM = 128;
 
 struct GemmParams {
@@ -124,7 +127,7 @@ struct Cfg {
   static constexpr int kSfColsPerStage = kFp4 ? kSfaCols + kSfbCols : 0;
   static_assert(kAccCols + kStages * kSfColsPerStage <= 512, "TMEM budget exceeded");
   static_assert(BN == 128 || BN == 256, "BN must be 128 or 256");
-    static_assert(kSmemBytes <= 227 * 1024, "shared memory budget exceeded");
+  static_assert(kSmemBytes <= 227 * 1024, "shared memory budget exceeded");
 };
 
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
@@ -432,7 +435,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         if (++as == kAccStages) { as = 0; aphase ^= 1; }
       }
     }
-  }  // warps 2 and 3 of the NVFP4 control warpgroup are idle
+  }  // warp 3 of the NVFP4 control warpgroup is idle
   } else if (is_mover) {
     // ------------------------------- scale movers (NVFP4) ------------------------------------
     // Two sets of four warps (one warp per TMEM lane quarter), since one trip of this loop

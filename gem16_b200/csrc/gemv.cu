@@ -475,13 +475,6 @@ int32_t launch_fp8_gemv_batch_variant(const char* op, const uint8_t* act, const 
 // 2 t, 2 t + 1, c2 / c3 to row g + 8.  The result differs from the single-token kernel's only in the
 // order of the fp32 additions.
 // ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ void mma_e4m3_m16n8k32(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                                   uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k32.row.col.f32.e4m3.e4m3.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
 constexpr int kMmaPieces = 4;                  // 64-byte pieces per span: eight 16-byte weight loads in flight per lane
 constexpr int kMmaSpan = kMmaPieces * 64;      // bytes of K one warp takes per step
 
@@ -539,8 +532,8 @@ fp8_gemv_mma_kernel(const uint8_t* __restrict__ act, const float* __restrict__ a
         if (kb + u * 64 < k) {   // warp-uniform; K is a multiple of 16, lanes past it hold zero weights
           uint4 xv = make_uint4(0, 0, 0, 0);
           if (token_live && kb + u * 64 + t4 * 16 < k) xv = ld_dep(reinterpret_cast<const uint4*>(xrow + kb + u * 64));
-          mma_e4m3_m16n8k32(acc, wa[u].x, wb[u].x, wa[u].y, wb[u].y, xv.x, xv.y);
-          mma_e4m3_m16n8k32(acc, wa[u].z, wb[u].z, wa[u].w, wb[u].w, xv.z, xv.w);
+          ptx::mma_e4m3(acc, wa[u].x, wb[u].x, wa[u].y, wb[u].y, xv.x, xv.y);
+          ptx::mma_e4m3(acc, wa[u].z, wb[u].z, wa[u].w, wb[u].w, xv.z, xv.w);
         }
       }
     }

@@ -27,6 +27,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "ptx.cuh"
 
 namespace gemb {
 namespace {
@@ -56,18 +57,6 @@ __device__ __forceinline__ void scale_pairs(uint32_t two_bytes, uint32_t& first,
   first = __byte_perm(h, h, 0x1010);
   second = __byte_perm(h, h, 0x3232);
 }
-// c = A B (first of a chain) and c += A B.
-__device__ __forceinline__ void mma_first(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-      : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.0f));
-}
-__device__ __forceinline__ void mma_next(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
 struct Fp4Matrix {
   const uint8_t* w;
   const uint8_t* ws;
@@ -90,11 +79,11 @@ struct Run {
 };
 __device__ __forceinline__ void load_run(Run& r, const uint8_t* w, const uint8_t* s, bool in, bool wide) {
   if (wide) {
-    asm volatile("{ .reg .pred p; setp.ne.b32 p, %11, 0;\n"
-                 "@p ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%9];\n"
-                 "@p ld.global.nc.b32 %8, [%10]; }"
-                 : "+r"(r.w[0]), "+r"(r.w[1]), "+r"(r.w[2]), "+r"(r.w[3]), "+r"(r.w[4]), "+r"(r.w[5]), "+r"(r.w[6]), "+r"(r.w[7]), "+r"(r.s)
-                 : "l"(w), "l"(s), "r"(static_cast<uint32_t>(in)));
+    ptx::ld_stream_32_if(r.w, w, in);
+    asm volatile("{ .reg .pred p; setp.ne.b32 p, %2, 0;\n"
+                 "@p ld.global.nc.b32 %0, [%1]; }"
+                 : "+r"(r.s)
+                 : "l"(s), "r"(static_cast<uint32_t>(in)));
   } else if (in) {
     asm volatile("ld.global.nc.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r.w[0]), "=r"(r.w[1]), "=r"(r.w[2]), "=r"(r.w[3]) : "l"(w));
     asm volatile("ld.global.nc.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r.w[4]), "=r"(r.w[5]), "=r"(r.w[6]), "=r"(r.w[7]) : "l"(w + 16));
@@ -156,9 +145,9 @@ __device__ __forceinline__ void dot_piece(float (&acc)[4], const Run& ra, const 
           ha[j] = mul_half2(ha[j], sa[b]);
           hb[j] = mul_half2(hb[j], sb[b]);
         }
-        if (i == 0) mma_first(c, ha[0], hb[0], ha[1], hb[1], xv.x, xv.y);
-        else mma_next(c, ha[0], hb[0], ha[1], hb[1], xv.x, xv.y);
-        mma_next(c, ha[2], hb[2], ha[3], hb[3], xv.z, xv.w);
+        if (i == 0) ptx::mma_f16_first(c, ha[0], hb[0], ha[1], hb[1], xv.x, xv.y);
+        else ptx::mma_f16(c, ha[0], hb[0], ha[1], hb[1], xv.x, xv.y);
+        ptx::mma_f16(c, ha[2], hb[2], ha[3], hb[3], xv.z, xv.w);
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j) acc[j] = __fadd_rn(acc[j], c[j]);

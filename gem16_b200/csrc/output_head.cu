@@ -14,6 +14,7 @@
 #include <cfloat>
 
 #include "common.cuh"
+#include "ptx.cuh"
 
 namespace gemb {
 namespace {
@@ -178,17 +179,6 @@ constexpr uint32_t kHmMinRows = 3;
 constexpr uint32_t kHmPairs = kOhBlocks / 2;               // pairs of candidate blocks
 constexpr uint32_t kHmStepTokens = kOhBlocks * kOhWarps;   // tokens all blocks take in one step
 
-__device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void load_32_bytes(uint32_t (&r)[8], const uint16_t* w, bool in) {
-  asm volatile("{ .reg .pred p; setp.ne.b32 p, %9, 0;\n"
-               "@p ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8]; }"
-               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
-               : "l"(w), "r"(static_cast<uint32_t>(in)));
-}
 __host__ __device__ inline uint32_t head_mma_tasks(uint32_t ctas, uint32_t vocab) {   // of the CTA that has the most
   return (kHmPairs + ctas - 1) / ctas * ((vocab + kHmStepTokens - 1) / kHmStepTokens);
 }
@@ -226,8 +216,8 @@ output_head_mma_kernel(const uint16_t* __restrict__ weights, const float* __rest
 #pragma unroll
       for (int i = 0; i < 8; ++i) wa[u][i] = wb[u][i] = 0;
     }
-    load_32_bytes(wa[u], pw[0] + lc * 64, in);
-    load_32_bytes(wb[u], pw[1] + lc * 64, in);
+    ptx::ld_stream_32_if(wa[u], pw[0] + lc * 64, in);
+    ptx::ld_stream_32_if(wb[u], pw[1] + lc * 64, in);
     if (++lc == chunks) {
       lc = 0;
       lt += kHmWarps;
@@ -301,10 +291,10 @@ output_head_mma_kernel(const uint16_t* __restrict__ weights, const float* __rest
       for (int q = 0; q < 3; ++q) {
         const uint4 b0 = bs[((cc * 3 + q) * 2) * 32 + lane], b1 = bs[((cc * 3 + q) * 2 + 1) * 32 + lane];
         float c[4] = {0.0f, 0.0f, 0.0f, 0.0f}, d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        mma_bf16(c, wa[u][0], wb[u][0], wa[u][1], wb[u][1], b0.x, b0.y);
-        mma_bf16(d, wa[u][4], wb[u][4], wa[u][5], wb[u][5], b1.x, b1.y);
-        mma_bf16(c, wa[u][2], wb[u][2], wa[u][3], wb[u][3], b0.z, b0.w);
-        mma_bf16(d, wa[u][6], wb[u][6], wa[u][7], wb[u][7], b1.z, b1.w);
+        ptx::mma_bf16(c, wa[u][0], wb[u][0], wa[u][1], wb[u][1], b0.x, b0.y);
+        ptx::mma_bf16(d, wa[u][4], wb[u][4], wa[u][5], wb[u][5], b1.x, b1.y);
+        ptx::mma_bf16(c, wa[u][2], wb[u][2], wa[u][3], wb[u][3], b0.z, b0.w);
+        ptx::mma_bf16(d, wa[u][6], wb[u][6], wa[u][7], wb[u][7], b1.z, b1.w);
 #pragma unroll
         for (int i = 0; i < 4; ++i) acc[q][i] = __fadd_rn(acc[q][i], __fadd_rn(c[i], d[i]));
       }
