@@ -136,9 +136,10 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   return r;
 }
 
-// kSplit > 1: a cluster of that many CTAs shares one tile of a dense call, each a contiguous part of K; the fp32 partial
-// accumulators meet in shared memory (see the epilogue).
-template <bool kFp4, int BN, int kStages, int kAccStages, bool kPair, int kSplit = 1>
+// kSplit > 1: a cluster of that many CTAs shares one tile of a dense call, each a contiguous share of K; kParts > 1: a CTA
+// accumulates its share in that many parts, each in an accumulator of its own.  The kSplit x kParts fp32 partial accumulators meet in shared
+// memory (see the epilogue).
+template <bool kFp4, int BN, int kStages, int kAccStages, bool kPair, int kSplit = 1, int kParts = 1>
 __global__ void __launch_bounds__(kFp4 ? kGemmThreadsFp4 : kGemmThreadsFp8, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
             const __grid_constant__ CUtensorMap map_part, const __grid_constant__ CUtensorMap map_out, const GemmParams p) {
@@ -224,14 +225,17 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     }
   }
   const uint32_t num_tiles = m_units * n_tiles;
-  static_assert(kSplit == 1 || !kPair, "a tile is shared along K or along its rows");
+  constexpr uint32_t kCuts = kSplit * kParts;   // parts of a row's sum
+  static_assert(kCuts == 1 || !kPair, "a tile is shared along K or along its rows");
+  static_assert(kAccStages % kParts == 0, "one accumulator per part");
   const uint32_t first_tile = kPair ? blockIdx.x >> 1 : blockIdx.x / kSplit;
   const uint32_t tile_stride = kPair ? gridDim.x >> 1 : gridDim.x / kSplit;
   const uint32_t my_tiles = first_tile < num_tiles ? (num_tiles - first_tile + tile_stride - 1) / tile_stride : 0;
   const uint32_t k_stages_all = (p.k + C::kKPerStage - 1) / C::kKPerStage;
   const uint32_t split = kSplit > 1 ? ptx::cluster_ctarank() : 0u;
-  const uint32_t ks0 = kSplit > 1 ? split * k_stages_all / kSplit : 0u;   // this CTA's part of K
-  const uint32_t k_stages = kSplit > 1 ? (split + 1) * k_stages_all / kSplit - ks0 : k_stages_all;
+  auto part_start = [&](uint32_t part) { return part * k_stages_all / kCuts; };
+  const uint32_t ks0 = kCuts > 1 ? part_start(split * kParts) : 0u;   // this CTA's share of K
+  const uint32_t k_stages = kCuts > 1 ? part_start((split + 1) * kParts) - ks0 : k_stages_all;
   const uint32_t k_groups_pad = (p.k / 16 + 3) / 4;  // 512-byte scale chunks per 128-row group
   auto tile_expert_of = [&](uint32_t mt) -> int32_t {
     return ld_dep(tile_expert + 2 * (kPair ? (mt & ~1u) : mt));
@@ -370,12 +374,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
       uint32_t as = 0, aphase = 0;
       uint32_t stage = 0, phase = 0;
       bool ready = false;
-      for (uint32_t t = 0; t < my_tiles && !*abort_flag; ++t) {
+      for (uint32_t t = 0; t < my_tiles * kParts && !*abort_flag; ++t) {   // a part is a tile of its own here
         if (!wait_issuer(&acc_empty[as], aphase ^ 1)) { fail_wait(2); break; }
         const uint32_t tmem_acc = tmem_base + as * BN;
-        uint32_t k_left = p.k - ks0 * C::kKPerStage;
+        const uint32_t first = kParts > 1 ? part_start(split * kParts + t % kParts) : ks0;
+        const uint32_t steps = kParts > 1 ? part_start(split * kParts + t % kParts + 1) - first : k_stages;
+        uint32_t k_left = p.k - first * C::kKPerStage;
         bool ok = true;
-        for (uint32_t ks = 0; ks < k_stages; ++ks, k_left -= C::kKPerStage) {
+        for (uint32_t ks = 0; ks < steps; ++ks, k_left -= C::kKPerStage) {
           if (!ready) {   // the operands and, NVFP4, their scales
             ok = wait_issuer(&full[stage], phase);
             if constexpr (kFp4) ok = ok && wait_issuer(&sf_ready[stage], phase);
@@ -509,28 +515,30 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     uint8_t* my_stage = epi_stage + (set * 4 + quarter) * 4096;
     uint32_t as = 0, aphase = 0;
     if constexpr (kSplit > 1) {
-      // Every CTA leaves its partial accumulator in shared memory (the operand stages are free: its last MMA has
+      // Every CTA leaves its partial accumulators in shared memory (the operand stages are free: its last MMA has
       // completed; rows of 132 words are conflict-free for a lane per row), then takes BN / kSplit columns and adds the
       // parts of all CTAs in K order, read through the cluster's shared window.  The forms that quantise the GELU product need whole
       // blocks of columns: there a CTA takes every kSplit-th row.
       uint32_t mt, nt;
       tile_coords(first_tile, mt, nt);
       constexpr int kStride = BN + 4;
-      static_assert(128 * kStride * 4 <= kStages * (C::kABytes + C::kBBytes), "the partial sums replace the operand stages");
-      float* part = reinterpret_cast<float*>(smem) + (quarter * 32 + lane) * kStride;
-      if (!ptx::mbar_wait(&acc_full[0], 0)) fail_wait(4);
+      constexpr int kPartFloats = 128 * kStride;
+      static_assert(kParts * kPartFloats * 4 <= kStages * (C::kABytes + C::kBBytes), "the partial sums replace the operand stages");
+      if (!ptx::mbar_wait(&acc_full[kParts - 1], 0)) fail_wait(4);   // commits are in order: the earlier parts are complete too
       ptx::tc_fence_after();
 #pragma unroll 1
-      for (uint32_t c = set; c < BN / 64; c += 2) {
+      for (uint32_t i = set; i < kParts * (BN / 64); i += 2) {
         if (mt * BM + quarter * 32 >= p.m) break;   // warp-uniform
+        const uint32_t q = i / (BN / 64), c = i % (BN / 64);
+        float* part = reinterpret_cast<float*>(smem) + q * kPartFloats + (quarter * 32 + lane) * kStride;
         uint32_t v0[32], v1[32];
-        ptx::tc_ld_32x32b_x32(tmem_base + ((quarter * 32) << 16) + c * 64, v0);
-        ptx::tc_ld_32x32b_x32(tmem_base + ((quarter * 32) << 16) + c * 64 + 32, v1);
+        ptx::tc_ld_32x32b_x32(tmem_base + q * BN + ((quarter * 32) << 16) + c * 64, v0);
+        ptx::tc_ld_32x32b_x32(tmem_base + q * BN + ((quarter * 32) << 16) + c * 64 + 32, v1);
         ptx::tc_wait_ld();
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          *reinterpret_cast<uint4*>(part + c * 64 + 4 * q) = make_uint4(v0[4 * q], v0[4 * q + 1], v0[4 * q + 2], v0[4 * q + 3]);
-          *reinterpret_cast<uint4*>(part + c * 64 + 32 + 4 * q) = make_uint4(v1[4 * q], v1[4 * q + 1], v1[4 * q + 2], v1[4 * q + 3]);
+        for (int j = 0; j < 8; ++j) {
+          *reinterpret_cast<uint4*>(part + c * 64 + 4 * j) = make_uint4(v0[4 * j], v0[4 * j + 1], v0[4 * j + 2], v0[4 * j + 3]);
+          *reinterpret_cast<uint4*>(part + c * 64 + 32 + 4 * j) = make_uint4(v1[4 * j], v1[4 * j + 1], v1[4 * j + 2], v1[4 * j + 3]);
         }
       }
       ptx::tc_fence_before();
@@ -538,11 +546,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
       ptx::cluster_sync();
       const uint32_t rows = min(static_cast<uint32_t>(BM), p.m - mt * BM);
       auto row_sum = [&](uint32_t r, uint32_t col) {   // four columns of a row, the parts added in K order
-        float4 v[kSplit];
+        float4 v[kCuts];
+        float* cell = reinterpret_cast<float*>(smem) + r * kStride + col;
 #pragma unroll
-        for (int c = 0; c < kSplit; ++c) v[c] = ptx::ld_cluster_f4(ptx::cluster_map(reinterpret_cast<float*>(smem) + r * kStride + col, c));
+        for (int c = 0; c < static_cast<int>(kCuts); ++c) v[c] = ptx::ld_cluster_f4(ptx::cluster_map(cell + c % kParts * kPartFloats, c / kParts));
 #pragma unroll
-        for (int c = 1; c < kSplit; ++c) {
+        for (int c = 1; c < static_cast<int>(kCuts); ++c) {
           v[0].x = __fadd_rn(v[0].x, v[c].x);
           v[0].y = __fadd_rn(v[0].y, v[c].y);
           v[0].z = __fadd_rn(v[0].z, v[c].z);
@@ -558,6 +567,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         const uint32_t f = p.gated ? nt * (BN / 2) + lane / 16 * 32 + lane % 8 * 4 : nt * BN + col;
         const bool holds_up = p.gated && (lane & 8) != 0, live = f < feats && !holds_up;
         const float alpha = holds_up ? p.alpha_up : p.alpha;
+#pragma unroll 2
         for (uint32_t r = split + kSplit * (set * 4 + quarter); r < rows; r += kSplit * 8) {   // warp-uniform
           const uint64_t row = mt * BM + r;
           uint2 gate = make_uint2(0, 0);
@@ -630,10 +640,31 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         row_scale = __fdiv_rn(1.0f, __fmul_rn(p.ga, __ldg(p.w_divisors + (tile_expert ? min(static_cast<uint32_t>(tile_expert_of(mt)), p.experts - 1) : 0u))));
       if (lane == 0) ptx::bulk_wait_group_read<0>();
       __syncwarp();
-      if (!ptx::mbar_wait(&acc_full[as], aphase)) { fail_wait(4); break; }
+      if (!ptx::mbar_wait(&acc_full[as + kParts - 1], aphase)) { fail_wait(4); break; }   // commits are in order: so are the parts before
       ptx::tc_fence_after();
       const uint32_t tmem_acc = tmem_base + as * BN + ((quarter * 32) << 16);
       bool released = false, pending = false;
+      // The accumulators of a CTA's further parts, added in K order.
+      auto add_parts = [&](uint32_t c, uint32_t (&v0)[32], uint32_t (&v1)[32]) {
+        uint32_t w[32];
+#pragma unroll
+        for (int q = 1; q < kParts; ++q) {
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            ptx::tc_ld_32x32b_x32(tmem_acc + q * BN + c * 64 + half * 32, w);
+            ptx::tc_wait_ld();
+            uint32_t* v = half ? v1 : v0;
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__fadd_rn(__uint_as_float(v[i]), __uint_as_float(w[i])));
+          }
+        }
+      };
+      auto release = [&]() {
+        ptx::tc_fence_before();
+        __syncwarp();
+        if (lane == 0)
+          for (int q = 0; q < kParts; ++q) arrive_issuer(&acc_empty[as + q]);
+      };
       uint32_t pending_col = 0;
       uint32_t packed[32];  // one converted sub-tile: 16-byte chunk j of this lane's row = packed[4j .. 4j+3]
       // Stages `packed` in this warp's swizzled buffer and hands it to a TMA store.
@@ -721,6 +752,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         uint32_t v0[32], v1[32];
         ptx::tc_ld_32x32b_x32(tmem_acc + c * 64, v0);
         ptx::tc_ld_32x32b_x32(tmem_acc + c * 64 + 32, v1);
+        if constexpr (kParts > 1) add_parts(c, v0, v1);
         uint32_t ws_pair = 0;  // FP8: lane l holds the bf16 scales of columns col0 + 2l, col0 + 2l + 1
         if constexpr (!kFp4) {
           const uint32_t c0 = min(col0 + 2 * lane, p.n - 2);
@@ -734,9 +766,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
           // after the warp's last sub-tile is in registers and the accumulator has been released.
           ptx::tc_wait_ld();
           if (c + 2 >= BN / 64 || col0 + 128 >= p.n) {
-            ptx::tc_fence_before();
-            __syncwarp();
-            if (lane == 0) arrive_issuer(&acc_empty[as]);
+            release();
             released = true;
           }
           if (pending) emit_gated(pending_col);
@@ -753,9 +783,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
           // features comes from memory (bf16, 128 bytes of the token's row).
           ptx::tc_wait_ld();
           if (c + 2 >= BN / 64 || col0 + 128 >= p.n) {
-            ptx::tc_fence_before();
-            __syncwarp();
-            if (lane == 0) arrive_issuer(&acc_empty[as]);
+            release();
             released = true;
           }
           const uint32_t row = row0 + lane;
@@ -816,9 +844,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         // released, and the staging and the TMA stores of both follow.
         ptx::tc_wait_ld();
         if (c + 2 >= BN / 64) {
-          ptx::tc_fence_before();
-          __syncwarp();
-          if (lane == 0) arrive_issuer(&acc_empty[as]);
+          release();
           released = true;
         }
         if (pending) stage_and_store(pending_col);
@@ -852,11 +878,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         else stage_and_store(pending_col);
       }
       if (!released) {
-        ptx::tc_fence_before();
-        __syncwarp();
-        if (lane == 0) arrive_issuer(&acc_empty[as]);
+        release();
       }
-      if (++as == kAccStages) { as = 0; aphase ^= 1; }
+      if ((as += kParts) == kAccStages) { as = 0; aphase ^= 1; }
     }
     if (lane == 0) ptx::bulk_wait_group_all();
   }
@@ -980,10 +1004,10 @@ bool grouped_pairs(uint64_t padded_rows_max, uint64_t experts) {
   return g_gemm_pair == 2 || rows >= 768 * experts;
 }
 
-template <bool kFp4, int BN, int kStages, int kAccStages, bool kPair = false, int kSplit = 1>
+template <bool kFp4, int BN, int kStages, int kAccStages, bool kPair = false, int kSplit = 1, int kParts = 1>
 int32_t launch_gemm(const char* op, const void* a, const void* b, const GemmParams& p, cudaStream_t stream) {
   using C = Cfg<kFp4, BN, kStages, kAccStages, kPair>;
-  auto kern = gemm_kernel<kFp4, BN, kStages, kAccStages, kPair, kSplit>;
+  auto kern = gemm_kernel<kFp4, BN, kStages, kAccStages, kPair, kSplit, kParts>;
   constexpr unsigned kThreads = kFp4 ? kGemmThreadsFp4 : kGemmThreadsFp8;
   // First call per device and kernel variant: shared-memory opt-in and the pair occupancy,
   // serialised so that two host threads cannot race on it.
@@ -1064,9 +1088,11 @@ int32_t launch_gemm(const char* op, const void* a, const void* b, const GemmPara
 // them are resident at once (a few SMs are left: clusters cannot use every one) and each keeps at least eight K steps to cover
 // the ring's fill.  77 tokens, weights cold: FP8 8,192 x 3,840 15.4 -> 10.8 us (two parts), 3,840 x 4,096 15.2 -> 7.8 and NVFP4
 // 3,840 x 15,360 20.8 -> 12.4 (four).  (A lane per row instead of eight or sixteen in the reduction: 5-6 us more.)
-// The parts of a row's sum are part of the result: a call that fuses the GELU product shares its tiles exactly where the separate
-// gate and up projections (half the columns each) would, whatever that does to its own number of tiles, so that both forms
-// give the same bytes.  The shared branch of a mixture-of-experts layer never shares (g_whole_k): its bits must depend neither on how
+// The parts of a row's sum are part of the result: a call that fuses the GELU product cuts its sums exactly where the separate
+// gate and up projections (half the columns each) would, so that both forms give the same bytes.  Where its own, twice as many tiles
+// leave no room for as many CTAs each, a CTA takes two neighbouring parts, one per accumulator (77 tokens, cold: 2 x 8,960 x 4,096
+// 20.5 us, 2 x 3,840 x 8,192 22.5, as without parts; a CTA per part in two rounds of CTAs 28.7 and 26.6).
+// The shared branch of a mixture-of-experts layer never shares (g_whole_k): its bits must depend neither on how
 // the layer's tokens are spread over ranks nor on the form its weights are stored in.
 int dense_split(const GemmParams& p, uint32_t k_per_stage) {
   if (p.plan != nullptr || p.out_f32 || g_whole_k || g_gemm_bn != 0 || g_gemm_pair != 0) return 1;
@@ -1088,10 +1114,12 @@ int32_t launch_fp4(const char* op, const void* act, const void* w, const GemmPar
     p.expert_lo = g_expert_lo;
     p.expert_hi = g_expert_hi;
   }
-  switch (dense_split(p, 256)) {
-    case 4: return launch_gemm<true, 128, 5, 2, false, 4>(op, act, w, p, stream);
-    case 2: return launch_gemm<true, 128, 5, 2, false, 2>(op, act, w, p, stream);
-    default: break;
+  const int parts = dense_split(p, 256);
+  if (parts > 1) {
+    const uint64_t tiles = static_cast<uint64_t>((p.m + BM - 1) / BM) * ((p.n + 127) / 128);
+    const bool room = tiles * parts + 8 <= static_cast<uint64_t>(sm_count());   // always, unless gated
+    if (parts == 4) return room ? launch_gemm<true, 128, 5, 2, false, 4>(op, act, w, p, stream) : launch_gemm<true, 128, 5, 2, false, 2, 2>(op, act, w, p, stream);
+    return room ? launch_gemm<true, 128, 5, 2, false, 2>(op, act, w, p, stream) : launch_gemm<true, 128, 5, 2, false, 1, 2>(op, act, w, p, stream);
   }
   int bn = g_gemm_bn;
   if (bn == 0) {
