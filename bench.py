@@ -614,7 +614,8 @@ def moe_headline(args):
                     "tensor_at_nominal": sum(flops.values()) / world / (FP4_NOMINAL_TFLOPS * 1e12) * 1e6,
                     "weights_over_hbm": moe_layer_weight_bytes() / world / (peaks["hbm_gbs"] * 1e9) * 1e6,
                     "nvlink_combine": (tokens / world) * MOE["topk"] * (world - 1) / world * MOE["hidden"] * 2 / 770e9 * 1e6}}
-    launches_per_layer = (11 if args.fused else 12) + (3 if world > 1 else 0)
+    # shared branch 3, router 1, top-k 1, permutation 3, dispatch 1, experts 2, combine 1; unfused: two GELU quantisers more
+    launches_per_layer = (12 if args.fused else 14) + (3 if world > 1 else 0)
     line = {
         "metric": "MoE stack tokens/s", "value": value, "unit": "tokens/s", "n_gpus": world, "steps": args.steps,
         "warmup": max(args.warmup, 3), "ms_per_step": pre["secs_per_step"] * 1e3, "higher_is_better": True,
