@@ -141,10 +141,12 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 // The decode GEMVs read their weights ahead of pdl_wait.  A quantiser, whose output may be a weight matrix, therefore lets
 // its dependents start early only for fewer rows than an NVFP4 weight matrix can have (its rows are a multiple of 8; an FP8
 // matrix gets its bf16 scales from a kernel outside this library, which lets nothing start early); otherwise they start
-// when its CTAs have ended.  Kernels whose output is no weight (norms, GEMVs, the expert path) trigger always.
-constexpr uint32_t kFewRows = 7;
+// when its CTAs have ended.  Where the output is no GEMV weight (interleaved scales, a GELU product) the line is a decode batch's
+// 16 rows.  Kernels whose output is no weight at all (norms, GEMVs, the expert path) trigger always.
+constexpr uint32_t kFewRows = 7, kDecodeRows = 16;
+template <bool kMayBeWeight = true>
 __device__ __forceinline__ void pdl_trigger_few_rows(uint32_t rows) {
-  if (rows <= kFewRows) pdl_trigger();
+  if (rows <= (kMayBeWeight ? kFewRows : kDecodeRows)) pdl_trigger();
 }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Loads of data an earlier kernel of the stream produced (volatile: they stay behind pdl_wait).

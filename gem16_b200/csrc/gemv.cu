@@ -894,7 +894,7 @@ __global__ void __launch_bounds__(1024)
 fp8_quantize_decode_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ out,
                            float* __restrict__ scales, uint32_t k) {
   __shared__ float red[32];
-  pdl_trigger_few_rows(gridDim.x);
+  pdl_trigger_few_rows<>(gridDim.x);
   pdl_wait();
   const uint64_t t = blockIdx.x;
   const uint4* xp = reinterpret_cast<const uint4*>(x + t * k);

@@ -46,6 +46,7 @@ __device__ __forceinline__ void load16(const uint16_t* p, float (&v)[16]) {
 
 template <typename In>
 struct PlainLoader {
+  static constexpr bool kMayBeWeight = true;
   const In* x;
   __device__ __forceinline__ void operator()(uint64_t offset, float (&v)[16]) const {
     load16(x + offset, v);
@@ -55,6 +56,7 @@ struct PlainLoader {
 // src/cuda/nvfp4/reference.cu:177-190.  For fp32 inputs gate/up are first rounded to bf16.
 template <typename In>
 struct GatedGeluLoader {
+  static constexpr bool kMayBeWeight = false;
   const In* gate;
   const In* up;
   __device__ __forceinline__ void operator()(uint64_t offset, float (&v)[16]) const {
@@ -90,7 +92,7 @@ template <class Loader, bool kRcp, bool kInterleaved>
 __global__ void __launch_bounds__(256)
 nvfp4_quantize_kernel(Loader loader, uint8_t* __restrict__ packed, uint8_t* __restrict__ scales,
                       uint32_t tokens, uint64_t k, uint32_t blocks_pad, uint64_t cells, float g) {
-  pdl_trigger_few_rows(tokens);
+  pdl_trigger_few_rows<Loader::kMayBeWeight && !kInterleaved>(tokens);   // the GEMVs take compact scales only
   pdl_wait();
   // blockDim and cells are multiples of 4: quads stay whole.  A 64-bit division costs as much as the
   // quantisation of a block, so it is left to tensors that need it.
@@ -624,7 +626,7 @@ fp8_quantize_kernel(const In* x, const uint16_t* __restrict__ w, uint8_t* out, f
   __shared__ float red2[8];
   __shared__ __align__(16) float xs[kNorm && kShort ? kShortRow : 4];
   if constexpr (kNorm) pdl_trigger();
-  else pdl_trigger_few_rows(gridDim.x);
+  else pdl_trigger_few_rows<>(gridDim.x);
   const uint64_t r = blockIdx.x;
   const In* row = x + r * k;
   constexpr bool short_row = kNorm && kShort;
