@@ -107,7 +107,8 @@ int32_t allow_full_smem(const char* op) {
 //     stream may still be writing.  Every kernel of the chain waits, so "my predecessor has completed" implies that
 //     everything before it has.
 //   - What may be read before pdl_wait is what no early-triggering kernel writes: weight matrices with their scales (the GEMVs'
-//     first pieces) and norm weights, straight into registers.  A kernel that writes such data must not trigger.
+//     first pieces; see pdl_trigger_few_rows for small ones) and norm weights, straight into registers.  A kernel that writes such
+//     data must not trigger.
 //   - What an earlier kernel wrote is read with ld_dep, not __ldg: the read-only path promises that the data does not change
 //     while the kernel is resident, which starts before pdl_wait here.
 template <typename... P, typename... A>
@@ -139,16 +140,19 @@ int32_t launch_pdl(const char* op, void (*kern)(P...), dim3 grid, dim3 block, si
 
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
 // The decode GEMVs read their weights ahead of pdl_wait.  A quantiser, whose output may be a weight matrix, therefore lets
-// its dependents start early only for fewer rows than an NVFP4 weight matrix can have (its rows are a multiple of 8; an FP8
-// matrix gets its bf16 scales from a kernel outside this library, which lets nothing start early); otherwise they start
-// when its CTAs have ended.  Where the output is no GEMV weight (interleaved scales, a GELU product) the line is a decode batch's
-// 16 rows.  Kernels whose output is no weight at all (norms, GEMVs, the expert path) trigger always.
-constexpr uint32_t kFewRows = 7, kDecodeRows = 16;
-template <bool kMayBeWeight = true>
+// its dependents start early only for a decode batch's few rows; otherwise they start when its CTAs have ended.  A GEMV whose
+// matrix has no more rows than that, so that such a call may have written it whole, waits first (pdl_wait_small_weights).
+// (Drawing the line below the smallest matrix, at seven rows, instead costs batches of 8 to 16 tokens 1.7 us per quantiser: 13 tokens x
+// 10,040 x 9,664 22.8 -> 24.5 us.)  Kernels whose output is no weight (norms, GEMVs, the expert path) trigger always.
+constexpr uint32_t kFewRows = 16;
 __device__ __forceinline__ void pdl_trigger_few_rows(uint32_t rows) {
-  if (rows <= (kMayBeWeight ? kFewRows : kDecodeRows)) pdl_trigger();
+  if (rows <= kFewRows) pdl_trigger();
 }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Ahead of a GEMV's early weight loads; `rows` of the weight matrix.
+__device__ __forceinline__ void pdl_wait_small_weights(uint64_t rows) {
+  if (rows <= kFewRows) pdl_wait();
+}
 // Loads of data an earlier kernel of the stream produced (volatile: they stay behind pdl_wait).
 __device__ __forceinline__ uint4 ld_dep(const uint4* p) {
   uint4 v;

@@ -72,6 +72,13 @@ struct Fp8Group {
   int n;
 };
 
+// Ahead of the early weight loads: see pdl_trigger_few_rows.
+__device__ __forceinline__ void wait_small_weights(const Fp8Group& grp) {
+  uint64_t fewest = grp.p[0].rows;
+  for (int i = 1; i < grp.n; ++i) fewest = min(fewest, grp.p[i].rows);
+  pdl_wait_small_weights(fewest);
+}
+
 // Shared-memory layout of the staged activation: per 512-element segment, lane l's sixteen
 // values are split into two 8-value halves stored at [l*8, l*8+8) and [256 + l*8, 256 + l*8 + 8)
 // so that each 128-bit shared load of a warp touches 512 contiguous bytes (no bank conflicts).
@@ -223,11 +230,12 @@ fp8_gemv_kernel(const void* __restrict__ act, const float* __restrict__ act_scal
   };
 
   // Programmatic dependent launch: let the next kernel in the stream start its own weight
-  // prefetch as soon as SM slots free up; weights are immutable so they may be read before the
+  // prefetch as soon as SM slots free up; weights are at rest so they may be read before the
   // previous kernel has finished, everything else waits for it.  (Loading them behind the wait, with an L2
   // prefetch in front of it, cost a four-layer FP8 decode pass 21 of 209 us.)  No kernel that could be writing
   // weights triggers its dependents early: see pdl_trigger_few_rows.
   pdl_trigger();
+  wait_small_weights(grp);
   uint64_t task = static_cast<uint64_t>(blockIdx.x) * kW + warp;
   bool prefetched = false;
   if (task < num_tasks) {
@@ -377,6 +385,7 @@ fp8_gemv_batch_kernel(const uint8_t* __restrict__ act, const float* __restrict__
       wv[u] = kb + u * 512 + lane * 16 < k ? ldg_stream(wp + u * 512) : make_uint4(0, 0, 0, 0);
   };
   pdl_trigger();
+  wait_small_weights(grp);
   uint64_t task = static_cast<uint64_t>(blockIdx.x) * kWarps + warp;
   bool prefetched = false;
   if (task < total_rows) {
@@ -502,6 +511,7 @@ fp8_gemv_mma_kernel(const uint8_t* __restrict__ act, const float* __restrict__ a
     }
   };
   pdl_trigger();
+  wait_small_weights(grp);
   uint64_t task = blockIdx.x;
   const uint64_t first_kb = static_cast<uint64_t>(warp) * kMmaSpan;
   const uint8_t* ra = nullptr;
@@ -613,7 +623,7 @@ int32_t launch_fp8_gemv_batch(const char* op, const uint8_t* act, const float* a
 // producer streams chunk after chunk into a ring of shared-memory stages with 1-D bulk copies
 // (cp.async.bulk, completion on an mbarrier), so the bytes in flight are bounded by shared
 // memory (about 190 KB per SM), not by registers, and keep flowing while the consumers quantise
-// the activation or wait for the previous kernel (weights are immutable, so the producer starts
+// the activation or wait for the previous kernel (weights are at rest, so the producer starts
 // before griddepcontrol.wait).  Consumer warp w owns stage w, i.e. the CTA's chunks w, w+12, ...
 // (an mbarrier parity wait may run at most one phase ahead, so a warp must see every phase of
 // the stages it waits on): it dots every row of the chunk from shared memory and releases the
@@ -684,6 +694,7 @@ fp8_gemv_ring_kernel(const void* __restrict__ act, const float* __restrict__ act
 
   if (warp == 0) {
     if (lane == 0) {
+      wait_small_weights(grp);
       uint32_t stage = 0, phase = 0;
       for (uint32_t j = 0; j < my_chunks && !*abort_flag; ++j) {
         if (!ptx::mbar_wait(&empty[stage], phase ^ 1, 1u << 18)) {
@@ -699,7 +710,7 @@ fp8_gemv_ring_kernel(const void* __restrict__ act, const float* __restrict__ act
       }
     }
   } else {
-    // Everything that is not an immutable weight is read only after the previous kernel is done.
+    // Everything that is not a weight is read only after the previous kernel is done.
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int ctid = threadIdx.x - 32, cthreads = kRingConsumers * 32;
     float a_scale;
@@ -894,7 +905,7 @@ __global__ void __launch_bounds__(1024)
 fp8_quantize_decode_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ out,
                            float* __restrict__ scales, uint32_t k) {
   __shared__ float red[32];
-  pdl_trigger_few_rows<>(gridDim.x);
+  pdl_trigger_few_rows(gridDim.x);
   pdl_wait();
   const uint64_t t = blockIdx.x;
   const uint4* xp = reinterpret_cast<const uint4*>(x + t * k);

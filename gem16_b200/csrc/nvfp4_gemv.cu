@@ -17,7 +17,8 @@
 // work cost as much as SMs without loads.  Measured, weights cold, in a chain of launches: gate / up 2 x 15,360 x 3,840 in
 // 18 us for one token and 20 us for five (23 us per token before, one launch each), down 3,840 x 15,360 in 12 and
 // 14 us (11 and 67 us before); without the loads the arithmetic takes 12 us, without the arithmetic
-// the loads 8.  A warp's first pieces are loaded ahead of pdl_wait (weights are immutable): 7 % of a decode pass.
+// the loads 8.  A warp's first pieces are loaded ahead of pdl_wait (weights are at rest, see pdl_trigger_few_rows): 7 % of a
+// decode pass.
 // Requesting all weights into L2 ahead of it changed nothing: the kernels before
 // this one then wait for HBM instead.  Lane 4g + t loads 32 contiguous bytes of rows g and g + 8 per piece
 // (four scale blocks each) and the four scale bytes that go with them; MMA j takes bytes 2j, 2j + 1 of that run as
@@ -175,6 +176,7 @@ nvfp4_gemv_kernel(const __grid_constant__ Fp4GemvArgs a) {
   auto share = [&](uint32_t w) { return list * w / kFpWarps; };
   const uint64_t lo = share(warp), hi = share(warp + 1);
   pdl_trigger();
+  pdl_wait_small_weights(a.rows);
   // Load cursor: piece `next` of the list = piece `np` of the tile whose rows the pointers stand on.
   uint64_t next = lo;
   uint32_t ntile = static_cast<uint32_t>(lo / pieces), np = static_cast<uint32_t>(lo % pieces);

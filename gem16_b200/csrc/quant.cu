@@ -46,7 +46,6 @@ __device__ __forceinline__ void load16(const uint16_t* p, float (&v)[16]) {
 
 template <typename In>
 struct PlainLoader {
-  static constexpr bool kMayBeWeight = true;
   const In* x;
   __device__ __forceinline__ void operator()(uint64_t offset, float (&v)[16]) const {
     load16(x + offset, v);
@@ -56,7 +55,6 @@ struct PlainLoader {
 // src/cuda/nvfp4/reference.cu:177-190.  For fp32 inputs gate/up are first rounded to bf16.
 template <typename In>
 struct GatedGeluLoader {
-  static constexpr bool kMayBeWeight = false;
   const In* gate;
   const In* up;
   __device__ __forceinline__ void operator()(uint64_t offset, float (&v)[16]) const {
@@ -92,7 +90,7 @@ template <class Loader, bool kRcp, bool kInterleaved>
 __global__ void __launch_bounds__(256)
 nvfp4_quantize_kernel(Loader loader, uint8_t* __restrict__ packed, uint8_t* __restrict__ scales,
                       uint32_t tokens, uint64_t k, uint32_t blocks_pad, uint64_t cells, float g) {
-  pdl_trigger_few_rows<Loader::kMayBeWeight && !kInterleaved>(tokens);   // the GEMVs take compact scales only
+  pdl_trigger_few_rows(tokens);
   pdl_wait();
   // blockDim and cells are multiples of 4: quads stay whole.  A 64-bit division costs as much as the
   // quantisation of a block, so it is left to tensors that need it.
@@ -446,7 +444,7 @@ __device__ __forceinline__ float load_short_row(const In* row, uint32_t k, float
   }
   return ss;
 }
-// The norm weights of elements 16 c .. 16 c + 15, before the wait for the previous kernel (weights are immutable).
+// The norm weights of elements 16 c .. 16 c + 15, before the wait for the previous kernel (they are at rest).
 __device__ __forceinline__ void load_norm_weights(const uint16_t* w, uint32_t c, uint32_t k, uint16_t (&wv)[16]) {
   if (w && c * 16 < k && (reinterpret_cast<uintptr_t>(w) & 15) == 0) {   // k is a multiple of 16
     const uint4 a = __ldg(reinterpret_cast<const uint4*>(w) + 2 * c), b = __ldg(reinterpret_cast<const uint4*>(w) + 2 * c + 1);
@@ -626,7 +624,7 @@ fp8_quantize_kernel(const In* x, const uint16_t* __restrict__ w, uint8_t* out, f
   __shared__ float red2[8];
   __shared__ __align__(16) float xs[kNorm && kShort ? kShortRow : 4];
   if constexpr (kNorm) pdl_trigger();
-  else pdl_trigger_few_rows<>(gridDim.x);
+  else pdl_trigger_few_rows(gridDim.x);
   const uint64_t r = blockIdx.x;
   const In* row = x + r * k;
   constexpr bool short_row = kNorm && kShort;

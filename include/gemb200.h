@@ -198,10 +198,9 @@ int32_t gemb_add_residual_f32(const float* values, const float* residual, float*
  * Weights are taken to be at rest: these calls request their first weight bytes (gemb_rmsnorm_residual and the
  * RMSNorm quantizers their norm weights) while the kernels in front of them in the stream still run.  What a copy, a memset,
  * a kernel from elsewhere or a call of this library that writes a whole weight matrix has written by then is
- * always seen (gemb_nvfp4_quantize with COMPACT scales and gemb_fp8_quantize of eight rows or more,
- * gemb_nvfp4_interleave_scales, gemb_nvfp4_pack_gate_up).  Only a matrix that is being quantised in pieces of fewer than eight
- * rows -- the size of a decode step's activations, whose quantizers overlap the projection behind them -- or one of up
- * to 16 rows whose payload comes from a call with INTERLEAVED scales must be separated from
+ * always seen (gemb_nvfp4_quantize, gemb_fp8_quantize, gemb_nvfp4_interleave_scales, gemb_nvfp4_pack_gate_up).
+ * Only a matrix of more than 16 rows that is being quantised in pieces of 16 rows or fewer -- the size of a decode
+ * batch's activations, whose quantizers overlap the projection behind them -- must be separated from
  * the first call that uses it as a weight by a synchronisation or a copy, or be used with GEMB_TUNE_GEMV_PDL 0.
  * ---------------------------------------------------------------------------------------- */
 

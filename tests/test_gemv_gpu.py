@@ -292,7 +292,7 @@ def test_nvfp4_gemv_tiles_and_token_counts(lib, dev, orc, rows, k, shift):
         assert all(torch.equal(a, b[:t]) for a, b in zip(o, outs[t_max]))
 
 
-@pytest.mark.parametrize("rows,k", [(8, 64), (8, 15360), (16, 3840), (24, 8192)])
+@pytest.mark.parametrize("rows,k", [(8, 64), (8, 15360), (16, 3840), (24, 8192), (32, 16384)])
 @pytest.mark.parametrize("act_first", [False, True])
 def test_weight_quantised_on_the_device_is_seen_at_once(lib, dev, rows, k, act_first):
     """A whole weight matrix, however small, may be quantised right in front of the GEMV that uses it, although the GEMV
