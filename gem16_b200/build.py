@@ -1,16 +1,18 @@
-"""In-tree build of libgemb200.so (sm_100a only) with plain nvcc.
+"""In-tree build of libgemb200.so (sm_100a only) with plain nvcc, and of the Python binding beside it.
 
     python -m gem16_b200.build [--force] [--verbose]
     GEMB_NVTX=1 python -m gem16_b200.build --force      (NVTX range around every entry point)
 
 The shared object lands next to this file so it travels with the source tree.  It links the
-CUDA runtime statically and has no Python or torch dependency.
+CUDA runtime statically and has no Python or torch dependency.  The binding (_binding, a CPython extension
+generated from the header) links against it and is only needed by lib.py.
 """
 from __future__ import annotations
 
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
@@ -29,6 +31,42 @@ def sources() -> list[str]:
 def headers() -> list[str]:
     hs = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
     return hs + [os.path.join(ROOT, "include", "gemb200.h")]
+
+
+BINDING = os.path.join(HERE, "_binding" + sysconfig.get_config_var("EXT_SUFFIX"))
+
+
+def binding_source() -> str:
+    """C++ of the extension: one METH_FASTCALL function per entry point that returns a status."""
+    from .lib import parse_header
+    functions, table = [], []
+    for name, (ret, params) in parse_header().items():
+        if ret != "int32_t":
+            continue
+        decl, args = [], []
+        for i, (ctype, _) in enumerate(params):
+            kind = "stream" if ctype == "gemb_stream_t" else "pointer" if "*" in ctype else "real" if ctype == "float" else "integer"
+            decl.append(f"  {'double' if kind == 'real' else 'unsigned long long'} a{i};\n  if (!{kind}(args[{i}], &a{i})) return nullptr;\n")
+            args.append(f"({ctype})a{i}" if kind in ("real", "integer") else f"reinterpret_cast<{ctype}>(a{i})")
+        functions.append(f"PyObject* py_{name}(PyObject*, PyObject* const* args, Py_ssize_t n) {{\n"
+                         f"  if (n != {len(params)}) return wrong_count(\"{name}\", {len(params)}, n);\n{''.join(decl)}"
+                         f"  int32_t rc;\n  Py_BEGIN_ALLOW_THREADS\n  rc = {name}({', '.join(args)});\n  Py_END_ALLOW_THREADS\n"
+                         "  return finish(rc);\n}\n")
+        table.append(f'  {{"{name}", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_{name})), METH_FASTCALL, nullptr}},\n')
+    with open(os.path.join(CSRC, "binding.inc")) as f:
+        return f.read().replace("@FUNCTIONS@", "".join(functions)).replace("@TABLE@", "".join(table))
+
+
+def build_binding(force: bool = False) -> None:
+    template, header = os.path.join(CSRC, "binding.inc"), os.path.join(ROOT, "include", "gemb200.h")
+    newest = max(os.path.getmtime(f) for f in (template, header, os.path.abspath(__file__)))
+    if not force and os.path.exists(BINDING) and os.path.getmtime(BINDING) >= newest:
+        return
+    src = os.path.join(OBJ, "binding.cpp")
+    with open(src, "w") as f:
+        f.write(binding_source())
+    subprocess.check_call(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-I", os.path.join(ROOT, "include"), "-I",
+                           sysconfig.get_paths()["include"], src, "-o", BINDING, "-L", HERE, "-l:libgemb200.so", "-Wl,-rpath,$ORIGIN"])
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -54,6 +92,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         subprocess.check_call([NVCC, "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-o", LIB, *objs,
                                "-cudart", "static",
                                "-Xlinker", "--no-undefined", "-ldl", "-lpthread", "-lrt"])
+    build_binding(force)
     return LIB
 
 

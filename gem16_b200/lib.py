@@ -1,7 +1,7 @@
-"""ctypes loader for libgemb200.so.
+"""Loader for libgemb200.so.
 
 Prototypes are derived from include/gemb200.h itself, so the binding cannot drift from the
-header.  Every call checks the returned gemb_status and raises GembError carrying the status
+header: checked calls go through an extension that build.py generates from it, everything else through ctypes.  Every call checks the returned gemb_status and raises GembError carrying the status
 name and gemb_last_error().  A missing library is a hard error: nothing here falls back to
 another implementation.
 """
@@ -95,9 +95,6 @@ def _ctype(t: str):
     return _SCALARS[t.replace("const ", "")]
 
 
-_PLAIN = frozenset((int, float, type(None)))
-
-
 def _as_arg(v):
     if v is None:
         return None
@@ -113,6 +110,15 @@ def _as_arg(v):
     return v
 
 
+def _as_address(v):
+    """What the binding cannot convert by itself: ctypes structures, arrays, pointers and references, and bytes."""
+    if type(v).__name__ == "CArgObject":   # byref()
+        return C.addressof(v._obj)
+    if isinstance(v, bytes) or hasattr(v, "contents") or isinstance(v, (C.c_void_p, C.c_char_p)):
+        return C.cast(v, C.c_void_p).value
+    return _as_arg(v)
+
+
 class Lib:
     def __init__(self, path: str = LIB_PATH):
         if not os.path.exists(path):
@@ -120,6 +126,12 @@ class Lib:
                 f"{path} is missing: build it with `python -m gem16_b200.build` (no fallback exists)")
         self.path = path
         self.cdll = C.CDLL(path)
+        try:
+            from . import _binding
+        except ImportError as e:
+            raise RuntimeError(f"the Python binding is missing: build it with `python -m gem16_b200.build` ({e})") from e
+        _binding.setup(_as_address, self._raise)
+        self.binding = _binding
         self.protos = parse_header()
         for name, (ret, params) in self.protos.items():
             fn = getattr(self.cdll, name)
@@ -135,24 +147,21 @@ class Lib:
         return getattr(self.cdll, name)(*[_as_arg(a) for a in args])
 
     def __getattr__(self, name: str):
-        """The checked call of an entry point, built once and kept on the instance: a decode call is a few
-        microseconds on the GPU, so the host path must not cost more.  Plain numbers, None and
-        tensors (by far the most arguments) are converted without going through _as_arg."""
+        """The checked call of an entry point, kept on the instance."""
         if not name.startswith("gemb_"):
             raise AttributeError(name)
-        fn = getattr(self.cdll, name)
-        plain, convert = _PLAIN, _as_arg
         if self.protos[name][0] == "int32_t":
-            def call(*args):
-                rc = fn(*[a if type(a) in plain else convert(a) for a in args])
-                if rc:
-                    raise GembError(rc, self.last_error())
-                return rc
+            call = getattr(self.binding, name)
         else:
+            fn = getattr(self.cdll, name)
+
             def call(*args):
-                return fn(*[a if type(a) in plain else convert(a) for a in args])
+                return fn(*[_as_arg(a) for a in args])
         setattr(self, name, call)
         return call
+
+    def _raise(self, rc: int):
+        raise GembError(rc, self.last_error())
 
 
 _LIB: Lib | None = None

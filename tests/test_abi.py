@@ -115,3 +115,24 @@ def test_plan_record_and_abi_version(lib):
         tiles = lib.cdll.gemb_moe_padded_rows_max(tokens, experts, topk) // 128
         assert lib.cdll.gemb_moe_plan_ints(tokens, experts, topk) == 2 + experts + 1 + 2 * tiles + 1 + tiles
         assert lib.cdll.gemb_moe_ep_plan_ints(tokens * topk, experts) >= 2 + experts + 1 + 2 * (tokens * topk // 128) + 1 + tokens * topk // 128
+
+
+def test_checked_calls_convert_their_arguments(lib):
+    """The generated binding: addresses as numbers, tensors or ctypes objects, status errors with the library's message, and
+    arguments that fit no parameter refused before the call."""
+    import ctypes as C
+    import torch
+    from gem16_b200.lib import GembError
+    t, buf = torch.zeros(64, dtype=torch.uint8), (C.c_uint8 * 64)()
+    for p in (64, t, buf, C.c_void_p(64), C.byref(buf), b"x" * 64):
+        with pytest.raises(GembError, match="multiple of 16") as e:
+            lib.gemb_fp8_gemv(p, p, p, p, p, 8, 24, None)      # K % 16: refused on the host
+        assert e.value.status_name == "kInvalidArgument"
+    with pytest.raises(GembError, match="nonnull"):
+        lib.gemb_fp8_gemv(None, t, t, t, t, 8, 32, None)
+    with pytest.raises(TypeError):
+        lib.gemb_fp8_gemv(t, t, t, t, t, 8, 32)
+    with pytest.raises(TypeError):
+        lib.gemb_fp8_gemv(t, t, t, t, t, 8.5, 32, None)
+    with pytest.raises(TypeError):
+        lib.gemb_nvfp4_gemv(t, t, t, t, t, 8, 64, "1", 1.0, None)
