@@ -111,24 +111,34 @@ int32_t allow_full_smem(const char* op) {
 //     data must not trigger.
 //   - What an earlier kernel wrote is read with ld_dep, not __ldg: the read-only path promises that the data does not change
 //     while the kernel is resident, which starts before pdl_wait here.
+// `beside`: a kernel of a few CTAs that runs while the CTAs of a decode projection (decode_gemv.cu), which want nearly all shared memory of
+// an SM, become resident: it takes the SM's largest shared-memory split too, because an SM changes its split only when it is empty.
+// Not for kernels that stream through registers: their loads in flight live in what is left to L1 (fp8_gemv_kernel 173 -> 213 us
+// for sixteen projections).
 template <typename... P, typename... A>
-int32_t launch_pdl(const char* op, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+int32_t launch_pdl_split(const char* op, bool beside, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+  attr[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+  attr[1].val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = beside ? 2 : 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(GEMB_INTERNAL, "%s: %s: %s", op, cudaGetErrorName(e), cudaGetErrorString(e));
   }
   return GEMB_OK;
+}
+template <typename... P, typename... A>
+int32_t launch_pdl(const char* op, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+  return launch_pdl_split(op, false, kern, grid, block, smem, stream, args...);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -152,6 +162,13 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 // Ahead of a GEMV's early weight loads; `rows` of the weight matrix.
 __device__ __forceinline__ void pdl_wait_small_weights(uint64_t rows) {
   if (rows <= kFewRows) pdl_wait();
+}
+// A line that will be read behind pdl_wait, into L2 ahead of it.  L2 is where all SMs meet, so it does not matter whether the line is
+// still being written.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+// The lines of `bytes` bytes, shared among the CTA's threads.
+__device__ __forceinline__ void prefetch_l2_span(const void* p, uint64_t bytes) {
+  for (uint64_t i = threadIdx.x * 128ull; i < bytes; i += blockDim.x * 128ull) prefetch_l2(static_cast<const uint8_t*>(p) + i);
 }
 // Loads of data an earlier kernel of the stream produced (volatile: they stay behind pdl_wait).
 __device__ __forceinline__ uint4 ld_dep(const uint4* p) {

@@ -1,0 +1,652 @@
+// Decode projections for 1 .. 8 tokens on tcgen05: y[t, r] = sum_k x[t, k] w[r, k], NVFP4 (kind::mxf4nvf4, block scales in
+// tensor memory) and FP8 (kind::f8f6f4).  The weights are the 128-row side of the MMA and go from memory to the tensor core as
+// they lie, by TMA: no thread converts, scales or even sees a weight.
+//
+// A CTA per SM owns whole output rows, in tiles of up to 32, so that no partial sum leaves the SM.  32 rows would fill a quarter of
+// the MMA; the 128 rows are therefore the same rows at four places of K: group q (MMA rows 32 q ..) takes the 128-byte
+// chunks 4 s + q of step s.  The other side holds one column per token and group, (t, q) = the token's values at group q's place of
+// K, and of the accumulator only the cells where the groups agree are used.  The partial sums of a row meet in the
+// epilogue.  The tensor core does four times the work that is wanted, for 16 or 32 columns, which is nothing: a step of four chunks (13 KB
+// for 26 rows) takes its two issuing threads 0.1 us, a third of the time that HBM needs to deliver it.
+//
+// Large matrices stream at the copy rate (FP8 30,720 x 3,840: 6.7 TB/s between the first tile and the last).  What bounds a decode step is
+// the way from one projection to the next: the previous kernel's end, the quantisers between, the activations' way into shared memory.
+//   - The producer requests the first 80 KB of an SM's weights before the previous kernel has ended (weights are at rest, see
+//     pdl_trigger_few_rows).  More (120, 160 KB) makes the row kernels' own loads wait for HBM: a mixed decode pass 188 -> 193 -> 195 us;
+//     40 KB: 189, FP8 193 instead of 189.
+//   - Weights and block scales carry an evict-first policy: without it they take the code of the kernels between out of L2 and
+//     every small kernel fetches its instructions from memory (with the policy 206 -> 188 us for the mixed pass, 232 -> 215 for five tokens).
+//   - The row kernels run with the largest shared-memory split too (launch_pdl_split), otherwise the SM they sit on gets its CTA of this kernel
+//     last, with nothing requested.
+// Four layers of a decode pass, start -> now: FP8 204 -> 188 us, FP8 attention with NVFP4 MLP 216 -> 187, the latter with five tokens
+// 264 -> 217 (mma.sync kernels with weights through registers before).
+//
+// Sums: the steps alternate between two issuing threads, each with accumulators of its own; FP8 cuts a thread's share into further
+// chains, because the tensor core truncates where an IEEE addition rounds, and the epilogue keeps what its additions round off (relative
+// error against binary64 4.5 .. 5.5e-8 for K 1,024 .. 15,360 and one token; 4.7 .. 7.3e-8 with fp32 fma chains; NVFP4: sums of a decode
+// projection are exact almost everywhere, the final division is what rounds).  How NVFP4 sums are cut depends on K alone, and a token's
+// columns on the token alone: a result is the same bits for every batch size.  FP8: the same bits for 1 .. 4 and for 5 .. 8 tokens.
+//
+// Warps: 0 producer (TMA), 1 and 6 MMA issuers, 2-5 stage the activations (and, NVFP4, their scales into tensor memory), then the
+// epilogue, 7-14 NVFP4 block scales (through registers into the order that tcgen05.cp wants: 4-byte loads, since a scale row is only
+// 4-byte aligned; eight warps with two steps each in flight, four warps cost the mixed pass 8 us).
+#include <algorithm>
+#include <type_traits>
+
+#include "decode_gemv.h"
+#include "ptx.cuh"
+#include "tensor_map.h"
+
+namespace gemb {
+
+__device__ int g_decode_error = 0;
+
+namespace {
+
+constexpr uint32_t kGroups = 4, kGroupRows = 32;
+constexpr uint32_t kStageBytes = kGroups * kGroupRows * 128;
+constexpr uint32_t kSfStageBytes = 2048;      // four chunks of 32 rows x 16 bytes, one per MMA
+constexpr uint32_t kEarlyBytes = 80 * 1024;   // weights requested ahead of the wait for the previous kernel
+constexpr uint32_t kMaxStages = 12, kMinStages = 4;
+constexpr uint32_t kScaleWarps = 8;
+constexpr uint32_t kThreadsFp8 = 224, kThreadsFp4 = 224 + 32 * kScaleWarps;
+constexpr size_t kSmemBudget = 204 * 1024;    // leaves room for a row kernel's CTA on the same SM
+// TMEM columns: two accumulator slots ([matrix][issuer][chain]), NVFP4 two regions of weight scales per issuer, then the tokens' scales.
+constexpr uint32_t kIssuers = 2, kChainCols = 64;   // FP8 chains of a sum: what fits these columns, per issuer
+constexpr uint32_t kSfaCols = kIssuers * 2 * 16;
+// NVFP4, tensor memory: 20 steps' token scales beside the accumulators of one matrix, 12 beside those of two.
+constexpr uint64_t kFp4MaxK = 20480, kFp4MaxKTwo = 12288;
+
+template <int kMaps>
+struct Maps {
+  CUtensorMap m[kMaps];
+};
+struct Args {
+  const void* act;
+  const void* act_scales;
+  const void* scales[3];
+  void* out[3];
+  float div[2];
+  float* product;
+  uint32_t rows[3], tile_start[4];
+  uint32_t tile_rows, k, tokens, columns, stages, early, fewest_rows;
+  bool words;      // NVFP4: the tokens' scales are 4-byte aligned
+  bool bf16_out;   // FP8, kQuant
+};
+
+// Barrier of the four staging / epilogue warps; true in all of them when one of them says so.
+__device__ __forceinline__ bool epi_barrier_or(bool v) {
+  uint32_t r;
+  asm volatile("{ .reg .pred p, q; setp.ne.b32 q, %1, 0;\n"
+               "barrier.cta.red.or.pred p, 2, 128, q;\n"
+               "selp.u32 %0, 1, 0, p; }"
+               : "=r"(r)
+               : "r"(static_cast<uint32_t>(v))
+               : "memory");
+  return r != 0;
+}
+
+// a + b; what the rounding lost (Knuth's two-sum) goes to `lost`.
+__device__ __forceinline__ float add_keep(float a, float b, float& lost) {
+  const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
+  lost = __fadd_rn(lost, __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb)));
+  return s;
+}
+
+template <bool kFp4, int kMats, bool kQuant, int kMaps>
+__global__ void __maxnreg__(96)   // 448 threads: leaves the registers for a row kernel's CTA beside it
+decode_gemv_kernel(const __grid_constant__ Maps<kMaps> maps, const __grid_constant__ Args a) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const uint32_t row_bytes = kFp4 ? a.k / 2 : a.k;
+  const uint32_t steps = (row_bytes + kGroups * 128 - 1) / (kGroups * 128);
+  const uint32_t stages = a.stages, b_step = (a.tokens + 1) / 2 * 1024;
+  uint8_t* stage_w = smem;
+  uint8_t* stage_sf = stage_w + stages * kStageBytes;
+  uint8_t* xb = stage_sf + (kFp4 ? stages * kSfStageBytes : 0);
+  // Eight columns are 1,024 bytes.  Where fewer than `columns` hold tokens the MMA reads on into the next step's: cells nobody uses.
+  float* part = reinterpret_cast<float*>(xb + steps * b_step);     // [2][matrix, or FP8: sums and what they lost][group][token][32]
+  const uint32_t part_floats = (kFp4 ? kMats : 2) * kGroups * a.tokens * kGroupRows;   // the room is at least steps x 512 bytes (NVFP4)
+  uint64_t* full = reinterpret_cast<uint64_t*>(part + max(2 * part_floats, kFp4 ? steps * 128 : 0u));
+  uint64_t* empty = full + kMaxStages;
+  uint64_t* acc_full = empty + kMaxStages;
+  uint64_t* acc_empty = acc_full + 2;
+  uint64_t* x_ready = acc_empty + 2;
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(x_ready + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
+
+  // The scale warps have nothing else to do while the activations are staged.
+  constexpr uint32_t kStagingThreads = 128 + (kFp4 ? 32 * kScaleWarps : 0);
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (uint32_t s = 0; s < stages; ++s) {
+      ptx::mbar_init(&full[s], kFp4 ? 2 : 1);
+      ptx::mbar_init(&empty[s], 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      ptx::mbar_init(&acc_full[s], kIssuers);
+      ptx::mbar_init(&acc_empty[s], 4);
+    }
+    ptx::mbar_init(x_ready, kStagingThreads / 32);
+    *abort_flag = 0;
+    ptx::fence_barrier_init();
+  }
+  __syncthreads();
+  // FP8: a sum's MMAs form chains of a few steps, each in an accumulator of its own, because the tensor core truncates where the
+  // epilogue's additions round.
+  const uint32_t own = (steps + kIssuers - 1) / kIssuers;
+  const uint32_t chain_steps = kFp4 ? own : (own * a.columns + kChainCols - 1) / kChainCols;
+  const uint32_t chains = kFp4 ? 1 : (own + chain_steps - 1) / chain_steps;
+  const uint32_t acc_cols = chains * a.columns, slot_cols = kMats * kIssuers * acc_cols;   // [slot][matrix][issuer][chain]
+  const uint32_t sfa_col = 2 * slot_cols, sfb_col = sfa_col + kSfaCols;
+  const uint32_t tmem_want = kFp4 ? sfb_col + steps * 16 : 2 * slot_cols;
+  const uint32_t tmem_cols = tmem_want <= 64 ? 64u : tmem_want <= 128 ? 128u : tmem_want <= 256 ? 256u : 512u;
+  const uint32_t tiles = a.tile_start[kFp4 ? 1 : 3];
+  const uint32_t my_tiles = (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x;
+  auto fail_wait = [&](int code) {
+    atomicCAS(&g_decode_error, 0, code);
+    *abort_flag = 1;
+  };
+  auto problem_of = [&](uint32_t tile) -> uint32_t {   // FP8: the matrix whose rows the tile holds
+    if constexpr (kMaps == 1 || kFp4) return 0;
+    return (tile >= a.tile_start[1] ? 1u : 0u) + (tile >= a.tile_start[2] ? 1u : 0u);
+  };
+
+  // 16-byte pieces of the tokens, in the 128-byte swizzle of the K-major operand; zeros past K.  Up to eight loads of a thread in flight.
+  const uint32_t pieces = steps * kGroups * 8;   // per token
+  auto place = [&](uint32_t token, uint32_t piece, const uint4& v) {
+    const uint32_t chunk = piece / 8, col = (chunk % kGroups) * a.tokens + token;
+    *reinterpret_cast<uint4*>(xb + (chunk / kGroups) * b_step + col * 128 + ((piece % 8 ^ (col & 7)) << 4)) = v;
+  };
+  auto stage_activations = [&](uint32_t tid) {
+    const uint32_t stride = row_bytes / 16;
+    const uint4* x = static_cast<const uint4*>(a.act);
+    if (a.tokens == 1) {
+#pragma unroll 1
+      for (uint32_t p0 = tid; p0 < pieces; p0 += 4 * kStagingThreads) {
+        uint4 v[4];
+#pragma unroll
+        for (uint32_t u = 0; u < 4; ++u) v[u] = p0 + u * kStagingThreads < stride ? ld_dep(x + p0 + u * kStagingThreads) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (uint32_t u = 0; u < 4; ++u)
+          if (p0 + u * kStagingThreads < pieces) place(0, p0 + u * kStagingThreads, v[u]);
+      }
+    } else {
+#pragma unroll 1
+      for (uint32_t p = tid; p < pieces; p += kStagingThreads) {
+        uint4 v[8];
+#pragma unroll
+        for (uint32_t t = 0; t < 8; ++t) v[t] = t < a.tokens && p < stride ? ld_dep(x + t * stride + p) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (uint32_t t = 0; t < 8; ++t)
+          if (t < a.tokens) place(t, p, v[t]);
+      }
+    }
+  };
+  // kQuant: one bf16 token, quantised as gemb_fp8_quantize does it; returns the scale.
+  auto quantise_activation = [&](uint32_t tid, uint32_t group, uint32_t lane) {
+    const uint4* x = static_cast<const uint4*>(a.act);
+    const uint32_t words = a.k / 8;   // of eight elements
+    float amax = 0.0f;
+    for (uint32_t w0 = tid; w0 < words; w0 += 4 * 128) {
+      uint4 v[4];
+#pragma unroll
+      for (uint32_t u = 0; u < 4; ++u) v[u] = w0 + u * 128 < words ? ld_dep(x + w0 + u * 128) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (uint32_t u = 0; u < 4; ++u) {
+        const uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) amax = fmaxf(amax, fmaxf(fabsf(__uint_as_float(w[j] << 16)), fabsf(__uint_as_float(w[j] & 0xFFFF0000u))));
+      }
+    }
+    amax = warp_max(amax);
+    if (lane == 0) part[group] = amax;
+    epi_barrier_or(false);
+    const Quotient q = token_quotient(fmaxf(fmaxf(part[0], part[1]), fmaxf(part[2], part[3])));
+    epi_barrier_or(false);   // `part` is free
+    for (uint32_t p = tid; p < pieces; p += 128) {
+      uint4 v = make_uint4(0, 0, 0, 0);
+      if (p * 16 < a.k) {
+        const uint4 lo = ld_dep(x + 2 * p), hi = ld_dep(x + 2 * p + 1);
+        const uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+        uint32_t c[8];
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) {
+          const float2 e = make_float2(__uint_as_float(w[j] << 16), __uint_as_float(w[j] & 0xFFFF0000u));
+          c[j] = q.divide ? e4m3x2_divided(e.x, e.y, q.scale) : e4m3_of_quotients(e, q);
+        }
+        v = make_uint4(c[0] | c[1] << 16, c[2] | c[3] << 16, c[4] | c[5] << 16, c[6] | c[7] << 16);
+      }
+      place(0, p, v);
+    }
+    return q.scale;
+  };
+
+  if (warp == 0) {
+    // ------------------------------- weights --------------------------------------------------
+    if (ptx::elect_one()) {
+      if (a.fewest_rows <= kFewRows) pdl_wait();
+      const uint64_t policy = ptx::evict_first_policy();   // the weights' stream must not take the code and the activations out of L2
+      uint32_t stage = 0, phase = 0, n = 0;
+      for (uint32_t t = 0; t < my_tiles && !*abort_flag; ++t) {
+        const uint32_t tile = blockIdx.x + t * gridDim.x, p = problem_of(tile);
+        const int32_t row0 = static_cast<int32_t>((tile - a.tile_start[p]) * a.tile_rows);
+        for (uint32_t i = 0; i < kMats * steps; ++i, ++n) {
+          const uint32_t mat = i >= steps ? 1u : 0u, s = i - mat * steps;
+          if (n == a.early) pdl_wait();   // `early` <= `stages`: from there on this thread waits for MMAs that wait for the previous kernel
+          if (n >= stages && !ptx::mbar_wait(&empty[stage], phase ^ 1)) { fail_wait(11); break; }
+          ptx::mbar_expect_tx(&full[stage], kGroups * a.tile_rows * 128);
+          // Chunks past the end of a row arrive as zeros, rows past the matrix too.
+#pragma unroll
+          for (uint32_t q = 0; q < kGroups; ++q)
+            ptx::tma_load_2d_hint(stage_w + stage * kStageBytes + q * (kGroupRows * 128), &maps.m[kMaps == 1 ? 0 : kFp4 ? mat : p], ptx::smem_addr(&full[stage]),
+                                  static_cast<int32_t>((s * kGroups + q) * 128), row0, policy);
+          if (++stage == stages) { stage = 0; phase ^= 1; }
+        }
+      }
+    }
+  } else if (warp == 1 || warp == 6) {
+    // ------------------------------- MMA issuers ----------------------------------------------
+    // An MMA takes about 80 clocks to issue and few to execute: two threads share the steps, each with accumulators of its own.  The
+    // number of stages is even, so that a stage always belongs to the same thread (a parity wait must see every phase).
+    const uint32_t issuer = warp == 1 ? 0u : 1u;
+    if (issuer == 0) {
+      ptx::tmem_alloc(tmem_holder, tmem_cols);
+      // Only now may the kernel behind this one start: where its CTAs fit beside these they allocate tensor memory too, and keep it
+      // until this kernel has ended.
+      pdl_trigger();
+    }
+    ptx::tc_fence_before();
+    asm volatile("bar.sync 1, 192;" ::: "memory");
+    ptx::tc_fence_after();
+    const uint32_t tmem = *tmem_holder;
+    if (ptx::elect_one()) {
+      pdl_wait();
+      const uint32_t idesc = kFp4 ? ptx::idesc_nvfp4(128, a.columns) : ptx::idesc_e4m3(128, a.columns);
+      uint32_t stage = issuer, phase = 0, slot = 0, slot_phase = 0, sfa_buf = 0;
+      uint32_t ready = 0;   // own steps from here on whose barriers have been seen complete
+      // An answer of a barrier takes longer than a step's MMAs: after the one that is waited for, the next four are asked for together.
+      auto wait_steps = [&]() {
+        if (!ptx::mbar_wait(&full[stage], phase)) return false;
+        bool seen[4];
+        uint32_t st = stage, ph = phase;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if ((st += kIssuers) >= stages) { st = issuer; ph ^= 1; }
+          seen[i] = ptx::mbar_test_wait(&full[st], ph);
+        }
+        ready = 1 + (seen[0] ? 1 + (seen[1] ? 1 + (seen[2] ? 1 + (seen[3] ? 1 : 0) : 0) : 0) : 0);
+        return true;
+      };
+      if (issuer < my_tiles * kMats * steps && !wait_steps()) fail_wait(14);
+      if (!ptx::mbar_wait(x_ready, 0)) fail_wait(12);
+      ptx::tc_fence_after();
+      uint32_t first = issuer;   // this thread's first step of the matrix at hand
+      for (uint32_t t = 0; t < my_tiles && !*abort_flag; ++t) {
+        if (t >= 2 && !ptx::mbar_wait(&acc_empty[slot], slot_phase ^ 1)) { fail_wait(13); break; }
+        bool ok = true;
+        for (uint32_t mat = 0; mat < kMats && ok; ++mat) {
+          uint32_t acc = tmem + slot * slot_cols + (mat * kIssuers + issuer) * acc_cols, in_chain = 0;
+          uint32_t s = first;
+          for (; s < steps; s += kIssuers) {
+            if (ready == 0) {
+              if (!wait_steps()) { fail_wait(14); ok = false; break; }
+              ptx::tc_fence_after();
+            }
+            --ready;
+            const uint64_t a_desc = ptx::smem_desc_k128_swizzled(ptx::smem_addr(stage_w + stage * kStageBytes));
+            const uint64_t b_desc = ptx::smem_desc_k128_swizzled(ptx::smem_addr(xb + s * b_step));
+            if constexpr (kFp4) {
+              const uint32_t sfa = tmem + sfa_col + (issuer * 2 + sfa_buf) * 16, sfb = tmem + sfb_col + s * 16;
+              const uint64_t sf_desc = ptx::smem_desc_scale_block(ptx::smem_addr(stage_sf + stage * kSfStageBytes));
+#pragma unroll
+              for (uint32_t j = 0; j < 4; ++j) ptx::tc_cp_scale_block(sfa + 4 * j, sf_desc + j * (512 >> 4));
+#pragma unroll
+              for (uint32_t j = 0; j < 4; ++j)
+                ptx::tc_mma_nvfp4(acc, a_desc + 2 * j, b_desc + 2 * j, idesc, sfa + 4 * j, sfb + 4 * j, (in_chain | j) != 0 ? 1u : 0u);
+              sfa_buf ^= 1;
+              ++in_chain;
+            } else {
+#pragma unroll
+              for (uint32_t j = 0; j < 4; ++j) ptx::tc_mma_f8(acc, a_desc + 2 * j, b_desc + 2 * j, idesc, (in_chain | j) != 0 ? 1u : 0u);
+              if (++in_chain == chain_steps) { in_chain = 0; acc += a.columns; }
+            }
+            ptx::tc_commit(&empty[stage]);
+            if ((stage += kIssuers) >= stages) { stage = issuer; phase ^= 1; }
+          }
+          first = s - steps;
+        }
+        if (!ok) break;
+        ptx::tc_commit(&acc_full[slot]);
+        if (++slot == 2) { slot = 0; slot_phase ^= 1; }
+      }
+    }
+  } else if (warp < 6) {
+    // ------------------------------- activations, then the epilogue ----------------------------
+    asm volatile("bar.sync 1, 192;" ::: "memory");
+    ptx::tc_fence_after();
+    const uint32_t tmem = *tmem_holder;
+    const uint32_t tid = threadIdx.x - 64, group = warp & 3;   // this warp's TMEM lanes are MMA rows 32 group ..
+    const uint32_t lanes = tmem + ((group * 32) << 16);
+    float a_scale[8];
+    pdl_wait();
+    if constexpr (kFp4) {
+      // The tokens' block scales are requested ahead of the activations, so that all loads share a round trip; then through shared
+      // memory ([step][MMA][column], where the epilogue's partial sums come later) into tensor memory, lane = column, the same in all
+      // four lane quarters.
+      constexpr uint32_t kWords = 4;
+      const uint32_t srow = a.k / 16, sf_words = steps * kGroups * 4;   // words of a token: [step][group][MMA]
+      uint32_t sw[kWords], token0 = 0, word0 = tid;
+      auto each_word = [&](auto f) {   // this thread's next words; returns where they end
+        uint32_t token = token0, word = word0;
+#pragma unroll
+        for (uint32_t u = 0; u < kWords; ++u, word += 128) {
+          while (word >= sf_words) { word -= sf_words; ++token; }
+          f(u, token, word);
+        }
+        return make_uint2(token, word);
+      };
+      auto load_scales = [&]() {
+        each_word([&](uint32_t u, uint32_t token, uint32_t word) {
+          sw[u] = 0;
+          if (token >= a.tokens || word * 4 >= srow) return;
+          const uint8_t* src = static_cast<const uint8_t*>(a.act_scales) + token * srow + word * 4;
+          if (a.words) sw[u] = static_cast<uint32_t>(ld_dep(reinterpret_cast<const int32_t*>(src)));
+          else sw[u] = ld_dep(src) | ld_dep(src + 1) << 8 | ld_dep(src + 2) << 16 | static_cast<uint32_t>(ld_dep(src + 3)) << 24;
+        });
+      };
+      load_scales();
+      stage_activations(tid);
+      uint32_t* sf = reinterpret_cast<uint32_t*>(part);
+      while (true) {
+        const uint2 end = each_word([&](uint32_t u, uint32_t token, uint32_t word) {
+          if (token < a.tokens) sf[(word / 16 * 4 + word % 4) * kGroupRows + word / 4 % kGroups * a.tokens + token] = sw[u];
+        });
+        token0 = end.x;
+        word0 = end.y;
+        while (word0 >= sf_words) { word0 -= sf_words; ++token0; }
+        if (token0 >= a.tokens) break;
+        load_scales();
+      }
+      epi_barrier_or(false);
+      const bool live = lane < kGroups * a.tokens;
+#pragma unroll 1
+      for (uint32_t s = 0; s < steps; ++s) {
+        uint4 v[4];
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) v[j] = make_uint4(live ? sf[(s * 4 + j) * kGroupRows + lane] : 0, 0, 0, 0);
+        ptx::tc_st_32x32b_x16(lanes + sfb_col + s * 16, v);
+      }
+      ptx::tc_wait_st();
+    } else if constexpr (kQuant) {
+      a_scale[0] = quantise_activation(tid, group, lane);
+    } else {
+#pragma unroll
+      for (uint32_t t = 0; t < 8; ++t) a_scale[t] = t < a.tokens ? ld_dep(static_cast<const float*>(a.act_scales) + t) : 0.0f;
+      stage_activations(tid);
+    }
+    ptx::fence_proxy_async_smem();
+    ptx::tc_fence_before();
+    if constexpr (kFp4) epi_barrier_or(false);   // everybody has read the scales: `part` is free
+    __syncwarp();
+    if (lane == 0) ptx::mbar_arrive(x_ready);
+
+    uint32_t slot = 0, slot_phase = 0;
+    for (uint32_t t = 0; t < my_tiles; ++t) {
+      const uint32_t tile = blockIdx.x + t * gridDim.x, p = problem_of(tile), rows = a.rows[p];
+      const uint32_t row = (tile - a.tile_start[p]) * a.tile_rows + lane;
+      const bool live = lane < a.tile_rows && row < rows;
+      float w_scale = 0.0f;
+      if constexpr (!kFp4) {
+        if (live) w_scale = bf16_bits_to_float(__ldg(static_cast<const uint16_t*>(a.scales[p]) + row));   // under the tile's MMAs
+      }
+      const bool failed = !ptx::mbar_wait(&acc_full[slot], slot_phase);
+      if (failed) fail_wait(15);
+      ptx::tc_fence_after();
+      float* mine = part + (t & 1) * part_floats;
+#pragma unroll
+      for (int mat = 0; mat < kMats; ++mat) {
+        // The chains of the two issuers, even steps first (of a sum of one step only one has anything).
+        const uint32_t cells = lanes + slot * slot_cols + mat * kIssuers * acc_cols + group * a.tokens;
+        const uint32_t first = (t * kMats + mat) * steps & 1;
+        auto gather = [&](auto cell_count) {
+          constexpr int kCells = decltype(cell_count)::value;
+          uint32_t v[kCells];
+          ptx::tc_ld_32x32b(cells + first * acc_cols, v);
+          // Pairs of chains (even steps, odd steps), two pairs in flight.  FP8: what an addition rounds off is kept and added at the end.
+          float lost[kCells];
+#pragma unroll
+          for (int e = 0; e < kCells; ++e) lost[e] = 0.0f;
+#pragma unroll 1
+          for (uint32_t c0 = 0; c0 < chains; c0 += 2) {
+            uint32_t w[4][kCells];
+            bool has[4];
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) {
+              const uint32_t c = c0 + i / 2;
+              has[i] = c < chains && (i % 2 == 0 ? c != 0 : 2 * c * chain_steps + 1 < steps);   // chain 0 of the even steps is in v
+              if (has[i]) ptx::tc_ld_32x32b(cells + (first ^ (i & 1)) * acc_cols + c * a.columns, w[i]);
+            }
+            ptx::tc_wait_ld();
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) {
+              if (!has[i]) continue;
+#pragma unroll
+              for (int e = 0; e < kCells; ++e) {
+                if constexpr (kFp4) v[e] = __float_as_uint(__fadd_rn(__uint_as_float(v[e]), __uint_as_float(w[i][e])));
+                else v[e] = __float_as_uint(add_keep(__uint_as_float(v[e]), __uint_as_float(w[i][e]), lost[e]));
+              }
+            }
+          }
+#pragma unroll
+          for (uint32_t token = 0; token < kCells; ++token) {
+            if (token >= a.tokens) continue;
+            mine[((mat * kGroups + group) * a.tokens + token) * kGroupRows + lane] = __uint_as_float(v[token]);
+            if constexpr (!kFp4) mine[part_floats / 2 + (group * a.tokens + token) * kGroupRows + lane] = lost[token];
+          }
+        };
+        if (a.tokens == 1) gather(std::integral_constant<int, 1>{});
+        else gather(std::integral_constant<int, 8>{});
+      }
+      ptx::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(&acc_empty[slot]);
+      // The next tile writes the other half of `part`; the barrier of the one after it lies behind these reads.
+      if (epi_barrier_or(failed || *abort_flag != 0)) break;
+      if (++slot == 2) { slot = 0; slot_phase ^= 1; }
+      auto sum = [&](uint32_t mat, uint32_t token) {
+        const float* c = mine + (mat * kGroups * a.tokens + token) * kGroupRows + lane;
+        const uint32_t d = a.tokens * kGroupRows;
+        if constexpr (kFp4) return __fadd_rn(__fadd_rn(c[0], c[d]), __fadd_rn(c[2 * d], c[3 * d]));
+        const float* l = c + part_floats / 2;
+        float lost = __fadd_rn(__fadd_rn(l[0], l[d]), __fadd_rn(l[2 * d], l[3 * d]));
+        const float lo = add_keep(c[0], c[d], lost), hi = add_keep(c[2 * d], c[3 * d], lost);
+        const float total = add_keep(lo, hi, lost);
+        return __fadd_rn(total, lost);
+      };
+#pragma unroll
+      for (uint32_t u = 0; u < 2; ++u) {
+        const uint32_t token = group + 4 * u;
+        if (token >= a.tokens || !live) continue;
+        const uint64_t o = static_cast<uint64_t>(token) * rows + row;
+        if constexpr (kFp4) {
+          const float y0 = __fdiv_rn(sum(0, token), a.div[0]);   // single final division by ga*gw: src/cuda/nvfp4/sm120.cu:243
+          if constexpr (kMats == 2) {
+            const float y1 = __fdiv_rn(sum(1, token), a.div[1]);
+            if (a.out[0]) static_cast<float*>(a.out[0])[o] = y0;
+            if (a.out[1]) static_cast<float*>(a.out[1])[o] = y1;
+            // bf16 boundaries and GELU-tanh product: src/cuda/nvfp4/sm120.cu:375-386.
+            a.product[o] = gelu_tanh_product(bf16_round(y0), bf16_round(y1));
+          } else {
+            static_cast<float*>(a.out[0])[o] = y0;
+          }
+        } else {
+          // (acc * a_scale) * w_scale, in that order: src/cuda/fp8/sm120.cu:234-239.
+          float xs = a_scale[0];
+#pragma unroll
+          for (uint32_t i = 1; i < 8; ++i)
+            if (i == token) xs = a_scale[i];
+          const float y = __fmul_rn(__fmul_rn(sum(0, token), xs), w_scale);
+          if (kQuant && a.bf16_out) static_cast<uint16_t*>(a.out[p])[o] = float_to_bf16_bits(y);
+          else static_cast<float*>(a.out[p])[o] = y;
+        }
+      }
+    }
+  } else if constexpr (kFp4) {
+    // ------------------------------- block scales of the weights -------------------------------
+    // Warp v takes the steps v, v + 8, ...: lane l loads word l % 16 (chunk group l % 16 / 4, MMA l % 4) of every other row, 64 contiguous
+    // bytes per row, and puts it where tcgen05.cp wants it: [MMA][row][group].  The next step's words are requested before this
+    // one's are stored, sixteen steps are in flight per SM.
+    if (a.fewest_rows <= kFewRows) pdl_wait();
+    const uint32_t srow = a.k / 16, word = lane & 15, half = lane >> 4, rounds = (a.tile_rows + 1) / 2;
+    const uint32_t per_tile = kMats * steps, total = my_tiles * per_tile;
+    const uint64_t policy = ptx::evict_first_policy();
+    const uint32_t active = min(kScaleWarps, stages);   // a warp sees every phase of the stages it waits on only if it laps none of them
+    uint32_t n = warp - 7, next = n < active ? n : total, stage = n % stages, use = 0;   // `next`: the step whose words are requested next
+    uint32_t v[16];
+    bool loaded = false, staged = false;
+    while (true) {
+      if (loaded) {   // v holds step n
+        if (use != 0) {
+          const bool ok = ptx::mbar_wait(&empty[stage], (use ^ 1) & 1);
+          if (!__all_sync(0xFFFFFFFFu, ok)) { fail_wait(16); break; }
+        }
+        uint8_t* dst = stage_sf + stage * kSfStageBytes + (word & 3) * 512 + half * 16 + (word >> 2) * 4;
+#pragma unroll
+        for (uint32_t u = 0; u < 16; ++u)
+          if (u < rounds) *reinterpret_cast<uint32_t*>(dst + u * 32) = v[u];
+        ptx::fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(&full[stage]);
+        n = next;
+        stage += active;
+        if (stage >= stages) { stage -= stages; ++use; }
+      }
+      loaded = next < total;
+      if (loaded) {
+        const uint32_t t = next / per_tile, i = next - t * per_tile, mat = i >= steps ? 1u : 0u, at = (i - mat * steps) * (kGroups * 16) + word * 4;
+        const uint32_t row0 = (blockIdx.x + t * gridDim.x) * a.tile_rows + half;
+        const uint8_t* src = static_cast<const uint8_t*>(a.scales[mat]) + static_cast<uint64_t>(row0) * srow + at;
+#pragma unroll
+        for (uint32_t u = 0; u < 16; ++u) {
+          v[u] = 0;
+          if (u < rounds && at < srow && row0 + 2 * u < a.rows[0]) v[u] = ptx::ld_stream_4(src + static_cast<uint64_t>(2 * u) * srow, policy);
+        }
+        next += active;
+      }
+      if (!staged && (!loaded || n >= a.early)) {   // the activations: this thread's share lies behind that of warps 2-5, see there
+        pdl_wait();
+        stage_activations(threadIdx.x - 96);
+        ptx::fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(x_ready);
+        staged = true;
+      }
+      if (!loaded || *abort_flag) break;
+    }
+  }
+
+  ptx::tc_fence_before();
+  __syncthreads();
+  if (*abort_flag) {
+    // Give copies that are still in flight a bounded time to land before the CTA exits.
+    for (int i = 0; i < 2000; ++i) __nanosleep(1000);
+    __syncthreads();
+  }
+  if (warp == 1) {
+    ptx::tc_fence_after();
+    ptx::tmem_dealloc(*tmem_holder, tmem_cols);
+  }
+}
+
+// Rows per tile: the fewest tiles per CTA that hold all rows at 32 each, then the fewest rows that still do, so that the
+// CTAs' shares are even.
+uint32_t pick_tile_rows(const uint64_t* rows, int n, uint64_t ctas) {
+  auto tiles = [&](uint64_t r) {
+    uint64_t t = 0;
+    for (int i = 0; i < n; ++i) t += (rows[i] + r - 1) / r;
+    return t;
+  };
+  const uint64_t per_cta = (tiles(kGroupRows) + ctas - 1) / ctas;
+  uint64_t r = std::max<uint64_t>(1, tiles(1) / (per_cta * ctas));
+  while (tiles(r) > per_cta * ctas) ++r;   // r = 32 is enough
+  return static_cast<uint32_t>(r);
+}
+
+template <bool kFp4, int kMats, bool kQuant, int kMaps>
+int32_t launch(const char* op, const DecodeCall& c, cudaStream_t stream, bool* taken) {
+  const uint64_t row_bytes = kFp4 ? c.k / 2 : c.k, steps = (row_bytes + 511) / 512;
+  const uint64_t columns = c.tokens <= 4 ? 16 : 32;
+  const size_t part = std::max<size_t>(2 * (kFp4 ? kMats : 2) * kGroups * c.tokens * kGroupRows * sizeof(float), kFp4 ? steps * 512 : 0);
+  const size_t fixed = steps * ((c.tokens + 1) / 2) * 1024 + part + (2 * kMaxStages + 5) * 8 + 64 + 1024;
+  const size_t per_stage = kStageBytes + (kFp4 ? kSfStageBytes : 0);
+  if (fixed + kMinStages * per_stage > kSmemBudget) return GEMB_OK;
+  Maps<kMaps> maps;
+  Args a{};
+  a.act = c.act;
+  a.act_scales = c.act_scales;
+  a.product = c.product;
+  a.k = static_cast<uint32_t>(c.k);
+  a.tokens = static_cast<uint32_t>(c.tokens);
+  a.columns = static_cast<uint32_t>(columns);
+  a.stages = static_cast<uint32_t>(std::min<uint64_t>(kMaxStages, (kSmemBudget - fixed) / per_stage)) & ~1u;
+  a.words = reinterpret_cast<uintptr_t>(c.act_scales) % 4 == 0;
+  a.bf16_out = c.bf16_out;
+  uint64_t rows[3] = {c.m[0].rows, c.m[1].rows, c.m[2].rows};
+  const int spaces = kFp4 ? 1 : c.n;   // gate and up share their rows' tiles
+  a.tile_rows = pick_tile_rows(rows, spaces, static_cast<uint64_t>(sm_count()));
+  uint32_t tiles = 0;
+  a.fewest_rows = UINT32_MAX;
+  for (int i = 0; i < 3; ++i) {
+    const DecodeMatrix& m = c.m[std::min(i, c.n - 1)];
+    a.tile_start[i] = tiles;
+    if (i < spaces) tiles += static_cast<uint32_t>((m.rows + a.tile_rows - 1) / a.tile_rows);
+    a.rows[i] = static_cast<uint32_t>(m.rows);
+    a.scales[i] = m.scales;
+    a.out[i] = m.out;
+    if (i < 2) a.div[i] = m.div;
+    a.fewest_rows = std::min(a.fewest_rows, a.rows[i]);
+    if (i < c.n) GEMB_TRY(make_byte_map(op, &maps.m[i], m.w, m.rows, row_bytes, a.tile_rows));
+  }
+  a.tile_start[3] = tiles;
+  if (kFp4) a.tile_start[1] = tiles;
+  const uint32_t ctas = std::min(tiles, static_cast<uint32_t>(sm_count()));
+  a.stages = static_cast<uint32_t>(std::min<uint64_t>(a.stages, ((tiles + ctas - 1) / ctas * kMats * steps + 1) & ~1ull));   // no more than a CTA has steps
+  a.early = std::min(a.stages, (kEarlyBytes + kGroups * a.tile_rows * 128 - 1) / (kGroups * a.tile_rows * 128));
+  const size_t smem = fixed + a.stages * per_stage;
+  GEMB_TRY((allow_full_smem<decode_gemv_kernel<kFp4, kMats, kQuant, kMaps>>(op)));
+  GEMB_TRY(launch_pdl_split(op, true, decode_gemv_kernel<kFp4, kMats, kQuant, kMaps>, dim3(ctas),
+                      dim3(kFp4 ? kThreadsFp4 : kThreadsFp8), smem, stream, maps, a));
+  *taken = true;
+  return check_launch(op);
+}
+
+}  // namespace
+
+// Reads and clears the kernels' bounded-wait flag (0 = clean, -1 = could not read).
+int decode_take_device_error() {
+  int code = 0;
+  if (cudaMemcpyFromSymbol(&code, g_decode_error, sizeof code) != cudaSuccess) return -1;
+  if (code != 0) {
+    const int zero = 0;
+    cudaMemcpyToSymbol(g_decode_error, &zero, sizeof zero);
+  }
+  return code;
+}
+
+int32_t launch_decode_fp4(const char* op, const DecodeCall& c, cudaStream_t stream, bool* taken) {
+  *taken = false;
+  // K alone decides (and the weights' alignment), never the token count: every batch size gives the same bits.
+  if (c.k > (c.n == 2 ? kFp4MaxKTwo : kFp4MaxK)) return GEMB_OK;
+  for (int i = 0; i < c.n; ++i)
+    if (reinterpret_cast<uintptr_t>(c.m[i].scales) % 4 != 0) return GEMB_OK;
+  return c.n == 2 ? launch<true, 2, false, 2>(op, c, stream, taken) : launch<true, 1, false, 1>(op, c, stream, taken);
+}
+
+int32_t launch_decode_fp8(const char* op, const DecodeCall& c, cudaStream_t stream, bool* taken) {
+  *taken = false;
+  if (c.quantize) return launch<false, 1, true, 1>(op, c, stream, taken);   // never more than one matrix
+  return c.n == 1 ? launch<false, 1, false, 1>(op, c, stream, taken) : launch<false, 1, false, 3>(op, c, stream, taken);
+}
+
+}  // namespace gemb

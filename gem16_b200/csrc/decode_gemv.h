@@ -1,0 +1,30 @@
+// Internal: the decode projections on tcgen05 (decode_gemv.cu), behind the entry points of gemv.cu and nvfp4_gemv.cu.
+#pragma once
+
+#include "common.cuh"
+
+namespace gemb {
+
+struct DecodeMatrix {
+  const uint8_t* w;
+  const void* scales;   // NVFP4: compact E4M3 block scales; FP8: bf16 per row
+  void* out;            // [tokens, rows]; NVFP4 gate / up form: may be null
+  uint64_t rows;
+  float div;            // NVFP4: ga * gw
+};
+struct DecodeCall {
+  const void* act;          // E2M1 / E4M3 bytes; bf16 when `quantize` is set
+  const void* act_scales;   // NVFP4: compact E4M3 block scales; FP8: fp32 per token
+  DecodeMatrix m[3];
+  int n;                    // matrices: 1, 2 (NVFP4: gate and up of the same rows), up to 3 (FP8: rows of their own)
+  float* product;           // NVFP4 gate / up form
+  uint64_t k, tokens;
+  bool quantize;            // FP8, one token: quantised in the kernel
+  bool bf16_out;            // with `quantize`
+};
+// *taken = false: the call is not one for these kernels, nothing was launched.
+int32_t launch_decode_fp4(const char* op, const DecodeCall& c, cudaStream_t stream, bool* taken);
+int32_t launch_decode_fp8(const char* op, const DecodeCall& c, cudaStream_t stream, bool* taken);
+int decode_take_device_error();
+
+}  // namespace gemb

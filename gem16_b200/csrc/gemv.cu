@@ -1,7 +1,8 @@
-// Batch-1 decode projections: HBM-streaming, warp-reduced GEMV kernels for FP8 (W8A8) weights in the
-// checkpoint's row-major source layout (NVFP4 weights: nvfp4_gemv.cu).
+// Entry points of the FP8 (W8A8) decode projections, weights in the checkpoint's row-major source layout, and the forms that are left
+// beside the tcgen05 kernel of decode_gemv.cu: contracting extents whose staged activations leave it no room (one token beyond
+// about 50,000, five and more beyond about 14,000) and what the tuning knobs ask for.  (NVFP4 weights: nvfp4_gemv.cu.)
 //
-// A CTA of 8 warps stages the activation vector once in shared memory (decoded to fp16, which holds every
+// One token: a CTA of 8 warps stages the activation vector once in shared memory (decoded to fp16, which holds every
 // E4M3 value exactly), then each warp streams kRows weight rows with coalesced 128-bit loads (lane l reads
 // bytes [16 l, 16 l + 16) of each 512-byte row segment, `no_allocate` so the stream does not evict the
 // activation from L1), accumulates in fp32 and folds the 32 lanes with an xor butterfly.  Weights are read
@@ -11,6 +12,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "decode_gemv.h"
 #include "ptx.cuh"
 
 namespace gemb {
@@ -334,21 +336,7 @@ int32_t launch_fp8_gemv_variant(const char* op, const void* act, const float* ac
   const uint64_t tasks = (grp.row_start[grp.n] + kRows - 1) / kRows;
   const uint64_t wave = static_cast<uint64_t>(sm_count()) * resident;
   const unsigned blocks = static_cast<unsigned>(std::min<uint64_t>((tasks + kW - 1) / kW, wave));
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(blocks);
-  cfg.blockDim = dim3(kW * 32);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = g_pdl ? 1 : 0;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaError_t le = cudaLaunchKernelEx(&cfg, kern, act, act_scale, grp, k);
-  if (le != cudaSuccess) {
-    cudaGetLastError();
-    return fail(GEMB_INTERNAL, "%s: %s: %s", op, cudaGetErrorName(le), cudaGetErrorString(le));
-  }
+  GEMB_TRY(launch_pdl(op, kern, dim3(blocks), dim3(kW * 32), smem, stream, act, act_scale, grp, k));
   return check_launch(op);
 }
 
@@ -601,8 +589,28 @@ int32_t launch_fp8_gemv_mma(const char* op, const uint8_t* act, const float* act
   return check_launch(op);
 }
 
+// The tcgen05 kernel (decode_gemv.cu) for a group of projections, unless a knob asks for another form.
+int32_t launch_fp8_decode(const char* op, const void* act, const float* act_scales, const Fp8Group& grp, uint64_t tokens, uint64_t k,
+                          bool quantize, bool bf16_out, cudaStream_t stream, bool* taken) {
+  *taken = false;
+  if (g_gemv_impl != 0 || g_rows_override != 0) return GEMB_OK;
+  DecodeCall c{};
+  c.act = act;
+  c.act_scales = act_scales;
+  for (int i = 0; i < grp.n; ++i) c.m[i] = {grp.p[i].w, grp.p[i].w_scales, grp.p[i].out, grp.p[i].rows, 1.0f};
+  c.n = grp.n;
+  c.k = k;
+  c.tokens = tokens;
+  c.quantize = quantize;
+  c.bf16_out = bf16_out;
+  return launch_decode_fp8(op, c, stream, taken);
+}
+
 int32_t launch_fp8_gemv_batch(const char* op, const uint8_t* act, const float* act_scales, const Fp8Group& grp,
                               uint64_t tokens, uint64_t k, cudaStream_t stream) {
+  bool taken = false;
+  GEMB_TRY(launch_fp8_decode(op, act, act_scales, grp, tokens, k, false, false, stream, &taken));
+  if (taken) return GEMB_OK;
   // Tensor-core form by default; GEMB_TUNE_GEMV_IMPL = 1 keeps the SIMT form, whose per-token results
   // are bit-identical to the single-token kernel.
   if (g_gemv_impl != 1) return launch_fp8_gemv_mma(op, act, act_scales, grp, tokens, k, stream);
@@ -873,6 +881,8 @@ int32_t launch_fp8_gemv(const char* op, const void* act, const float* act_scale,
   }
   grp.row_start[grp.n] = total_rows;
   bool launched = false;
+  GEMB_TRY(launch_fp8_decode(op, act, act_scale, grp, 1, k, kFusedQuant, kBf16Out, stream, &launched));
+  if (launched) return GEMB_OK;
   GEMB_TRY((launch_fp8_gemv_ring<kFusedQuant, kBf16Out>(op, act, act_scale, grp, k, stream, &launched)));
   if (launched) return GEMB_OK;
   const int rpw = pick_rows_per_warp(total_rows, k);
@@ -906,10 +916,11 @@ fp8_quantize_decode_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__
                            float* __restrict__ scales, uint32_t k) {
   __shared__ float red[32];
   pdl_trigger_few_rows(gridDim.x);
-  pdl_wait();
   const uint64_t t = blockIdx.x;
+  prefetch_l2_span(x + t * k, k * 2ull);
   const uint4* xp = reinterpret_cast<const uint4*>(x + t * k);
   const uint32_t chunks = k / 8;
+  pdl_wait();
   uint4 v[2];
   float amax = 0.0f;
 #pragma unroll
@@ -949,20 +960,8 @@ bool pdl_enabled() { return g_pdl != 0; }
 
 int32_t launch_fp8_quantize_decode(const char* op, const uint16_t* x, uint8_t* out, float* scales, uint64_t tokens,
                                    uint64_t k, cudaStream_t stream) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(static_cast<unsigned>(tokens));
-  cfg.blockDim = dim3(1024);
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = g_pdl ? 1 : 0;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaError_t le = cudaLaunchKernelEx(&cfg, fp8_quantize_decode_kernel, x, out, scales, static_cast<uint32_t>(k));
-  if (le != cudaSuccess) {
-    cudaGetLastError();
-    return fail(GEMB_INTERNAL, "%s: %s: %s", op, cudaGetErrorName(le), cudaGetErrorString(le));
-  }
+  GEMB_TRY(launch_pdl_split(op, true, fp8_quantize_decode_kernel, dim3(static_cast<unsigned>(tokens)), dim3(1024), 0, stream, x, out, scales,
+                            static_cast<uint32_t>(k)));
   return check_launch(op);
 }
 
@@ -974,7 +973,7 @@ int gemv_take_device_error() {
     const int zero = 0;
     cudaMemcpyToSymbol(g_gemv_error, &zero, sizeof zero);
   }
-  return code;
+  return code != 0 ? code : decode_take_device_error();
 }
 
 }  // namespace gemb

@@ -1,6 +1,7 @@
-// Decode projections with NVFP4 weights (W4A4) for 1 .. 8 tokens: y = (sum_k qa sa qw sw) / (ga * gw), and the fused
+// Entry points of the decode projections with NVFP4 weights (W4A4) for 1 .. 8 tokens: y = (sum_k qa sa qw sw) / (ga * gw), and the fused
 // gate / up form with the GELU-tanh product.  Weights in the checkpoint's row-major layout with COMPACT
-// block scales; every weight byte is read once whatever the token count.
+// block scales; every weight byte is read once whatever the token count.  The kernel here is the one for what the tcgen05 kernel of
+// decode_gemv.cu does not take: K beyond its tensor memory (20,480; gate / up 12,288) and block scales that are not 4-byte aligned.
 //
 // The dot products run on the warp-level tensor-core path (mma.sync m16n8k16, fp16 x fp16 -> fp32): the weights
 // are the M side as they lie in memory, the tokens its eight columns, so the arithmetic is the same for
@@ -15,9 +16,8 @@
 // 128-byte pieces along K.  The tiles are dealt out over the SMs and the pieces of an SM's tiles over its warps in
 // equal contiguous shares: the kernel is as much bound by the conversions as by the loads, so warps without
 // work cost as much as SMs without loads.  Measured, weights cold, in a chain of launches: gate / up 2 x 15,360 x 3,840 in
-// 18 us for one token and 20 us for five (23 us per token before, one launch each), down 3,840 x 15,360 in 12 and
-// 14 us (11 and 67 us before); without the loads the arithmetic takes 12 us, without the arithmetic
-// the loads 8.  A warp's first pieces are loaded ahead of pdl_wait (weights are at rest, see pdl_trigger_few_rows): 7 % of a
+// 18 us for one token and 20 us for five, down 3,840 x 15,360 in 12 and
+// 14 us; without the loads the arithmetic takes 12 us, without the arithmetic the loads 8 (the tcgen05 kernel, which has none: 14 and 9).  A warp's first pieces are loaded ahead of pdl_wait (weights are at rest, see pdl_trigger_few_rows): 7 % of a
 // decode pass.
 // Requesting all weights into L2 ahead of it changed nothing: the kernels before
 // this one then wait for HBM instead.  Lane 4g + t loads 32 contiguous bytes of rows g and g + 8 per piece
@@ -28,6 +28,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "decode_gemv.h"
 #include "ptx.cuh"
 
 namespace gemb {
@@ -291,6 +292,17 @@ uint64_t fp4_stage_bytes(uint64_t tokens, uint64_t k) { return tokens * ((k + kP
 
 template <bool kGateUp>
 int32_t launch_nvfp4_gemv(const char* op, Fp4GemvArgs a, cudaStream_t stream) {
+  DecodeCall c{};
+  c.act = a.act;
+  c.act_scales = a.act_scales;
+  c.n = kGateUp ? 2 : 1;
+  for (int m = 0; m < c.n; ++m) c.m[m] = {a.m[m].w, a.m[m].ws, a.m[m].out, a.rows, a.m[m].div};
+  c.product = a.product;
+  c.k = a.k;
+  c.tokens = a.tokens;
+  bool taken = false;
+  GEMB_TRY(launch_decode_fp4(op, c, stream, &taken));
+  if (taken) return GEMB_OK;
   a.wide = true;
   for (int m = 0; m < (kGateUp ? 2 : 1); ++m)
     a.wide = a.wide && reinterpret_cast<uintptr_t>(a.m[m].w) % 32 == 0 && reinterpret_cast<uintptr_t>(a.m[m].ws) % 4 == 0;

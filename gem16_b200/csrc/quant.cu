@@ -133,8 +133,8 @@ int32_t launch_nvfp4_quantize(const char* op, Loader loader, uint8_t* packed, ui
   const uint64_t cells = (inter ? (tokens + 127) / 128 * 128 : tokens) * blocks_pad;
   // Few cells (a decode token): small CTAs, so that they spread over the SMs and load side by side.
   const unsigned threads = cells <= 16384 ? 64 : 256;
-  GEMB_TRY(launch_pdl(op, kern, dim3(static_cast<unsigned>((cells + threads - 1) / threads)), dim3(threads), 0, stream,
-                      loader, packed, scales, static_cast<uint32_t>(tokens), k, static_cast<uint32_t>(blocks_pad), cells, g));
+  GEMB_TRY(launch_pdl_split(op, tokens <= kFewRows, kern, dim3(static_cast<unsigned>((cells + threads - 1) / threads)), dim3(threads), 0, stream,
+                            loader, packed, scales, static_cast<uint32_t>(tokens), k, static_cast<uint32_t>(blocks_pad), cells, g));
   return check_launch(op);
 }
 
@@ -515,6 +515,7 @@ rmsnorm_residual_kernel(const In* x, const uint16_t* __restrict__ w, const Res* 
 #pragma unroll
     for (int j = 0; j < 16; ++j) wv[j] = w && threadIdx.x + j * 256 < k ? __ldg(w + threadIdx.x + j * 256) : uint16_t(0x3F80);
     const float layer_scale = scalar ? bf16_bits_to_float(__ldg(scalar)) : 1.0f;
+    prefetch_l2_span(residual + base, k * sizeof(Res));
     pdl_wait();
     Res rv[16];
 #pragma unroll
@@ -631,6 +632,7 @@ fp8_quantize_kernel(const In* x, const uint16_t* __restrict__ w, uint8_t* out, f
   float inv = 1.0f;
   uint16_t wv[16];
   if (short_row) load_norm_weights(w, threadIdx.x, static_cast<uint32_t>(k), wv);
+  if (gridDim.x <= kFewRows) prefetch_l2_span(row, k * sizeof(In));
   pdl_wait();
   if constexpr (kNorm) inv = short_row ? stage_short_row(row, static_cast<uint32_t>(k), eps, xs, red) : rmsnorm_inverse(row, k, eps, red);
   const uint32_t blocks = static_cast<uint32_t>(k / 16);
@@ -777,8 +779,8 @@ int32_t gemb_nvfp4_rmsnorm_quantize(const void* input, int32_t input_dtype, cons
                       : (rcp ? rmsnorm_nvfp4_quantize_kernel<T, true, false, false> : rmsnorm_nvfp4_quantize_kernel<T, false, false, false>);
     if (short_rows(rows_out, k))   // the interleaved layout pads to 128 rows: never
       kern = rcp ? rmsnorm_nvfp4_quantize_kernel<T, true, false, true> : rmsnorm_nvfp4_quantize_kernel<T, false, false, true>;
-    GEMB_TRY(launch_pdl(op, kern, dim3(static_cast<unsigned>(rows_out)), dim3(256), 0, stream, x, weight, packed, scales,
-                        static_cast<uint32_t>(tokens), k, eps, g, static_cast<uint32_t>(c_pad)));
+    GEMB_TRY(launch_pdl_split(op, rows_out <= kFewRows, kern, dim3(static_cast<unsigned>(rows_out)), dim3(256), 0, stream, x, weight, packed, scales,
+                              static_cast<uint32_t>(tokens), k, eps, g, static_cast<uint32_t>(c_pad)));
     return check_launch(op);
   };
   return input_dtype == GEMB_F32 ? launch(static_cast<const float*>(input)) : launch(static_cast<const uint16_t*>(input));
@@ -829,7 +831,7 @@ int32_t launch_fp8_rows(const char* op, const void* input, int32_t input_dtype, 
   auto launch = [&](auto* x) -> int32_t {
     using T = std::remove_const_t<std::remove_pointer_t<decltype(x)>>;
     auto kern = kNorm && short_rows(tokens, k) ? fp8_quantize_kernel<T, kNorm, kNorm> : fp8_quantize_kernel<T, kNorm, false>;
-    return launch_pdl(op, kern, grid, dim3(256), 0, stream, x, weight, out, scales, k, eps);
+    return launch_pdl_split(op, tokens <= kFewRows, kern, grid, dim3(256), 0, stream, x, weight, out, scales, k, eps);
   };
   GEMB_TRY(input_dtype == GEMB_F32 ? launch(static_cast<const float*>(input)) : launch(static_cast<const uint16_t*>(input)));
   return check_launch(op);
@@ -887,7 +889,7 @@ int32_t gemb_rmsnorm_residual(const void* input, int32_t input_dtype, const uint
     using Res = std::remove_const_t<std::remove_pointer_t<decltype(res)>>;
     using Out = std::remove_pointer_t<decltype(o)>;
     auto kern = short_rows(vectors, width) ? rmsnorm_residual_kernel<In, Res, Out, true> : rmsnorm_residual_kernel<In, Res, Out, false>;
-    return launch_pdl(op, kern, grid, dim3(256), 0, stream, x, weight_bf16, res, normalized_output, o, width, epsilon, scalar_bf16);
+    return launch_pdl_split(op, vectors <= kFewRows, kern, grid, dim3(256), 0, stream, x, weight_bf16, res, normalized_output, o, width, epsilon, scalar_bf16);
   };
   const auto* xb = static_cast<const uint16_t*>(input);
   if (bf16_out)

@@ -358,3 +358,83 @@ def test_nvfp4_gemv_batch_takes_what_fits_the_staging(lib, dev):
         assert torch.equal(one, y[t]), t
     with pytest.raises(GembError):
         lib.gemb_nvfp4_gemv_batch(act, acts, w, ws, torch.zeros((7, rows), device=dev), 7, rows, k, 100.0, 100.0, None)
+
+
+def _dequantised(q, s, rows, k):
+    """NVFP4 codes and compact scales -> binary64 on the device."""
+    grid = torch.tensor([0, .5, 1, 1.5, 2, 3, 4, 6, 0, -.5, -1, -1.5, -2, -3, -4, -6], dtype=torch.float64, device=q.device)
+    v = torch.stack([grid[(q & 15).long()], grid[(q >> 4).long()]], -1).reshape(rows, k)
+    return v * s.view(torch.float8_e4m3fn).double().reshape(rows, k // 16).repeat_interleave(16, 1)
+
+
+# One row, rows that are no multiple of a tile, one tile per SM and one row more, several tiles with a short last one; K of one MMA, of a
+# part of a chunk, of a part of a step, of odd and even numbers of steps, at the limits of the tensor-core kernel and past them
+# (gate / up 12,288, one matrix 20,480; FP8 what shared memory holds), and the pipeline's shortest rings (six tokens x 15,360).
+@pytest.mark.parametrize("tokens,rows,k", [(1, 8, 64), (8, 8, 64), (1, 152, 192), (3, 4736, 832), (4, 4744, 1024), (5, 9480, 1088), (2, 1000, 2112),
+                                           (8, 320, 12288), (1, 320, 12352), (6, 24, 15360), (1, 64, 20480), (1, 64, 20544)])
+def test_decode_projections_over_tiles_steps_and_limits(lib, dev, tokens, rows, k):
+    """Both formats of the decode projections against binary64, within the GEMV budget; every token of an NVFP4 batch
+    bit-identical to the single-token call."""
+    gen = torch.Generator(device=dev).manual_seed(rows * 31 + k)
+    x = torch.randn((tokens, k), device=dev, generator=gen).to(torch.bfloat16).view(torch.int16)
+    w = [torch.randn((rows, k), device=dev, generator=gen) * 0.02 for _ in range(2)]
+    u8, f32 = torch.uint8, torch.float32
+    ga, gw = 448.0, 20000.0
+
+    def nvfp4(t, n, dtype, g):
+        q, s = torch.empty((n, k // 2), dtype=u8, device=dev), torch.empty((n, k // 16), dtype=u8, device=dev)
+        lib.gemb_nvfp4_quantize(t, dtype, q, s, n, k, g, 0, 0, None)
+        return q, s
+
+    def close(y, want):
+        assert ((y.double() - want).norm() <= 1e-6 * want.norm()).item()
+
+    (xq, xs), ws = nvfp4(x, tokens, 1, ga), [nvfp4(t, rows, 0, gw) for t in w]
+    want = [_dequantised(xq, xs, tokens, k) @ _dequantised(q, s, rows, k).T / (ga * gw) for q, s in ws]
+    y, g, u, p = (torch.full((tokens, rows), float("nan"), device=dev) for _ in range(4))
+    lib.gemb_nvfp4_gemv_batch(xq, xs, *ws[0], y, tokens, rows, k, ga, gw, None)
+    lib.gemb_nvfp4_gemv_gate_up_batch(xq, xs, *ws[0], *ws[1], g, u, p, tokens, rows, k, ga, gw, ga, gw, None)
+    for got, ref in ((y, want[0]), (g, want[0]), (u, want[1])):
+        close(got, ref)
+    assert torch.isfinite(p).all()
+    for t in range(tokens):
+        one = torch.zeros((rows,), device=dev)
+        lib.gemb_nvfp4_gemv(xq[t], xs[t], *ws[0], one, rows, k, ga, gw, None)
+        assert torch.equal(one, y[t]), t
+
+    q8, s8 = torch.empty((rows, k), dtype=u8, device=dev), torch.empty((rows,), dtype=f32, device=dev)
+    x8, t8 = torch.empty((tokens, k), dtype=u8, device=dev), torch.empty((tokens,), dtype=f32, device=dev)
+    lib.gemb_fp8_quantize(w[0], 0, q8, s8, rows, k, None)
+    lib.gemb_fp8_quantize(x, 1, x8, t8, tokens, k, None)
+    sb = s8.to(torch.bfloat16)
+    ref = (x8.view(torch.float8_e4m3fn).double() @ q8.view(torch.float8_e4m3fn).double().T) * t8.double()[:, None] * sb.double()
+    if tokens * ((k + 511) // 512 * 512) <= 102400:
+        lib.gemb_fp8_gemv_batch(x8, t8, q8, sb.view(torch.int16), y, tokens, rows, k, None)
+        close(y, ref)
+    one, fused = torch.zeros((rows,), device=dev), torch.zeros((rows,), device=dev)
+    lib.gemb_fp8_gemv(x8[0], t8, q8, sb.view(torch.int16), one, rows, k, None)
+    lib.gemb_fp8_gemv_bf16in(x[0], q8, sb.view(torch.int16), fused, 0, rows, k, None)
+    close(one, ref[0])
+    assert torch.equal(one, fused)
+
+
+@pytest.mark.parametrize("tokens,k", [(1, 528), (5, 3840)])
+def test_fp8_nan_stays_in_its_row(lib, dev, tokens, k):
+    """Rows share a matrix instruction with other places of K and columns with other tokens: a NaN code must not leave its row,
+    nor a NaN token its column."""
+    rows = 72
+    gen = torch.Generator(device=dev).manual_seed(k)
+    w = (torch.randn((rows, k), device=dev, generator=gen) * 0.5).to(torch.float8_e4m3fn).view(torch.uint8)
+    x = torch.randn((tokens, k), device=dev, generator=gen).to(torch.float8_e4m3fn).view(torch.uint8)
+    w[17, k - 1] = 0x7F
+    ones = torch.full((rows,), 0x3F80, dtype=torch.int16, device=dev)
+    xs = torch.ones((tokens,), device=dev)
+    y = torch.zeros((tokens, rows), device=dev)
+    lib.gemb_fp8_gemv_batch(x, xs, w, ones, y, tokens, rows, k, None)
+    bad = torch.isnan(y)
+    assert bad[:, 17].all() and bad.sum() == tokens
+    if tokens > 1:
+        x[2, 3] = 0xFF
+        lib.gemb_fp8_gemv_batch(x, xs, w, ones, y, tokens, rows, k, None)
+        bad = torch.isnan(y)
+        assert bad[2].all() and bad[:, 17].all() and bad.sum() == rows + tokens - 1
