@@ -669,8 +669,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
               make_uint2(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]));
         }
       }
-    } else
-    for (uint32_t tile = first_tile; tile < num_tiles && !*abort_flag; tile += tile_stride) {
+    } else {
+    // Dry run: until the first accumulator is full these warps have nothing to do, and their code (20 KB of straight line in the GELU form) has
+    // been taken out of the instruction caches by the kernels in between.  So they go through it once on whatever tensor memory holds, without
+    // waiting, releasing or storing.  Cold, the GELU epilogue of a tile takes 7 us, warm 1.6.  For the small tiles of short calls only: where a
+    // CTA walks many tiles, the condition costs more than the first tile's fetches (16,384 tokens 1 - 2 %).
+    constexpr bool kDryRun = BN == 128 && !kPair;
+    bool dry = kDryRun && my_tiles != 0;
+    for (uint32_t tile = first_tile; tile < num_tiles && !*abort_flag;) {
       uint32_t mt, nt;
       tile_coords(tile, mt, nt);
       // In a pair the odd CTA may own a padding-only tile: it takes part in the barriers, nothing else.
@@ -686,7 +692,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         row_scale = __fdiv_rn(1.0f, __fmul_rn(p.ga, __ldg(p.w_divisors + (tile_expert ? min(static_cast<uint32_t>(tile_expert_of(mt)), p.experts - 1) : 0u))));
       if (lane == 0) ptx::bulk_wait_group_read<0>();
       __syncwarp();
-      if (!ptx::mbar_wait(&acc_full[as + kParts - 1], aphase)) { fail_wait(4); break; }   // commits are in order: so are the parts before
+      if (!dry && !ptx::mbar_wait(&acc_full[as + kParts - 1], aphase)) { fail_wait(4); break; }   // commits are in order: so are the parts before
       ptx::tc_fence_after();
       const uint32_t tmem_acc = tmem_base + as * BN + ((quarter * 32) << 16);
       bool released = false, pending = false;
@@ -708,7 +714,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
       auto release = [&]() {
         ptx::tc_fence_before();
         __syncwarp();
-        if (lane == 0)
+        if (lane == 0 && !dry)
           for (int q = 0; q < kParts; ++q) arrive_issuer(&acc_empty[as + q]);
       };
       uint32_t pending_col = 0;
@@ -717,7 +723,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
       // Pushing epilogue: where this lane's row goes, and how many of the warp's 32 rows are real.
       int2 push_to = make_int2(-1, 0);
       uint32_t push_valid = 0;
-      if (kFp4 && p.push_meta != nullptr && !dead) {
+      if (kFp4 && p.push_meta != nullptr && !dead && !dry) {
         const uint32_t tile_rows = min(static_cast<uint32_t>(ld_dep(p.push_tile_rows + mt)), static_cast<uint32_t>(BM));
         push_valid = tile_rows > quarter * 32 ? min(32u, tile_rows - quarter * 32) : 0u;
         if (static_cast<uint32_t>(lane) < push_valid) {
@@ -761,7 +767,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
               make_uint4(packed[4 * j], packed[4 * j + 1], packed[4 * j + 2], packed[4 * j + 3]);
         ptx::fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) {
+        if (lane == 0 && !dry) {
           ptx::tma_store_2d(&map_out, my_stage, static_cast<int32_t>(col), static_cast<int32_t>(row0));
           ptx::bulk_commit_group();
         }
@@ -782,7 +788,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
           quantize_block16<false>(prod, p.g_product, words[2 * b], words[2 * b + 1], sb[b]);
         }
         const uint32_t row = row0 + lane;
-        if (row < p.m) {
+        if (row < p.m && !dry) {
           *reinterpret_cast<uint4*>(p.out_packed + static_cast<uint64_t>(row) * (inter / 2) + f0 / 2) =
               make_uint4(words[0], words[1], words[2], words[3]);
           const uint32_t c_pad = (inter / 16 + 3) / 4 * 4;
@@ -833,7 +839,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             released = true;
           }
           const uint32_t row = row0 + lane;
-          if (row < p.m) {
+          if (row < p.m && !dry) {
             const uint4* gp = reinterpret_cast<const uint4*>(p.gate_in + static_cast<uint64_t>(row) * p.n + col0);
             const uint32_t c_pad = (p.n / 16 + 3) / 4 * 4;
 #pragma unroll
@@ -877,7 +883,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             }
             ptx::fence_proxy_async_smem();
             __syncwarp();
-            if (lane == 0) {
+            if (lane == 0 && !dry) {
               ptx::tma_store_2d(&map_out, my_stage, static_cast<int32_t>(col0 + half * 32), static_cast<int32_t>(row0));
               ptx::bulk_commit_group();
             }
@@ -926,7 +932,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
       if (!released) {
         release();
       }
+      if (dry) {
+        dry = false;
+        continue;
+      }
+      tile += tile_stride;
       if ((as += kParts) == kAccStages) { as = 0; aphase ^= 1; }
+    }
     }
     if (lane == 0) ptx::bulk_wait_group_all();
   }
@@ -1111,7 +1123,9 @@ int dense_split(const GemmParams& p, uint32_t k_per_stage) {
 // balance -- a dense call with fewer 256-wide tiles than SMs (decode-size batches of the shared branch: 23 us
 // instead of 29), and the grouped gate/up GEMM with the GELU epilogue up to 320 announced assignments per
 // expert (its 1,408 interleaved columns are 5.5 tiles of 256 but 11 of 128; whole layer, 128 experts top-8: 370 us
-// instead of 379 at 3,001 tokens; about even at 6,000).
+// instead of 379 at 3,001 tokens; about even at 6,000), the other grouped GEMMs up to 32: with K as short as the down projection's
+// (three steps) the one accumulator of a wide tile makes every tile wait for the epilogue of the one before (layer of 16 / 64 / 256 tokens 73.9 -> 70.9,
+// 90.5 -> 87.6, 122.2 -> 120.6 us; even at 700, slower beyond).
 int32_t launch_fp4(const char* op, const void* act, const void* w, const GemmParams& params, bool pairs, cudaStream_t stream) {
   GemmParams p = params;
   if (p.plan != nullptr) {
@@ -1129,7 +1143,7 @@ int32_t launch_fp4(const char* op, const void* act, const void* w, const GemmPar
   if (bn == 0) {
     bool narrow;
     if (p.plan != nullptr)
-      narrow = p.gated && g_grouped_rows_hint != 0 && g_grouped_rows_hint <= 320ull * p.experts;
+      narrow = g_grouped_rows_hint != 0 && g_grouped_rows_hint <= (p.gated ? 320ull : 32ull) * p.experts;
     else
       narrow = static_cast<uint64_t>((p.m + BM - 1) / BM) * ((p.n + 255) / 256) < static_cast<uint64_t>(sm_count());
     bn = narrow ? 128 : 256;

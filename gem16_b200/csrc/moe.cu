@@ -387,7 +387,6 @@ permute_small_kernel(const int32_t* ids, int32_t* __restrict__ counts, int32_t* 
   int* totals = loff + experts + 1;     // [3 * 33]
   int* warp_counts = totals + 3 * 33;   // [4][experts]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  pdl_trigger();
   for (uint32_t i = threadIdx.x; i < 5 * experts; i += 128) (i < experts ? cnt[i] : warp_counts[i - experts]) = 0;
   pdl_wait();
   __syncthreads();
@@ -420,6 +419,9 @@ permute_small_kernel(const int32_t* ids, int32_t* __restrict__ counts, int32_t* 
     }
   }
   __syncthreads();
+  // Only now: the dispatch's CTAs, one per token, would wait on SMs that the shared branch's GEMMs on the other stream need (64-token layer
+  // 91.2 -> 90.4 us).
+  pdl_trigger();
   int* running = warp_counts + warp * experts;
 #pragma unroll
   for (int c = 0; c < 8; ++c) {
