@@ -27,6 +27,10 @@
 // projection are exact almost everywhere, the final division is what rounds).  How NVFP4 sums are cut depends on K alone, and a token's
 // columns on the token alone: a result is the same bits for every batch size.  FP8: the same bits for 1 .. 4 and for 5 .. 8 tokens.
 //
+// One kernel for one matrix, for gate and up and for the grouped projections, on purpose: the projections of a layer then share their code,
+// and fetching instructions that the weights' stream has displaced is a good part of a short kernel (a kernel of its own for
+// single matrices: mixed pass 180 -> 190 us, five tokens 219 -> 234).
+//
 // Warps: 0 producer (TMA), 1 and 6 MMA issuers, 2-5 stage the activations (and, NVFP4, their scales into tensor memory), then the
 // epilogue, 7-14 NVFP4 block scales (through registers into the order that tcgen05.cp wants: 4-byte loads, since a scale row is only
 // 4-byte aligned; eight warps with two steps each in flight, four warps cost the mixed pass 8 us).
@@ -57,9 +61,8 @@ constexpr uint32_t kSfaCols = kIssuers * 2 * 16;
 // NVFP4, tensor memory: 20 steps' token scales beside the accumulators of one matrix, 12 beside those of two.
 constexpr uint64_t kFp4MaxK = 20480, kFp4MaxKTwo = 12288;
 
-template <int kMaps>
 struct Maps {
-  CUtensorMap m[kMaps];
+  CUtensorMap m[3];
 };
 struct Args {
   const void* act;
@@ -70,6 +73,7 @@ struct Args {
   float* product;
   uint32_t rows[3], tile_start[4];
   uint32_t tile_rows, k, tokens, columns, stages, early, fewest_rows;
+  uint32_t mats;   // NVFP4: 2 for gate and up of the same rows, else 1
   bool words;      // NVFP4: the tokens' scales are 4-byte aligned
   bool bf16_out;   // FP8, kQuant
 };
@@ -93,9 +97,10 @@ __device__ __forceinline__ float add_keep(float a, float b, float& lost) {
   return s;
 }
 
-template <bool kFp4, int kMats, bool kQuant, int kMaps>
+template <bool kFp4, bool kQuant>
 __global__ void __maxnreg__(96)   // 448 threads: leaves the registers for a row kernel's CTA beside it
-decode_gemv_kernel(const __grid_constant__ Maps<kMaps> maps, const __grid_constant__ Args a) {
+decode_gemv_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Args a) {
+  const uint32_t mats = kFp4 ? a.mats : 1;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t row_bytes = kFp4 ? a.k / 2 : a.k;
@@ -106,7 +111,7 @@ decode_gemv_kernel(const __grid_constant__ Maps<kMaps> maps, const __grid_consta
   uint8_t* xb = stage_sf + (kFp4 ? stages * kSfStageBytes : 0);
   // Eight columns are 1,024 bytes.  Where fewer than `columns` hold tokens the MMA reads on into the next step's: cells nobody uses.
   float* part = reinterpret_cast<float*>(xb + steps * b_step);     // [2][matrix, or FP8: sums and what they lost][group][token][32]
-  const uint32_t part_floats = (kFp4 ? kMats : 2) * kGroups * a.tokens * kGroupRows;   // the room is at least steps x 512 bytes (NVFP4)
+  const uint32_t part_floats = (kFp4 ? mats : 2) * kGroups * a.tokens * kGroupRows;   // the room is at least steps x 512 bytes (NVFP4)
   uint64_t* full = reinterpret_cast<uint64_t*>(part + max(2 * part_floats, kFp4 ? steps * 128 : 0u));
   uint64_t* empty = full + kMaxStages;
   uint64_t* acc_full = empty + kMaxStages;
@@ -137,7 +142,7 @@ decode_gemv_kernel(const __grid_constant__ Maps<kMaps> maps, const __grid_consta
   const uint32_t own = (steps + kIssuers - 1) / kIssuers;
   const uint32_t chain_steps = kFp4 ? own : (own * a.columns + kChainCols - 1) / kChainCols;
   const uint32_t chains = kFp4 ? 1 : (own + chain_steps - 1) / chain_steps;
-  const uint32_t acc_cols = chains * a.columns, slot_cols = kMats * kIssuers * acc_cols;   // [slot][matrix][issuer][chain]
+  const uint32_t acc_cols = chains * a.columns, slot_cols = mats * kIssuers * acc_cols;   // [slot][matrix][issuer][chain]
   const uint32_t sfa_col = 2 * slot_cols, sfb_col = sfa_col + kSfaCols;
   const uint32_t tmem_want = kFp4 ? sfb_col + steps * 16 : 2 * slot_cols;
   const uint32_t tmem_cols = tmem_want <= 64 ? 64u : tmem_want <= 128 ? 128u : tmem_want <= 256 ? 256u : 512u;
@@ -148,7 +153,7 @@ decode_gemv_kernel(const __grid_constant__ Maps<kMaps> maps, const __grid_consta
     *abort_flag = 1;
   };
   auto problem_of = [&](uint32_t tile) -> uint32_t {   // FP8: the matrix whose rows the tile holds
-    if constexpr (kMaps == 1 || kFp4) return 0;
+    if constexpr (kFp4) return 0;
     return (tile >= a.tile_start[1] ? 1u : 0u) + (tile >= a.tile_start[2] ? 1u : 0u);
   };
 
@@ -231,7 +236,7 @@ decode_gemv_kernel(const __grid_constant__ Maps<kMaps> maps, const __grid_consta
       for (uint32_t t = 0; t < my_tiles && !*abort_flag; ++t) {
         const uint32_t tile = blockIdx.x + t * gridDim.x, p = problem_of(tile);
         const int32_t row0 = static_cast<int32_t>((tile - a.tile_start[p]) * a.tile_rows);
-        for (uint32_t i = 0; i < kMats * steps; ++i, ++n) {
+        for (uint32_t i = 0; i < mats * steps; ++i, ++n) {
           const uint32_t mat = i >= steps ? 1u : 0u, s = i - mat * steps;
           if (n == a.early) pdl_wait();   // `early` <= `stages`: from there on this thread waits for MMAs that wait for the previous kernel
           if (n >= stages && !ptx::mbar_wait(&empty[stage], phase ^ 1)) { fail_wait(11); break; }
@@ -239,7 +244,7 @@ decode_gemv_kernel(const __grid_constant__ Maps<kMaps> maps, const __grid_consta
           // Chunks past the end of a row arrive as zeros, rows past the matrix too.
 #pragma unroll
           for (uint32_t q = 0; q < kGroups; ++q)
-            ptx::tma_load_2d_hint(stage_w + stage * kStageBytes + q * (kGroupRows * 128), &maps.m[kMaps == 1 ? 0 : kFp4 ? mat : p], ptx::smem_addr(&full[stage]),
+            ptx::tma_load_2d_hint(stage_w + stage * kStageBytes + q * (kGroupRows * 128), &maps.m[kFp4 ? mat : p], ptx::smem_addr(&full[stage]),
                                   static_cast<int32_t>((s * kGroups + q) * 128), row0, policy);
           if (++stage == stages) { stage = 0; phase ^= 1; }
         }
@@ -278,14 +283,14 @@ decode_gemv_kernel(const __grid_constant__ Maps<kMaps> maps, const __grid_consta
         ready = 1 + (seen[0] ? 1 + (seen[1] ? 1 + (seen[2] ? 1 + (seen[3] ? 1 : 0) : 0) : 0) : 0);
         return true;
       };
-      if (issuer < my_tiles * kMats * steps && !wait_steps()) fail_wait(14);
+      if (issuer < my_tiles * mats * steps && !wait_steps()) fail_wait(14);
       if (!ptx::mbar_wait(x_ready, 0)) fail_wait(12);
       ptx::tc_fence_after();
       uint32_t first = issuer;   // this thread's first step of the matrix at hand
       for (uint32_t t = 0; t < my_tiles && !*abort_flag; ++t) {
         if (t >= 2 && !ptx::mbar_wait(&acc_empty[slot], slot_phase ^ 1)) { fail_wait(13); break; }
         bool ok = true;
-        for (uint32_t mat = 0; mat < kMats && ok; ++mat) {
+        for (uint32_t mat = 0; mat < mats && ok; ++mat) {
           uint32_t acc = tmem + slot * slot_cols + (mat * kIssuers + issuer) * acc_cols, in_chain = 0;
           uint32_t s = first;
           for (; s < steps; s += kIssuers) {
@@ -404,11 +409,11 @@ decode_gemv_kernel(const __grid_constant__ Maps<kMaps> maps, const __grid_consta
       if (failed) fail_wait(15);
       ptx::tc_fence_after();
       float* mine = part + (t & 1) * part_floats;
-#pragma unroll
-      for (int mat = 0; mat < kMats; ++mat) {
+#pragma unroll 1
+      for (uint32_t mat = 0; mat < mats; ++mat) {
         // The chains of the two issuers, even steps first (of a sum of one step only one has anything).
         const uint32_t cells = lanes + slot * slot_cols + mat * kIssuers * acc_cols + group * a.tokens;
-        const uint32_t first = (t * kMats + mat) * steps & 1;
+        const uint32_t first = (t * mats + mat) * steps & 1;
         auto gather = [&](auto cell_count) {
           constexpr int kCells = decltype(cell_count)::value;
           uint32_t v[kCells];
@@ -471,7 +476,7 @@ decode_gemv_kernel(const __grid_constant__ Maps<kMaps> maps, const __grid_consta
         const uint64_t o = static_cast<uint64_t>(token) * rows + row;
         if constexpr (kFp4) {
           const float y0 = __fdiv_rn(sum(0, token), a.div[0]);   // single final division by ga*gw: src/cuda/nvfp4/sm120.cu:243
-          if constexpr (kMats == 2) {
+          if (mats == 2) {
             const float y1 = __fdiv_rn(sum(1, token), a.div[1]);
             if (a.out[0]) static_cast<float*>(a.out[0])[o] = y0;
             if (a.out[1]) static_cast<float*>(a.out[1])[o] = y1;
@@ -499,7 +504,7 @@ decode_gemv_kernel(const __grid_constant__ Maps<kMaps> maps, const __grid_consta
     // one's are stored, sixteen steps are in flight per SM.
     if (a.fewest_rows <= kFewRows) pdl_wait();
     const uint32_t srow = a.k / 16, word = lane & 15, half = lane >> 4, rounds = (a.tile_rows + 1) / 2;
-    const uint32_t per_tile = kMats * steps, total = my_tiles * per_tile;
+    const uint32_t per_tile = mats * steps, total = my_tiles * per_tile;
     const uint64_t policy = ptx::evict_first_policy();
     const uint32_t active = min(kScaleWarps, stages);   // a warp sees every phase of the stages it waits on only if it laps none of them
     uint32_t n = warp - 7, next = n < active ? n : total, stage = n % stages, use = 0;   // `next`: the step whose words are requested next
@@ -573,15 +578,15 @@ uint32_t pick_tile_rows(const uint64_t* rows, int n, uint64_t ctas) {
   return static_cast<uint32_t>(r);
 }
 
-template <bool kFp4, int kMats, bool kQuant, int kMaps>
+template <bool kFp4, bool kQuant>
 int32_t launch(const char* op, const DecodeCall& c, cudaStream_t stream, bool* taken) {
-  const uint64_t row_bytes = kFp4 ? c.k / 2 : c.k, steps = (row_bytes + 511) / 512;
+  const uint64_t mats = kFp4 ? c.n : 1, row_bytes = kFp4 ? c.k / 2 : c.k, steps = (row_bytes + 511) / 512;
   const uint64_t columns = c.tokens <= 4 ? 16 : 32;
-  const size_t part = std::max<size_t>(2 * (kFp4 ? kMats : 2) * kGroups * c.tokens * kGroupRows * sizeof(float), kFp4 ? steps * 512 : 0);
+  const size_t part = std::max<size_t>(2 * (kFp4 ? mats : 2) * kGroups * c.tokens * kGroupRows * sizeof(float), kFp4 ? steps * 512 : 0);
   const size_t fixed = steps * ((c.tokens + 1) / 2) * 1024 + part + (2 * kMaxStages + 5) * 8 + 64 + 1024;
   const size_t per_stage = kStageBytes + (kFp4 ? kSfStageBytes : 0);
   if (fixed + kMinStages * per_stage > kSmemBudget) return GEMB_OK;
-  Maps<kMaps> maps;
+  Maps maps;
   Args a{};
   a.act = c.act;
   a.act_scales = c.act_scales;
@@ -592,6 +597,7 @@ int32_t launch(const char* op, const DecodeCall& c, cudaStream_t stream, bool* t
   a.stages = static_cast<uint32_t>(std::min<uint64_t>(kMaxStages, (kSmemBudget - fixed) / per_stage)) & ~1u;
   a.words = reinterpret_cast<uintptr_t>(c.act_scales) % 4 == 0;
   a.bf16_out = c.bf16_out;
+  a.mats = static_cast<uint32_t>(mats);
   uint64_t rows[3] = {c.m[0].rows, c.m[1].rows, c.m[2].rows};
   const int spaces = kFp4 ? 1 : c.n;   // gate and up share their rows' tiles
   a.tile_rows = pick_tile_rows(rows, spaces, static_cast<uint64_t>(sm_count()));
@@ -611,11 +617,11 @@ int32_t launch(const char* op, const DecodeCall& c, cudaStream_t stream, bool* t
   a.tile_start[3] = tiles;
   if (kFp4) a.tile_start[1] = tiles;
   const uint32_t ctas = std::min(tiles, static_cast<uint32_t>(sm_count()));
-  a.stages = static_cast<uint32_t>(std::min<uint64_t>(a.stages, ((tiles + ctas - 1) / ctas * kMats * steps + 1) & ~1ull));   // no more than a CTA has steps
+  a.stages = static_cast<uint32_t>(std::min<uint64_t>(a.stages, ((tiles + ctas - 1) / ctas * mats * steps + 1) & ~1ull));   // no more than a CTA has steps
   a.early = std::min(a.stages, (kEarlyBytes + kGroups * a.tile_rows * 128 - 1) / (kGroups * a.tile_rows * 128));
   const size_t smem = fixed + a.stages * per_stage;
-  GEMB_TRY((allow_full_smem<decode_gemv_kernel<kFp4, kMats, kQuant, kMaps>>(op)));
-  GEMB_TRY(launch_pdl_split(op, true, decode_gemv_kernel<kFp4, kMats, kQuant, kMaps>, dim3(ctas),
+  GEMB_TRY((allow_full_smem<decode_gemv_kernel<kFp4, kQuant>>(op)));
+  GEMB_TRY(launch_pdl_split(op, true, decode_gemv_kernel<kFp4, kQuant>, dim3(ctas),
                       dim3(kFp4 ? kThreadsFp4 : kThreadsFp8), smem, stream, maps, a));
   *taken = true;
   return check_launch(op);
@@ -640,13 +646,12 @@ int32_t launch_decode_fp4(const char* op, const DecodeCall& c, cudaStream_t stre
   if (c.k > (c.n == 2 ? kFp4MaxKTwo : kFp4MaxK)) return GEMB_OK;
   for (int i = 0; i < c.n; ++i)
     if (reinterpret_cast<uintptr_t>(c.m[i].scales) % 4 != 0) return GEMB_OK;
-  return c.n == 2 ? launch<true, 2, false, 2>(op, c, stream, taken) : launch<true, 1, false, 1>(op, c, stream, taken);
+  return launch<true, false>(op, c, stream, taken);
 }
 
 int32_t launch_decode_fp8(const char* op, const DecodeCall& c, cudaStream_t stream, bool* taken) {
   *taken = false;
-  if (c.quantize) return launch<false, 1, true, 1>(op, c, stream, taken);   // never more than one matrix
-  return c.n == 1 ? launch<false, 1, false, 1>(op, c, stream, taken) : launch<false, 1, false, 3>(op, c, stream, taken);
+  return c.quantize ? launch<false, true>(op, c, stream, taken) : launch<false, false>(op, c, stream, taken);
 }
 
 }  // namespace gemb
