@@ -49,6 +49,7 @@ int gemv_take_device_error();
 int ep_take_device_error();
 int moe_take_device_error();
 int router_input_take_device_error();
+int router_take_device_error();
 
 inline bool positive_finite(float v) { return std::isfinite(v) && v > 0.0f; }
 

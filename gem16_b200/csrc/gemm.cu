@@ -76,13 +76,13 @@ static EncodeTiledFn encode_tiled_fn() {
   return fn;
 }
 
-// 2-D map with the 128-byte swizzle.  The encoder wants a current context, which a host thread has only after its first call that
+// 2-D map.  The encoder wants a current context, which a host thread has only after its first call that
 // needs one: cudaSetDevice makes the thread's device current for the driver too.
 static CUresult encode(EncodeTiledFn fn, CUtensorMap* map, CUtensorMapDataType type, void* base, const cuuint64_t* dims,
-                       const cuuint64_t* strides, const cuuint32_t* box, CUtensorMapL2promotion promotion) {
+                       const cuuint64_t* strides, const cuuint32_t* box, CUtensorMapSwizzle swizzle, CUtensorMapL2promotion promotion) {
   const cuuint32_t estr[2] = {1, 1};
   for (int attempt = 0;; ++attempt) {
-    const CUresult r = fn(map, type, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, promotion,
+    const CUresult r = fn(map, type, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, promotion,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     int dev = 0;
     if (r != CUDA_ERROR_INVALID_CONTEXT || attempt != 0 || cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) return r;
@@ -96,7 +96,21 @@ int32_t make_byte_map(const char* op, CUtensorMap* map, const void* base, uint64
   const cuuint64_t dims[2] = {row_bytes, rows};
   const cuuint64_t strides[1] = {row_bytes};
   const cuuint32_t box[2] = {128, box_rows};
-  CUresult r = encode(fn, map, CU_TENSOR_MAP_DATA_TYPE_UINT8, const_cast<void*>(base), dims, strides, box, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+  CUresult r = encode(fn, map, CU_TENSOR_MAP_DATA_TYPE_UINT8, const_cast<void*>(base), dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B,
+                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+  if (r != CUDA_SUCCESS) return fail(GEMB_INTERNAL, "%s: cuTensorMapEncodeTiled failed with CUresult %d", op, int(r));
+  return GEMB_OK;
+}
+
+int32_t make_word_map(const char* op, CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t word_bytes, uint32_t box_cols,
+                      uint32_t box_rows, bool swizzle) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (!fn) return fail(GEMB_UNSUPPORTED, "%s: cuTensorMapEncodeTiled is not available from the driver", op);
+  const cuuint64_t dims[2] = {cols, rows};
+  const cuuint64_t strides[1] = {cols * word_bytes};
+  const cuuint32_t box[2] = {box_cols, box_rows};
+  CUresult r = encode(fn, map, word_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_UINT32, const_cast<void*>(base), dims, strides,
+                      box, swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
   if (r != CUDA_SUCCESS) return fail(GEMB_INTERNAL, "%s: cuTensorMapEncodeTiled failed with CUresult %d", op, int(r));
   return GEMB_OK;
 }
@@ -977,7 +991,8 @@ int32_t make_out_map(const char* op, CUtensorMap* map, void* base, uint64_t rows
   const cuuint64_t dims[2] = {cols, rows};
   const cuuint64_t strides[1] = {cols * 2};
   const cuuint32_t box[2] = {64, 32};
-  CUresult r = encode(fn, map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, base, dims, strides, box, CU_TENSOR_MAP_L2_PROMOTION_NONE);
+  CUresult r = encode(fn, map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B,
+                      CU_TENSOR_MAP_L2_PROMOTION_NONE);
   if (r != CUDA_SUCCESS) return fail(GEMB_INTERNAL, "%s: cuTensorMapEncodeTiled failed with CUresult %d", op, int(r));
   return GEMB_OK;
 }
@@ -989,7 +1004,8 @@ int32_t make_out_map_f32(const char* op, CUtensorMap* map, void* base, uint64_t 
   const cuuint64_t dims[2] = {cols, rows};
   const cuuint64_t strides[1] = {cols * 4};
   const cuuint32_t box[2] = {32, 32};
-  CUresult r = encode(fn, map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, base, dims, strides, box, CU_TENSOR_MAP_L2_PROMOTION_NONE);
+  CUresult r = encode(fn, map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B,
+                      CU_TENSOR_MAP_L2_PROMOTION_NONE);
   if (r != CUDA_SUCCESS) return fail(GEMB_INTERNAL, "%s: cuTensorMapEncodeTiled failed with CUresult %d", op, int(r));
   return GEMB_OK;
 }
@@ -1540,6 +1556,8 @@ int32_t gemb_check_device_status(void) {
     return fail(GEMB_INTERNAL, "%s: an expert-parallel kernel met positions outside its buffers and skipped or clamped them (check %d)", op, ep_code);
   if (router_input_take_device_error() != 0)
     return fail(GEMB_INTERNAL, "%s: the router's input transform gave up waiting for its rows", op);
+  const int router_code = router_take_device_error();
+  if (router_code != 0) return fail(GEMB_INTERNAL, "%s: a router-logits kernel gave up waiting on its ring (role %d)", op, router_code);
   const int moe_code = moe_take_device_error();
   if (moe_code == 1)
     return fail(GEMB_DATA_LOSS, "%s: the router met a non-finite logit; the token got zero routing weights", op);

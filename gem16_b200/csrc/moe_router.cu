@@ -5,43 +5,54 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "ptx.cuh"
+#include "tensor_map.h"
 
 namespace gemb {
 
 // Benchmark hook (GEMB_TUNE_ROUTER_TILE): 0 = automatic, otherwise one of the shapes below.  All give the same bits.
 int g_router_tile = 0;
 
+// Set when a wait on the operands' ring runs out (1: the producer's, 2: a reader's); gemb_check_device_status() reports and clears it.
+__device__ int g_router_error = 0;
+
+int router_take_device_error() {
+  int code = 0;
+  if (cudaMemcpyFromSymbol(&code, g_router_error, sizeof code) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  if (code != 0) {
+    const int zero = 0;
+    cudaMemcpyToSymbol(g_router_error, &zero, sizeof zero);
+  }
+  return code;
+}
+
 namespace {
 
-__device__ __forceinline__ void cp_async_16(void* smem_dst, const void* src, bool valid) {
-  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst));
-  const uint32_t n = valid ? 16u : 0u;   // 0 source bytes: the destination is zero filled
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+// Eight bytes, global -> shared; `bar` gets an arrival of this thread once everything that it has copied so has landed.
+__device__ __forceinline__ void cp_async_8(void* smem_dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(ptx::smem_addr(smem_dst)), "l"(src) : "memory");
 }
-__device__ __forceinline__ void cp_async_8(void* smem_dst, const void* src, bool valid) {
-  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst));
-  const uint32_t n = valid ? 8u : 0u;
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(ptx::smem_addr(bar)) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int kPending>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory"); }
 
 // ---------------------------------------------------------------------------------------------
-// CTA = four warps = 4 kTok tokens x 32 kExp experts: a warp owns kTok tokens, a lane the experts lane + 32 j, so a
+// CTA = four computing warps = 4 kTok tokens x 32 kExp experts: a warp owns kTok tokens, a lane the experts lane + 32 j, so a
 // thread carries kTok x kExp independent chains.  What bounds it, per k and SM: kTok kExp clocks of fma, 4 kExp + 2 kTok
-// clocks of shared-memory reads (a read returns 128 bytes per clock, broadcast or not; that, 40 clocks
-// against 28 of fma per 14 x 4 outputs of a thread, bound the former kernel, which read fp32 tokens), and four clocks of fma latency.
-// So the activations stay bf16 in shared memory (one read brings four k of a token) and are widened in
-// registers, the weights keep the order memory has them in (rows padded by four words: the lanes' 16-byte reads
-// along k are conflict free), and nothing is transposed.
-//
-// Tiles of 128 / kExp k run through a ring of four buffers by cp.async; one barrier per tile, taken while the tile's
-// last operands are in registers, so that neither it nor a shared-memory read is waited for: the
-// operands of the next step are always requested before the current step is computed.  2,816 x 128, us before -> now:
-// 64 tokens 22.6 -> 14, 256: 29 -> 17, 512: 41 -> 26, 1,024: 53 -> 36, 2,048: 74 -> 57, 3,001: 112 -> 77,
-// 6,000: 164 -> 131.  (Loops of two steps instead of the whole tile unrolled: 20-50 % slower; scalar fma
-// outgrows the instruction cache with ten and more tokens per warp.)
+// clocks of shared-memory reads (a read returns 128 bytes per clock, broadcast or not), and four clocks of fma latency; with one
+// warp per scheduler whatever else a warp issues or waits for adds to the fma.  So
+// - the activations stay bf16 in shared memory (one read brings four k of a token) and are widened in registers;
+// - a fifth warp does all the copying: tiles of 128 / kExp k by TMA through a ring of four buffers, two barriers per buffer.  The
+//   computing warps spent 200 ns per tile of 6 x 4 outputs and 32 k on addresses, cp.async and a barrier, of 880 in all.  (The copying
+//   warp with one bulk copy per row instead: 33 ns per copy, 440 us for 3,001 tokens.)
+// - the next step's operands are requested between the products of the current one, not in a burst before them.
+// The weights' rows are 128-byte pieces in TMA's swizzle: the lanes' 16-byte reads along k are conflict free.
+// 2,816 x 128, us with cp.async -> now: 16 tokens 14.6 -> 12.4, 256: 18.5 -> 14.4, 512: 27.6 -> 20.6, 1,024: 37 -> 31, 2,048: 59 -> 50,
+// 3,001: 78 -> 65, 6,000: 133 -> 115.  (Steps of 8 k with 16-byte reads of the activations, or the products in serpentine order: no
+// gain.  Scalar fma instead of packed: 84 us for 3,001.)
 // ---------------------------------------------------------------------------------------------
 constexpr int kRtWarps = 4, kRtThreads = kRtWarps * 32, kRtDepth = 4, kRtSteps = 8;
 
@@ -52,8 +63,9 @@ struct RouterShape {
   static constexpr int kG = kStepK / 4;            // groups of four k per step
   static constexpr int kTokens = kRtWarps * kTok, kExperts = 32 * kExp;
   struct Smem {
-    float w[kRtDepth][kExperts][kK + 4];
+    float w[kRtDepth][kK / 32][kExperts][32];   // 128-byte swizzle: 16-byte piece c of row r lies at c ^ (r & 7)
     uint16_t x[kRtDepth][kTokens][kK];
+    uint64_t full[kRtDepth], empty[kRtDepth];
   };
 };
 
@@ -68,87 +80,124 @@ template <int kTok, int kExp, int kG, typename S>
 __device__ __forceinline__ void router_load(RouterOps<kTok, kExp, kG>& o, const typename S::Smem& sm, uint32_t buf, int k, int warp, int lane) {
 #pragma unroll
   for (int g = 0; g < kG; ++g) {
+    const int at = k + 4 * g;
 #pragma unroll
-    for (int j = 0; j < kExp; ++j) o.w[g][j] = *reinterpret_cast<const float4*>(&sm.w[buf][lane + 32 * j][k + 4 * g]);
+    for (int j = 0; j < kExp; ++j) o.w[g][j] = *reinterpret_cast<const float4*>(&sm.w[buf][at / 32][lane + 32 * j][(at / 4 % 8 ^ (lane & 7)) * 4]);
 #pragma unroll
-    for (int i = 0; i < kTok; ++i) o.x[g][i] = *reinterpret_cast<const uint2*>(&sm.x[buf][warp * kTok + i][k + 4 * g]);
+    for (int i = 0; i < kTok; ++i) o.x[g][i] = *reinterpret_cast<const uint2*>(&sm.x[buf][warp * kTok + i][at]);
   }
 }
 
-// Two tokens share an instruction: the packed fp32 fma is one IEEE fma per half.
+// The products of one k.  Two tokens share an instruction: the packed fp32 fma is one IEEE fma per half.
 template <int kTok, int kExp, int kG>
-__device__ __forceinline__ void router_compute(float2 (&acc)[(kTok + 1) / 2][kExp], const RouterOps<kTok, kExp, kG>& o) {
+__device__ __forceinline__ void router_products(float2 (&acc)[(kTok + 1) / 2][kExp], const RouterOps<kTok, kExp, kG>& o, int g, int q) {
+  float wq[kExp], xq[kTok];
 #pragma unroll
-  for (int g = 0; g < kG; ++g)
+  for (int j = 0; j < kExp; ++j) wq[j] = q == 0 ? o.w[g][j].x : q == 1 ? o.w[g][j].y : q == 2 ? o.w[g][j].z : o.w[g][j].w;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      float wq[kExp], xq[kTok];
+  for (int i = 0; i < kTok; ++i) {
+    const uint32_t two = q < 2 ? o.x[g][i].x : o.x[g][i].y;
+    xq[i] = __uint_as_float((q & 1) ? (two & 0xFFFF0000u) : (two << 16));
+  }
+  if constexpr (kTok == 1) {
 #pragma unroll
-      for (int j = 0; j < kExp; ++j) wq[j] = q == 0 ? o.w[g][j].x : q == 1 ? o.w[g][j].y : q == 2 ? o.w[g][j].z : o.w[g][j].w;
+    for (int j = 0; j < kExp; ++j) acc[0][j].x = fmaf(xq[0], wq[j], acc[0][j].x);
+  } else {
 #pragma unroll
-      for (int i = 0; i < kTok; ++i) {
-        const uint32_t two = q < 2 ? o.x[g][i].x : o.x[g][i].y;
-        xq[i] = __uint_as_float((q & 1) ? (two & 0xFFFF0000u) : (two << 16));
-      }
-      if constexpr (kTok == 1) {
+    for (int j = 0; j < kExp; ++j) {
+      const float2 wp = make_float2(wq[j], wq[j]);
 #pragma unroll
-        for (int j = 0; j < kExp; ++j) acc[0][j].x = fmaf(xq[0], wq[j], acc[0][j].x);
-      } else {
-#pragma unroll
-        for (int j = 0; j < kExp; ++j) {
-          const float2 wp = make_float2(wq[j], wq[j]);
-#pragma unroll
-          for (int p = 0; p < kTok / 2; ++p) acc[p][j] = __ffma2_rn(make_float2(xq[2 * p], xq[2 * p + 1]), wp, acc[p][j]);
-        }
-      }
+      for (int p = 0; p < kTok / 2; ++p) acc[p][j] = __ffma2_rn(make_float2(xq[2 * p], xq[2 * p + 1]), wp, acc[p][j]);
     }
+  }
+}
+
+// Reads that stay where they are written: the compiler would gather them before the products.
+__device__ __forceinline__ float4 lds_16(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ uint2 lds_8(uint32_t addr) {
+  uint2 v;
+  asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
+  return v;
+}
+
+// One step's products (`cur`), with the operands of the step at k of a tile (`next`) requested between them.  w_tile is the address of
+// the lane's row and x_tile that of the warp's first token in that tile.
+template <int kTok, int kExp, int kG, typename S>
+__device__ __forceinline__ void router_step(float2 (&acc)[(kTok + 1) / 2][kExp], const RouterOps<kTok, kExp, kG>& cur, RouterOps<kTok, kExp, kG>& next,
+                                            uint32_t w_tile, uint32_t x_tile, uint32_t k) {
+  constexpr int kLoads = kG * (kExp + kTok), kSlots = 4 * kG;
+  auto load = [&](int i) {
+    const uint32_t g = i / (kExp + kTok), r = i % (kExp + kTok), at = k + 4 * g;
+    if (r < kExp) next.w[g][r] = lds_16((w_tile ^ (at / 4 % 8 << 4)) + at / 32 * S::kExperts * 128 + r * 32 * 128);
+    else next.x[g][r - kExp] = lds_8(x_tile + at * 2 + (r - kExp) * S::kK * 2);
+  };
+#pragma unroll
+  for (int slot = 0; slot < kSlots; ++slot) {
+#pragma unroll
+    for (int i = 0; i < kLoads; ++i)
+      if (i * kSlots / kLoads == slot) load(i);
+    router_products<kTok, kExp, kG>(acc, cur, slot / 4, slot % 4);
+  }
 }
 
 template <int kTok, int kExp>
-__global__ void __launch_bounds__(kRtThreads, kTok * kExp >= 24 ? 2 : 3)
-router_logits_kernel(const uint16_t* x, const float* __restrict__ w, const float* __restrict__ bias, float* logits,
-                     uint32_t tokens, uint32_t hidden, uint32_t experts, bool x_wide) {
+__global__ void __launch_bounds__(kRtThreads + 32, kTok * kExp >= 24 ? 2 : 3)
+router_logits_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const uint16_t* x,
+                     const float* __restrict__ bias, float* logits, uint32_t tokens, uint32_t hidden, uint32_t experts, bool x_wide) {
   using S = RouterShape<kTok, kExp>;
   constexpr int kK = S::kK, kG = S::kG;
   static_assert(kTok == 1 || kTok % 2 == 0, "tokens go in pairs");
   extern __shared__ __align__(16) uint8_t router_smem[];
-  auto& sm = *reinterpret_cast<typename S::Smem*>(router_smem);
+  auto& sm = *reinterpret_cast<typename S::Smem*>((reinterpret_cast<uintptr_t>(router_smem) + 1023) & ~uintptr_t(1023));
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t tok0 = blockIdx.x * S::kTokens, exp0 = blockIdx.y * S::kExperts;
   const uint32_t tiles = (hidden + kK - 1) / kK, full = hidden / kK;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kRtDepth; ++i) {
+      ptx::mbar_init(&sm.full[i], x_wide ? 1 : 33);
+      ptx::mbar_init(&sm.empty[i], kRtWarps);
+    }
+    ptx::fence_barrier_init();
+  }
+  __syncthreads();
   pdl_trigger();
   pdl_wait();
-  // A weight tile is kExperts rows of kK / 4 16-byte pieces (1,024 in all, eight per thread), an activation tile
-  // kTokens rows of kK / 8 16-byte pieces (or twice as many halves where rows are only 8-byte aligned).
-  constexpr int kWp = kK / 4, kXp = kK / 8;
-  const uint32_t wrow = threadIdx.x / kWp, wcol = threadIdx.x % kWp * 4;
-  auto issue = [&](uint32_t t) {
-    if (t < tiles) {
-      const uint32_t k0 = t * kK, buf = t % kRtDepth;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const uint32_t row = wrow + i * (kRtThreads / kWp);
-        const bool ok = k0 + wcol < hidden && exp0 + row < experts;
-        cp_async_16(&sm.w[buf][row][wcol], w + static_cast<uint64_t>(ok ? exp0 + row : 0) * hidden + (ok ? k0 + wcol : 0), ok);
+  if (warp == kRtWarps) {
+    const uint32_t rows = min(static_cast<uint32_t>(S::kTokens), tokens - tok0);
+    for (uint32_t t = 0; t < tiles; ++t) {
+      const uint32_t buf = t % kRtDepth, k0 = t * kK;
+      if (t >= kRtDepth && !ptx::mbar_wait(&sm.empty[buf], (t / kRtDepth - 1) & 1)) {
+        atomicCAS(&g_router_error, 0, 1);
+        break;
       }
-      if (x_wide) {
+      if (lane == 0) {   // past the matrices' edges TMA writes zeros, which count
+        const uint32_t bar = ptx::smem_addr(&sm.full[buf]);
+        ptx::mbar_expect_tx(&sm.full[buf], S::kExperts * kK * 4 + (x_wide ? S::kTokens * kK * 2 : 0));
 #pragma unroll
-        for (int i = 0; i < (S::kTokens * kXp + kRtThreads - 1) / kRtThreads; ++i) {
-          const uint32_t idx = threadIdx.x + i * kRtThreads, row = idx / kXp, col = idx % kXp * 8;
-          if (row >= static_cast<uint32_t>(S::kTokens)) break;
-          const bool ok = k0 + col < hidden && tok0 + row < tokens;
-          cp_async_16(&sm.x[buf][row][col], x + static_cast<uint64_t>(ok ? tok0 + row : 0) * hidden + (ok ? k0 + col : 0), ok);
+        for (int b = 0; b < kK / 32; ++b) ptx::tma_load_2d<false>(&sm.w[buf][b][0][0], &map_w, bar, k0 + b * 32, exp0);
+        if (x_wide) ptx::tma_load_2d<false>(&sm.x[buf][0][0], &map_x, bar, k0, tok0);
+      }
+      if (!x_wide) {   // rows that are only 8-byte aligned
+        const uint32_t n = min(static_cast<uint32_t>(kK), hidden - k0) / 4;
+        for (uint32_t i = lane; i < rows * n; i += 32) {
+          const uint32_t row = i / n, col = i % n * 4;
+          cp_async_8(&sm.x[buf][row][col], x + static_cast<uint64_t>(tok0 + row) * hidden + k0 + col);
         }
-      } else {
-#pragma unroll 1
-        for (uint32_t idx = threadIdx.x; idx < S::kTokens * kXp * 2u; idx += kRtThreads) {
-          const uint32_t row = idx / (kXp * 2), col = idx % (kXp * 2) * 4;
-          const bool ok = k0 + col < hidden && tok0 + row < tokens;
-          cp_async_8(&sm.x[buf][row][col], x + static_cast<uint64_t>(ok ? tok0 + row : 0) * hidden + (ok ? k0 + col : 0), ok);
-        }
+        cp_async_arrive(&sm.full[buf]);
       }
     }
-    cp_async_commit();   // one group per call, empty past the last tile, so the counting stays uniform
+    return;
+  }
+  bool ok = true;
+  auto landed = [&](uint32_t t) {
+    if (!ptx::mbar_wait(&sm.full[t % kRtDepth], t / kRtDepth & 1)) {
+      atomicCAS(&g_router_error, 0, 2);
+      ok = false;
+    }
   };
   float2 acc[(kTok + 1) / 2][kExp];
 #pragma unroll
@@ -158,36 +207,32 @@ router_logits_kernel(const uint16_t* x, const float* __restrict__ w, const float
 #pragma unroll
     for (int p = 0; p < (kTok + 1) / 2; ++p) acc[p][j] = make_float2(b, b);
   }
-#pragma unroll
-  for (int t = 0; t < kRtDepth; ++t) issue(t);
-  cp_async_wait<kRtDepth - 1>();
-  __syncthreads();
+  landed(0);
   RouterOps<kTok, kExp, kG> ops[2];
+  const uint32_t w_lane = ptx::smem_addr(&sm.w[0][0][lane][(lane & 7) * 4]), x_warp = ptx::smem_addr(&sm.x[0][warp * kTok][0]);
   router_load<kTok, kExp, kG, S>(ops[0], sm, 0, 0, warp, lane);
-  for (uint32_t t = 0; t < full; ++t) {
+  for (uint32_t t = 0; t < full && ok; ++t) {
     const uint32_t buf = t % kRtDepth;
 #pragma unroll
     for (int s = 0; s < kRtSteps; ++s) {
-      if (s + 1 < kRtSteps) {
-        router_load<kTok, kExp, kG, S>(ops[(s + 1) & 1], sm, buf, (s + 1) * S::kStepK, warp, lane);
-      } else {
-        cp_async_wait<kRtDepth - 2>();   // tile t + 1 has landed (this thread's pieces)
-        __syncthreads();                 // everyone's; and everyone has read all of tile t
-        issue(t + kRtDepth);             // into the buffer of tile t
-        router_load<kTok, kExp, kG, S>(ops[0], sm, (t + 1) % kRtDepth, 0, warp, lane);   // past the last tile: old bytes, not used
-      }
-      router_compute<kTok, kExp, kG>(acc, ops[s & 1]);
+      const bool last = s + 1 == kRtSteps;
+      if (last && t + 1 < tiles) landed(t + 1);   // past the last tile: old bytes, not used
+      const uint32_t next = last ? (t + 1) % kRtDepth : buf;
+      router_step<kTok, kExp, kG, S>(acc, ops[s & 1], ops[(s + 1) & 1], w_lane + next * (S::kExperts * kK * 4), x_warp + next * (S::kTokens * kK * 2),
+                                     last ? 0 : (s + 1) * S::kStepK);
     }
+    __syncwarp();
+    if (lane == 0) ptx::mbar_arrive(&sm.empty[buf]);   // all of tile t has been read
   }
   if (full < tiles) {   // the rest of K, a multiple of four: its tile has landed
     RouterOps<kTok, kExp, 1> o;
 #pragma unroll 1
     for (uint32_t k = 0; k < hidden - full * kK; k += 4) {
       router_load<kTok, kExp, 1, S>(o, sm, full % kRtDepth, static_cast<int>(k), warp, lane);
-      router_compute<kTok, kExp, 1>(acc, o);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) router_products<kTok, kExp, 1>(acc, o, 0, q);
     }
   }
-  cp_async_wait<0>();
 #pragma unroll
   for (int i = 0; i < kTok; ++i) {
     const uint32_t t = tok0 + warp * kTok + i;
@@ -204,8 +249,8 @@ router_logits_kernel(const uint16_t* x, const float* __restrict__ w, const float
 // The largest batches: CTA = 64 or 56 tokens x 128 experts, thread = 16 or 14 tokens x 4 experts, fp32 tiles of 32 k
 // transposed on the way into shared memory, the next tile's global loads in registers.  56 tokens even out
 // batches that 64-token CTAs would spread unevenly over the SMs.  Slower than the kernel above while an SM
-// has one CTA at most (its loads are then not covered), 15 % faster with two: 16,384 x 2,816 x 128 in 234 us
-// (90 of 128 fma per clock and SM) against 274 us, which pays there for widening the activations.  Shared tiles are
+// has one CTA at most (its loads are then not covered), 15 % faster with two: 16,384 x 2,816 x 128 in 235 us
+// (90 of 128 fma per clock and SM) against 276 us, which pays there for widening the activations.  Shared tiles are
 // stored k-major with an xor swizzle of the column (multiples of 4 / 8 keep each thread's float4 groups
 // intact) so that both the transposing stores and the float4 loads are bank-conflict free.
 // ---------------------------------------------------------------------------------------------
@@ -358,10 +403,13 @@ int32_t launch_router(const char* op, const RouterArgs& a, cudaStream_t stream) 
   auto kern = router_logits_kernel<kTok, kExp>;
   GEMB_TRY((allow_full_smem<router_logits_kernel<kTok, kExp>>(op)));
   const bool x_wide = a.hidden % 8 == 0 && reinterpret_cast<uintptr_t>(a.x) % 16 == 0;
+  CUtensorMap map_w, map_x{};
+  GEMB_TRY(make_word_map(op, &map_w, a.w, a.experts, a.hidden, 4, 32, S::kExperts, true));
+  if (x_wide) GEMB_TRY(make_word_map(op, &map_x, a.x, a.tokens, a.hidden, 2, S::kK, S::kTokens, false));
   // Not a dependent launch: CTAs placed while the kernel before this one still fills SMs end up two on one SM and none on
   // another (2,048 tokens: 57 us this way, 81 us behind a kernel that triggers early).
-  kern<<<dim3((a.tokens + S::kTokens - 1) / S::kTokens, (a.experts + S::kExperts - 1) / S::kExperts), kRtThreads, sizeof(typename S::Smem),
-         stream>>>(a.x, a.w, a.bias, a.logits, a.tokens, a.hidden, a.experts, x_wide);
+  kern<<<dim3((a.tokens + S::kTokens - 1) / S::kTokens, (a.experts + S::kExperts - 1) / S::kExperts), kRtThreads + 32, sizeof(typename S::Smem) + 1024,
+         stream>>>(map_w, map_x, a.x, a.bias, a.logits, a.tokens, a.hidden, a.experts, x_wide);
   return check_launch(op);
 }
 template <int kTok>
@@ -380,9 +428,9 @@ struct RouterShapeCost {
   int32_t (*launch)(const char*, const RouterArgs&, cudaStream_t);
 };
 constexpr RouterShapeCost kRouterShapes[] = {
-    {4, 32, 14, 10, launch_router<1, 1>},      {8, 32, 16, 11, launch_router<2, 1>},      {8, 64, 26, 17, launch_router<2, 2>},
-    {16, 64, 35, 27, launch_router<4, 2>},     {32, 64, 57, 46, launch_router<8, 2>},     {24, 128, 77, 64, launch_router<6, 4>},
-    {32, 128, 96, 77, launch_router<8, 4>},    {40, 128, 113, 95, launch_router<10, 4>},  {48, 128, 131, 110, launch_router<12, 4>},
+    {4, 32, 12, 9, launch_router<1, 1>},       {8, 32, 14, 9, launch_router<2, 1>},       {8, 64, 21, 14, launch_router<2, 2>},
+    {16, 64, 30, 22, launch_router<4, 2>},     {32, 64, 49, 42, launch_router<8, 2>},     {24, 128, 65, 53, launch_router<6, 4>},
+    {32, 128, 81, 70, launch_router<8, 4>},    {40, 128, 98, 87, launch_router<10, 4>},   {48, 128, 116, 105, launch_router<12, 4>},
     {56, 128, 135, 98, launch_router_wide<56>}, {64, 128, 136, 110, launch_router_wide<64>},
 };
 

@@ -92,6 +92,30 @@ def test_every_router_kernel_variant_gives_the_same_bits(lib, dev, orc, tokens, 
         lib.gemb_set_tuning(8, 0)
 
 
+@pytest.mark.parametrize("hidden", [4, 36, 128, 260, 544, 2820])
+@pytest.mark.parametrize("tokens,experts,shift", [(1, 128, 0), (25, 33, 4), (49, 160, 0), (130, 128, 4)])
+def test_router_rings_over_edges(lib, dev, orc, tokens, hidden, experts, shift):
+    """Tiles and rings of every logits kernel: K below one tile, with a rest, past the ring's depth; rows of 8-byte alignment only
+    (hidden % 8 = 4, or a view that starts `shift` values in); token and expert tails.  Bit for bit, as one chain in ascending k."""
+    rng = np.random.default_rng(tokens * hidden)
+    x = bf16_bits(rng.standard_normal((tokens, hidden)).astype(np.float32))
+    w = (rng.standard_normal((experts, hidden)) * 0.02).astype(np.float32)
+    want = orc.moe_router_logits(x, w, None)
+    room = torch.zeros(tokens * hidden + 8, dtype=torch.uint16, device=dev)
+    xd = room[shift:shift + tokens * hidden]
+    xd.copy_(to_dev(x, dev).view(torch.uint16).reshape(-1))
+    wd = to_dev(w, dev)
+    try:
+        for tile in (0, 1, 2, 3, 4, 24, 32, 40, 48, 56, 64):
+            lib.gemb_set_tuning(8, tile)
+            out = torch.full((tokens, experts), float("nan"), device=dev)
+            lib.gemb_moe_router_logits(xd, wd, None, out, tokens, hidden, experts, None)
+            assert np.array_equal(to_np(out).view(np.uint32), want.view(np.uint32)), tile
+    finally:
+        lib.gemb_set_tuning(8, 0)
+    lib.gemb_check_device_status()
+
+
 @pytest.mark.parametrize("tokens", [1, 17, 511, 512, 1023, 4096])
 def test_permutation_bit_exact(lib, dev, orc, tokens):
     rng = np.random.default_rng(tokens)
