@@ -124,6 +124,14 @@ def test_permutation_bit_exact(lib, dev, orc, tokens):
     check_permute(lib, dev, orc, ids, 128)
 
 
+@pytest.mark.parametrize("assignments,experts", [(1025, 1), (2048, 33), (3 * 1024 + 7, 1024), (17 * 1024 + 1, 128), (147 * 1024, 160),
+                                                 (147 * 1024 + 1, 128), (300 * 1024 + 9, 128)])
+def test_permutation_over_segments(lib, dev, orc, assignments, experts):
+    """Segments of 1,024 assignments: two to the most that one launch places (a CTA per SM), and more (scan and scatter in two launches)."""
+    rng = np.random.default_rng(assignments)
+    check_permute(lib, dev, orc, rng.integers(0, experts, (assignments, 1)).astype(np.int32), experts)
+
+
 def test_permutation_zero_hit_and_single_expert(lib, dev, orc):
     check_permute(lib, dev, orc, np.tile(np.arange(8, dtype=np.int32), (700, 1)), 128)      # 120 experts empty
     check_permute(lib, dev, orc, (np.arange(128 * 8, dtype=np.int32).reshape(128, 8)) % 128, 128)
