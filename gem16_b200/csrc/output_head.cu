@@ -32,11 +32,25 @@ __device__ __forceinline__ bool better(float v, uint32_t t, const Candidate& c) 
   return v > c.value || (v == c.value && t < c.token);
 }
 
-__device__ __forceinline__ bool is_suppressed(uint32_t token, const uint32_t* __restrict__ list, uint32_t n) {
-  for (uint32_t i = 0; i < n; ++i)
-    if (__ldg(list + i) == token) return true;
-  return false;
-}
+// The suppression list as a warp sees it: its first 32 entries in the lanes' registers.
+struct Suppressed {
+  const int32_t* list;
+  uint32_t count, mine;
+  __device__ __forceinline__ Suppressed(const uint32_t* suppressed, uint32_t n, const uint32_t* dynamic_n)
+      : list(reinterpret_cast<const int32_t*>(suppressed)),
+        count(dynamic_n != nullptr ? static_cast<uint32_t>(ld_dep(reinterpret_cast<const int32_t*>(dynamic_n))) : n) {
+    const uint32_t lane = threadIdx.x & 31;
+    mine = lane < count ? static_cast<uint32_t>(ld_dep(list + lane)) : ~0u;   // no token
+  }
+  // The bits of all entries, `bit_of` giving an entry's.  Whole warps only.
+  template <typename F>
+  __device__ __forceinline__ uint32_t mask(F bit_of) const {
+    uint32_t bits = bit_of(mine);
+    for (uint32_t i = 32 + (threadIdx.x & 31); i - (threadIdx.x & 31) < count; i += 32)
+      if (i < count) bits |= bit_of(static_cast<uint32_t>(ld_dep(list + i)));
+    return __reduce_or_sync(0xFFFFFFFFu, bits);
+  }
+};
 
 // kRows hidden vectors share one pass over the weights.  A warp takes kTok vocabulary rows at a time
 // (kTok * kU 16-byte loads per lane in flight before any arithmetic) so that each shared-memory read
@@ -44,9 +58,9 @@ __device__ __forceinline__ bool is_suppressed(uint32_t token, const uint32_t* __
 // kernel is bound by shared-memory bandwidth, not by HBM.
 template <int kRows>
 __global__ void __launch_bounds__(kOhThreads)
-output_head_kernel(const uint16_t* __restrict__ weights, const float* __restrict__ hidden_rows,
-                   const uint32_t* __restrict__ suppressed, uint32_t suppressed_count,
-                   const uint32_t* __restrict__ dynamic_suppressed_count, Candidate* __restrict__ candidates,
+output_head_kernel(const uint16_t* __restrict__ weights, const float* hidden_rows,
+                   const uint32_t* suppressed, uint32_t suppressed_count,
+                   const uint32_t* dynamic_suppressed_count, Candidate* __restrict__ candidates,
                    float* __restrict__ logits_out, uint32_t vocab, uint32_t hidden) {
   constexpr int kTok = kRows >= 3 ? 4 : kRows;   // weight rows per warp iteration
   constexpr int kU = 8 / kTok;                   // 16-byte pieces per lane, weight row and pass
@@ -56,12 +70,14 @@ output_head_kernel(const uint16_t* __restrict__ weights, const float* __restrict
   __shared__ Candidate warp_best[kRows][kOhWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t pieces = hidden / 8;   // 16-byte pieces per weight row
+  pdl_trigger();
+  pdl_wait();
   for (uint32_t i = threadIdx.x; i < kRows * hidden / 4; i += kOhThreads) {
     const uint32_t r = i / (hidden / 4), q = i % (hidden / 4);
-    hs[(r * 2 + (q & 1)) * pieces + (q >> 1)] = __ldg(reinterpret_cast<const float4*>(hidden_rows) + i);
+    hs[(r * 2 + (q & 1)) * pieces + (q >> 1)] = ld_dep(reinterpret_cast<const float4*>(hidden_rows) + i);
   }
   __syncthreads();
-  const uint32_t n_sup = dynamic_suppressed_count != nullptr ? __ldg(dynamic_suppressed_count) : suppressed_count;
+  const Suppressed sup(suppressed, suppressed_count, dynamic_suppressed_count);
   Candidate best[kRows];
 #pragma unroll
   for (int r = 0; r < kRows; ++r) best[r] = {-FLT_MAX, 0u};
@@ -123,12 +139,18 @@ output_head_kernel(const uint16_t* __restrict__ weights, const float* __restrict
 #pragma unroll
         for (int off = 16; off != 0; off >>= 1) sum[j][r] += __shfl_xor_sync(0xFFFFFFFFu, sum[j][r], off);
       }
+    const uint32_t barred = sup.mask([&](uint32_t entry) {
+      uint32_t bits = 0;
+#pragma unroll
+      for (int j = 0; j < kTok; ++j) bits |= entry == token0 + j * stride ? 1u << j : 0u;
+      return bits;
+    });
     if (lane == 0) {
 #pragma unroll
       for (int j = 0; j < kTok; ++j) {
         if (!live[j]) continue;
         const uint32_t token = token0 + j * stride;
-        const bool allowed = !is_suppressed(token, suppressed, n_sup);
+        const bool allowed = (barred >> j & 1) == 0;
 #pragma unroll
         for (int r = 0; r < kRows; ++r) {
           const float capped = tanhf(sum[j][r] / 30.0f) * 30.0f;   // src/cuda/output_head.cu:53,88
@@ -159,23 +181,28 @@ output_head_kernel(const uint16_t* __restrict__ weights, const float* __restrict
 }
 
 // ---------------------------------------------------------------------------------------------
-// Three to eight hidden rows on the warp-level tensor-core path (mma.sync m16n8k16, bf16 x bf16 -> fp32): the weights are the M
-// side as they lie in memory, the hidden rows its eight columns.  An fp32 hidden value is the exact sum of three bf16 values
-// (its mantissa cut into eight bits each), so three MMAs per 16 k give the fp32 products; two chains of two (32 products each)
-// start from zero and join the running fp32 sum with IEEE additions.  The fma form above spends an fma and its share of
-// the unpacking per hidden row and weight: 262,144 x 3,840 with 3 / 5 / 8 rows 437 / 507 / 1,045 us there, 322 here (2.01 GB: 312 at the
-// copy rate).
+// Two to eight hidden rows on the warp-level tensor-core path (mma.sync m16n8k16, bf16 x bf16 -> fp32): the weights are the M
+// side as they lie in memory.  An fp32 hidden value is the exact sum of three bf16 values (its mantissa cut into eight bits each), and
+// the three parts of every hidden row are columns of the N side: one tile of eight columns for two rows, two for up to five, three for
+// up to eight.  Two chains of two MMAs (32 products each) start from zero and join the running fp32 sum with IEEE additions.  The fma
+// form above spends an fma and its share of the unpacking per hidden row and weight: 262,144 x 3,840 with 3 / 5 / 8 rows 440 / 508 /
+// 1,035 us there, 320 / 322 / 328 here (2.01 GB: 307 at the copy rate); the rate of these MMAs is what is left (with three tiles
+// for all 336 / 338 / 338).
 //
 // One CTA of sixteen warps per SM, the split hidden rows in shared memory in MMA order.  A task is sixteen vocabulary rows = the
-// eight tokens that two neighbouring candidate blocks take in one of their steps; a CTA owns whole pairs of blocks and
-// deals their tasks to its warps, so that a block's candidate is found inside the CTA.  Lane 4g + t loads 32 bytes of rows g
-// and g + 8 per 64 k, three such pieces ahead.
+// eight tokens that two neighbouring candidate blocks take in one of their steps; a CTA owns whole pairs of blocks, so that a block's
+// candidate is found inside the CTA, and its tasks' pieces of 64 k are shared evenly and contiguously over its warps: whole tasks per
+// warp left most of them idle in the last round (eight rows x 3,840, us before -> now: 32,000 tokens 62 -> 56, 50,000: 94 -> 79,
+// 92,548: 141 -> 129, 151,936: 223 -> 201, 262,144: 338 -> 328, the launches behind one another included).  Parts of a task
+// that lies across warps meet in shared memory, in order.  Lane 4g + t loads 32 bytes of rows g and g + 8 per 64 k, three such pieces
+// ahead (eight warps with bursts of four: 15 % slower).
 // ---------------------------------------------------------------------------------------------
 constexpr int kHmWarps = 16, kHmThreads = kHmWarps * 32, kHmAhead = 3;
-// Two rows take the fma form: 262,144 / 131,072 / 100,000 / 50,000 x 3,840 take 326 / 178 / 154 / 96 us there and 342 / 197 / 156 / 102
-// here (2,048 wide: 178 / 100 / 92 / 59 and 199 / 119 / 94 / 61); only where all blocks have one step (32,000 tokens) is it 80
-// there and 66 here.  Three rows are faster here at every size (8,000 x 2,048: 51 and 25; 262,144 x 3,840: 424 and 342; all cold).
-constexpr uint32_t kHmMinRows = 3;
+// One row takes the fma form (32,000 / 92,548 / 262,144 x 3,840: 43 / 104 / 278 us there, 52 / 120 / 306 here), three and more this one.
+// Two rows: 32,000 / 92,548 / 151,936 x 3,840 75 / 135 / 196 there and 54 / 124 / 193 here (2,048 wide: 49 / 81 / 113 and 33 / 72 / 109;
+// beyond that the forms are level); the line lies at six steps of all candidate blocks, 196,608 tokens.  Error of two rows against
+// binary64, weights of 0.02 and 0.05, 1,536 to 3,840 wide: rms 0.12-0.66 e-6 there, 0.07-0.35 e-6 here, largest 0.72-4.07 and 0.74-3.47.
+constexpr uint32_t kHmTwoRowSteps = 6;
 constexpr uint32_t kHmPairs = kOhBlocks / 2;               // pairs of candidate blocks
 constexpr uint32_t kHmStepTokens = kOhBlocks * kOhWarps;   // tokens all blocks take in one step
 
@@ -183,15 +210,27 @@ __host__ __device__ inline uint32_t head_mma_tasks(uint32_t ctas, uint32_t vocab
   return (kHmPairs + ctas - 1) / ctas * ((vocab + kHmStepTokens - 1) / kHmStepTokens);
 }
 
+// The parts of the hidden rows are the columns: all first parts, all second ones, all third ones, eight to a tile of the MMA's N side;
+// with three tiles one for each.
+__host__ __device__ inline uint32_t head_mma_tiles(uint32_t rows) { return (3 * rows + 7) / 8; }
+// Split hidden rows in MMA order; afterwards a 16-byte part of a task per thread.
+__host__ __device__ inline uint32_t head_mma_row_bytes(uint32_t rows, uint32_t hidden) {
+  const uint32_t bytes = (hidden + 63) / 64 * head_mma_tiles(rows) * 2 * 32 * 16;
+  return bytes > kHmThreads * 16 ? bytes : kHmThreads * 16;
+}
+
+template <int kTiles>
 __global__ void __launch_bounds__(kHmThreads, 1)
-output_head_mma_kernel(const uint16_t* __restrict__ weights, const float* __restrict__ hidden_rows, uint32_t rows,
-                       const uint32_t* __restrict__ suppressed, uint32_t suppressed_count,
-                       const uint32_t* __restrict__ dynamic_suppressed_count, Candidate* __restrict__ candidates,
+output_head_mma_kernel(const uint16_t* __restrict__ weights, const float* hidden_rows, uint32_t rows,
+                       const uint32_t* suppressed, uint32_t suppressed_count,
+                       const uint32_t* dynamic_suppressed_count, Candidate* __restrict__ candidates,
                        float* __restrict__ logits_out, uint32_t vocab, uint32_t hidden) {
   extern __shared__ __align__(16) uint4 hm_smem[];
+  pdl_trigger();
+  pdl_wait();   // the weights too: a bf16 matrix may be any kernel's output
   const uint32_t chunks = (hidden + 63) / 64, steps = (vocab + kHmStepTokens - 1) / kHmStepTokens;
-  uint4* bs = hm_smem;   // [chunk][split][half of the chunk's MMAs][lane]
-  Candidate* best = reinterpret_cast<Candidate*>(bs + static_cast<size_t>(chunks) * 3 * 2 * 32);   // [task][block of the pair][8]
+  uint4* bs = hm_smem;   // [chunk][tile][half of the chunk's MMAs][lane]
+  Candidate* best = reinterpret_cast<Candidate*>(reinterpret_cast<uint8_t*>(hm_smem) + head_mma_row_bytes(rows, hidden));   // [task][block of the pair][8]
   const uint32_t warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   // Tasks in the order of their steps: every step but the last is whole, and of the last one the pairs that still hold tokens come
@@ -199,28 +238,30 @@ output_head_mma_kernel(const uint16_t* __restrict__ weights, const float* __rest
   const uint32_t pairs = (kHmPairs - blockIdx.x + gridDim.x - 1) / gridDim.x;
   const uint32_t last_live = (vocab - (steps - 1) * kHmStepTokens + 15) / 16;   // pairs of the whole grid that the last step reaches
   const uint32_t tasks = pairs * (steps - 1) + (last_live > blockIdx.x ? (last_live - blockIdx.x + gridDim.x - 1) / gridDim.x : 0);
-  // Load cursor: piece `lc` of task `lt`.
-  uint32_t lt = warp, lc = 0;
+  // The warp's share: pieces [lo, hi) of the CTA's tasks x chunks.  Load cursor: piece `lc` of task `lt`, `left` pieces to come.
+  const uint32_t lo = tasks * chunks * warp / kHmWarps, hi = tasks * chunks * (warp + 1) / kHmWarps;
+  uint32_t lt = lo / chunks, lc = lo % chunks, left = hi - lo;
   const uint16_t* pw[2] = {weights, weights};
   auto first_token = [&](uint32_t task) { return task / pairs * kHmStepTokens + (blockIdx.x + gridDim.x * (task % pairs)) * 16; };
   auto aim = [&]() {
-    if (lt >= tasks) return;
+    if (left == 0) return;
     const uint32_t tok0 = first_token(lt);
     pw[0] = weights + static_cast<uint64_t>(min(tok0 + g, vocab - 1)) * hidden + t * 16;
     pw[1] = weights + static_cast<uint64_t>(min(tok0 + 8 + g, vocab - 1)) * hidden + t * 16;
   };
   uint32_t wa[kHmAhead][8], wb[kHmAhead][8];
   auto load = [&](int u) {
-    const bool in = lt < tasks && lc * 64 + t * 16 < hidden;
+    const bool in = left != 0 && lc * 64 + t * 16 < hidden;
     if (lc * 64 + 64 > hidden) {   // past K zero weights meet zero activations
 #pragma unroll
       for (int i = 0; i < 8; ++i) wa[u][i] = wb[u][i] = 0;
     }
     ptx::ld_stream_32_if(wa[u], pw[0] + lc * 64, in);
     ptx::ld_stream_32_if(wb[u], pw[1] + lc * 64, in);
+    if (left != 0) --left;
     if (++lc == chunks) {
       lc = 0;
-      lt += kHmWarps;
+      ++lt;
       aim();
     }
   };
@@ -234,41 +275,45 @@ output_head_mma_kernel(const uint16_t* __restrict__ weights, const float* __rest
   // under the first loads
   for (uint32_t idx = threadIdx.x; idx < chunks * 64; idx += kHmThreads) {
     const uint32_t chunk = idx / 64, half = idx / 32 & 1, cg = (idx & 31) >> 2, ct = idx & 3, k = chunk * 64 + ct * 16 + half * 8;
-    uint32_t out[3][4] = {};
-    if (cg < rows && k < hidden) {
-      const float4 a = __ldg(reinterpret_cast<const float4*>(hidden_rows + static_cast<uint64_t>(cg) * hidden + k));
-      const float4 b = __ldg(reinterpret_cast<const float4*>(hidden_rows + static_cast<uint64_t>(cg) * hidden + k) + 1);
-      const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        float rest = v[i];
+    for (uint32_t n = 0; n < kTiles; ++n) {
+      const uint32_t col = n * 8 + cg, part = kTiles == 3 ? n : col / rows, r = kTiles == 3 ? cg : col % rows;
+      uint32_t out[4] = {};
+      if (part < 3 && r < rows && k < hidden) {
+        const float* src = hidden_rows + static_cast<uint64_t>(r) * hidden + k;
+        const float4 a = ld_dep(reinterpret_cast<const float4*>(src)), b = ld_dep(reinterpret_cast<const float4*>(src) + 1);
+        const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          const uint32_t top = __float_as_uint(rest) & 0xFFFF0000u;
-          out[q][i / 2] |= (i & 1) ? top : top >> 16;
-          rest = isfinite(v[i]) ? __fsub_rn(rest, __uint_as_float(top)) : 0.0f;
+        for (int i = 0; i < 8; ++i) {
+          float rest = v[i];
+          uint32_t top = __float_as_uint(rest) & 0xFFFF0000u;
+#pragma unroll
+          for (uint32_t q = 1; q < 3; ++q) {
+            if (q > part) break;
+            rest = isfinite(v[i]) ? __fsub_rn(rest, __uint_as_float(top)) : 0.0f;
+            top = __float_as_uint(rest) & 0xFFFF0000u;
+          }
+          out[i / 2] |= (i & 1) ? top : top >> 16;
         }
       }
+      bs[((chunk * kTiles + n) * 2 + half) * 32 + (idx & 31)] = make_uint4(out[0], out[1], out[2], out[3]);
     }
-#pragma unroll
-    for (int q = 0; q < 3; ++q) bs[((chunk * 3 + q) * 2 + half) * 32 + (idx & 31)] = make_uint4(out[q][0], out[q][1], out[q][2], out[q][3]);
   }
   __syncthreads();
-  const uint32_t n_sup = dynamic_suppressed_count != nullptr ? __ldg(dynamic_suppressed_count) : suppressed_count;
+  const Suppressed sup(suppressed, suppressed_count, dynamic_suppressed_count);
 
-  float acc[3][4] = {};
-  // acc[.][0], acc[.][1]: token g, hidden rows 2t, 2t + 1; acc[.][2], acc[.][3]: token g + 8
-  auto emit = [&](uint32_t task) {
+  // v[0], v[1]: token g, hidden rows 2t, 2t + 1; v[2], v[3]: token g + 8
+  auto emit = [&](uint32_t task, const float (&v)[4]) {
     const uint32_t tok0 = first_token(task);
+    const uint32_t barred = sup.mask([&](uint32_t entry) { return entry - tok0 < 16 ? 1u << (entry - tok0) : 0u; });
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const uint32_t token = tok0 + g + 8 * h;
-      const bool live = token < vocab, allowed = live && !is_suppressed(token, suppressed, n_sup);
+      const bool live = token < vocab, allowed = live && (barred >> (g + 8 * h) & 1) == 0;
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         const uint32_t r = 2 * t + j;
-        const int i = 2 * h + j;
-        const float capped = tanhf(__fadd_rn(acc[0][i], __fadd_rn(acc[1][i], acc[2][i])) / 30.0f) * 30.0f;   // src/cuda/output_head.cu:53,88
+        const float capped = tanhf(v[2 * h + j] / 30.0f) * 30.0f;   // src/cuda/output_head.cu:53,88
         if (logits_out != nullptr && live && r < rows) logits_out[static_cast<uint64_t>(r) * vocab + token] = capped;
         Candidate c{-FLT_MAX, 0u};
         if (allowed && better(capped, token, c)) c = {capped, token};
@@ -282,33 +327,112 @@ output_head_mma_kernel(const uint16_t* __restrict__ weights, const float* __rest
       }
     }
   };
-  uint32_t task = warp, cc = 0;
-  while (task < tasks) {
+  // Two rows have the registers for three running sums (pieces in turn): shorter chains of additions than the fma form's lanes and tree.
+  constexpr int kSums = kTiles == 1 ? kHmAhead : 1;
+  float acc[kSums][kTiles][4] = {}, head[4] = {};
+  // The three parts of this thread's hidden rows, which lie with the lanes 4g .. 4g + 3.
+  auto total = [&](float (&v)[4]) {
+#pragma unroll
+    for (int m = 1; m < kSums; ++m)
+#pragma unroll
+      for (int n = 0; n < kTiles; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          acc[0][n][i] = __fadd_rn(acc[0][n][i], acc[m][n][i]);
+          acc[m][n][i] = 0.0f;
+        }
+    if constexpr (kTiles == 3) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[i] = __fadd_rn(acc[0][0][i], __fadd_rn(acc[0][1][i], acc[0][2][i]));
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float x[3];
+#pragma unroll
+        for (uint32_t q = 0; q < 3; ++q) {
+          const uint32_t col = min(q * rows + 2 * t + i % 2, kTiles * 8 - 1u);   // rows past the last one: anything
+          x[q] = 0.0f;
+#pragma unroll
+          for (int n = 0; n < kTiles; ++n) {
+            const float even = __shfl_sync(0xFFFFFFFFu, acc[0][n][i & 2], 4 * g + col % 8 / 2), odd = __shfl_sync(0xFFFFFFFFu, acc[0][n][(i & 2) + 1], 4 * g + col % 8 / 2);
+            if (col / 8 == n) x[q] = (col & 1) ? odd : even;
+          }
+        }
+        v[i] = __fadd_rn(x[0], __fadd_rn(x[1], x[2]));
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < kTiles; ++n)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[0][n][i] = 0.0f;
+  };
+  uint32_t task = lo / chunks, cc = lo % chunks, todo = hi - lo;
+  bool whole = cc == 0;   // the current task's first piece is the warp's
+  while (todo != 0) {
 #pragma unroll
     for (int u = 0; u < kHmAhead; ++u) {
-      if (task >= tasks) break;   // warp-uniform
+      if (todo == 0) break;   // warp-uniform
 #pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        const uint4 b0 = bs[((cc * 3 + q) * 2) * 32 + lane], b1 = bs[((cc * 3 + q) * 2 + 1) * 32 + lane];
+      for (int n = 0; n < kTiles; ++n) {
+        const uint4 b0 = bs[((cc * kTiles + n) * 2) * 32 + lane], b1 = bs[((cc * kTiles + n) * 2 + 1) * 32 + lane];
         float c[4] = {0.0f, 0.0f, 0.0f, 0.0f}, d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         ptx::mma_bf16(c, wa[u][0], wb[u][0], wa[u][1], wb[u][1], b0.x, b0.y);
         ptx::mma_bf16(d, wa[u][4], wb[u][4], wa[u][5], wb[u][5], b1.x, b1.y);
-        ptx::mma_bf16(c, wa[u][2], wb[u][2], wa[u][3], wb[u][3], b0.z, b0.w);
-        ptx::mma_bf16(d, wa[u][6], wb[u][6], wa[u][7], wb[u][7], b1.z, b1.w);
+        if constexpr (kSums > 1) {   // as many chains as MMAs: what the tensor core cuts off stays below the additions' rounding
+          float c2[4] = {0.0f, 0.0f, 0.0f, 0.0f}, d2[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+          ptx::mma_bf16(c2, wa[u][2], wb[u][2], wa[u][3], wb[u][3], b0.z, b0.w);
+          ptx::mma_bf16(d2, wa[u][6], wb[u][6], wa[u][7], wb[u][7], b1.z, b1.w);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) acc[q][i] = __fadd_rn(acc[q][i], __fadd_rn(c[i], d[i]));
+          for (int i = 0; i < 4; ++i) {
+            c[i] = __fadd_rn(c[i], c2[i]);
+            d[i] = __fadd_rn(d[i], d2[i]);
+          }
+        } else {
+          ptx::mma_bf16(c, wa[u][2], wb[u][2], wa[u][3], wb[u][3], b0.z, b0.w);
+          ptx::mma_bf16(d, wa[u][6], wb[u][6], wa[u][7], wb[u][7], b1.z, b1.w);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[u % kSums][n][i] = __fadd_rn(acc[u % kSums][n][i], __fadd_rn(c[i], d[i]));
       }
       load(u);
+      --todo;
       if (++cc == chunks) {
-        emit(task);
+        float v[4];
+        total(v);
+        if (whole) {
+          emit(task, v);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) head[i] = v[i];
+        }
+        whole = true;
         cc = 0;
-        task += kHmWarps;
-#pragma unroll
-        for (int q = 0; q < 3; ++q)
-#pragma unroll
-          for (int i = 0; i < 4; ++i) acc[q][i] = 0.0f;
+        ++task;
       }
     }
+  }
+  // Tasks that lie across warps: everybody but the task's first warp leaves its part (its first task's, which it did not begin) where
+  // the hidden rows were, the first one adds the parts in order.
+  float tail[4];
+  total(tail);
+  const bool opens = cc != 0 && whole && hi != lo;
+  if (cc != 0 && !whole) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) head[i] = tail[i];
+  }
+  __syncthreads();
+  float4* parts = reinterpret_cast<float4*>(bs);
+  parts[warp * 32 + lane] = make_float4(head[0], head[1], head[2], head[3]);
+  __syncthreads();
+  if (opens) {
+    for (uint32_t w = warp + 1; w < kHmWarps && tasks * chunks * w / kHmWarps < (task + 1) * chunks; ++w) {
+      const float4 v = parts[w * 32 + lane];
+      tail[0] = __fadd_rn(tail[0], v.x);
+      tail[1] = __fadd_rn(tail[1], v.y);
+      tail[2] = __fadd_rn(tail[2], v.z);
+      tail[3] = __fadd_rn(tail[3], v.w);
+    }
+    emit(task, tail);
   }
   __syncthreads();
   if (candidates == nullptr) return;
@@ -323,33 +447,39 @@ output_head_mma_kernel(const uint16_t* __restrict__ weights, const float* __rest
   }
 }
 
-// One CTA per hidden row: best of its 4,096 candidates.
-__global__ void __launch_bounds__(kOhThreads)
-output_head_argmax_kernel(const Candidate* __restrict__ candidates, uint32_t* __restrict__ selected) {
-  __shared__ Candidate scratch[kOhWarps];
-  const Candidate* row = candidates + static_cast<uint64_t>(blockIdx.x) * kOhBlocks;
+// One CTA per hidden row: best of its 4,096 candidates, all of them in flight at once (latency is all there is: with 256 threads that
+// took one after the other 6.5 us, behind a head of 32,000 x 3,840 of 44).
+constexpr int kOaThreads = 1024;
+__global__ void __launch_bounds__(kOaThreads)
+output_head_argmax_kernel(const Candidate* candidates, uint32_t* __restrict__ selected) {
+  __shared__ Candidate scratch[kOaThreads / 32];
+  const int2* row = reinterpret_cast<const int2*>(candidates + static_cast<uint64_t>(blockIdx.x) * kOhBlocks);
+  pdl_trigger();
+  pdl_wait();
+  int2 raw[kOhBlocks / kOaThreads];
+#pragma unroll
+  for (int i = 0; i < kOhBlocks / kOaThreads; ++i) raw[i] = ld_dep(row + threadIdx.x + i * kOaThreads);
   Candidate c{-FLT_MAX, 0u};
-  for (uint32_t i = threadIdx.x; i < kOhBlocks; i += kOhThreads) {
-    const Candidate o = row[i];
+#pragma unroll
+  for (int i = 0; i < kOhBlocks / kOaThreads; ++i) {
+    const Candidate o{__int_as_float(raw[i].x), static_cast<uint32_t>(raw[i].y)};
     if (better(o.value, o.token, c)) c = o;
   }
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-#pragma unroll
-  for (int off = 16; off != 0; off >>= 1) {
-    const float ov = __shfl_down_sync(0xFFFFFFFFu, c.value, off);
-    const uint32_t ot = __shfl_down_sync(0xFFFFFFFFu, c.token, off);
-    if (better(ov, ot, c)) c = {ov, ot};
-  }
-  if (lane == 0) scratch[warp] = c;
-  __syncthreads();
-  if (warp == 0) {
-    c = lane < kOhWarps ? scratch[lane] : Candidate{-FLT_MAX, 0u};
+  auto fold = [&]() {
 #pragma unroll
     for (int off = 16; off != 0; off >>= 1) {
       const float ov = __shfl_down_sync(0xFFFFFFFFu, c.value, off);
       const uint32_t ot = __shfl_down_sync(0xFFFFFFFFu, c.token, off);
       if (better(ov, ot, c)) c = {ov, ot};
     }
+  };
+  fold();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (lane == 0) scratch[warp] = c;
+  __syncthreads();
+  if (warp == 0) {
+    c = scratch[lane];
+    fold();
     if (lane == 0) selected[blockIdx.x] = c.token;
   }
 }
@@ -360,18 +490,27 @@ int32_t launch_output_head(const char* op, const uint16_t* weights, const float*
                            float* logits, uint32_t vocab, uint32_t hidden, cudaStream_t stream) {
   const size_t smem = static_cast<size_t>(kRows) * hidden * sizeof(float);
   GEMB_TRY(allow_full_smem<output_head_kernel<kRows>>(op));
-  output_head_kernel<kRows><<<kOhBlocks, kOhThreads, smem, stream>>>(weights, hidden_rows, suppressed, suppressed_count,
-                                                                    dynamic_count, candidates, logits, vocab, hidden);
-  return check_launch(op);
+  return launch_pdl(op, output_head_kernel<kRows>, dim3(kOhBlocks), dim3(kOhThreads), smem, stream, weights, hidden_rows, suppressed,
+                    suppressed_count, dynamic_count, candidates, logits, vocab, hidden);
 }
 
-// false: the shapes the tensor-core form does not take (rows that are not whole 32-byte pieces, hidden rows or candidates that do
-// not fit the shared memory of one CTA: 48 bytes per hidden element whatever the number of rows, so hidden up to 4,544 at
-// 262,144 tokens and 4,736 at 65,536).  They run in the fma form, which takes 1.2 (three rows) to 3 times (eight) as long.
+template <int kTiles>
+int32_t launch_head_mma(const char* op, size_t smem, const uint16_t* weights, const float* hidden_rows, uint32_t rows, const uint32_t* suppressed,
+                        uint32_t suppressed_count, const uint32_t* dynamic_count, Candidate* candidates, float* logits, uint32_t vocab,
+                        uint32_t hidden, cudaStream_t stream) {
+  GEMB_TRY(allow_full_smem<output_head_mma_kernel<kTiles>>(op));
+  return launch_pdl(op, output_head_mma_kernel<kTiles>, dim3(sm_count()), dim3(kHmThreads), smem, stream, weights, hidden_rows, rows, suppressed,
+                    suppressed_count, dynamic_count, candidates, logits, vocab, hidden);
+}
+
+// false: the shapes the tensor-core form does not take (see above; rows that are not whole 32-byte pieces; hidden rows or candidates that
+// do not fit the shared memory of one CTA: 16 bytes per hidden element and tile, so hidden up to 4,544 at 262,144 tokens and 4,736 at
+// 65,536 for six rows and more, 6,784 and 7,104 for three to five).  They run in the fma form.
 bool head_mma_fits(const uint16_t* weights, uint32_t rows, uint32_t vocab, uint32_t hidden, size_t* smem) {
-  *smem = static_cast<size_t>((hidden + 63) / 64) * 3 * 2 * 32 * sizeof(uint4) +
+  *smem = head_mma_row_bytes(rows, hidden) +
           static_cast<size_t>(head_mma_tasks(static_cast<uint32_t>(sm_count()), vocab)) * 2 * 8 * sizeof(Candidate);
-  return rows >= kHmMinRows && hidden % 16 == 0 && reinterpret_cast<uintptr_t>(weights) % 32 == 0 && *smem <= 227 * 1024;
+  const bool pays = rows >= 3 || (rows == 2 && vocab <= kHmTwoRowSteps * kHmStepTokens);
+  return pays && hidden % 16 == 0 && reinterpret_cast<uintptr_t>(weights) % 32 == 0 && *smem <= 227 * 1024;
 }
 
 }  // namespace
@@ -406,10 +545,11 @@ int32_t gemb_output_head_candidates(const uint16_t* weights_bf16, const float* h
                  h = static_cast<uint32_t>(hidden);
   size_t smem = 0;
   if (head_mma_fits(weights_bf16, static_cast<uint32_t>(rows), v, h, &smem)) {
-    GEMB_TRY(allow_full_smem<output_head_mma_kernel>(op));
-    output_head_mma_kernel<<<sm_count(), kHmThreads, smem, stream>>>(weights_bf16, hidden_rows, static_cast<uint32_t>(rows), suppressed, sc,
-                                                                     dynamic_suppressed_count, c, diagnostic_logits, v, h);
-    return check_launch(op);
+    switch (head_mma_tiles(static_cast<uint32_t>(rows))) {
+      case 1: return launch_head_mma<1>(op, smem, weights_bf16, hidden_rows, static_cast<uint32_t>(rows), suppressed, sc, dynamic_suppressed_count, c, diagnostic_logits, v, h, stream);
+      case 2: return launch_head_mma<2>(op, smem, weights_bf16, hidden_rows, static_cast<uint32_t>(rows), suppressed, sc, dynamic_suppressed_count, c, diagnostic_logits, v, h, stream);
+      default: return launch_head_mma<3>(op, smem, weights_bf16, hidden_rows, static_cast<uint32_t>(rows), suppressed, sc, dynamic_suppressed_count, c, diagnostic_logits, v, h, stream);
+    }
   }
   switch (rows) {
     case 1: return launch_output_head<1>(op, weights_bf16, hidden_rows, suppressed, sc, dynamic_suppressed_count, c, diagnostic_logits, v, h, stream);
@@ -428,8 +568,8 @@ int32_t gemb_output_head_argmax(const void* candidates, uint64_t rows, uint32_t*
   GEMB_REQUIRE(candidates && selected, "%s: pointers must be nonnull", op);
   GEMB_REQUIRE(rows >= 1 && rows <= kOhMaxRows, "%s: between 1 and %d rows", op, kOhMaxRows);
   GEMB_ENTER(op);
-  output_head_argmax_kernel<<<static_cast<unsigned>(rows), kOhThreads, 0, stream>>>(static_cast<const Candidate*>(candidates), selected);
-  return check_launch(op);
+  return launch_pdl(op, output_head_argmax_kernel, dim3(static_cast<unsigned>(rows)), dim3(kOaThreads), 0, stream,
+                    static_cast<const Candidate*>(candidates), selected);
 }
 
 }  // extern "C"

@@ -129,3 +129,27 @@ def test_output_head_rows_sharing_a_pass_at_the_edges(lib, dev, orc, rows, vocab
         best = np.full(4096, -np.finfo(np.float32).max, np.float32)
         np.maximum.at(best, block, got[r])
         assert np.array_equal(values[r], best)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,vocab,hidden", [(1, 33000, 264), (2, 17, 3840), (2, 4096 * 8 * 6, 16), (2, 4096 * 8 * 6 + 1, 16),
+                                               (2, 40000, 1040), (3, 70, 64), (4, 32768 * 3 + 100, 208), (5, 2368 * 16, 1936),
+                                               (6, 37000, 3840), (2, 300, 7104)])
+def test_output_head_tasks_across_warps_and_long_lists(lib, dev, orc, rows, vocab, hidden):
+    """Every number of column tiles; fewer pieces than warps, tasks that lie across warps, two rows on both sides of the line between
+    the forms; a suppression list longer than a warp whose last entries are the best tokens, its length read on the device."""
+    w, h = make_case(orc, rows, vocab, hidden, rows + vocab)
+    want, _ = orc.output_head(w, h)
+    best = list(dict.fromkeys(int(np.argmax(want[r])) for r in range(rows)))
+    sup = [t for t in range(vocab) if t % 3 == 0 and t not in best][:max(0, min(40, vocab // 3) - len(best))] + best
+    sd = torch.tensor(sup + [0, 1], dtype=torch.int32, device=dev)
+    count = torch.tensor([len(sup)], dtype=torch.int32, device=dev)
+    cand = torch.full((rows, 4096, 2), -1, dtype=torch.int32, device=dev)
+    logits = torch.full((rows, vocab), float("nan"), device=dev)
+    selected = torch.full((rows,), -1, dtype=torch.int32, device=dev)
+    lib.gemb_output_head_candidates(torch.from_numpy(w.view(np.int16)).to(dev), torch.from_numpy(h).to(dev), rows, sd, len(sup) + 2, count,
+                                    cand, logits, vocab, hidden, None)
+    lib.gemb_output_head_argmax(cand, rows, selected, None)
+    got = logits.cpu().numpy()
+    assert np.abs(got - want).max() <= 2e-5 * max(1.0, np.abs(want).max())
+    assert np.array_equal(selected.cpu().numpy().astype(np.uint32), select(got, sup))
