@@ -18,8 +18,8 @@
 //     every small kernel fetches its instructions from memory (with the policy 206 -> 188 us for the mixed pass, 232 -> 215 for five tokens).
 //   - The row kernels run with the largest shared-memory split too (launch_pdl_split), otherwise the SM they sit on gets its CTA of this kernel
 //     last, with nothing requested.
-// Four layers of a decode pass, start -> now: FP8 204 -> 188 us, FP8 attention with NVFP4 MLP 216 -> 187, the latter with five tokens
-// 264 -> 217 (mma.sync kernels with weights through registers before).
+// Four layers of a decode pass, before -> now: FP8 204 -> 183 us, FP8 attention with NVFP4 MLP 216 -> 175, the latter with five tokens
+// 264 -> 210 (mma.sync kernels with weights through registers before).
 //
 // Sums: the steps alternate between two issuing threads, each with accumulators of its own; FP8 cuts a thread's share into further
 // chains, because the tensor core truncates where an IEEE addition rounds, and the epilogue keeps what its additions round off (relative
@@ -33,7 +33,8 @@
 //
 // Warps: 0 producer (TMA), 1 and 6 MMA issuers, 2-5 stage the activations (and, NVFP4, their scales into tensor memory), then the
 // epilogue, 7-14 NVFP4 block scales (through registers into the order that tcgen05.cp wants: 4-byte loads, since a scale row is only
-// 4-byte aligned; eight warps with two steps each in flight, four warps cost the mixed pass 8 us).
+// 4-byte aligned; eight warps with two steps each in flight, four warps cost the mixed pass 8 us; 16-byte loads and stores without
+// bank conflicts where the rows allow them: 183.4 -> 185.0 on one GPU, so this is not what a step waits for).
 #include <algorithm>
 #include <type_traits>
 

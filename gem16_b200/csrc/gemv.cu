@@ -1,6 +1,6 @@
 // Entry points of the FP8 (W8A8) decode projections, weights in the checkpoint's row-major source layout, and the forms that are left
-// beside the tcgen05 kernel of decode_gemv.cu: contracting extents whose staged activations leave it no room (one token beyond
-// about 50,000, five and more beyond about 14,000) and what the tuning knobs ask for.  (NVFP4 weights: nvfp4_gemv.cu.)
+// beside the tcgen05 kernel of decode_gemv.cu: one token of a contracting extent whose staged activations leave it no room (beyond
+// 69,632; the batches that are accepted always fit) and what the tuning knobs ask for.  (NVFP4 weights: nvfp4_gemv.cu.)
 //
 // One token: a CTA of 8 warps stages the activation vector once in shared memory (decoded to fp16, which holds every
 // E4M3 value exactly), then each warp streams kRows weight rows with coalesced 128-bit loads (lane l reads
