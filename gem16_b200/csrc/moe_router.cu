@@ -147,7 +147,7 @@ __device__ __forceinline__ void router_step(float2 (&acc)[(kTok + 1) / 2][kExp],
 template <int kTok, int kExp>
 __global__ void __launch_bounds__(kRtThreads + 32, kTok * kExp >= 24 ? 2 : 3)
 router_logits_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const uint16_t* x,
-                     const float* __restrict__ bias, float* logits, uint32_t tokens, uint32_t hidden, uint32_t experts, bool x_wide) {
+                     const float* bias, float* logits, uint32_t tokens, uint32_t hidden, uint32_t experts, bool x_wide) {
   using S = RouterShape<kTok, kExp>;
   constexpr int kK = S::kK, kG = S::kG;
   static_assert(kTok == 1 || kTok % 2 == 0, "tokens go in pairs");
@@ -203,7 +203,7 @@ router_logits_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
 #pragma unroll
   for (int j = 0; j < kExp; ++j) {
     const uint32_t e = exp0 + lane + 32 * j;
-    const float b = (bias != nullptr && e < experts) ? __ldg(bias + e) : 0.0f;
+    const float b = (bias != nullptr && e < experts) ? ld_dep(bias + e) : 0.0f;
 #pragma unroll
     for (int p = 0; p < (kTok + 1) / 2; ++p) acc[p][j] = make_float2(b, b);
   }
@@ -406,10 +406,15 @@ int32_t launch_router(const char* op, const RouterArgs& a, cudaStream_t stream) 
   CUtensorMap map_w, map_x{};
   GEMB_TRY(make_word_map(op, &map_w, a.w, a.experts, a.hidden, 4, 32, S::kExperts, true));
   if (x_wide) GEMB_TRY(make_word_map(op, &map_x, a.x, a.tokens, a.hidden, 2, S::kK, S::kTokens, false));
-  // Not a dependent launch: CTAs placed while the kernel before this one still fills SMs end up two on one SM and none on
-  // another (2,048 tokens: 57 us this way, 81 us behind a kernel that triggers early).
-  kern<<<dim3((a.tokens + S::kTokens - 1) / S::kTokens, (a.experts + S::kExperts - 1) / S::kExperts), kRtThreads + 32, sizeof(typename S::Smem) + 1024,
-         stream>>>(map_w, map_x, a.x, a.bias, a.logits, a.tokens, a.hidden, a.experts, x_wide);
+  const dim3 grid((a.tokens + S::kTokens - 1) / S::kTokens, (a.experts + S::kExperts - 1) / S::kExperts);
+  // A few CTAs start behind the previous kernel's last ones (layer of 1 / 16 / 48 tokens 49.3 -> 47.0, 68.1 -> 64.9, 80.4 -> 76.3 us).  More of
+  // them would wait on SMs that the GEMMs of the other stream want (64 tokens, 64 CTAs: 85.0 -> 88.5), and those of a large batch,
+  // placed while the kernel before this one still fills SMs, end up two on one SM and none on another (2,048 tokens: 57 us
+  // this way, 81 us behind a kernel that triggers early).
+  if (grid.x * grid.y * 3ull <= static_cast<uint64_t>(sm_count()))
+    return launch_pdl(op, kern, grid, dim3(kRtThreads + 32), sizeof(typename S::Smem) + 1024, stream, map_w, map_x, a.x, a.bias, a.logits, a.tokens,
+                      a.hidden, a.experts, x_wide);
+  kern<<<grid, kRtThreads + 32, sizeof(typename S::Smem) + 1024, stream>>>(map_w, map_x, a.x, a.bias, a.logits, a.tokens, a.hidden, a.experts, x_wide);
   return check_launch(op);
 }
 template <int kTok>
