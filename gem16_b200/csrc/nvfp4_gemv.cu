@@ -81,7 +81,7 @@ struct Run {
 };
 __device__ __forceinline__ void load_run(Run& r, const uint8_t* w, const uint8_t* s, bool in, bool wide) {
   if (wide) {
-    ptx::ld_stream_32_if(r.w, w, in);
+    ptx::ld_stream_32_if<true>(r.w, w, in);
     asm volatile("{ .reg .pred p; setp.ne.b32 p, %2, 0;\n"
                  "@p ld.global.nc.b32 %0, [%1]; }"
                  : "+r"(r.s)

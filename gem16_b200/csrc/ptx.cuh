@@ -537,12 +537,20 @@ __device__ __forceinline__ uint32_t ld_stream_4(const void* p, uint64_t policy) 
   asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.b32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(policy));
   return v;
 }
-// 32 weight bytes (32-byte aligned) past L1; the registers stay as they are when `in` is false.
+// 32 weight bytes (32-byte aligned) past L1; the registers stay as they are when `in` is false.  kAtRest: bytes that nothing writes while
+// the kernel is resident (the read-only path); otherwise what a kernel before a programmatic launch may have written.
+template <bool kAtRest>
 __device__ __forceinline__ void ld_stream_32_if(uint32_t (&r)[8], const void* p, bool in) {
-  asm volatile("{ .reg .pred p; setp.ne.b32 p, %9, 0;\n"
-               "@p ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8]; }"
-               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
-               : "l"(p), "r"(static_cast<uint32_t>(in)));
+  if constexpr (kAtRest)
+    asm volatile("{ .reg .pred p; setp.ne.b32 p, %9, 0;\n"
+                 "@p ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8]; }"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
+                 : "l"(p), "r"(static_cast<uint32_t>(in)));
+  else
+    asm volatile("{ .reg .pred p; setp.ne.b32 p, %9, 0;\n"
+                 "@p ld.global.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8]; }"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
+                 : "l"(p), "r"(static_cast<uint32_t>(in)));
 }
 
 }  // namespace ptx
